@@ -1,7 +1,7 @@
-// Token sampling on the device, one CTA per request row:
+// Token sampling on the device:
 //   * greedy arg-max (lowest index wins ties),
 //   * temperature + top-k + top-p sampling by the exponential-race (Gumbel-max)
-//     method: the kept set is found with radix selection over the logit bits
+//     method: the kept set is found with counters over the logits
 //     (counts for top-k, probability mass for top-p), then the winner is
 //     argmax(logit / T + Gumbel noise) over the kept tokens, noise from a
 //     counter-based Philox4x32-10 generator keyed per row.
@@ -13,6 +13,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include "../common/device_once.h"
 
 namespace b200 {
 
@@ -66,19 +68,6 @@ __device__ __forceinline__ MaxIdx block_argmax(MaxIdx m, MaxIdx* red) {
   return t;
 }
 
-__device__ __forceinline__ float block_reduce_sum(float v, float* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  float t = (l < (blockDim.x >> 5)) ? red[l] : 0.f;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  __syncthreads();
-  return t;
-}
-
 // Philox4x32-10 (Salmon et al., SC'11): 128-bit counter, 64-bit key.
 __device__ __forceinline__ uint4 philox4x32(uint4 ctr, uint2 key) {
   const uint32_t M0 = 0xD2511F53u, M1 = 0xCD9E8D57u, W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;
@@ -110,136 +99,350 @@ argmax_kernel(const T* __restrict__ logits, int* __restrict__ out, int V, long l
   if (threadIdx.x == 0) out[blockIdx.x] = m.i == 0x7fffffff ? 0 : m.i;
 }
 
-// Radix selection state shared by the block.
-struct SelectShared {
-  float hist[2048];
-  uint32_t prefix;
-  uint32_t prefix_mask;
-  float remaining;
-  int done;
+// ---------------------------------------------------------------------------------------------- sampling
+// A thread-block cluster of eight CTAs per row.  Each CTA keeps its eighth of the row in shared memory, so
+// that a row of 128 k fp32 logits is read from device memory once and the later passes (threshold of top-k,
+// threshold of top-p, draw) run from shared memory on eight SMs.  One CTA of 1024 threads per row, reading
+// the row from memory in every pass, took 615 us for 128 rows x 128256 (its histogram over the leading key bits
+// put most of the vocabulary into some thirty counters, and one thread walked the 2048 counters); this form is
+// bound by the passes over shared memory.
+static constexpr int kRowCtas = 8;
+static constexpr int kRowThreads = 512;
+static constexpr int kBins = 2048;
+static constexpr int kMaxKeys = kBins / 2;
+static constexpr int kMaxSlice = 50 * 1024;     // logits of a slice that fit shared memory
+
+struct RowShared {
+  union {
+    float mass[kBins];           // of this CTA's slice
+    uint32_t count[kBins];
+    struct {                     // CTA 0, after the counters have been read: the logits of the chosen bin
+      uint32_t key[kMaxKeys];
+      float weight[kMaxKeys];
+    } list;
+  };
+  MaxIdx top;                    // of this CTA's slice
+  MaxIdx red[32];
+  float warp_sum[kRowThreads / 32];
+  // written by CTA 0, read by all
+  int bin;
+  float above, target;
+  int num_keys;
+  uint32_t threshold;
 };
 
-// Finds the largest key threshold `thr` such that the total weight of elements with key >= thr
-// is >= target, where weight is 1 (COUNT) or exp2(x*s - m) (mass).  Elements below
-// `floor_key` are ignored.  Returns the threshold key.
-template <typename T, bool MASS>
-__device__ uint32_t radix_select(const T* row, int V, float target, uint32_t floor_key,
-                                 float scale_log2, float max_scaled, SelectShared* sh) {
-  if (threadIdx.x == 0) {
-    sh->prefix = 0;
-    sh->prefix_mask = 0;
-    sh->remaining = target;
-  }
-  const int shifts[3] = {21, 10, 0};
-  const int widths[3] = {11, 11, 10};
-  for (int pass = 0; pass < 3; ++pass) {
-    const int shift = shifts[pass];
-    const int bins = 1 << widths[pass];
-    for (int i = threadIdx.x; i < 2048; i += blockDim.x) sh->hist[i] = 0.f;
-    __syncthreads();
-    const uint32_t prefix = sh->prefix, mask = sh->prefix_mask;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-      const float x = load_logit<T>(row, i);
-      const uint32_t key = float_key(x);
-      if (key < floor_key || (key & mask) != prefix) continue;
-      const int b = (key >> shift) & (bins - 1);
-      const float wgt = MASS ? exp2f(x * scale_log2 - max_scaled) : 1.f;
-      atomicAdd(&sh->hist[b], wgt);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float rem = sh->remaining;
-      int b = bins - 1;
-      for (; b > 0; --b) {
-        const float h = sh->hist[b];
-        if (h >= rem) break;
-        rem -= h;
-      }
-      sh->remaining = rem;
-      sh->prefix = prefix | (static_cast<uint32_t>(b) << shift);
-      sh->prefix_mask = mask | (static_cast<uint32_t>(bins - 1) << shift);
-    }
-    __syncthreads();
-  }
-  return sh->prefix;
+__device__ __forceinline__ uint32_t remote_smem(const void* p, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;"
+      : "=r"(a)
+      : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ uint32_t remote_u32(const void* p, int rank) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(remote_smem(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ float remote_f32(const void* p, int rank) { return __uint_as_float(remote_u32(p, rank)); }
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kSampleThreads)
+// Best of the eight slices' entries (every thread of every CTA gets it); ends with all CTAs past the exchange.
+__device__ __forceinline__ MaxIdx row_best(MaxIdx m, RowShared* sh) {
+  m = block_argmax(m, sh->red);
+  if (threadIdx.x == 0) sh->top = m;
+  cluster_barrier();
+#pragma unroll
+  for (int r = 0; r < kRowCtas; ++r)
+    m = better(m, MaxIdx{remote_f32(&sh->top.v, r), static_cast<int>(remote_u32(&sh->top.i, r))});
+  cluster_barrier();
+  return m;
+}
+
+// One pass of counters over the slices: ``bin_of(x)`` in [0, kBins) grows as logits fall, or is negative for
+// logits that take no part.  Finds the first bin at which the weight of the bins up to it reaches the target
+// (``target`` times the whole weight if SHARE); leaves bin, the weight before it and the target in CTA 0's
+// shared memory, bin = -1 if rounding keeps the sum below the target.
+template <bool MASS, bool SHARE, typename Load, typename Bin>
+__device__ void count_pass(Load load, int n, int rank, Bin bin_of, float target, float scale_log2, float max_scaled,
+                           RowShared* sh) {
+  for (int i = threadIdx.x; i < kBins; i += kRowThreads) sh->count[i] = 0u;    // also 0.f
+  __syncthreads();
+  // the last bin takes whatever lies far below the maximum, often most of the row: added up in registers
+  float far = 0.f;
+  for (int i = threadIdx.x; i < n; i += kRowThreads) {
+    const float x = load(i);
+    const int b = bin_of(x);
+    if (b < 0) continue;
+    const float w = MASS ? exp2f(__fmaf_rn(x, scale_log2, -max_scaled)) : 1.f;
+    if (b == kBins - 1)
+      far += w;
+    else if (MASS)
+      atomicAdd(&sh->mass[b], w);
+    else
+      atomicAdd(&sh->count[b], 1u);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) far += __shfl_xor_sync(0xffffffffu, far, o);
+  if ((threadIdx.x & 31) == 0 && far > 0.f) {
+    if (MASS)
+      atomicAdd(&sh->mass[kBins - 1], far);
+    else
+      atomicAdd(&sh->count[kBins - 1], static_cast<uint32_t>(far));
+  }
+  cluster_barrier();
+  if (rank == 0) {
+    constexpr int PER = kBins / kRowThreads;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float w[PER], own = 0.f;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      w[j] = 0.f;
+#pragma unroll
+      for (int r = 0; r < kRowCtas; ++r) {
+        const uint32_t v = remote_u32(&sh->count[threadIdx.x * PER + j], r);
+        w[j] += MASS ? __uint_as_float(v) : static_cast<float>(v);
+      }
+      own += w[j];
+    }
+    float incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    if (lane == 31) sh->warp_sum[warp] = incl;
+    if (threadIdx.x == 0) {
+      sh->bin = 0x7fffffff;
+      sh->num_keys = 0;
+      sh->threshold = 0u;
+    }
+    __syncthreads();
+    float before = incl - own, total = 0.f;
+    for (int i = 0; i < kRowThreads / 32; ++i) {
+      if (i < warp) before += sh->warp_sum[i];
+      total += sh->warp_sum[i];
+    }
+    if (SHARE) target *= total;
+    // an empty bin is never chosen; the smallest bin that qualifies is
+    int mine = 0x7fffffff;
+    float run = before, mine_above = 0.f;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      if (mine == 0x7fffffff && w[j] > 0.f && run + w[j] >= target) {
+        mine = static_cast<int>(threadIdx.x) * PER + j;
+        mine_above = run;
+      }
+      run += w[j];
+    }
+    if (mine != 0x7fffffff) atomicMin(&sh->bin, mine);
+    __syncthreads();
+    const int chosen = sh->bin;
+    __syncthreads();
+    if (mine == chosen && mine != 0x7fffffff) sh->above = mine_above;
+    if (threadIdx.x == 0) {
+      sh->target = target;
+      if (chosen == 0x7fffffff) sh->bin = -1;
+    }
+  }
+  cluster_barrier();
+}
+
+// Largest key threshold such that the weight of the logits with key >= threshold is >= the target (as in
+// count_pass), over the logits with key >= floor_key; 0 if there is none.  Weight: 1 or, MASS, exp2(x s - m).
+// The first counters are linear in the logit (1/32 of a power of two of probability below the maximum), which
+// spreads a vocabulary over them; the keys of the chosen bin are then compared with one another, or, if there are
+// more than kMaxKeys of them (equal logits), go through counters of their key bits.
+template <bool MASS, typename Load>
+__device__ uint32_t row_threshold(Load load, int n, int rank, float target, uint32_t floor_key, float scale_log2,
+                                  float max_scaled, RowShared* sh) {
+  const auto linear = [=](float x) {
+    const int b = static_cast<int>(__fmaf_rn(-x, scale_log2, max_scaled) * 32.f);
+    return float_key(x) < floor_key ? -1 : min(max(b, 0), kBins - 1);
+  };
+  if (!(target > 0.f)) return 0xffffffffu;      // top_p <= 0: nothing qualifies, the caller falls back to the maximum
+  count_pass<MASS, MASS>(load, n, rank, linear, target, scale_log2, max_scaled, sh);
+  const int bin = static_cast<int>(remote_u32(&sh->bin, 0));
+  if (bin < 0) return 0u;
+  target = remote_f32(&sh->target, 0);
+  float above = remote_f32(&sh->above, 0);
+  const uint32_t counter = remote_smem(&sh->num_keys, 0);
+  for (int i = threadIdx.x; i < n; i += kRowThreads) {
+    const float x = load(i);
+    if (linear(x) != bin) continue;
+    uint32_t at;
+    asm volatile("atom.shared::cluster.add.u32 %0, [%1], 1;" : "=r"(at) : "r"(counter) : "memory");
+    if (at < kMaxKeys)
+      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote_smem(&sh->list.key[at], 0)), "r"(float_key(x))
+                   : "memory");
+  }
+  cluster_barrier();
+  const int found = static_cast<int>(remote_u32(&sh->num_keys, 0));
+  if (found <= kMaxKeys) {
+    if (rank == 0) {
+      for (int i = threadIdx.x; i < found; i += kRowThreads) {
+        const uint32_t key = sh->list.key[i];
+        const float x = __uint_as_float((key & 0x80000000u) ? key & 0x7fffffffu : ~key);
+        sh->list.weight[i] = MASS ? exp2f(__fmaf_rn(x, scale_log2, -max_scaled)) : 1.f;
+      }
+      __syncthreads();
+      for (int i = threadIdx.x; i < found; i += kRowThreads) {
+        const uint32_t key = sh->list.key[i];
+        float sum = above;
+        uint32_t least = key;
+#pragma unroll 4
+        for (int j = 0; j < found; ++j) {
+          const uint32_t other = sh->list.key[j];
+          least = min(least, other);
+          if (other >= key) sum += sh->list.weight[j];
+        }
+        // (the least key qualifies by the choice of the bin, whatever the order of the sums says)
+        if (sum >= target || key == least) atomicMax(&sh->threshold, key);
+      }
+    }
+    cluster_barrier();
+    return remote_u32(&sh->threshold, 0);      // reset behind the first barrier of the next count_pass
+  }
+  uint32_t prefix = 0u, mask = 0u;
+  for (int shift = 22; shift >= 0; shift = shift == 2 ? -1 : shift - 10) {
+    // digits of 10, 10, 10 and the last 2 bits
+    const auto digit = [=](float x) {
+      const uint32_t key = float_key(x);
+      return linear(x) != bin || (key & mask) != prefix ? -1 : 1023 - static_cast<int>((key >> shift) & 1023u);
+    };
+    count_pass<MASS, false>(load, n, rank, digit, target - above, scale_log2, max_scaled, sh);
+    const int b = static_cast<int>(remote_u32(&sh->bin, 0));
+    if (b >= 0) above += remote_f32(&sh->above, 0);
+    const uint32_t d = b < 0 ? 0u : static_cast<uint32_t>(1023 - b);
+    prefix |= d << shift;
+    mask |= 1023u << shift;
+  }
+  const auto tail = [=](float x) {
+    const uint32_t key = float_key(x);
+    return linear(x) != bin || (key & mask) != prefix ? -1 : 3 - static_cast<int>(key & 3u);
+  };
+  count_pass<MASS, false>(load, n, rank, tail, target - above, scale_log2, max_scaled, sh);
+  const int b = static_cast<int>(remote_u32(&sh->bin, 0));
+  return prefix | (b < 0 ? 0u : static_cast<uint32_t>(3 - b));
+}
+
+template <typename T, bool CACHED>
+__global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
 sample_kernel(const T* __restrict__ logits, int* __restrict__ out, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
               const long long* __restrict__ seeds, const long long* __restrict__ step_offset, int V,
-              long long stride) {
-  __shared__ MaxIdx red_mi[32];
-  __shared__ float red_f[32];
-  __shared__ SelectShared sh;
-  const int rowi = blockIdx.x;
-  const T* row = logits + static_cast<long long>(rowi) * stride;
+              long long stride, int slice) {
+  extern __shared__ __align__(16) float cached[];
+  __shared__ RowShared sh;
+  const int rowi = blockIdx.x / kRowCtas;
+  const int rank = blockIdx.x % kRowCtas;
+  const int lo = min(V, rank * slice), n = min(V, lo + slice) - lo;
+  const T* row = logits + static_cast<long long>(rowi) * stride + lo;
   const float temp = temperature ? temperature[rowi] : 1.f;
+  const bool greedy = temp < 1e-5f;
 
-  // pass 1: max (and greedy answer)
+  // the maximum (the greedy answer), and the slice into shared memory
   MaxIdx m{-INFINITY, 0x7fffffff};
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    const float v = load_logit<T>(row, i);
+  const auto see = [&](float v, int i) {
     if (v > m.v) {
       m.v = v;
       m.i = i;
     }
+  };
+  int i0 = 0;
+  if (sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+    const float4* row4 = reinterpret_cast<const float4*>(row);
+    const int n4 = n / 4;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n4; i += kRowThreads) {
+      const float4 v = row4[i];
+      if (CACHED && !greedy) reinterpret_cast<float4*>(cached)[i] = v;
+      see(v.x, lo + 4 * i);
+      see(v.y, lo + 4 * i + 1);
+      see(v.z, lo + 4 * i + 2);
+      see(v.w, lo + 4 * i + 3);
+    }
+    i0 = n4 * 4;
   }
-  m = block_argmax(m, red_mi);
-  if (temp < 1e-5f) {
-    if (threadIdx.x == 0) out[rowi] = m.i == 0x7fffffff ? 0 : m.i;
+#pragma unroll 4
+  for (int i = i0 + threadIdx.x; i < n; i += kRowThreads) {
+    const float v = load_logit<T>(row, i);
+    if (CACHED && !greedy) cached[i] = v;
+    see(v, lo + i);
+  }
+  m = row_best(m, &sh);
+  if (greedy) {
+    if (rank == 0 && threadIdx.x == 0) out[rowi] = m.i == 0x7fffffff ? 0 : m.i;
     return;
   }
+  const auto load = [&](int i) { return CACHED ? cached[i] : load_logit<T>(row, i); };
   const float scale_log2 = 1.4426950408889634f / temp;
   const float max_scaled = m.v * scale_log2;
 
   uint32_t floor_key = 0;  // keep keys >= floor_key
   const int k = top_k ? top_k[rowi] : 0;
-  if (k > 0 && k < V) {
-    floor_key = radix_select<T, false>(row, V, static_cast<float>(k), 0u, scale_log2, max_scaled, &sh);
-  }
+  if (k > 0 && k < V)
+    floor_key = row_threshold<false>(load, n, rank, static_cast<float>(k), 0u, scale_log2, max_scaled, &sh);
   const float p = top_p ? top_p[rowi] : 1.f;
-  if (p < 1.f) {
-    float z = 0.f;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-      const float x = load_logit<T>(row, i);
-      if (float_key(x) >= floor_key) z += exp2f(x * scale_log2 - max_scaled);
-    }
-    z = block_reduce_sum(z, red_f);
-    const uint32_t kp =
-        radix_select<T, true>(row, V, p * z, floor_key, scale_log2, max_scaled, &sh);
-    if (kp > floor_key) floor_key = kp;
-  }
+  if (p < 1.f) floor_key = max(floor_key, row_threshold<true>(load, n, rank, p, floor_key, scale_log2, max_scaled, &sh));
 
-  // final pass: Gumbel-max over the kept set
+  // Gumbel-max over the kept set; four neighbours share a counter value
   const uint64_t seed = seeds ? static_cast<uint64_t>(seeds[rowi]) : 0x9E3779B97F4A7C15ull;
   const uint64_t off = step_offset ? static_cast<uint64_t>(step_offset[0]) : 0ull;
   const uint2 key = make_uint2(static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
   MaxIdx best{-INFINITY, 0x7fffffff};
-  for (int i4 = threadIdx.x; i4 * 4 < V; i4 += blockDim.x) {
-    const uint4 r = philox4x32(make_uint4(static_cast<uint32_t>(i4), static_cast<uint32_t>(off),
+  for (int i4 = threadIdx.x; i4 * 4 < n; i4 += kRowThreads) {
+    float x[4];
+    bool any = false;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      x[j] = i4 * 4 + j < n ? load(i4 * 4 + j) : 0.f;
+      any |= i4 * 4 + j < n && float_key(x[j]) >= floor_key;
+    }
+    if (!any) continue;
+    const uint4 r = philox4x32(make_uint4(static_cast<uint32_t>(lo / 4 + i4), static_cast<uint32_t>(off),
                                           static_cast<uint32_t>(off >> 32), static_cast<uint32_t>(rowi)),
                                key);
     const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int i = i4 * 4 + j;
-      if (i >= V) break;
-      const float x = load_logit<T>(row, i);
-      if (float_key(x) < floor_key) continue;
+      const int i = lo + i4 * 4 + j;
+      if (i4 * 4 + j >= n || float_key(x[j]) < floor_key) continue;
       // u in (0,1]; e = -log(u) ~ Exp(1); score = x/T - log(e)
       const float u = (static_cast<float>(rr[j] >> 8) + 1.0f) * (1.0f / 16777216.0f);
       const float e = -__logf(u);
-      const float score = x / temp - __logf(fmaxf(e, 1e-30f));
+      const float score = x[j] / temp - __logf(fmaxf(e, 1e-30f));
       if (score > best.v || (score == best.v && i < best.i)) {
         best.v = score;
         best.i = i;
       }
     }
   }
-  best = block_argmax(best, red_mi);
-  if (threadIdx.x == 0) out[rowi] = best.i == 0x7fffffff ? (m.i == 0x7fffffff ? 0 : m.i) : best.i;
+  best = row_best(best, &sh);
+  if (rank == 0 && threadIdx.x == 0) out[rowi] = best.i == 0x7fffffff ? (m.i == 0x7fffffff ? 0 : m.i) : best.i;
+}
+
+template <typename T>
+int launch_sample(const void* logits, int* out, const float* temperature, const int* top_k, const float* top_p,
+                  const long long* seeds, const long long* step_offset, int B, int V, long long stride,
+                  cudaStream_t stream) {
+  // slices begin at a multiple of the four logits that share a draw
+  const int slice = ((V + kRowCtas - 1) / kRowCtas + 3) / 4 * 4;
+  const bool fits = slice <= kMaxSlice;
+  const auto kern = fits ? sample_kernel<T, true> : sample_kernel<T, false>;
+  const int smem = fits ? slice * 4 : 0;
+  static DeviceOnce once;
+  int dev = 0;
+  if (once.needed(&dev)) {
+    if (cudaFuncSetAttribute(sample_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSlice * 4) !=
+        cudaSuccess)
+      return -4;
+    once.mark(dev);
+  }
+  kern<<<B * kRowCtas, kRowThreads, smem, stream>>>(static_cast<const T*>(logits), out, temperature, top_k, top_p,
+                                                    seeds, step_offset, V, stride, slice);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
 }  // namespace b200
@@ -261,13 +464,7 @@ extern "C" int b200_sample(const void* logits, int* out, const float* temperatur
                            const float* top_p, const long long* seeds, const long long* step_offset,
                            int B, int V, long long stride, int is_fp32, cudaStream_t stream) {
   if (B <= 0) return 0;
-  if (is_fp32)
-    sample_kernel<float><<<B, kSampleThreads, 0, stream>>>(static_cast<const float*>(logits), out,
-                                                           temperature, top_k, top_p, seeds,
-                                                           step_offset, V, stride);
-  else
-    sample_kernel<__nv_bfloat16><<<B, kSampleThreads, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(logits), out, temperature, top_k, top_p, seeds,
-        step_offset, V, stride);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return is_fp32 ? launch_sample<float>(logits, out, temperature, top_k, top_p, seeds, step_offset, B, V, stride, stream)
+                 : launch_sample<__nv_bfloat16>(logits, out, temperature, top_k, top_p, seeds, step_offset, B, V,
+                                                stride, stream);
 }

@@ -531,6 +531,61 @@ def test_sample_respects_top_k_top_p_and_distribution():
     assert (other != got).float().mean() > 0.3
 
 
+def _philox_u(seed, row, groups):
+    """Uniform numbers (0, 1] of the sampling kernel's draw: Philox4x32-10, a counter per four logits."""
+    import numpy as np
+    c = [np.arange(groups, dtype=np.uint64), np.zeros(groups, np.uint64), np.zeros(groups, np.uint64),
+         np.full(groups, row, np.uint64)]
+    k0, k1 = seed & 0xFFFFFFFF, (seed >> 32) & 0xFFFFFFFF
+    for _ in range(10):
+        a, b = c[0] * np.uint64(0xD2511F53), c[2] * np.uint64(0xCD9E8D57)
+        lo, hi = np.uint64(0xFFFFFFFF), np.uint64(32)
+        c = [(b >> hi) ^ c[1] ^ np.uint64(k0), b & lo, (a >> hi) ^ c[3] ^ np.uint64(k1), a & lo]
+        k0, k1 = (k0 + 0x9E3779B9) & 0xFFFFFFFF, (k1 + 0xBB67AE85) & 0xFFFFFFFF
+    return (torch.from_numpy((np.stack(c, 1).reshape(-1) >> np.uint64(8)).astype(np.float64)) + 1) / 2 ** 24
+
+
+@pytest.mark.parametrize("v,dtype,pad", [(1, torch.float32, 0), (7, torch.float32, 1), (1000, torch.bfloat16, 0),
+                                         (4097, torch.float32, 3), (128256, torch.float32, 0),
+                                         (151936, torch.bfloat16, 8), (410001, torch.float32, 3)])
+def test_sample_draws_the_best_race_among_the_kept_logits(v, dtype, pad):
+    """Slices with remainders, rows off 16-byte boundaries, a row too long for shared memory, equal logits; rows take
+    turns in top-k, top-p, both, neither."""
+    torch.manual_seed(v)
+    n = 10
+    logits = (torch.randn(n, v + pad, device=DEV) * 2).to(dtype)[:, :v]
+    logits[8:] = 1.5                                            # all equal: the chosen bin holds the whole row
+    row = torch.arange(n, device=DEV)
+    temp = 0.3 + 0.15 * row
+    top_k = torch.where(row % 4 == 1, 50, torch.where(row % 4 == 3, 1, 0)).int()
+    top_p = torch.where(row % 4 >= 2, 0.9, 1.0).float()
+    top_p[9], top_k[5], top_p[6] = 0.5, v, 0.0
+    seeds = torch.arange(n, device=DEV) * 0x123456789 + 5
+    got = ops.sample(logits, temp, top_k, top_p, seeds, None).tolist()
+    for i in range(n):
+        x = logits[i].double().cpu()
+        k, p, t = int(top_k[i]), float(top_p[i]), float(temp[i])
+        if p == 0.0:
+            assert got[i] == int(x.argmax())
+            continue
+        order = x.sort(descending=True).values
+        floor = order[k - 1] if 0 < k < v else order[-1]
+        if p < 1:
+            w = torch.where(order >= floor, ((order - order[0]) / t).exp(), 0.0).cumsum(0)
+            # 1e-5: fp32 sums of positive numbers and the 2^-22 of exp2
+            lowest = order[min(v - 1, int((w < p * w[-1] * (1 + 1e-5)).sum()))]
+            surest = order[int((w < p * w[-1] * (1 - 1e-5)).sum())]
+        else:
+            lowest = surest = floor
+        u = _philox_u(int(seeds[i]), i, -(-v // 4))[:v]
+        score = x / t - (-u.log()).clamp_min(1e-30).log()
+        assert x[got[i]] >= max(lowest, floor)
+        # fp32: x / t within 2^-22 of it, a logarithm within 2^-20 (u near 1 keeps 24 bits of it)
+        best = float(score[x >= max(surest, floor)].max())
+        e = float(-u[got[i]].log())
+        assert float(score[got[i]]) >= best - 1e-4 - 2e-6 / max(e, 1e-7)
+
+
 # --------------------------------------------------------------------- MoE
 @pytest.mark.parametrize("e,k,sigmoid,groups,bias", [(64, 6, False, (1, 1), False), (128, 8, False, (1, 1), False),
                                                       (256, 8, True, (8, 4), True), (8, 2, True, (4, 2), False)])
