@@ -1,4 +1,6 @@
-// Paged GQA prefill attention on the 5th-generation tensor cores (head size 128, bf16).
+// Gated / windowed paged GQA prefill attention on the 5th-generation tensor cores (head size 128, bf16): what
+// gqa_gated.cuh describes, a sliding window (tiles before it are skipped), a softmax sink without a value, and the
+// output gate.  (Plain causal attention: gqa_prefill_two_tiles.cu.)
 //
 // One CTA = 128 query rows of one (sequence, query head).  Both products of every 64-key tile
 // run as tcgen05.mma with the accumulators in tensor memory:
@@ -17,13 +19,6 @@
 // Warp roles (192 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 softmax.
 // Every wait is bounded; on expiry the CTA records a status code, stops issuing, waits for what
 // is in flight, frees its TMEM and returns (its output rows are then not valid).
-//
-// Same operation as gqa_prefill_kernel (which stays for other head sizes, sliding windows and
-// sinks).  The EXT form adds what gqa_gated.cuh describes: a sliding window (tiles before it are
-// skipped), a softmax sink without a value, and the output gate; replaces npu_fused_infer_attention_score in its TND paged prefill form
-// (omni_npu/attention/backends/attention.py:216-281).
-
-#include <cstdlib>
 
 #include "attn_params.cuh"
 #include "gqa_gated.cuh"
@@ -31,6 +26,7 @@
 #include "../common/pdl.cuh"
 #include "../common/ptx.cuh"
 #include "../common/tensormap.h"
+#include "umma_desc.cuh"
 
 namespace b200 {
 
@@ -47,60 +43,24 @@ constexpr int NUM_BARS = 1 + 4 * STAGES + 2 * 2 + 3;   // q_full; k/v full+empty
 constexpr int TMEM_COLS = 256;          // S0 [0,64) S1 [64,128) O [128,256)
 constexpr int COL_S = 0, COL_O = 128;
 
-// DQK: query / key head size, 128 (GQA models) or 192 (non-absorbed latent attention: 128 nope + 64 rope)
-template <int DQK>
-struct Cfg {
-  static constexpr int QK_SLABS = DQK / 64;
-  static constexpr int Q_BYTES = QK_SLABS * SLAB;
-  static constexpr int K_BYTES = QK_SLABS * KV_SLAB;
-  static constexpr int V_BYTES = 2 * KV_SLAB;
-  static constexpr int OFF_Q = 0;
-  static constexpr int OFF_K = OFF_Q + Q_BYTES;
-  static constexpr int OFF_V = OFF_K + STAGES * K_BYTES;
-  static constexpr int OFF_P = OFF_V + STAGES * V_BYTES;
-  static constexpr int OFF_BAR = OFF_P + P_BYTES;
-  static constexpr int SMEM = OFF_BAR + NUM_BARS * 8 + 16;
-  static constexpr int CTAS_PER_SM = SMEM <= 115 * 1024 ? 2 : 1;
-};
+constexpr int QK_SLABS = 2;
+constexpr int Q_BYTES = QK_SLABS * SLAB;
+constexpr int K_BYTES = QK_SLABS * KV_SLAB;
+constexpr int V_BYTES = 2 * KV_SLAB;
+constexpr int OFF_Q = 0;
+constexpr int OFF_K = OFF_Q + Q_BYTES;
+constexpr int OFF_V = OFF_K + STAGES * K_BYTES;
+constexpr int OFF_P = OFF_V + STAGES * V_BYTES;
+constexpr int OFF_BAR = OFF_P + P_BYTES;
+constexpr int SMEM = OFF_BAR + NUM_BARS * 8 + 16;
 }  // namespace tcp
 
 enum : int { kStatusPrefillTimeout = 41, kStatusPrefillSmemAlign = 42 };
 
-__device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-      :
-      : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]),
-        "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]),
-        "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// K-major, 128-byte rows, 128B swizzle (what TMA writes): 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t desc_kmajor(uint32_t smem_addr) {
-  return make_smem_desc_sw128(smem_addr);
-}
-// MN-major, 128B swizzle: a "row" is one K index holding 64 MN elements (128 bytes); 8 K rows form a
-// 1024-byte atom; the next 8 K rows follow at the stride byte offset (1024), the next 64 MN elements at
-// the leading byte offset.
-__device__ __forceinline__ uint64_t desc_mnmajor(uint32_t smem_addr, uint32_t lbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFF) >> 4);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
-}
-
 // Launch bounds name 256 threads although 192 are launched: the register file is split over the
 // four sub-partitions of an SM, and two CTAs of six warps put four warps on one of them, which only
 // fits with at most 128 registers per thread (the bound a 256-thread, two-per-SM kernel gets).
-// What the EXT form takes beyond AttnParams.
+// What the kernel takes beyond AttnParams.
 struct PrefillExt {
   const __nv_bfloat16* gate;   // or null
   long long g_stride;
@@ -108,15 +68,12 @@ struct PrefillExt {
   float sink_log2;
 };
 
-template <int DQK, bool EXT>
-__global__ void __launch_bounds__(256, tcp::Cfg<DQK>::CTAS_PER_SM)
+__global__ void __launch_bounds__(256, 2)
 gqa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_v, const AttnParams p, const int box_rows,
                       const int m_tiles, const PrefillExt x) {
   using namespace tcp;
-  using C = Cfg<DQK>;
-  constexpr int OFF_Q = C::OFF_Q, OFF_K = C::OFF_K, OFF_V = C::OFF_V, OFF_P = C::OFF_P, OFF_BAR = C::OFF_BAR;
-  constexpr int Q_BYTES = C::Q_BYTES, K_BYTES = C::K_BYTES, V_BYTES = C::V_BYTES, D = DV;
+  constexpr int D = DV;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint64_t* q_full = bars;
@@ -193,7 +150,7 @@ gqa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   // keys this tile can see: causal rows reach position ctx + m0 + BM - 1 at most
   const int kv_hi = p.causal ? min(kv_len, ctx + m0 + BM) : kv_len;
   // first tile: with a window, the one that holds the oldest key of the tile's first row
-  const int j0 = EXT && p.window > 0 ? max(0, ctx + m0 - p.window + 1) / BN : 0;
+  const int j0 = p.window > 0 ? max(0, ctx + m0 - p.window + 1) / BN : 0;
   const int n_tiles = active ? (kv_hi + BN - 1) / BN - j0 : 0;
 
   int issued = 0;          // tiles whose copies were started (producer lane only)
@@ -203,8 +160,8 @@ gqa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       const int* bt = p.block_tables + static_cast<long long>(b) * p.max_blocks;
       mbar_arrive_expect_tx(q_full, Q_BYTES);
 #pragma unroll
-      for (int sl = 0; sl < C::QK_SLABS; ++sl)
-        tma_load_2d(smem + OFF_Q + sl * SLAB, &tm_q, q_full, h * DQK + sl * 64, q_begin + m0);
+      for (int sl = 0; sl < QK_SLABS; ++sl)
+        tma_load_2d(smem + OFF_Q + sl * SLAB, &tm_q, q_full, h * D + sl * 64, q_begin + m0);
       for (int j = 0; j < n_tiles; ++j) {
         const int st = j % STAGES;
         if (j >= STAGES) {
@@ -219,14 +176,14 @@ gqa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         const int nvalid = min(BN, kv_len - n0);
         const int nboxes = (nvalid + box_rows - 1) / box_rows;
         const uint32_t box_bytes = static_cast<uint32_t>(nboxes * box_rows * 128);
-        mbar_arrive_expect_tx(&k_full[st], box_bytes * C::QK_SLABS);
+        mbar_arrive_expect_tx(&k_full[st], box_bytes * QK_SLABS);
         mbar_arrive_expect_tx(&v_full[st], box_bytes * 2);
         for (int i = 0; i < nboxes; ++i) {
           const int key = n0 + i * box_rows;
           const int blk = bt[key / p.block_size];
           const int row = (blk * p.Hk + kvh) * p.block_size + key % p.block_size;
 #pragma unroll
-          for (int sl = 0; sl < C::QK_SLABS; ++sl)
+          for (int sl = 0; sl < QK_SLABS; ++sl)
             tma_load_2d(smem + OFF_K + st * K_BYTES + sl * KV_SLAB + i * box_rows * 128, &tm_k, &k_full[st],
                         sl * 64, row);
 #pragma unroll
@@ -275,7 +232,7 @@ gqa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         tc_fence_after_sync();
         const uint32_t k_addr = smem_u32(smem + OFF_K + st * K_BYTES);
 #pragma unroll
-        for (int kk = 0; kk < DQK / 16; ++kk) {
+        for (int kk = 0; kk < D / 16; ++kk) {
           const int slab = kk >> 2, off = (kk & 3) * 32;
           umma_f16(tmem_base + COL_S + sb * BN, desc_kmajor(q_addr + slab * SLAB + off),
                    desc_kmajor(k_addr + slab * KV_SLAB + off), idesc_s, kk > 0 ? 1u : 0u);
@@ -298,7 +255,7 @@ gqa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const int q_pos = ctx + m0 + r;                       // position of this row's token
     const bool row_valid = m0 + r < q_len;
     // the sink is a key seen from the start
-    float row_max = EXT && x.has_sink ? x.sink_log2 : -INFINITY, row_sum = EXT && x.has_sink ? 1.f : 0.f;
+    float row_max = x.has_sink ? x.sink_log2 : -INFINITY, row_sum = x.has_sink ? 1.f : 0.f;
     uint8_t* p_row = smem + OFF_P + r * 128;
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
@@ -320,7 +277,7 @@ gqa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       // tiles that lie entirely below the diagonal and inside the sequence need no mask
       const int row_lo = ctx + m0 + quarter * 32;                      // smallest position in this warp
       const bool interior = n0 + BN <= kv_len && (!p.causal || n0 + BN - 1 <= row_lo) &&
-                            (!EXT || p.window <= 0 || n0 > row_lo + 31 - p.window);
+                            (p.window <= 0 || n0 > row_lo + 31 - p.window);
       if (interior) {
 #pragma unroll
         for (int c = 0; c < 64; ++c) {
@@ -333,7 +290,7 @@ gqa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         for (int c = 0; c < 64; ++c) {
           const int key = n0 + c;
           const bool keep = key < kv_len && (!p.causal || key <= q_pos) &&
-                            (!EXT || p.window <= 0 || key > q_pos - p.window);
+                            (p.window <= 0 || key > q_pos - p.window);
           const float v = keep ? __uint_as_float(sv[c >> 5][c & 31]) * p.scale_log2 : -INFINITY;
           s[c] = v;
           tile_max = fmaxf(tile_max, v);
@@ -404,7 +361,7 @@ gqa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         tmem_ld_32x32b_x32(tmem_base + lane_base + COL_O + c * 32, ov);
         tmem_ld_wait();
         if (row_valid) {
-          if constexpr (EXT) {
+          {
             if (x.gate) {
               const uint4* g = reinterpret_cast<const uint4*>(x.gate + static_cast<long long>(q_begin + m0 + r) * x.g_stride +
                                                               static_cast<long long>(h) * D + c * 32);
@@ -469,112 +426,24 @@ gqa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
 using namespace b200;
 
-// CTAs of the kernel that fit one SM (2 for head size 128: 112 KB of shared memory, 256 TMEM columns each).
-// smem_bytes = 0: the kernel's own size; another value asks what a CTA of that size would get.
-extern "C" int b200_gqa_prefill_tc_ctas_per_sm(int smem_bytes) {
-  int n = 0;
-  auto kern = gqa_prefill_tc_kernel<128, false>;
-  if (smem_bytes <= 0) smem_bytes = tcp::Cfg<128>::SMEM;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, tcp::Cfg<128>::SMEM);
-  cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, tcp::THREADS, smem_bytes) != cudaSuccess) return -1;
-  return n;
-}
-
-// What the occupancy figure is made of: out[0..7] = registers per thread, static shared bytes, max dynamic
-// shared bytes, shared memory per SM, registers per SM, reserved shared bytes per block, max blocks per SM,
-// local (spill) bytes per thread.
-extern "C" int b200_gqa_prefill_tc_resources(int* out) {
-  cudaFuncAttributes fa{};
-  if (cudaFuncGetAttributes(&fa, gqa_prefill_tc_kernel<128, false>) != cudaSuccess) return -1;
-  int dev = 0, v = 0;
-  cudaGetDevice(&dev);
-  out[0] = fa.numRegs;
-  out[1] = static_cast<int>(fa.sharedSizeBytes);
-  out[2] = fa.maxDynamicSharedSizeBytes;
-  cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-  out[3] = v;
-  cudaDeviceGetAttribute(&v, cudaDevAttrMaxRegistersPerMultiprocessor, dev);
-  out[4] = v;
-  cudaDeviceGetAttribute(&v, cudaDevAttrReservedSharedMemoryPerBlock, dev);
-  out[5] = v;
-  cudaDeviceGetAttribute(&v, cudaDevAttrMaxBlocksPerMultiprocessor, dev);
-  out[6] = v;
-  out[7] = static_cast<int>(fa.localSizeBytes);
-  return 0;
-}
-
-template <int DQK, bool EXT = false>
 static int launch_prefill_tc(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p,
-                             int box_rows, dim3 grid, cudaStream_t stream, const PrefillExt& x = PrefillExt{}) {
-  auto kern = gqa_prefill_tc_kernel<DQK, EXT>;
+                             int box_rows, dim3 grid, cudaStream_t stream, const PrefillExt& x) {
+  auto kern = gqa_prefill_tc_kernel;
   static DeviceOnce once;
   int dev = 0;
   if (once.needed(&dev)) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, tcp::Cfg<DQK>::SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, tcp::SMEM) != cudaSuccess)
       return -20;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     once.mark(dev);
   }
-  return launch_pdl(kern, grid, dim3(tcp::THREADS), tcp::Cfg<DQK>::SMEM, stream, 1, tq, tk, tv, p, box_rows,
+  return launch_pdl(kern, grid, dim3(tcp::THREADS), tcp::SMEM, stream, 1, tq, tk, tv, p, box_rows,
                     static_cast<int>(grid.x), x) == cudaSuccess
              ? 0
              : -21;
 }
 
-// Returns 0 when the kernel ran, 1 when the problem is not one it takes (caller falls back), < 0 on error.
-// Takes query / key head sizes 128 and 192 with value head size 128, no sliding window.
-extern "C" int b200_gqa_prefill_tc(const void* q, const void* k_cache, const void* v_cache, void* out, float* lse,
-                                   const int* block_tables, const int* cu_q, const int* seq_lens, int B,
-                                   int max_q_len, int max_blocks, int block_size, int Hq, int Hk, int Dqk, int Dv,
-                                   long long q_stride, long long out_stride, float scale, int causal, int window,
-                                   long long total_q_rows, int num_cache_blocks, int* status, cudaStream_t stream) {
-  if ((Dqk != 128 && Dqk != 192) || Dv != 128 || window != 0 || Hq % Hk != 0) return 1;
-  const bool tma_ok = (block_size % 8) == 0 && (block_size <= 64 ? (64 % block_size) == 0 : (block_size % 64) == 0) &&
-                      (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0 && (reinterpret_cast<uintptr_t>(v_cache) & 15) == 0 &&
-                      (reinterpret_cast<uintptr_t>(q) & 15) == 0 && ((q_stride * 2) & 15) == 0 &&
-                      ((out_stride * 2) & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-  if (!tma_ok || num_cache_blocks <= 0 || total_q_rows <= 0) return 1;
-  if (B <= 0 || max_q_len <= 0) return 0;
-  AttnParams p{};
-  p.q = static_cast<const __nv_bfloat16*>(q);
-  p.k_cache = static_cast<const __nv_bfloat16*>(k_cache);
-  p.v_cache = static_cast<const __nv_bfloat16*>(v_cache);
-  p.out = static_cast<__nv_bfloat16*>(out);
-  p.lse = lse;
-  p.block_tables = block_tables;
-  p.cu_q = cu_q;
-  p.seq_lens = seq_lens;
-  p.max_blocks = max_blocks;
-  p.block_size = block_size;
-  p.Hq = Hq;
-  p.Hk = Hk;
-  p.q_stride = q_stride;
-  p.out_stride = out_stride;
-  p.scale_log2 = scale * kLog2e;
-  p.causal = causal;
-  p.status = status;
-  p.num_cache_blocks = num_cache_blocks;
-  const int box_rows = block_size < 64 ? block_size : 64;
-  CUtensorMap tq, tk, tv;
-  int r = make_tensormap_2d(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, q, static_cast<uint64_t>(total_q_rows),
-                            static_cast<uint64_t>(Hq) * Dqk, static_cast<uint64_t>(q_stride), tcp::BM, 64,
-                            CU_TENSOR_MAP_SWIZZLE_128B);
-  if (r) return r - 1000;
-  const uint64_t rows = static_cast<uint64_t>(num_cache_blocks) * Hk * block_size;
-  r = make_tensormap_2d(&tk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, k_cache, rows, Dqk, Dqk, box_rows, 64,
-                        CU_TENSOR_MAP_SWIZZLE_128B);
-  if (r) return r - 2000;
-  r = make_tensormap_2d(&tv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, v_cache, rows, 128, 128, box_rows, 64,
-                        CU_TENSOR_MAP_SWIZZLE_128B);
-  if (r) return r - 3000;
-  const int m_tiles = (max_q_len + tcp::BM - 1) / tcp::BM;
-  dim3 grid(m_tiles, Hq, B);
-  return Dqk == 128 ? launch_prefill_tc<128>(tq, tk, tv, p, box_rows, grid, stream)
-                    : launch_prefill_tc<192>(tq, tk, tv, p, box_rows, grid, stream);
-}
-
-// The EXT form: gated, windowed attention with head sizes 128.  Returns 1 when the problem is not one it takes.
+// Gated, windowed attention with head sizes 128.  Returns 1 when the problem is not one it takes.
 namespace b200 {
 int gated_prefill_tc(const GatedAttnParams& g, int max_q_len, long long total_q_rows, int* status,
                      cudaStream_t stream) {
@@ -621,6 +490,6 @@ int gated_prefill_tc(const GatedAttnParams& g, int max_q_len, long long total_q_
                         CU_TENSOR_MAP_SWIZZLE_128B);
   if (r) return -3000;
   const dim3 grid((max_q_len + tcp::BM - 1) / tcp::BM, g.Hq, g.B);
-  return launch_prefill_tc<128, true>(tq, tk, tv, p, box_rows, grid, stream, x);
+  return launch_prefill_tc(tq, tk, tv, p, box_rows, grid, stream, x);
 }
 }  // namespace b200

@@ -281,6 +281,27 @@ def test_gqa_prefill_tcgen05_matches_reference(seq_lens, q_lens, hq, hk, bs, cau
     _close(got2, want, 2e-2, 2e-2)
 
 
+@pytest.mark.parametrize("d,hq,hk,bs,seq_lens,q_lens", [
+    (128, 8, 2, 16, [129, 128, 127, 257], [129, 128, 1, 256]),      # heads in pairs: edges of the 128-row / -key tiles
+    (128, 6, 2, 16, [257, 255, 400], [257, 129, 128]),              # three heads per key head: row tiles in pairs
+    (192, 4, 4, 16, [256, 385, 130], [256, 300, 2]),                # latent prompt sizes, one head per key head
+    (192, 4, 2, 64, [140], [140]),
+    (128, 4, 1, 128, [300], [300]),                                 # copies of 128 rows
+    (128, 32, 4, 8, [700, 1, 650, 90, 513], [700, 1, 600, 5, 513]),  # more items than SMs, smallest copies
+])
+@pytest.mark.parametrize("causal", [True, False])
+def test_gqa_prefill_two_tiles(d, hq, hk, bs, seq_lens, q_lens, causal):
+    q, kc, vc, bt, cu, sl = _paged_setup(seq_lens, q_lens, hq, hk, d, bs, dv=128, seed=3)
+    q[: q_lens[0]] *= 4.0                      # scores far apart: the reference maximum moves
+    want, lse_want = ref.paged_attention(q, kc, vc, bt, cu, sl, hq, d ** -0.5, causal, 0, True)
+    for _ in range(2):
+        got, lse = ops.gqa_prefill(q.to(DEV), kc.to(DEV), vc.to(DEV), bt.to(DEV), cu.to(DEV), sl.to(DEV),
+                                   len(seq_lens), max(q_lens), hq, d ** -0.5, causal, 0, True)
+        # P and the result are rounded to bf16 (2^-9 each) of values up to about 4
+        _close(got, want, 2e-2, 2e-2)
+        _close(lse, lse_want, 2e-2, 1e-2)
+
+
 @pytest.mark.parametrize("d,bs", [(128, 16), (64, 16), (128, 128)])
 def test_gqa_prefill(d, bs):
     seq_lens, q_lens = [130, 64, 517, 9], [130, 33, 200, 9]
