@@ -15,6 +15,12 @@ int b200_gemm(const void* A, const void* W, void* C, const void* bias, const voi
               int N, int K, int lda, int ldw, int ldc, int dtype_fp8, int out_fp32, int swiglu,
               int BN, int splits, int cluster_split, void* workspace, int* counters, int* status,
               int max_ctas, float act_alpha, float act_limit, cudaStream_t stream);
+int b200_gemm_stream(const void* A, const void* W, void* C, const void* bias, const void* residual, int M, int N, int K,
+                     int lda, int ldw, int ldc, int out_fp32, int act, int splits, int* status, int max_ctas,
+                     float act_alpha, float act_limit, cudaStream_t stream);
+int b200_grouped_gemm_stream(const void* A, const void* W, void* C, const int* expert_offsets, int num_experts,
+                             int total_rows, int N, int K, int lda, int ldc, int act, int tn, int* status, int max_ctas,
+                             float act_alpha, float act_limit, cudaStream_t stream);
 int b200_gemm_pair(const void* A, const void* W, void* C, const void* bias, const void* residual,
                    int M, int N, int K, int lda, int ldw, int ldc, int dtype_fp8, int out_fp32,
                    int swiglu, int BN, int* status, int max_ctas, float act_alpha, float act_limit,
@@ -208,6 +214,56 @@ Tensor gemm_pair(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& 
                        (int)act, (int)bn, status.data_ptr<int>(), (int)max_ctas,
                        (float)act_alpha, (float)act_limit, cur_stream()),
         "gemm_pair");
+  return c;
+}
+
+// Same contract as gemm() for at most 128 bf16 rows: the weights are the tensor cores' M operand (gemm/gemm_stream.cu).
+Tensor gemm_stream(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& bias,
+                   const c10::optional<Tensor>& residual, bool out_fp32, int64_t act, int64_t splits,
+                   const Tensor& status, int64_t max_ctas, double act_alpha, double act_limit) {
+  TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 2, "gemm_stream: 2-D CUDA tensors");
+  TORCH_CHECK(a.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16, "gemm_stream: bf16 inputs");
+  TORCH_CHECK(a.stride(1) == 1 && w.stride(1) == 1, "gemm_stream: K must be contiguous");
+  const int M = a.size(0), K = a.size(1), N = w.size(0);
+  TORCH_CHECK(w.size(1) == K, "gemm_stream: K mismatch");
+  c10::cuda::CUDAGuard guard(a.device());
+  const int n_out = gated(act) ? N / 2 : N;
+  Tensor c = torch::empty({M, n_out}, a.options().dtype(out_fp32 ? at::kFloat : at::kBFloat16));
+  const void* bias_p = nullptr;
+  const void* res_p = nullptr;
+  if (bias.has_value()) {
+    CHECK_CUDA_BF16(*bias);
+    TORCH_CHECK(bias->numel() == N && bias->is_contiguous(), "gemm_stream: bias [N]");
+    bias_p = bias->data_ptr();
+  }
+  if (residual.has_value()) {
+    CHECK_CUDA_BF16(*residual);
+    TORCH_CHECK(residual->is_contiguous() && residual->size(0) == M && residual->size(1) == n_out,
+                "gemm_stream: residual [M,N] contiguous");
+    res_p = residual->data_ptr();
+  }
+  check(b200_gemm_stream(a.data_ptr(), w.data_ptr(), c.data_ptr(), bias_p, res_p, M, N, K, (int)a.stride(0),
+                         (int)w.stride(0), n_out, out_fp32 ? 1 : 0, (int)act, (int)splits, status.data_ptr<int>(),
+                         (int)max_ctas, (float)act_alpha, (float)act_limit, cur_stream()),
+        "gemm_stream");
+  return c;
+}
+
+Tensor grouped_gemm_stream(const Tensor& a, const Tensor& w, const Tensor& expert_offsets, int64_t act, int64_t tn,
+                           const Tensor& status, int64_t max_ctas, double act_alpha, double act_limit) {
+  TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 3, "grouped_gemm: shapes");
+  TORCH_CHECK(a.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16, "grouped_gemm: bf16 inputs");
+  TORCH_CHECK(a.stride(1) == 1 && w.is_contiguous(), "grouped_gemm: contiguity");
+  CHECK_I32(expert_offsets);
+  const int E = w.size(0), N = w.size(1), K = w.size(2), rows = a.size(0);
+  TORCH_CHECK(a.size(1) == K && expert_offsets.numel() == E + 1, "grouped_gemm: size mismatch");
+  c10::cuda::CUDAGuard guard(a.device());
+  const int n_out = gated(act) ? N / 2 : N;
+  Tensor c = torch::empty({rows, n_out}, a.options());
+  check(b200_grouped_gemm_stream(a.data_ptr(), w.data_ptr(), c.data_ptr(), expert_offsets.data_ptr<int>(), E, rows, N, K,
+                                 (int)a.stride(0), n_out, (int)act, (int)tn, status.data_ptr<int>(), (int)max_ctas,
+                                 (float)act_alpha, (float)act_limit, cur_stream()),
+        "grouped_gemm_stream");
   return c;
 }
 
@@ -1066,6 +1122,8 @@ TORCH_LIBRARY(omni_b200, m) {
   m.def("gemm_plan", &gemm_plan);
   m.def("gemm", &gemm);
   m.def("gemm_pair", &gemm_pair);
+  m.def("gemm_stream", &gemm_stream);
+  m.def("grouped_gemm_stream", &grouped_gemm_stream);
   m.def("grouped_gemm", &grouped_gemm);
   m.def("moe_topk", &moe_topk);
   m.def("argmax", &argmax);

@@ -1,0 +1,502 @@
+// Products with few rows, dense and grouped:  C[M,N] = A[M,K] * W[N,K]^T, bf16 in, fp32 accumulate.
+//
+// What bounds them is the weight stream, so the weights are the M operand: a tile is 128 rows of W times the
+// (16 .. 128) rows of A, and a stage of the ring is 16 KB of weights and 2 KB per 16 rows of A.  (With the rows of A
+// as the M operand, gemm_tcgen05_kernel, every slab carries 16 KB of A whatever M is.)  A CTA takes half of an SM's
+// shared memory: two are resident, or one and the next kernel's, whose first ring of weights then flows while this
+// kernel finishes.
+//
+// Dense: N / 128 tiles; when these are fewer than the resident CTAs, the 2, 4 or 8 CTAs of a cluster share a tile's
+// K and sum their parts in rank order over distributed shared memory.  The split depends on N and K alone, so the
+// result of a row does not depend on the number of rows.
+// Grouped: tiles of all live experts, each read once; an expert with more rows than a tile takes several tiles side by
+// side, which share its weights in L2.
+//
+// Measured in a CUDA graph, one row (us, gemm_tcgen05_kernel / here / the weights at 6.4 TB/s): 4096 x 4096
+// 17.5 / 9.2 / 5.2, 6144 x 4096 22.7 / 12.5 / 7.8, 4096 x 14336 35.2 / 21.5 / 18.2, 28672 x 4096 with silu 71.5 / 41.4 /
+// 36.5, 128256 x 4096 193 / 162 / 163; 83 of 128 experts live, 1536 x 2048 with silu 121 / 83 / 81.
+// Against 8 CTAs per cluster throughout: 6144 x 4096 takes 16.0 (only what stays resident at once pays).
+//
+// Per CTA (192 threads): warp 0 TMA, warp 1 MMA, warps 2-5 epilogue (a thread holds one column of C and the rows of A
+// one after another).  Every wait is bounded; on expiry the CTA records a status code, waits for its copies in flight,
+// frees its TMEM and returns.
+
+#include "../common/device_once.h"
+#include "../common/pdl.cuh"
+#include "../common/ptx.cuh"
+#include "../common/tensormap.h"
+#include "gated_act.cuh"
+
+namespace b200 {
+
+namespace stream {
+constexpr int BW = 128;                  // rows of W per tile
+constexpr int SLAB_K = 64;               // elements of K per stage: 128 bytes
+constexpr int W_BYTES = BW * 128;
+constexpr int THREADS = 192;
+constexpr int RING = 108 * 1024;         // of a CTA, so that two fit an SM
+constexpr int MAX_EXPERTS = 512;
+}  // namespace stream
+
+struct StreamParams {
+  int M, N, K;
+  int tn;                 // rows of A per tile: 16, 32, 64 or 128
+  int box;                // rows of A per copy: dense tn (rows past the end cost nothing), grouped 16
+  int stages, k_slabs, splits, num_n_tiles;
+  int num_experts;
+  int ldc, out_fp32, act;
+  float act_alpha, act_limit;
+  void* C;
+  const __nv_bfloat16* bias;
+  const __nv_bfloat16* residual;
+  const int* expert_offsets;
+  int* status;
+};
+
+struct StreamTile {
+  int n0, row0, rows, expert;
+};
+
+template <bool GROUPED>
+__device__ __forceinline__ bool stream_tile(const StreamParams& p, const int* prefix, const int* first_row, int t,
+                                            int& cursor, StreamTile& tile) {
+  if constexpr (GROUPED) {
+    if (t >= prefix[p.num_experts]) return false;
+    while (prefix[cursor + 1] <= t) ++cursor;
+    const int row0 = first_row[cursor], rows = first_row[cursor + 1] - row0;
+    const int row_tiles = (rows + p.tn - 1) / p.tn;
+    const int local = t - prefix[cursor], rt = local % row_tiles;
+    tile.n0 = local / row_tiles * stream::BW;
+    tile.row0 = row0 + rt * p.tn;
+    tile.rows = min(p.tn, rows - rt * p.tn);
+    tile.expert = cursor;
+  } else {
+    if (t >= p.num_n_tiles) return false;
+    tile.n0 = t * stream::BW;
+    tile.row0 = 0;
+    tile.rows = p.M;
+    tile.expert = 0;
+  }
+  return true;
+}
+
+// One value of C per thread (column n; the 32 lanes of a warp hold neighbouring columns): epilogue and store.
+__device__ __forceinline__ void stream_store(const StreamParams& p, float v, int row, int n) {
+  const bool ok = n < p.N;
+  const float bias = p.bias && ok ? __bfloat162float(p.bias[n]) : 0.f;
+  if (act_is_gated(p.act)) {
+    v += bias;
+    // columns alternate in groups of eight: gate, up (N is a multiple of 16)
+    const float up = __shfl_xor_sync(0xffffffffu, v, 8);
+    if (ok && !(n & 8))
+      static_cast<__nv_bfloat16*>(p.C)[static_cast<size_t>(row) * p.ldc + (n >> 4) * 8 + (n & 7)] =
+          __float2bfloat16(gated_act(p.act, v, up, p.act_alpha, p.act_limit));
+    return;
+  }
+  if (act_is_unary(p.act)) v = unary_act(p.act, v, p.act_alpha, p.act_limit);
+  if (!ok) return;
+  v += bias;
+  const size_t at = static_cast<size_t>(row) * p.ldc + n;
+  if (p.residual) v += __bfloat162float(p.residual[at]);
+  if (p.out_fp32)
+    static_cast<float*>(p.C)[at] = v;
+  else
+    static_cast<__nv_bfloat16*>(p.C)[at] = __float2bfloat16(v);
+}
+
+template <bool GROUPED>
+__global__ void __launch_bounds__(stream::THREADS, 2)
+gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
+                   const StreamParams p) {
+  using namespace stream;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  const int stage_bytes = W_BYTES + p.tn * 128;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + p.stages * stage_bytes);
+  uint64_t* empty_bar = full_bar + p.stages;
+  uint64_t* tmem_full = empty_bar + p.stages;
+  uint64_t* tmem_empty = tmem_full + 2;
+  uint64_t* drain_bar = tmem_empty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* prefix = const_cast<int*>(abort_flag) + 1;       // grouped: tiles before an expert, [E + 1]
+  int* first_row = prefix + p.num_experts + 1;          // grouped: the offsets
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int acc_stride = p.tn;
+  const uint32_t tmem_cols = p.tn < 32 ? 32u : 2u * p.tn;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&tmem_full[i], 1);
+      mbar_init(&tmem_empty[i], 4);
+    }
+    mbar_init(drain_bar, 1);
+    *abort_flag = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tm_w);
+    tma_prefetch_desc(&tm_x);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, tmem_cols);
+    tmem_relinquish();
+  }
+  if constexpr (GROUPED) {
+    pdl_wait();      // the offsets come from an earlier kernel
+    if (warp == 2) {
+      const int per = (p.num_experts + 31) / 32;
+      const int e0 = min(p.num_experts, lane * per), e1 = min(p.num_experts, e0 + per);
+      int tiles = 0;
+      for (int e = e0; e < e1; ++e)
+        tiles += (p.expert_offsets[e + 1] - p.expert_offsets[e] + p.tn - 1) / p.tn * p.num_n_tiles;
+      int incl = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      int before = incl - tiles;
+      for (int e = e0; e < e1; ++e) {
+        const int a = p.expert_offsets[e], b = p.expert_offsets[e + 1];
+        prefix[e] = before;
+        first_row[e] = a;
+        before += (b - a + p.tn - 1) / p.tn * p.num_n_tiles;
+        if (e + 1 == p.num_experts) {
+          prefix[e + 1] = before;
+          first_row[e + 1] = b;
+        }
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  const int rank = p.splits > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int t_first = blockIdx.x / p.splits, t_stride = gridDim.x / p.splits;
+  const int per = (p.k_slabs + p.splits - 1) / p.splits;
+  const int k_begin = rank * per, k_end = min(p.k_slabs, k_begin + per);
+
+  pdl_trigger();
+  // the weights are written by no kernel ahead of this one: their first ring is under way before the wait
+  const bool early = !GROUPED && threadIdx.x == 0;
+  if (!early) pdl_wait();
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      int stage = 0, cursor = 0, preloaded = 0, issued = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      StreamTile tile;
+      if constexpr (!GROUPED) {
+        if (stream_tile<GROUPED>(p, prefix, first_row, t_first, cursor, tile)) {
+          const uint32_t bytes = W_BYTES + (tile.rows + p.box - 1) / p.box * p.box * 128;
+          for (; preloaded < p.stages && k_begin + preloaded < k_end; ++preloaded) {
+            mbar_arrive_expect_tx(&full_bar[preloaded], bytes);
+            tma_load_2d(smem + preloaded * stage_bytes, &tm_w, &full_bar[preloaded], (k_begin + preloaded) * SLAB_K,
+                        tile.n0);
+          }
+        }
+        pdl_wait();
+      }
+      for (int t = t_first; ok && stream_tile<GROUPED>(p, prefix, first_row, t, cursor, tile); t += t_stride) {
+        const int boxes = (tile.rows + p.box - 1) / p.box;
+        for (int k = k_begin; k < k_end; ++k) {
+          uint8_t* dst = smem + stage * stage_bytes;
+          if (issued >= preloaded) {
+            if (!mbar_wait(&empty_bar[stage], phase ^ 1)) {
+              atomicCAS(p.status, 0, kStatusTimeoutEmptyBarrier);
+              *abort_flag = 1;
+              ok = false;
+              break;
+            }
+            mbar_arrive_expect_tx(&full_bar[stage], static_cast<uint32_t>(W_BYTES + boxes * p.box * 128));
+            if constexpr (GROUPED)
+              tma_load_3d(dst, &tm_w, &full_bar[stage], k * SLAB_K, tile.n0, tile.expert);
+            else
+              tma_load_2d(dst, &tm_w, &full_bar[stage], k * SLAB_K, tile.n0);
+          }
+          for (int i = 0; i < boxes; ++i)
+            tma_load_2d(dst + W_BYTES + i * p.box * 128, &tm_x, &full_bar[stage], k * SLAB_K, tile.row0 + i * p.box);
+          ++issued;
+          if (++stage == p.stages) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+      if (!ok) {
+        // (only after the first ring, so every stage's last copies are complete sets): wait, bounded, until they land
+        int s = stage;
+        uint32_t ph = phase;
+        for (int i = 0; i < p.stages && i < issued; ++i) {
+          if (--s < 0) {
+            s = p.stages - 1;
+            ph ^= 1;
+          }
+          mbar_wait(&full_bar[s], ph);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      int stage = 0, cursor = 0, acc = 0;
+      uint32_t phase = 0, acc_phase = 0;
+      bool ok = true;
+      StreamTile tile;
+      const uint32_t lo0 = (smem_u32(smem) & 0x3FFFF) >> 4;
+      for (int t = t_first; ok && stream_tile<GROUPED>(p, prefix, first_row, t, cursor, tile); t += t_stride) {
+        if (*abort_flag || !mbar_wait(&tmem_empty[acc], acc_phase ^ 1)) {
+          if (!*abort_flag) atomicCAS(p.status, 0, kStatusTimeoutTmemEmpty);
+          *abort_flag = 1;
+          break;
+        }
+        tc_fence_after_sync();
+        const uint32_t idesc = make_idesc(1, 1, BW, (tile.rows + p.box - 1) / p.box * p.box);
+        const uint32_t d = tmem_base + static_cast<uint32_t>(acc * acc_stride);
+        for (int k = k_begin; k < k_end; ++k) {
+          if (!mbar_wait(&full_bar[stage], phase)) {
+            atomicCAS(p.status, 0, kStatusTimeoutFullBarrier);
+            *abort_flag = 1;
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();
+          const uint32_t w_lo = lo0 + ((stage * stage_bytes) >> 4), x_lo = w_lo + (W_BYTES >> 4);
+          umma_first<kKindBF16>(d, w_lo, x_lo, idesc, k > k_begin ? 1u : 0u);
+          umma_acc<kKindBF16>(d, w_lo + 2, x_lo + 2, idesc);
+          umma_acc<kKindBF16>(d, w_lo + 4, x_lo + 4, idesc);
+          umma_acc<kKindBF16>(d, w_lo + 6, x_lo + 6, idesc);
+          tc_commit(&empty_bar[stage]);
+          if (++stage == p.stages) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+        if (!ok) break;
+        tc_commit(&tmem_full[acc]);
+        if (++acc == 2) {
+          acc = 0;
+          acc_phase ^= 1;
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue
+    const int quarter = warp & 3;
+    const int r = quarter * 32 + lane;      // row of the W tile
+    int cursor = 0, acc = 0;
+    uint32_t acc_phase = 0;
+    StreamTile tile;
+    for (int t = t_first; stream_tile<GROUPED>(p, prefix, first_row, t, cursor, tile); t += t_stride) {
+      bool ok = !*abort_flag && mbar_wait(&tmem_full[acc], acc_phase);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        if (lane == 0 && !*abort_flag) atomicCAS(p.status, 0, kStatusTimeoutTmemFull);
+        *abort_flag = 1;
+        break;
+      }
+      tc_fence_after_sync();
+      const uint32_t col = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc * acc_stride);
+      float* part = reinterpret_cast<float*>(smem);      // split K: [row of A][128] (the ring has been read)
+      for (int c = 0; c < tile.rows; c += 16) {
+        uint32_t v[16];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+            : "r"(col + static_cast<uint32_t>(c))
+            : "memory");
+        tmem_ld_wait();
+        const int n = min(16, tile.rows - c);
+        if (p.splits > 1) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (i < n) part[(c + i) * BW + r] = __uint_as_float(v[i]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (i < n) stream_store(p, __uint_as_float(v[i]), tile.row0 + c + i, tile.n0 + r);
+        }
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tmem_empty[acc]);
+      if (++acc == 2) {
+        acc = 0;
+        acc_phase ^= 1;
+      }
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (p.splits > 1) {
+    // one tile per CTA: the CTAs of the cluster share out its rows of A
+    cluster_sync_all();
+    if (warp >= 2 && !*abort_flag) {
+      const int r = (warp & 3) * 32 + lane;
+      const int n = t_first * BW + r;
+      for (int row = rank; row < p.M; row += p.splits) {
+        const uint32_t at = smem_u32(smem) + static_cast<uint32_t>((row * BW + r) * 4);
+        float v[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          v[s] = 0.f;
+          if (s < p.splits)
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[s]) : "r"(mapa_shared(at, s)) : "memory");
+        }
+        float sum = v[0];
+#pragma unroll
+        for (int s = 1; s < 8; ++s) sum += v[s];
+        stream_store(p, sum, row, n);
+      }
+    }
+    cluster_sync_all();
+  }
+  if (warp == 1) {
+    if (*abort_flag && lane == 0) {
+      // products still in flight write tensor memory: wait (bounded) for them before it is freed
+      tc_commit(drain_bar);
+      mbar_wait(drain_bar, 0);
+    }
+    __syncwarp();
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, tmem_cols);
+  }
+}
+
+static int stream_stages(int tn) {
+  const int n = stream::RING / (stream::W_BYTES + tn * 128);
+  return n > 8 ? 8 : n;
+}
+
+static size_t stream_smem(int tn, int stages, int num_experts) {
+  return 1024 + static_cast<size_t>(stages) * (stream::W_BYTES + tn * 128) + (2 * stages + 5) * 8 + 8 +
+         (num_experts > 0 ? 2 * (num_experts + 1) * 4 : 0);
+}
+
+// CTAs that share a tile's K: as many (a power of two up to the portable cluster size) as keep all CTAs resident at two
+// per SM, with at least four slabs each.
+static int stream_splits(int n_tiles, int k_slabs) {
+  int best = 1;
+  for (int s = 2; s <= 8; s *= 2) {
+    const int per = (k_slabs + s - 1) / s;
+    if (n_tiles * s <= 2 * sm_count() && per >= 4 && (s - 1) * per < k_slabs) best = s;
+  }
+  return best;
+}
+
+template <bool GROUPED>
+static int launch_stream(const CUtensorMap& tw, const CUtensorMap& tx, const StreamParams& p, int grid,
+                         cudaStream_t stream) {
+  auto kern = gemm_stream_kernel<GROUPED>;
+  static DeviceOnce once;
+  int dev = 0;
+  if (once.needed(&dev)) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 114 * 1024) != cudaSuccess) return -20;
+    once.mark(dev);
+  }
+  return launch_pdl(kern, dim3(grid), dim3(stream::THREADS), stream_smem(p.tn, p.stages, p.num_experts), stream,
+                    p.splits, tw, tx, p) == cudaSuccess
+             ? 0
+             : -21;
+}
+
+}  // namespace b200
+
+using namespace b200;
+
+// A [M <= 128, K] (pitch lda), W [N, K] (pitch ldw), C [M, N, or N / 2 with a gated activation].  splits 0: by rule.
+extern "C" int b200_gemm_stream(const void* A, const void* W, void* C, const void* bias, const void* residual, int M,
+                                int N, int K, int lda, int ldw, int ldc, int out_fp32, int act, int splits, int* status,
+                                int max_ctas, float act_alpha, float act_limit, cudaStream_t cu_stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (M > 128) return -10;
+  if (act_is_gated(act) && ((N % 16) != 0 || out_fp32 || residual)) return -11;
+  StreamParams p{};
+  p.M = M;
+  p.N = N;
+  p.K = K;
+  p.tn = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
+  p.box = p.tn;
+  p.stages = stream_stages(p.tn);
+  p.k_slabs = (K + stream::SLAB_K - 1) / stream::SLAB_K;
+  p.num_n_tiles = (N + stream::BW - 1) / stream::BW;
+  p.splits = splits > 0 ? splits : stream_splits(p.num_n_tiles, p.k_slabs);
+  if (p.splits != 1 && p.splits != 2 && p.splits != 4 && p.splits != 8) return -12;
+  if ((p.splits - 1) * ((p.k_slabs + p.splits - 1) / p.splits) >= p.k_slabs) return -12;
+  p.ldc = ldc;
+  p.out_fp32 = out_fp32;
+  p.act = act;
+  p.act_alpha = act_alpha;
+  p.act_limit = act_limit;
+  p.C = C;
+  p.bias = static_cast<const __nv_bfloat16*>(bias);
+  p.residual = static_cast<const __nv_bfloat16*>(residual);
+  p.status = status;
+  CUtensorMap tw, tx;
+  int r = make_tensormap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, N, K, ldw, stream::BW, stream::SLAB_K,
+                            CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r) return r;
+  r = make_tensormap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, M, K, lda, p.box, stream::SLAB_K,
+                        CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r) return r - 1000;
+  int grid = p.num_n_tiles * p.splits;
+  if (p.splits == 1) {
+    const int most = max_ctas > 0 ? max_ctas : 2 * sm_count();
+    if (grid > most) grid = most;
+  }
+  return launch_stream<false>(tw, tx, p, grid, cu_stream);
+}
+
+// A [total_rows, K], W [E, N, K]; rows expert_offsets[e] .. expert_offsets[e + 1] (device) belong to expert e.
+// tn: rows of A per tile, 16, 32, 64 or 128.
+extern "C" int b200_grouped_gemm_stream(const void* A, const void* W, void* C, const int* expert_offsets,
+                                        int num_experts, int total_rows, int N, int K, int lda, int ldc, int act, int tn,
+                                        int* status, int max_ctas, float act_alpha, float act_limit,
+                                        cudaStream_t cu_stream) {
+  if (total_rows <= 0 || num_experts <= 0 || N <= 0 || K <= 0) return 0;
+  if (num_experts > stream::MAX_EXPERTS) return -13;
+  if (tn != 16 && tn != 32 && tn != 64 && tn != 128) return -10;
+  if (act_is_gated(act) && (N % 16) != 0) return -11;
+  StreamParams p{};
+  p.M = total_rows;
+  p.N = N;
+  p.K = K;
+  p.tn = tn;
+  p.box = 16;
+  p.stages = stream_stages(tn);
+  p.k_slabs = (K + stream::SLAB_K - 1) / stream::SLAB_K;
+  p.num_n_tiles = (N + stream::BW - 1) / stream::BW;
+  p.splits = 1;
+  p.num_experts = num_experts;
+  p.ldc = ldc;
+  p.act = act;
+  p.act_alpha = act_alpha;
+  p.act_limit = act_limit;
+  p.C = C;
+  p.expert_offsets = expert_offsets;
+  p.status = status;
+  // at most one row tile per expert beyond those that total_rows fill
+  const long long row_tiles = total_rows / tn + (num_experts < total_rows ? num_experts : total_rows);
+  if (row_tiles * p.num_n_tiles > 0x7fffffffll) return -14;
+  CUtensorMap tw, tx;
+  int r = make_tensormap_3d(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, num_experts, N, K, static_cast<uint64_t>(N) * K,
+                            K, stream::BW, stream::SLAB_K, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r) return r;
+  r = make_tensormap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, total_rows, K, lda, p.box, stream::SLAB_K,
+                        CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r) return r - 1000;
+  int grid = max_ctas > 0 ? max_ctas : 2 * sm_count();
+  if (row_tiles * p.num_n_tiles < grid) grid = static_cast<int>(row_tiles * p.num_n_tiles);
+  return launch_stream<true>(tw, tx, p, grid, cu_stream);
+}

@@ -198,6 +198,17 @@ PAIR_MIN_M = int(os.environ.get("OMNI_B200_GEMM_PAIR_MIN_M", "1024"))
 SMALL_M_GEMM = os.environ.get("OMNI_B200_SMALL_M_GEMM", "library")
 SMALL_M_LIBRARY_ROWS = (64, 256)
 
+# Products with fewer bf16 rows than this stream their weights through gemm_stream_kernel.  Measured in a CUDA graph
+# (us, gemm_tcgen05_kernel / gemm_stream_kernel) with 1 and 63 rows: 4096 x 4096 17.5 / 9.2 and 17.6 / 12.5,
+# 28672 x 4096 with silu 71.5 / 41.4 and 61.1 / 49.7, 128256 x 4096 193 / 162 and 178 / 177; with 128 rows the last is
+# 187 / 200: the rows of A, read again for every 128 columns, then weigh as much as the weights.
+STREAM_ROWS = 64
+# The grouped form pays up to this many rows per group on average (rows of A per tile: 64 up to half of it, then 128).
+# 128 groups 1536 x 2048 with silu: 121 / 83 us with 1 row per group, 169 / 127 with 8,
+# 172 / 136 with 32, 172 / 148 with 64; 208 / 211 with 128.  64 groups 2048 x 1408: 79.5 / 62 with 12 rows, 81 / 72
+# with 48, 85 / 88 with 96.
+STREAM_GROUP_ROWS = 64
+
 GELU_TANH = "gelu_tanh"    # gated activation gelu(gate) * up, gelu in its tanh form
 RELU = "relu"              # gated activation max(gate, 0) * up
 UNARY = {"relu2": 5, "tanh": 6}
@@ -260,6 +271,11 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
         return C.gemm_pair(a, w, bias, residual, out_dtype == torch.float32, kind[0], pbn, st.status, max_ctas,
                            kind[1], kind[2])
     fused, gated = kind[0] != 0, kind[0] in (1, 2, 4, 7)
+    if (m < STREAM_ROWS and a.dtype == torch.bfloat16 and bn == 0 and splits == 0
+            and not (gated and (residual is not None or out_dtype == torch.float32))):
+        _count(1)
+        return C.gemm_stream(a, w, bias, residual, out_dtype == torch.float32, kind[0], 0, st.status, max_ctas, kind[1],
+                             kind[2])
     key = (m, n, k, a.dtype.itemsize, kind[0], bn, splits)
     plan = st.plans.get(key)
     if plan is None:
@@ -407,10 +423,15 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, expert_offsets: torch.Tensor,
     if a.dtype == torch.float32:
         _count(1)
         return _core().gemm_simt(a, w, expert_offsets, *kind, None)
-    if bn <= 0:
-        bn = grouped_tile(a.shape[0], w.shape[0], w.shape[1], w.shape[2])
     st = device_state(a.device)
     _count(1)
+    rows, groups, n, k = a.shape[0], *w.shape
+    if bn <= 0 and a.dtype == torch.bfloat16 and rows <= STREAM_GROUP_ROWS * groups:
+        return _core().grouped_gemm_stream(a, w, expert_offsets, kind[0],
+                                           64 if 2 * rows <= STREAM_GROUP_ROWS * groups else 128, st.status, max_ctas,
+                                           kind[1], kind[2])
+    if bn <= 0:
+        bn = grouped_tile(rows, groups, n, k)
     return _core().grouped_gemm(a, w, expert_offsets, kind[0], bn, st.status, max_ctas, kind[1], kind[2])
 
 

@@ -169,6 +169,47 @@ def test_grouped_gemm():
     _close(out, want, 0.06, 3e-2)
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 128, 64), (1, 6144, 4096), (15, 1000, 520), (16, 4096, 14336), (17, 24, 2048),
+                                   (33, 28672, 256), (63, 40000, 128), (5, 130, 8)])
+def test_gemm_few_rows(m, n, k):
+    """Weights as the M operand: every tile width, K splits of 1 to 8, ragged N and K, all epilogues."""
+    torch.manual_seed(m + n + k)
+    a = torch.randn(m, k, device=DEV, dtype=torch.bfloat16)
+    w = (torch.randn(n, k, device=DEV) * k ** -0.5).bfloat16()
+    bias = torch.randn(n, device=DEV, dtype=torch.bfloat16)
+    res = torch.randn(m, n, device=DEV, dtype=torch.bfloat16)
+    exact = a.double() @ w.double().T
+    # fp32 sums of k products of size k ** -0.5: k * 2 ** -24 of their absolute sum at worst
+    _close(ops.gemm(a, w, out_dtype=torch.float32), exact.float(), k ** 0.5 * 2 ** -22 + 1e-6, 0)
+    # one rounding to bf16
+    _close(ops.gemm(a, w, bias, res), (exact + bias.double() + res.double()).float(), 1e-3, 2 ** -8)
+    _close(ops.gemm(a, w, bias, unary="relu2"), (exact.clamp_min(0) ** 2 + bias.double()).float(), 1e-3, 2 ** -8)
+    if n % 16 == 0:
+        gate, up = exact.view(m, -1, 2, 8).unbind(2)
+        _close(ops.gemm(a, w, swiglu=True), (torch.nn.functional.silu(gate) * up).reshape(m, -1).float(), 1e-3, 2 ** -7)
+    # a row's result does not depend on the rows beside it
+    assert torch.equal(ops.gemm(a[:1], w), ops.gemm(a, w)[:1])
+    ops.check_status()
+
+
+@pytest.mark.parametrize("counts,n,k", [([1], 128, 64), ([0, 16, 17, 0, 1, 200, 0], 256, 320), ([64, 65, 0, 63], 1000, 96),
+                                        ([0, 0, 0, 3], 48, 40), ([1] * 70, 144, 128), ([300] + [0] * 11, 384, 256)])
+def test_grouped_gemm_few_rows(counts, n, k):
+    torch.manual_seed(len(counts) + n)
+    offs = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32)
+    rows, e = int(offs[-1]), len(counts)
+    assert rows <= ops.STREAM_GROUP_ROWS * e
+    a = torch.randn(rows + 5, k, device=DEV, dtype=torch.bfloat16)      # rows past the last offset take no part
+    w = (torch.randn(e, n, k, device=DEV) * k ** -0.5).bfloat16()
+    exact = torch.cat([a[offs[i]: offs[i + 1]].double() @ w[i].double().T for i in range(e)])
+    _close(ops.grouped_gemm(a, w, offs.to(DEV))[:rows], exact.float(), 1e-3, 2 ** -8)
+    if n % 16 == 0:
+        gate, up = exact.view(rows, -1, 2, 8).unbind(2)
+        _close(ops.grouped_gemm(a, w, offs.to(DEV), swiglu=True)[:rows],
+               (torch.nn.functional.silu(gate) * up).reshape(rows, -1).float(), 1e-3, 2 ** -7)
+    ops.check_status()
+
+
 def test_gemm_fp8_plain():
     torch.manual_seed(4)
     m, n, k = 256, 512, 1024
