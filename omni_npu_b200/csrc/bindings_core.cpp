@@ -21,6 +21,9 @@ int b200_gemm_stream(const void* A, const void* W, void* C, const void* bias, co
 int b200_grouped_gemm_stream(const void* A, const void* W, void* C, const int* expert_offsets, int num_experts,
                              int total_rows, int N, int K, int lda, int ldc, int act, int tn, int* status, int max_ctas,
                              float act_alpha, float act_limit, cudaStream_t stream);
+int b200_grouped_gemm_pair(const void* A, const void* W, void* C, const int* expert_offsets, int num_experts,
+                           int total_rows, int N, int K, int lda, int ldc, int act, int* status, int max_ctas,
+                           float act_alpha, float act_limit, cudaStream_t stream);
 int b200_gemm_pair(const void* A, const void* W, void* C, const void* bias, const void* residual,
                    int M, int N, int K, int lda, int ldw, int ldc, int dtype_fp8, int out_fp32,
                    int swiglu, int BN, int* status, int max_ctas, float act_alpha, float act_limit,
@@ -249,8 +252,9 @@ Tensor gemm_stream(const Tensor& a, const Tensor& w, const c10::optional<Tensor>
   return c;
 }
 
-Tensor grouped_gemm_stream(const Tensor& a, const Tensor& w, const Tensor& expert_offsets, int64_t act, int64_t tn,
-                           const Tensor& status, int64_t max_ctas, double act_alpha, double act_limit) {
+// tn: rows per tile of the weight-streaming kernel (gemm/gemm_stream.cu), 0: the kernel on CTA pairs (gemm/grouped_pair.cu).
+Tensor grouped_gemm_rows(const Tensor& a, const Tensor& w, const Tensor& expert_offsets, int64_t act, int64_t tn,
+                         const Tensor& status, int64_t max_ctas, double act_alpha, double act_limit) {
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 3, "grouped_gemm: shapes");
   TORCH_CHECK(a.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16, "grouped_gemm: bf16 inputs");
   TORCH_CHECK(a.stride(1) == 1 && w.is_contiguous(), "grouped_gemm: contiguity");
@@ -260,10 +264,17 @@ Tensor grouped_gemm_stream(const Tensor& a, const Tensor& w, const Tensor& exper
   c10::cuda::CUDAGuard guard(a.device());
   const int n_out = gated(act) ? N / 2 : N;
   Tensor c = torch::empty({rows, n_out}, a.options());
-  check(b200_grouped_gemm_stream(a.data_ptr(), w.data_ptr(), c.data_ptr(), expert_offsets.data_ptr<int>(), E, rows, N, K,
-                                 (int)a.stride(0), n_out, (int)act, (int)tn, status.data_ptr<int>(), (int)max_ctas,
-                                 (float)act_alpha, (float)act_limit, cur_stream()),
-        "grouped_gemm_stream");
+  const int* offsets = expert_offsets.data_ptr<int>();
+  if (tn > 0)
+    check(b200_grouped_gemm_stream(a.data_ptr(), w.data_ptr(), c.data_ptr(), offsets, E, rows, N, K, (int)a.stride(0),
+                                   n_out, (int)act, (int)tn, status.data_ptr<int>(), (int)max_ctas, (float)act_alpha,
+                                   (float)act_limit, cur_stream()),
+          "grouped_gemm_stream");
+  else
+    check(b200_grouped_gemm_pair(a.data_ptr(), w.data_ptr(), c.data_ptr(), offsets, E, rows, N, K, (int)a.stride(0), n_out,
+                                 (int)act, status.data_ptr<int>(), (int)max_ctas, (float)act_alpha, (float)act_limit,
+                                 cur_stream()),
+          "grouped_gemm_pair");
   return c;
 }
 
@@ -1123,7 +1134,7 @@ TORCH_LIBRARY(omni_b200, m) {
   m.def("gemm", &gemm);
   m.def("gemm_pair", &gemm_pair);
   m.def("gemm_stream", &gemm_stream);
-  m.def("grouped_gemm_stream", &grouped_gemm_stream);
+  m.def("grouped_gemm_rows", &grouped_gemm_rows);
   m.def("grouped_gemm", &grouped_gemm);
   m.def("moe_topk", &moe_topk);
   m.def("argmax", &argmax);

@@ -25,7 +25,7 @@
 #include "../common/pdl.cuh"
 #include "../common/ptx.cuh"
 #include "../common/tensormap.h"
-#include "gated_act.cuh"
+#include "column_store.cuh"
 
 namespace b200 {
 
@@ -104,7 +104,8 @@ __device__ __forceinline__ void stream_store(const StreamParams& p, float v, int
     static_cast<__nv_bfloat16*>(p.C)[at] = __float2bfloat16(v);
 }
 
-template <bool GROUPED>
+// SPLIT: the CTAs of a cluster share a tile's K.
+template <bool GROUPED, bool SPLIT>
 __global__ void __launch_bounds__(stream::THREADS, 2)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                    const StreamParams p) {
@@ -177,9 +178,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  const int rank = p.splits > 1 ? static_cast<int>(cluster_ctarank()) : 0;
-  const int t_first = blockIdx.x / p.splits, t_stride = gridDim.x / p.splits;
-  const int per = (p.k_slabs + p.splits - 1) / p.splits;
+  const int rank = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
+  const int t_first = SPLIT ? blockIdx.x / p.splits : blockIdx.x, t_stride = SPLIT ? gridDim.x / p.splits : gridDim.x;
+  const int per = SPLIT ? (p.k_slabs + p.splits - 1) / p.splits : p.k_slabs;
   const int k_begin = rank * per, k_end = min(p.k_slabs, k_begin + per);
 
   pdl_trigger();
@@ -292,6 +293,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     // ------------------------------------------------------------ epilogue
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;      // row of the W tile
+    // bf16 results without a residual, and without a bias behind a unary activation: stored in pairs of columns
+    const bool plain = !p.out_fp32 && !p.residual && !(p.bias && act_is_unary(p.act));
+    const bool pairs = columns_pair(p.C, p.ldc, p.N, act_is_gated(p.act));
     int cursor = 0, acc = 0;
     uint32_t acc_phase = 0;
     StreamTile tile;
@@ -305,6 +309,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       }
       tc_fence_after_sync();
       const uint32_t col = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc * acc_stride);
+      const int col_n = tile.n0 + r;
+      const float bias = plain && p.bias && col_n < p.N ? __bfloat162float(p.bias[col_n]) : 0.f;
       float* part = reinterpret_cast<float*>(smem);      // split K: [row of A][128] (the ring has been read)
       for (int c = 0; c < tile.rows; c += 16) {
         uint32_t v[16];
@@ -317,14 +323,21 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             : "memory");
         tmem_ld_wait();
         const int n = min(16, tile.rows - c);
-        if (p.splits > 1) {
+        if constexpr (SPLIT) {
 #pragma unroll
           for (int i = 0; i < 16; ++i)
             if (i < n) part[(c + i) * BW + r] = __uint_as_float(v[i]);
+        } else if (plain) {
+          float x[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(v[i]) + bias;
+          store_act_columns(p.act, p.act_alpha, p.act_limit, x,
+                            static_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(tile.row0 + c) * p.ldc, p.ldc, col_n, p.N,
+                            n, pairs);
         } else {
 #pragma unroll
           for (int i = 0; i < 16; ++i)
-            if (i < n) stream_store(p, __uint_as_float(v[i]), tile.row0 + c + i, tile.n0 + r);
+            if (i < n) stream_store(p, __uint_as_float(v[i]), tile.row0 + c + i, col_n);
         }
       }
       tc_fence_before_sync();
@@ -339,7 +352,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 
   tc_fence_before_sync();
   __syncthreads();
-  if (p.splits > 1) {
+  if constexpr (SPLIT) {
     // one tile per CTA: the CTAs of the cluster share out its rows of A
     cluster_sync_all();
     if (warp >= 2 && !*abort_flag) {
@@ -395,10 +408,10 @@ static int stream_splits(int n_tiles, int k_slabs) {
   return best;
 }
 
-template <bool GROUPED>
+template <bool GROUPED, bool SPLIT>
 static int launch_stream(const CUtensorMap& tw, const CUtensorMap& tx, const StreamParams& p, int grid,
                          cudaStream_t stream) {
-  auto kern = gemm_stream_kernel<GROUPED>;
+  auto kern = gemm_stream_kernel<GROUPED, SPLIT>;
   static DeviceOnce once;
   int dev = 0;
   if (once.needed(&dev)) {
@@ -455,7 +468,8 @@ extern "C" int b200_gemm_stream(const void* A, const void* W, void* C, const voi
     const int most = max_ctas > 0 ? max_ctas : 2 * sm_count();
     if (grid > most) grid = most;
   }
-  return launch_stream<false>(tw, tx, p, grid, cu_stream);
+  return p.splits > 1 ? launch_stream<false, true>(tw, tx, p, grid, cu_stream)
+                      : launch_stream<false, false>(tw, tx, p, grid, cu_stream);
 }
 
 // A [total_rows, K], W [E, N, K]; rows expert_offsets[e] .. expert_offsets[e + 1] (device) belong to expert e.
@@ -498,5 +512,5 @@ extern "C" int b200_grouped_gemm_stream(const void* A, const void* W, void* C, c
   if (r) return r - 1000;
   int grid = max_ctas > 0 ? max_ctas : 2 * sm_count();
   if (row_tiles * p.num_n_tiles < grid) grid = static_cast<int>(row_tiles * p.num_n_tiles);
-  return launch_stream<true>(tw, tx, p, grid, cu_stream);
+  return launch_stream<true, false>(tw, tx, p, grid, cu_stream);
 }

@@ -198,16 +198,13 @@ PAIR_MIN_M = int(os.environ.get("OMNI_B200_GEMM_PAIR_MIN_M", "1024"))
 SMALL_M_GEMM = os.environ.get("OMNI_B200_SMALL_M_GEMM", "library")
 SMALL_M_LIBRARY_ROWS = (64, 256)
 
-# Products with fewer bf16 rows than this stream their weights through gemm_stream_kernel.  Measured in a CUDA graph
-# (us, gemm_tcgen05_kernel / gemm_stream_kernel) with 1 and 63 rows: 4096 x 4096 17.5 / 9.2 and 17.6 / 12.5,
-# 28672 x 4096 with silu 71.5 / 41.4 and 61.1 / 49.7, 128256 x 4096 193 / 162 and 178 / 177; with 128 rows the last is
-# 187 / 200: the rows of A, read again for every 128 columns, then weigh as much as the weights.
+# Products with fewer bf16 rows than this stream their weights through gemm_stream_kernel; up to 128 rows with this many
+# weight rows at least (every SM then has a tile without splitting K).  Measured in a CUDA graph (us,
+# gemm_tcgen05_kernel / gemm_stream_kernel) with 1 and 63 rows: 4096 x 4096 17.5 / 9.2 and 17.6 / 12.5, 28672 x 4096 with
+# silu 71 / 40.6 and 60 / 43.3, 128256 x 4096 190 / 163 and 176 / 169; with 128 rows 61 / 47.4 and 184 / 181, but
+# 6144 x 4096 20 / 24: the rows of A, read again for every 128 columns, then weigh as much as the weights.
 STREAM_ROWS = 64
-# The grouped form pays up to this many rows per group on average (rows of A per tile: 64 up to half of it, then 128).
-# 128 groups 1536 x 2048 with silu: 121 / 83 us with 1 row per group, 169 / 127 with 8,
-# 172 / 136 with 32, 172 / 148 with 64; 208 / 211 with 128.  64 groups 2048 x 1408: 79.5 / 62 with 12 rows, 81 / 72
-# with 48, 85 / 88 with 96.
-STREAM_GROUP_ROWS = 64
+STREAM_WIDE_ROWS, STREAM_WIDE_N = 128, 148 * 128
 
 GELU_TANH = "gelu_tanh"    # gated activation gelu(gate) * up, gelu in its tanh form
 RELU = "relu"              # gated activation max(gate, 0) * up
@@ -271,7 +268,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
         return C.gemm_pair(a, w, bias, residual, out_dtype == torch.float32, kind[0], pbn, st.status, max_ctas,
                            kind[1], kind[2])
     fused, gated = kind[0] != 0, kind[0] in (1, 2, 4, 7)
-    if (m < STREAM_ROWS and a.dtype == torch.bfloat16 and bn == 0 and splits == 0
+    if ((m < STREAM_ROWS or m <= STREAM_WIDE_ROWS and n >= STREAM_WIDE_N) and a.dtype == torch.bfloat16 and bn == 0 and splits == 0
             and not (gated and (residual is not None or out_dtype == torch.float32))):
         _count(1)
         return C.gemm_stream(a, w, bias, residual, out_dtype == torch.float32, kind[0], 0, st.status, max_ctas, kind[1],
@@ -395,7 +392,7 @@ def gemm_scaled(a_q: torch.Tensor, w_q: torch.Tensor, a_scale: torch.Tensor, w_s
 
 @functools.lru_cache(maxsize=4096)
 def grouped_tile(rows: int, groups: int, n: int, k: int, sms: int = 148) -> int:
-    """Tile width of a grouped bf16 product whose ``rows`` rows spread evenly over the groups: 256, or the largest
+    """Tile width of a grouped e4m3 product whose ``rows`` rows spread evenly over the groups: 256, or the largest
     power of two from 32 that divides n, unless another width is clearly better under the cost model of the
     dense plan (csrc/gemm/gemm_tcgen05.cu): fewer idle SMs in a decode step, less padding of n in a prompt."""
     live = max(1, min(groups, rows))
@@ -412,6 +409,21 @@ def grouped_tile(rows: int, groups: int, n: int, k: int, sms: int = 148) -> int:
     return best if cost(best) < 0.95 * cost(first) else first
 
 
+@functools.lru_cache(maxsize=4096)
+def grouped_rows_tile(rows: int, groups: int, n: int, sms: int = 148) -> int:
+    """Kernel of a grouped bf16 product: rows of A per tile of gemm_stream_kernel, or 0 for grouped_pair_kernel.
+
+    Streaming wins while the weights outweigh the rows (us, streaming / pair): 128 groups 1536 x 2048 with silu 132 / 136
+    at 32 rows per group, 64 groups 2816 x 2048 117 / 125 at 48, but 128 groups 2048 x 768 110 / 79 at 64; with too few
+    tiles for the SMs, 4 groups 2048 x 2048 at 48 rows, 16.3 / 14.1.  A pair's tile is 256 weight rows: 16 groups
+    128 x 512 at 4096 rows 20.1 / 26.8.  Narrow tiles fill the SMs: there at 128 rows 7.9 with 32 and 9.2 with 64."""
+    per = -(-rows // groups)
+    tiles = min(rows, groups) * -(-n // 128)
+    if n > 128 and per > (48 if tiles >= sms else 16):
+        return 0
+    return 32 if tiles * -(-per // 64) < sms else 64 if per <= 48 else 128
+
+
 def grouped_gemm(a: torch.Tensor, w: torch.Tensor, expert_offsets: torch.Tensor,
                  swiglu: bool = False, bn: int = 0, max_ctas: int = 0,
                  act=SILU, unary: Optional[str] = None) -> torch.Tensor:
@@ -426,10 +438,9 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, expert_offsets: torch.Tensor,
     st = device_state(a.device)
     _count(1)
     rows, groups, n, k = a.shape[0], *w.shape
-    if bn <= 0 and a.dtype == torch.bfloat16 and rows <= STREAM_GROUP_ROWS * groups:
-        return _core().grouped_gemm_stream(a, w, expert_offsets, kind[0],
-                                           64 if 2 * rows <= STREAM_GROUP_ROWS * groups else 128, st.status, max_ctas,
-                                           kind[1], kind[2])
+    if bn <= 0 and a.dtype == torch.bfloat16:
+        return _core().grouped_gemm_rows(a, w, expert_offsets, kind[0], grouped_rows_tile(rows, groups, n), st.status,
+                                         max_ctas, kind[1], kind[2])
     if bn <= 0:
         bn = grouped_tile(rows, groups, n, k)
     return _core().grouped_gemm(a, w, expert_offsets, kind[0], bn, st.status, max_ctas, kind[1], kind[2])

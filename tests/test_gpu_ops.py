@@ -170,7 +170,7 @@ def test_grouped_gemm():
 
 
 @pytest.mark.parametrize("m,n,k", [(1, 128, 64), (1, 6144, 4096), (15, 1000, 520), (16, 4096, 14336), (17, 24, 2048),
-                                   (33, 28672, 256), (63, 40000, 128), (5, 130, 8)])
+                                   (33, 28672, 256), (63, 40000, 128), (5, 130, 8), (128, 20000, 64), (100, 18945, 72)])
 def test_gemm_few_rows(m, n, k):
     """Weights as the M operand: every tile width, K splits of 1 to 8, ragged N and K, all epilogues."""
     torch.manual_seed(m + n + k)
@@ -192,17 +192,21 @@ def test_gemm_few_rows(m, n, k):
     ops.check_status()
 
 
-@pytest.mark.parametrize("counts,n,k", [([1], 128, 64), ([0, 16, 17, 0, 1, 200, 0], 256, 320), ([64, 65, 0, 63], 1000, 96),
-                                        ([0, 0, 0, 3], 48, 40), ([1] * 70, 144, 128), ([300] + [0] * 11, 384, 256)])
-def test_grouped_gemm_few_rows(counts, n, k):
+@pytest.mark.parametrize("counts,n,k", [
+    ([1], 128, 64), ([0, 16, 17, 0, 1, 200, 0], 256, 320), ([64, 65, 0, 63], 1000, 96), ([0, 0, 0, 3], 48, 40),
+    ([1] * 70, 144, 128), ([300] + [0] * 11, 384, 256), ([255, 256, 257, 0, 31, 33, 513], 304, 136), ([2049], 2048, 8),
+    ([2600, 3], 512, 200), ([900, 100], 100, 64), ([129] * 70, 135, 72), ([33] * 200, 264, 64)])
+def test_grouped_gemm_tiles(counts, n, k):
+    """The weight-streaming kernel and the one on CTA pairs: ragged rows, rows of a tile dealt out evenly, odd N."""
     torch.manual_seed(len(counts) + n)
     offs = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32)
     rows, e = int(offs[-1]), len(counts)
-    assert rows <= ops.STREAM_GROUP_ROWS * e
     a = torch.randn(rows + 5, k, device=DEV, dtype=torch.bfloat16)      # rows past the last offset take no part
     w = (torch.randn(e, n, k, device=DEV) * k ** -0.5).bfloat16()
     exact = torch.cat([a[offs[i]: offs[i + 1]].double() @ w[i].double().T for i in range(e)])
+    # one rounding to bf16 (2 ** -9 relative), and of two products of fp32 activations
     _close(ops.grouped_gemm(a, w, offs.to(DEV))[:rows], exact.float(), 1e-3, 2 ** -8)
+    _close(ops.grouped_gemm(a, w, offs.to(DEV), unary="relu2")[:rows], (exact.clamp_min(0) ** 2).float(), 1e-3, 2 ** -8)
     if n % 16 == 0:
         gate, up = exact.view(rows, -1, 2, 8).unbind(2)
         _close(ops.grouped_gemm(a, w, offs.to(DEV), swiglu=True)[:rows],
