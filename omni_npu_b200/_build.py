@@ -41,7 +41,7 @@ CORE_SOURCES = [
     "attn/gqa_gated.cu", "attn/gqa_gated_decode.cu", "attn/gqa_gated_prefill.cu", "attn/gqa_prefill_tcgen05.cu",
     "attn/latent_attn.cu", "attn/mixed_attn.cu", "attn/mixed_attn_decode.cu", "attn/mixed_attn_prefill.cu",
     "attn/mla_decode.cu", "attn/qk_norm_rope.cu",
-    "gemm/gemm_simt.cu", "gemm/gemm_stream.cu", "gemm/gemm_tcgen05.cu", "gemm/gemm_tcgen05_pair.cu", "gemm/grouped_pair.cu", "moe/moe_ep.cu",
+    "gemm/gemm_pair.cu", "gemm/gemm_simt.cu", "gemm/gemm_stream.cu", "gemm/gemm_tcgen05.cu", "moe/moe_ep.cu",
     "norm_rope/hyper_norm.cu", "norm_rope/post_norm.cu", "norm_rope/residual_norm.cu", "recurrent/decay_prep.cu", "recurrent/recurrent.cu",
     "sample/sampling.cu",
 ]

@@ -184,8 +184,7 @@ Tensor gemm(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& bias,
   return c;
 }
 
-// Same contract as gemm() without split-K, run by CTA pairs: one 256 x BN tile per pair of SMs
-// (tcgen05 cta_group::2), each SM staging half of the weight tile.
+// Same contract as gemm() without split-K, run by CTA pairs (gemm/gemm_pair.cu); bn: rows of a per tile, 0 by rule.
 Tensor gemm_pair(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& bias,
                  const c10::optional<Tensor>& residual, bool out_fp32, int64_t act, int64_t bn,
                  const Tensor& status, int64_t max_ctas, double act_alpha, double act_limit) {
@@ -252,7 +251,7 @@ Tensor gemm_stream(const Tensor& a, const Tensor& w, const c10::optional<Tensor>
   return c;
 }
 
-// tn: rows per tile of the weight-streaming kernel (gemm/gemm_stream.cu), 0: the kernel on CTA pairs (gemm/grouped_pair.cu).
+// tn: rows per tile of the weight-streaming kernel (gemm/gemm_stream.cu), 0: the kernel on CTA pairs (gemm/gemm_pair.cu).
 Tensor grouped_gemm_rows(const Tensor& a, const Tensor& w, const Tensor& expert_offsets, int64_t act, int64_t tn,
                          const Tensor& status, int64_t max_ctas, double act_alpha, double act_limit) {
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 3, "grouped_gemm: shapes");

@@ -185,8 +185,13 @@ def check_status(device: Optional[torch.device] = None) -> None:
 
 # ------------------------------------------------------------------------ GEMM
 SILU = (0.0, 0.0)          # gated activation silu(gate) * up: no slope, no limit
-# smallest M routed to the CTA-pair GEMM (0 = never); prefill-sized problems only
+# smallest M always routed to the CTA-pair GEMM (0 = never)
 PAIR_MIN_M = int(os.environ.get("OMNI_B200_GEMM_PAIR_MIN_M", "1024"))
+# ... and above this many bf16 rows products whose plan has no K split (gated, or wide enough to fill the SMs).  Us,
+# gemm_tcgen05_kernel / gemm_pair_kernel: 5632 x 2048 with silu 17.2 / 12.8 at 100 rows,
+# 24.6 / 16.7 at 512; 102400 x 2048 119 / 88.5 at 200, 317 / 223 at 700; 4096 x 4096 25.4 / 20.6 at 400.  With a split K
+# 128 x 2048 takes 7.9 / 10.6 at 200.
+PAIR_UNSPLIT_M = 64
 # Plain bf16 products (no residual, SwiGLU, scales or fused collective) of a decode-sized batch
 # whose plan here is a cluster split-K: "library" hands them to cuBLAS, "own" keeps them on
 # gemm_tcgen05_kernel.  Measured at M = 128 inside a CUDA graph (us, own / cuBLAS): 4096 x 4096
@@ -246,8 +251,8 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
     reduced-precision mode.
     ``splits`` > 1 forces split-K (as a thread-block cluster when it fits), a
     negative value forces the workspace variant with |splits| slices.
-    ``pair`` selects the CTA-pair kernel (256-row tiles over two SMs); by default
-    it runs for M >= PAIR_MIN_M when no split-K was asked for."""
+    ``pair`` selects the CTA-pair kernel (tiles over two SMs, ``bn`` rows of ``a`` each); by default it runs for
+    M >= PAIR_MIN_M, and for bf16 above PAIR_UNSPLIT_M where K is not split, when neither was asked for."""
     if not a.is_cuda:
         return ref.gemm(a, w, bias, residual, out_dtype, swiglu, act, xielu, unary)
     C = _core()
@@ -262,10 +267,8 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
     if pair is None:
         pair = PAIR_MIN_M > 0 and m >= PAIR_MIN_M and splits == 0 and bn == 0
     if pair:
-        n_eff = n
-        pbn = bn if bn > 0 else (256 if n_eff >= 256 else max(32, ((n_eff + 31) // 32) * 32))
         _count(1)
-        return C.gemm_pair(a, w, bias, residual, out_dtype == torch.float32, kind[0], pbn, st.status, max_ctas,
+        return C.gemm_pair(a, w, bias, residual, out_dtype == torch.float32, kind[0], bn, st.status, max_ctas,
                            kind[1], kind[2])
     fused, gated = kind[0] != 0, kind[0] in (1, 2, 4, 7)
     if ((m < STREAM_ROWS or m <= STREAM_WIDE_ROWS and n >= STREAM_WIDE_N) and a.dtype == torch.bfloat16 and bn == 0 and splits == 0
@@ -279,6 +282,11 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
         plan = C.gemm_plan(m, n, k, a.dtype.itemsize, gated, bn, 1 if gated else max(0, splits) if fused else splits)
         st.plans[key] = plan
     pbn, psplits, ws_bytes, ncnt, cluster = plan
+    if pair is None and m > PAIR_UNSPLIT_M and 0 < PAIR_MIN_M and a.dtype == torch.bfloat16 and bn == 0 and splits == 0 \
+            and psplits == 1:
+        _count(1)
+        return C.gemm_pair(a, w, bias, residual, out_dtype == torch.float32, kind[0], 0, st.status, max_ctas,
+                           kind[1], kind[2])
     if library_small_m(m, bool(cluster), residual is None and not fused and bn == 0
                        and splits == 0 and a.dtype == torch.bfloat16 and out_dtype in (None, torch.bfloat16)):
         return torch.nn.functional.linear(a, w, bias)    # a library kernel: not counted as a launch of ours

@@ -192,6 +192,28 @@ def test_gemm_few_rows(m, n, k):
     ops.check_status()
 
 
+@pytest.mark.parametrize("m,n,k", [(65, 18944, 72), (129, 20000, 200), (257, 130, 64), (300, 1000, 136), (1023, 384, 1048),
+                                   (1025, 257, 8), (2000, 48, 520), (33, 304, 128)])
+def test_gemm_pair_rows(m, n, k):
+    """Rows of A as the N operand of CTA pairs: every width of a tile, ragged M, N and K, all epilogues."""
+    torch.manual_seed(m + n)
+    a = torch.randn(m, k, device=DEV, dtype=torch.bfloat16)
+    w = (torch.randn(n, k, device=DEV) * k ** -0.5).bfloat16()
+    bias = torch.randn(n, device=DEV, dtype=torch.bfloat16)
+    res = torch.randn(m, n, device=DEV, dtype=torch.bfloat16)
+    exact = a.double() @ w.double().T
+    for bn in (0, 32, 160, 224, 256):
+        _close(ops.gemm(a, w, bn=bn, pair=True), exact.float(), 1e-3, 2 ** -8)
+    # fp32 sums of k products of size k ** -0.5; else one rounding to bf16
+    _close(ops.gemm(a, w, out_dtype=torch.float32, pair=True), exact.float(), k ** 0.5 * 2 ** -22 + 1e-6, 0)
+    _close(ops.gemm(a, w, bias, res, pair=True), (exact + bias.double() + res.double()).float(), 1e-3, 2 ** -8)
+    _close(ops.gemm(a, w, bias, unary="relu2", pair=True), (exact.clamp_min(0) ** 2 + bias.double()).float(), 1e-3, 2 ** -8)
+    if n % 16 == 0:
+        gate, up = (exact + bias.double()).view(m, -1, 2, 8).unbind(2)
+        _close(ops.gemm(a, w, bias, swiglu=True), (torch.nn.functional.silu(gate) * up).reshape(m, -1).float(), 1e-3, 2 ** -7)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("counts,n,k", [
     ([1], 128, 64), ([0, 16, 17, 0, 1, 200, 0], 256, 320), ([64, 65, 0, 63], 1000, 96), ([0, 0, 0, 3], 48, 40),
     ([1] * 70, 144, 128), ([300] + [0] * 11, 384, 256), ([255, 256, 257, 0, 31, 33, 513], 304, 136), ([2049], 2048, 8),
