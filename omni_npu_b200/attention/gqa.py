@@ -64,13 +64,18 @@ class GQAAttention(torch.nn.Module):
         self.window = sliding_window
 
     def forward(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
-                cos_sin: Optional[torch.Tensor], apply_rope: bool = True) -> torch.Tensor:
+                cos_sin: Optional[torch.Tensor], apply_rope: bool = True, norm=None) -> torch.Tensor:
         """q [T, Hq*D], k [T, Hk*D], v [T, Hk*Dv] (views into the fused QKV
-        projection are fine).  Returns [T, Hq*Dv]."""
+        projection are fine).  ``norm`` = (q weight, k weight, eps): every head of q and k is normed
+        first.  Returns [T, Hq*Dv]."""
         ctx = get_forward_context()
         md: AttentionMetadata = ctx.attn_metadata
         k_cache, v_cache = ctx.kv_caches[self.layer_idx]
         pc = md.extra.get("pcp") if md.is_prefill else None
+        fused = pc is None and apply_rope and cos_sin is not None and md.positions.dim() == 1
+        if norm is not None and not fused:
+            q, k = (ops.rms_norm(x.reshape(-1, self.head_dim), w, norm[2]).view(x.shape[0], -1)
+                    for x, w in ((q, norm[0]), (k, norm[1])))
         if pc is not None:
             # prefill context parallelism: this rank holds the query rows of its token shard; the
             # keys and values of the whole step are gathered, rotated with their own positions and
@@ -92,9 +97,9 @@ class GQAAttention(torch.nn.Module):
             ops.gqa_cache_write(k_all, v_all, k_cache, v_cache, pc["slot_all"])
             return ops.gqa_prefill(q, k_cache, v_cache, md.block_tables, md.cu_q, md.seq_lens,
                                    md.num_seqs, md.max_q_len, self.num_heads, self.scale, True, self.window)
-        if apply_rope and cos_sin is not None and md.positions.dim() == 1:
-            ops.rope_cache_gqa_(q, k, v, k_cache, v_cache, md.positions, md.slot_mapping, cos_sin,
-                                self.head_dim, self.rot_dim, self.neox)
+        if fused:
+            q = ops.rope_cache_gqa_(q, k, v, k_cache, v_cache, md.positions, md.slot_mapping, cos_sin,
+                                    self.head_dim, self.rot_dim, self.neox, norm)
         else:
             ops.gqa_cache_write(k, v, k_cache, v_cache, md.slot_mapping)
         nd = md.extra.get("num_decode_seqs", 0) if md.is_prefill else 0

@@ -52,8 +52,8 @@ int b200_rope_qk(void* q, void* k, const int* positions, const float* cos_sin, i
 int b200_rope_cache_gqa(void* q, const void* k, const void* v, void* k_cache, void* v_cache,
                         const int* positions, const int* slot_mapping, const float* cos_sin, int T,
                         int Hq, int Hk, int D, int rot_dim, int neox, long long q_stride,
-                        long long k_stride, long long v_stride, int block_size,
-                        cudaStream_t stream);
+                        long long k_stride, long long v_stride, int block_size, const void* q_w, const void* k_w,
+                        float eps, cudaStream_t stream);
 int b200_mla_kv_rmsnorm_rope_cache(const void* kv_c, const void* k_pe, const void* w, void* cache,
                                    void* kv_c_out, void* k_pe_out, const int* positions,
                                    const int* slot_mapping, const float* cos_sin, float eps, int T,
@@ -430,9 +430,12 @@ void rope_qk(Tensor q, Tensor k, const Tensor& positions, const Tensor& cos_sin,
         "rope_qk");
 }
 
-void rope_cache_gqa(Tensor q, const Tensor& k, const Tensor& v, Tensor k_cache, Tensor v_cache,
+// q_w, k_w: a norm of every head of q and k ahead of the rotation.  False (nothing done): heads that the fused kernel
+// does not take.
+bool rope_cache_gqa(Tensor q, const Tensor& k, const Tensor& v, Tensor k_cache, Tensor v_cache,
                     const Tensor& positions, const Tensor& slot_mapping, const Tensor& cos_sin,
-                    int64_t head_dim, int64_t rot_dim, bool neox) {
+                    int64_t head_dim, int64_t rot_dim, bool neox, const c10::optional<Tensor>& q_w,
+                    const c10::optional<Tensor>& k_w, double eps) {
   CHECK_CUDA_BF16(q);
   CHECK_CUDA_BF16(k);
   CHECK_CUDA_BF16(v);
@@ -446,12 +449,23 @@ void rope_cache_gqa(Tensor q, const Tensor& k, const Tensor& v, Tensor k_cache, 
   const int T = q.size(0);
   const int Hk = k_cache.size(1), bs = k_cache.size(2);
   c10::cuda::CUDAGuard guard(q.device());
-  check(b200_rope_cache_gqa(q.data_ptr(), k.data_ptr(), v.data_ptr(), k_cache.data_ptr(),
+  const void *qw = nullptr, *kw = nullptr;
+  if (q_w.has_value() && k_w.has_value()) {
+    CHECK_CUDA_BF16(*q_w);
+    CHECK_CUDA_BF16(*k_w);
+    TORCH_CHECK(q_w->is_contiguous() && k_w->is_contiguous() && q_w->numel() == head_dim && k_w->numel() == head_dim,
+                "rope_cache: norm weights [head_dim]");
+    qw = q_w->data_ptr();
+    kw = k_w->data_ptr();
+  }
+  const int rc = b200_rope_cache_gqa(q.data_ptr(), k.data_ptr(), v.data_ptr(), k_cache.data_ptr(),
                             v_cache.data_ptr(), positions.data_ptr<int>(),
                             slot_mapping.data_ptr<int>(), cos_sin.data_ptr<float>(), T,
                             (int)(q.size(1) / head_dim), Hk, (int)head_dim, (int)rot_dim,
-                            neox ? 1 : 0, q.stride(0), k.stride(0), v.stride(0), bs, cur_stream()),
-        "rope_cache_gqa");
+                            neox ? 1 : 0, q.stride(0), k.stride(0), v.stride(0), bs, qw, kw, (float)eps, cur_stream());
+  if (rc == 1) return false;
+  check(rc, "rope_cache_gqa");
+  return true;
 }
 
 void mla_kv_rmsnorm_rope_cache(const Tensor& kv_c, const Tensor& k_pe, const Tensor& w, Tensor cache,

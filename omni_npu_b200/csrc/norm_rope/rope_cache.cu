@@ -301,6 +301,94 @@ rope_cache_gqa_vec_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
   }
 }
 
+// ---- whole heads, neox pairing, rot_dim = D: norm of q and k per head, rotation and cache rows in one pass -------------
+// A head belongs to D / 16 lanes of a warp (a power of two), each with eight elements of the lower half and the eight
+// that they are paired with: one read and one write of everything, the sum of squares by shuffles among the lanes.
+// What bounds it: memory, 2 x (q + k + v) bytes a token.  8192 tokens of 32 + 2 x 4 heads of 128: copies of the q and k
+// views, norms, rotation and cache rows as kernels of their own took 260 us, this one 47 (26 at 6.4 TB/s; the items of the
+// kernel above without norms 52).  One token of 32 + 2 x 8 heads without norms: 2.3 us, 2.4 above.
+__global__ void __launch_bounds__(512)
+qk_norm_rope_cache_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
+                          const __nv_bfloat16* __restrict__ v, __nv_bfloat16* __restrict__ k_cache,
+                          __nv_bfloat16* __restrict__ v_cache, const int* __restrict__ positions,
+                          const int* __restrict__ slot_mapping, const float* __restrict__ cos_sin,
+                          const __nv_bfloat16* __restrict__ q_w, const __nv_bfloat16* __restrict__ k_w, float eps, int Hq,
+                          int Hk, int D, int lane_bits, long long q_stride, long long k_stride, long long v_stride,
+                          int block_size) {
+  b200::pdl_trigger();
+  b200::pdl_wait();
+  const int t = blockIdx.x;
+  const int slot = slot_mapping[t];
+  const int half = D >> 1, lanes = 1 << lane_bits;
+  const float* cs = cos_sin + static_cast<long long>(positions[t]) * D;
+  const bool store = slot >= 0;     // a padded token: q only
+  const long long blk = store ? slot / block_size : 0;
+  const long long cache_row = blk * Hk * block_size + (store ? slot - blk * block_size : 0);
+  const int total = (store ? Hq + 2 * Hk : Hq) << lane_bits;
+  for (int base = 0; base < total; base += blockDim.x) {      // (whole warps stay together for the shuffles)
+    const int idx = base + threadIdx.x;
+    const bool live = idx < total;
+    const int head = idx >> lane_bits, d = 8 * (idx & (lanes - 1));
+    const bool is_q = head < Hq, is_v = head >= Hq + Hk;
+    const int h = is_q ? head : is_v ? head - Hq - Hk : head - Hq;
+    const __nv_bfloat16* src = (is_q ? q + t * q_stride : is_v ? v + t * v_stride : k + t * k_stride) +
+                               static_cast<long long>(h) * D + d;
+    __nv_bfloat16* dst = is_q ? q + t * q_stride + static_cast<long long>(h) * D + d
+                              : (is_v ? v_cache : k_cache) + (cache_row + static_cast<long long>(h) * block_size) * D + d;
+    uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
+    if (live) {
+      a = *reinterpret_cast<const uint4*>(src);
+      b = *reinterpret_cast<const uint4*>(src + half);
+    }
+    float x[8], y[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 u = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&a)[j]);
+      const float2 w = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&b)[j]);
+      x[2 * j] = u.x, x[2 * j + 1] = u.y, y[2 * j] = w.x, y[2 * j + 1] = w.y;
+    }
+    if (q_w) {
+      float ss = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += x[j] * x[j] + y[j] * y[j];
+      for (int o = lanes >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (live && !is_v) {
+        const float inv = rsqrtf(ss / static_cast<float>(D) + eps);
+        const __nv_bfloat16* w = (is_q ? q_w : k_w) + d;
+        const uint4 wa = *reinterpret_cast<const uint4*>(w), wb = *reinterpret_cast<const uint4*>(w + half);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 ga = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&wa)[j]);
+          const float2 gb = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&wb)[j]);
+          x[2 * j] *= inv * ga.x, x[2 * j + 1] *= inv * ga.y;
+          y[2 * j] *= inv * gb.x, y[2 * j + 1] *= inv * gb.y;
+        }
+      }
+    }
+    if (!live) continue;
+    if (!is_v) {
+#pragma unroll
+      for (int j = 0; j < 8; j += 4) {
+        const float4 c4 = *reinterpret_cast<const float4*>(cs + d + j), s4 = *reinterpret_cast<const float4*>(cs + half + d + j);
+        const float c[4] = {c4.x, c4.y, c4.z, c4.w}, s[4] = {s4.x, s4.y, s4.z, s4.w};
+        float u[4], w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          u[i] = x[j + i] * c[i] - y[j + i] * s[i];
+          w[i] = y[j + i] * c[i] + x[j + i] * s[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i += 2) {
+          reinterpret_cast<__nv_bfloat162*>(&a)[(j + i) >> 1] = __floats2bfloat162_rn(u[i], u[i + 1]);
+          reinterpret_cast<__nv_bfloat162*>(&b)[(j + i) >> 1] = __floats2bfloat162_rn(w[i], w[i + 1]);
+        }
+      }
+    }
+    *reinterpret_cast<uint4*>(dst) = a;
+    *reinterpret_cast<uint4*>(dst + half) = b;
+  }
+}
+
 // MLA: kv_c [T, L] (L = 512) is RMS-normalised with weight w; k_pe [T, R] (R = 64)
 // gets RoPE (gpt-j/interleaved or neox pairing); the row [norm(kv_c) | rope(k_pe)]
 // is written to cache[slot].  kv_c_out / k_pe_out (optional) receive the same
@@ -416,16 +504,33 @@ extern "C" int b200_rope_qk(void* q, void* k, const int* positions, const float*
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
+// q_w, k_w [D]: weights of a norm per head ahead of the rotation, or null (then eps is not used).  Returns 1 when there
+// are norms and the heads are not ones that the fused kernel takes (the caller norms them first).
 extern "C" int b200_rope_cache_gqa(void* q, const void* k, const void* v, void* k_cache,
                                    void* v_cache, const int* positions, const int* slot_mapping,
                                    const float* cos_sin, int T, int Hq, int Hk, int D, int rot_dim,
                                    int neox, long long q_stride, long long k_stride,
-                                   long long v_stride, int block_size, cudaStream_t stream) {
+                                   long long v_stride, int block_size, const void* q_w, const void* k_w, float eps,
+                                   cudaStream_t stream) {
   if (T <= 0) return 0;
   if ((D & 7) != 0 || (rot_dim & 1) != 0 || rot_dim > D) return -1;
   const auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   const bool vec = (rot_dim & 15) == 0 && ((q_stride | k_stride | v_stride) & 7) == 0 && al16(q) && al16(k) &&
                    al16(v) && al16(k_cache) && al16(v_cache) && al16(cos_sin);
+  // whole heads on 1 to 32 lanes
+  if (vec && neox && rot_dim == D && (D & (D - 1)) == 0 && D >= 16 && D <= 512 && al16(q_w) && al16(k_w)) {
+    int lane_bits = 0;
+    while ((16 << lane_bits) < D) ++lane_bits;
+    const int items = (Hq + 2 * Hk) << lane_bits;
+    const int threads = items >= 512 ? 512 : (items + 31) / 32 * 32;
+    b200::launch_pdl(qk_norm_rope_cache_kernel, dim3(T), dim3(threads), 0, stream, 1, static_cast<__nv_bfloat16*>(q),
+                     static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v),
+                     static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), positions, slot_mapping,
+                     cos_sin, static_cast<const __nv_bfloat16*>(q_w), static_cast<const __nv_bfloat16*>(k_w), eps, Hq, Hk, D,
+                     lane_bits, q_stride, k_stride, v_stride, block_size);
+    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  }
+  if (q_w) return 1;
   b200::launch_pdl(vec ? rope_cache_gqa_vec_kernel : rope_cache_gqa_kernel, dim3(T), dim3(256), 0, stream, 1,
                    static_cast<__nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k),
                    static_cast<const __nv_bfloat16*>(v), static_cast<__nv_bfloat16*>(k_cache),

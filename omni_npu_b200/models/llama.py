@@ -48,11 +48,8 @@ class LlamaAttention(nn.Module):
 
     def forward(self, hidden: torch.Tensor, reduce: bool = True, fuse_norm=None):
         q, k, v = self.qkv_proj(hidden)
-        if self.qk_norm:
-            t = q.shape[0]
-            q = self.q_norm(q.reshape(-1, self.head_dim)).view(t, -1)
-            k = self.k_norm(k.reshape(-1, self.head_dim)).view(t, -1)
-        o = self.attn(q, k, v, self.rotary.cos_sin_cache)
+        norm = (self.q_norm.weight, self.k_norm.weight, self.q_norm.eps) if self.qk_norm else None
+        o = self.attn(q, k, v, self.rotary.cos_sin_cache, norm=norm)
         if fuse_norm is not None:
             # o_proj + tensor-parallel reduction + residual add + the following RMSNorm
             return row_parallel_add_rms_norm(self.o_proj, o, fuse_norm[0], fuse_norm[1])

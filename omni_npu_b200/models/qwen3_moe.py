@@ -65,11 +65,8 @@ class HeadToSequenceAttention(LlamaAttention):
         if stream is None or not stream.enabled:
             return super().forward(hidden, reduce=reduce, fuse_norm=fuse_norm)
         q, k, v = self.qkv_proj(hidden)
-        if self.qk_norm:
-            t = q.shape[0]
-            q = self.q_norm(q.reshape(-1, self.head_dim)).view(t, -1)
-            k = self.k_norm(k.reshape(-1, self.head_dim)).view(t, -1)
-        o = self.attn(q, k, v, self.rotary.cos_sin_cache)
+        norm = (self.q_norm.weight, self.k_norm.weight, self.q_norm.eps) if self.qk_norm else None
+        o = self.attn(q, k, v, self.rotary.cos_sin_cache, norm=norm)
         if o.shape[0] != stream.padded:
             o = torch.cat([o, o.new_zeros(stream.padded - o.shape[0], o.shape[1])], dim=0)
         o = self.tp.comm.all_to_all(o, scatter_dim=0, gather_dim=-1)        # [T/tp, heads * d]

@@ -510,16 +510,30 @@ def rope_qk_(q: torch.Tensor, k: torch.Tensor, positions: torch.Tensor, cos_sin:
 
 def rope_cache_gqa_(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor,
                     v_cache: torch.Tensor, positions: torch.Tensor, slot_mapping: torch.Tensor,
-                    cos_sin: torch.Tensor, head_dim: int, rot_dim: int, neox: bool = True) -> None:
-    """RoPE on q (in place) and k, then k / v stored into the paged cache."""
+                    cos_sin: torch.Tensor, head_dim: int, rot_dim: int, neox: bool = True,
+                    norm: Optional[Tuple[torch.Tensor, torch.Tensor, float]] = None) -> torch.Tensor:
+    """RoPE on q (in place) and k, then k / v stored into the paged cache.  ``norm`` = (q weight, k weight, eps): an
+    RMSNorm of every head of q and k ahead of the rotation.  Returns the rotated queries: ``q``, or new rows where the
+    norm is a kernel of its own."""
+    def normed(x, w, rms):
+        return rms(x.reshape(-1, head_dim), w, norm[2]).view(x.shape[0], -1)
+
     if not q.is_cuda:
+        if norm is not None:
+            q, k = normed(q, norm[0], ref.rms_norm), normed(k, norm[1], ref.rms_norm)
         qo, ko = ref.rope_qk(q, k, positions, cos_sin, head_dim, rot_dim, neox)
         q.copy_(qo)
         ref.gqa_cache_write(ko, v, k_cache, v_cache, slot_mapping)
-        return
+        return q
+    args = (v, k_cache, v_cache, positions, slot_mapping, cos_sin, head_dim, rot_dim, neox)
+    if norm is not None:
+        if _C().rope_cache_gqa(q, k, *args, *norm):
+            _count(1)
+            return q
+        q, k = normed(q, norm[0], rms_norm), normed(k, norm[1], rms_norm)
     _count(1)
-    _C().rope_cache_gqa(q, k, v, k_cache, v_cache, positions, slot_mapping, cos_sin, head_dim,
-                        rot_dim, neox)
+    _C().rope_cache_gqa(q, k, *args, None, None, 0.0)
+    return q
 
 
 def gqa_cache_write(k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,

@@ -540,6 +540,49 @@ def test_lse_merge_and_gather_cache():
     assert torch.equal(ops.gather_cache(cache, bt, sl).cpu(), ref.gather_cache(cache.cpu(), bt.cpu(), sl))
 
 
+@pytest.mark.parametrize("t,hq,hk,d,rot,neox", [(1, 32, 4, 128, 128, True), (37, 3, 1, 16, 16, True), (300, 5, 2, 64, 64, True),
+                                                (9, 2, 2, 256, 256, True), (3, 1, 1, 512, 512, True),
+                                                (17, 4, 2, 128, 64, True), (5, 4, 2, 96, 96, True), (6, 4, 2, 128, 128, False)])
+@pytest.mark.parametrize("normed", [True, False])
+def test_rope_cache_gqa_norm(t, hq, hk, d, rot, neox, normed):
+    """Norm per head, rotation and cache rows in one pass (and heads for which they are separate kernels)."""
+    torch.manual_seed(t + d)
+    bs = 16
+    qkv = torch.randn(t, (hq + 2 * hk) * d, device=DEV, dtype=torch.bfloat16) * 3
+    q, k, v = qkv.split([hq * d, hk * d, hk * d], 1)
+    w = [(torch.rand(d, device=DEV) + 0.5).bfloat16() for _ in range(2)]
+    eps = 1e-3
+    pos = torch.randint(0, 1000, (t,), device=DEV, dtype=torch.int32)
+    slots = torch.randperm(20 * bs)[:t].to(torch.int32)
+    if t > 3:
+        slots[3] = -1
+    cs = ref.build_cos_sin_cache(rot, 1024, 10000.0).to(DEV)
+
+    def exact(x, g):
+        x = x.double().view(t, -1, d)
+        if normed:
+            x = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps) * g.double()
+        c, s = cs.double()[pos.long()][:, None].chunk(2, -1)
+        r = x[..., :rot]
+        a, b = r.chunk(2, -1) if neox else (r[..., 0::2], r[..., 1::2])
+        u, y = a * c - b * s, b * c + a * s
+        r = torch.cat([u, y], -1) if neox else torch.stack([u, y], -1).flatten(-2)
+        return torch.cat([r, x[..., rot:]], -1)
+
+    want_q, want_k, want_v = exact(q, w[0]), exact(k, w[1]), v.reshape(t, hk, d).clone()
+    kc = torch.zeros(20, hk, bs, d, device=DEV, dtype=torch.bfloat16)
+    vc = torch.zeros_like(kc)
+    got = ops.rope_cache_gqa_(q, k, v, kc, vc, pos, slots.to(DEV), cs, d, rot, neox, (*w, eps) if normed else None)
+    # one rounding to bf16, of values up to some 12 times the weight; a second one where the norm is a kernel of its own
+    _close(got.view(t, hq, d), want_q.float(), 2e-2, 2 ** -8)
+    for i, s in enumerate(slots.tolist()):
+        if s >= 0:
+            _close(kc[s // bs, :, s % bs], want_k[i].float(), 2e-2, 2 ** -8)
+            assert torch.equal(vc[s // bs, :, s % bs], want_v[i])
+    written = (slots >= 0).sum().item()
+    assert int((vc != 0).any(-1).any(1).sum()) == written
+
+
 def test_rope_cache_gqa_and_cache_write():
     t, hq, hk, d, bs = 29, 8, 2, 128, 16
     qkv = torch.randn(t, (hq + 2 * hk) * d, device=DEV, dtype=torch.bfloat16)
