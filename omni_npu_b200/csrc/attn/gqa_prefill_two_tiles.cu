@@ -161,11 +161,6 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
   }
-  {
-    // value rows of a partly filled tile that no copy writes must hold finite values (their P is zero)
-    uint4* z = reinterpret_cast<uint4*>(smem + C::OFF_V);
-    for (int i = tid; i < VS * V_BYTES / 16; i += THREADS) z[i] = make_uint4(0u, 0u, 0u, 0u);
-  }
   if (warp == 9) {
     tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
@@ -228,6 +223,20 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
         if (v_loads >= VS) ok = !*abort_flag && mbar_wait(&v_empty[vs], ((v_loads / VS) - 1) & 1);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
+        // the product reads whole groups of 16 keys, and rows past the sequence would count if they were infinite or NaN
+        // (P is zero there): what no copy fills, with pages of 8 keys, is cleared; rows of other sequences never take part
+        {
+          const int filled = nboxes * box_rows, missing = ((min(BN, it.kv_len - n0) + 15) & ~15) - filled;
+          if (missing > 0) {
+            for (int i = lane; i < missing * 16; i += 32) {
+              const int sl = i / (missing * 8), at = i % (missing * 8);
+              *reinterpret_cast<uint4*>(smem + C::OFF_V + vs * V_BYTES + sl * SLAB + filled * 128 + at * 16) =
+                  make_uint4(0u, 0u, 0u, 0u);
+            }
+            fence_proxy_async();
+            __syncwarp();
+          }
+        }
         if (lane == 0) mbar_arrive_expect_tx(&v_full[vs], static_cast<uint32_t>(nboxes * box_rows * 128) * 2);
         __syncwarp();
         for (int l = lane; l < nboxes * 2; l += 32) {
@@ -283,8 +292,9 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
             ++pc[i];
             tc_fence_after_sync();
             const uint64_t vd = desc_mnmajor(v_base + (vc % VS) * V_BYTES, SLAB);
+            const int groups = (min(BN, it.kv_len - j * BN) + 15) / 16;
 #pragma unroll 2
-            for (int kk = 0; kk < BN / 16; ++kk)       // 16 keys: 8 columns of P, 16 rows of 128 bytes of V
+            for (int kk = 0; kk < groups; ++kk)        // 16 keys: 8 columns of P, 16 rows of 128 bytes of V
               umma_f16_ta(tmem_base + COL_O + i * 128, tmem_base + COL_S + i * 128 + kk * 8, vd + kk * 128, idesc_o,
                           (j > 0 || kk > 0) ? 1u : 0u);
             // in order behind the product that reads P: the next S may take its place

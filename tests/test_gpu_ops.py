@@ -540,6 +540,35 @@ def test_lse_merge_and_gather_cache():
     assert torch.equal(ops.gather_cache(cache, bt, sl).cpu(), ref.gather_cache(cache.cpu(), bt.cpu(), sl))
 
 
+@pytest.mark.parametrize("bs", [8, 16, 64])
+@pytest.mark.parametrize("dqk", [128, 192])
+def test_prefill_keeps_other_sequences_nans_out(bs, dqk):
+    """Rows of a key tile past the end of a sequence take no part, whatever other sequences left in shared memory."""
+    torch.manual_seed(bs)
+    hq = hk = 8
+    lens = [700] * 20 + [3, 17, 133, 250, 129, 8]            # more items than SMs: later ones follow the first
+    bad = 20                                                 # sequences whose values are NaN and infinite
+    nb = [-(-n // bs) for n in lens]
+    kc = torch.randn(sum(nb), hk, bs, dqk, device=DEV, dtype=torch.bfloat16)
+    vc = torch.randn(sum(nb), hk, bs, 128, device=DEV, dtype=torch.bfloat16)
+    vc[: sum(nb[:bad])] = float("nan")
+    vc[: nb[0]] = float("inf")
+    bt = torch.zeros(len(lens), max(nb), dtype=torch.int32)
+    at = 0
+    for i, n in enumerate(nb):
+        bt[i, :n] = torch.arange(at, at + n)
+        at += n
+    cu = torch.tensor([0] + lens).cumsum(0).int()
+    q = torch.randn(sum(lens), hq * dqk, device=DEV, dtype=torch.bfloat16)
+    out = ops.gqa_prefill(q, kc, vc, bt.to(DEV), cu.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV), len(lens),
+                          max(lens), hq, dqk ** -0.5)
+    assert not torch.isfinite(out[: cu[bad]].float()).any()
+    tail = slice(int(cu[bad]), None)
+    want = ref.paged_attention(q[tail].cpu(), kc.cpu(), vc.cpu(), bt[bad:], cu[bad:] - cu[bad],
+                               torch.tensor(lens[bad:], dtype=torch.int32), hq, dqk ** -0.5, True, 0, False, 0)
+    _close(out[tail], want, 2e-2, 2e-2)
+
+
 @pytest.mark.parametrize("t,hq,hk,d,rot,neox", [(1, 32, 4, 128, 128, True), (37, 3, 1, 16, 16, True), (300, 5, 2, 64, 64, True),
                                                 (9, 2, 2, 256, 256, True), (3, 1, 1, 512, 512, True),
                                                 (17, 4, 2, 128, 64, True), (5, 4, 2, 96, 96, True), (6, 4, 2, 128, 128, False)])
