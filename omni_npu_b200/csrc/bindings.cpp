@@ -263,9 +263,10 @@ Tensor gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tensor& w, c
 // Grouped block-scaled e4m3 GEMM (MoE experts): a [rows, K] e4m3 + a_scale [rows, K/128]; w [E, N, K] e4m3 +
 // w_scale [E, R, K/128]; expert e owns rows expert_offsets[e] .. [e + 1].  swiglu: gate / up rows of w are
 // interleaved in groups of 8, their scale rows are gate blocks then up blocks (from row up_scale_row0).
-Tensor grouped_gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tensor& w, const Tensor& w_scale,
-                              const Tensor& expert_offsets, bool swiglu, int64_t up_scale_row0, const Tensor& status,
-                              int64_t max_ctas) {
+// The result goes into c [rows, N, or N / 2 with swiglu] (rows may lie further apart).
+void grouped_gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tensor& w, const Tensor& w_scale,
+                            const Tensor& expert_offsets, Tensor c, bool swiglu, int64_t up_scale_row0,
+                            const Tensor& status, int64_t max_ctas) {
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 3, "grouped_gemm_fp8_block: shapes");
   TORCH_CHECK(a.scalar_type() == at::kFloat8_e4m3fn && w.scalar_type() == at::kFloat8_e4m3fn,
               "grouped_gemm_fp8_block: float8_e4m3fn operands");
@@ -283,13 +284,14 @@ Tensor grouped_gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tens
               "grouped_gemm_fp8_block: scale rows do not cover the weight rows");
   c10::cuda::CUDAGuard guard(a.device());
   const int64_t n_out = swiglu ? N / 2 : N;
-  Tensor c = torch::empty({rows, n_out}, a.options().dtype(at::kBFloat16));
+  TORCH_CHECK(c.is_cuda() && c.scalar_type() == at::kBFloat16 && c.dim() == 2 && c.size(0) == rows && c.size(1) == n_out &&
+                  c.stride(1) == 1 && c.stride(0) >= n_out && c.device() == a.device(),
+              "grouped_gemm_fp8_block: result bf16 [rows, N]");
   check(b200_grouped_gemm_fp8_block(a.data_ptr(), a_scale.data_ptr<float>(), w.data_ptr(), w_scale.data_ptr<float>(),
                                     c.data_ptr(), expert_offsets.data_ptr<int>(), (int)E, (int)rows, (int)N, (int)K,
-                                    (int)a.stride(0), (int)n_out, (int)R, swiglu ? 1 : 0, (int)up_scale_row0,
+                                    (int)a.stride(0), (int)c.stride(0), (int)R, swiglu ? 1 : 0, (int)up_scale_row0,
                                     status.data_ptr<int>(), (int)max_ctas, cur_stream()),
         "grouped_gemm_fp8_block");
-  return c;
 }
 
 // Sparse-attention indexer: scores on the tensor cores + radix select of the topk best key

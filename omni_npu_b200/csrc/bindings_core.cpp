@@ -252,8 +252,9 @@ Tensor gemm_stream(const Tensor& a, const Tensor& w, const c10::optional<Tensor>
 }
 
 // tn: rows per tile of the weight-streaming kernel (gemm/gemm_stream.cu), 0: the kernel on CTA pairs (gemm/gemm_pair.cu).
-Tensor grouped_gemm_rows(const Tensor& a, const Tensor& w, const Tensor& expert_offsets, int64_t act, int64_t tn,
-                         const Tensor& status, int64_t max_ctas, double act_alpha, double act_limit) {
+// The result goes into c [rows, N, or N / 2 with a gated activation] (rows may lie further apart).
+void grouped_gemm_rows(const Tensor& a, const Tensor& w, const Tensor& expert_offsets, Tensor c, int64_t act, int64_t tn,
+                       const Tensor& status, int64_t max_ctas, double act_alpha, double act_limit) {
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 3, "grouped_gemm: shapes");
   TORCH_CHECK(a.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16, "grouped_gemm: bf16 inputs");
   TORCH_CHECK(a.stride(1) == 1 && w.is_contiguous(), "grouped_gemm: contiguity");
@@ -262,19 +263,21 @@ Tensor grouped_gemm_rows(const Tensor& a, const Tensor& w, const Tensor& expert_
   TORCH_CHECK(a.size(1) == K && expert_offsets.numel() == E + 1, "grouped_gemm: size mismatch");
   c10::cuda::CUDAGuard guard(a.device());
   const int n_out = gated(act) ? N / 2 : N;
-  Tensor c = torch::empty({rows, n_out}, a.options());
+  TORCH_CHECK(c.is_cuda() && c.scalar_type() == at::kBFloat16 && c.dim() == 2 && c.size(0) == rows && c.size(1) == n_out &&
+                  c.stride(1) == 1 && c.stride(0) >= n_out && c.device() == a.device(),
+              "grouped_gemm: result bf16 [rows, N]");
+  const int ldc = (int)c.stride(0);
   const int* offsets = expert_offsets.data_ptr<int>();
   if (tn > 0)
     check(b200_grouped_gemm_stream(a.data_ptr(), w.data_ptr(), c.data_ptr(), offsets, E, rows, N, K, (int)a.stride(0),
-                                   n_out, (int)act, (int)tn, status.data_ptr<int>(), (int)max_ctas, (float)act_alpha,
+                                   ldc, (int)act, (int)tn, status.data_ptr<int>(), (int)max_ctas, (float)act_alpha,
                                    (float)act_limit, cur_stream()),
           "grouped_gemm_stream");
   else
-    check(b200_grouped_gemm_pair(a.data_ptr(), w.data_ptr(), c.data_ptr(), offsets, E, rows, N, K, (int)a.stride(0), n_out,
+    check(b200_grouped_gemm_pair(a.data_ptr(), w.data_ptr(), c.data_ptr(), offsets, E, rows, N, K, (int)a.stride(0), ldc,
                                  (int)act, status.data_ptr<int>(), (int)max_ctas, (float)act_alpha, (float)act_limit,
                                  cur_stream()),
           "grouped_gemm_pair");
-  return c;
 }
 
 Tensor grouped_gemm(const Tensor& a, const Tensor& w, const Tensor& expert_offsets, int64_t act,

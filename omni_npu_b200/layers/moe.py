@@ -228,9 +228,9 @@ class FusedMoE(nn.Module):
         return moved
 
     # ----------------------------------------------------------------- forward
-    def _expert_rows(self, rows: torch.Tensor, offsets: torch.Tensor) -> torch.Tensor:
+    def _expert_rows(self, rows: torch.Tensor, offsets: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         h = ops.grouped_gemm(rows, self.w13, offsets, swiglu=self.unary is None, act=self.act, unary=self.unary)
-        return ops.grouped_gemm(h, self.w2, offsets)
+        return ops.grouped_gemm(h, self.w2, offsets, out=out)
 
     def forward(self, hidden: torch.Tensor) -> torch.Tensor:
         """hidden [T,H] (replicated across TP ranks) -> [T,H]."""
@@ -303,6 +303,9 @@ class FusedMoE(nn.Module):
             fp8_rows = self.quant == "fp8" and self.buffers.fp8_dispatch
             rows, offsets, handle = ep_dispatch(comm, x, ids_local, w, self.num_physical, self.buffers,
                                                 fp8=fp8_rows)
+            # the second product writes where the combine reads: the peers' rows of this step have arrived, so their
+            # combines of the step before are over
+            y = self.buffers.expert_y[: handle.rows]
             if self.quant == "fp8":
                 # block-scaled e4m3 experts: the rows arrive quantised per token per 128 columns (the
                 # scatter kernel quantises them on the way; without fp8 buffers they are quantised
@@ -311,10 +314,9 @@ class FusedMoE(nn.Module):
                 h1 = ops.grouped_gemm_fp8_block(rq, rs, self.w13, self.w13_scale, offsets, swiglu=True,
                                                 up_scale_row0=(self.intermediate_size + 127) // 128)
                 hq, hs = ops.quant_fp8_1x128(h1)
-                y = ops.grouped_gemm_fp8_block(hq, hs, self.w2, self.w2_scale, offsets)
+                ops.grouped_gemm_fp8_block(hq, hs, self.w2, self.w2_scale, offsets, out=y)
             else:
-                y = self._expert_rows(rows, offsets)
-            self.buffers.expert_y[: y.shape[0]].copy_(y)
+                self._expert_rows(rows, offsets, out=y)
             if shared_out is not None:
                 torch.cuda.current_stream(x.device).wait_stream(self._side_stream)
             return ep_combine(comm, self.buffers.expert_y, handle, shared_out, self.buffers)

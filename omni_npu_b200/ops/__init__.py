@@ -321,17 +321,21 @@ def gemm_fp8_block(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.Tensor, 
 
 def grouped_gemm_fp8_block(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor,
                            expert_offsets: torch.Tensor, swiglu: bool = False, up_scale_row0: int = 0,
-                           max_ctas: int = 0) -> torch.Tensor:
+                           max_ctas: int = 0, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Per-expert block-scaled e4m3 GEMM: rows ``expert_offsets[e]:expert_offsets[e+1]`` of ``a_q`` times
     ``w_q[e].T`` with ``w_scale[e]`` (one scale per 128 x 128 block).  ``swiglu``: gate / up rows of
     ``w_q`` are interleaved in groups of 8 and the result is ``silu(gate) * up``; the scale rows are the
-    gate blocks followed, from row ``up_scale_row0``, by the up blocks."""
+    gate blocks followed, from row ``up_scale_row0``, by the up blocks.  ``out``: where the result goes."""
     if not a_q.is_cuda:
-        return ref.grouped_gemm_fp8_block(a_q, a_scale, w_q, w_scale, expert_offsets, swiglu, up_scale_row0)
+        y = ref.grouped_gemm_fp8_block(a_q, a_scale, w_q, w_scale, expert_offsets, swiglu, up_scale_row0)
+        return y if out is None else out.copy_(y)
     st = device_state(a_q.device)
+    if out is None:
+        out = torch.empty(a_q.shape[0], w_q.shape[1] // (2 if swiglu else 1), dtype=torch.bfloat16, device=a_q.device)
     _count(1)
-    return _C().grouped_gemm_fp8_block(a_q, a_scale.contiguous(), w_q, w_scale.contiguous(), expert_offsets, swiglu,
-                                       up_scale_row0, st.status, max_ctas)
+    _C().grouped_gemm_fp8_block(a_q, a_scale.contiguous(), w_q, w_scale.contiguous(), expert_offsets, out, swiglu,
+                                up_scale_row0, st.status, max_ctas)
+    return out
 
 
 def dsa_indexer_topk(q: torch.Tensor, w: torch.Tensor, index_cache: torch.Tensor, block_tables: torch.Tensor,
@@ -434,24 +438,30 @@ def grouped_rows_tile(rows: int, groups: int, n: int, sms: int = 148) -> int:
 
 def grouped_gemm(a: torch.Tensor, w: torch.Tensor, expert_offsets: torch.Tensor,
                  swiglu: bool = False, bn: int = 0, max_ctas: int = 0,
-                 act=SILU, unary: Optional[str] = None) -> torch.Tensor:
+                 act=SILU, unary: Optional[str] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Per-expert GEMM: rows expert_offsets[e]:expert_offsets[e+1] of ``a`` times ``w[e].T``
-    (``swiglu`` / ``act`` / ``unary`` as in :func:`gemm`)."""
-    if not a.is_cuda:
-        return ref.grouped_gemm(a, w, expert_offsets, swiglu, act, unary)
+    (``swiglu`` / ``act`` / ``unary`` as in :func:`gemm`).  ``out``: where the result goes."""
     kind = _act_kind(swiglu, act, None, unary)
-    if a.dtype == torch.float32:
+    if a.is_cuda and a.dtype == torch.bfloat16 and bn <= 0:
+        rows, groups, n = a.shape[0], w.shape[0], w.shape[1]
+        if out is None:
+            out = a.new_empty(rows, n // 2 if kind[0] in (1, 2, 4, 7) else n)
         _count(1)
-        return _core().gemm_simt(a, w, expert_offsets, *kind, None)
-    st = device_state(a.device)
-    _count(1)
-    rows, groups, n, k = a.shape[0], *w.shape
-    if bn <= 0 and a.dtype == torch.bfloat16:
-        return _core().grouped_gemm_rows(a, w, expert_offsets, kind[0], grouped_rows_tile(rows, groups, n), st.status,
-                                         max_ctas, kind[1], kind[2])
-    if bn <= 0:
-        bn = grouped_tile(rows, groups, n, k)
-    return _core().grouped_gemm(a, w, expert_offsets, kind[0], bn, st.status, max_ctas, kind[1], kind[2])
+        _core().grouped_gemm_rows(a, w, expert_offsets, out, kind[0], grouped_rows_tile(rows, groups, n),
+                                  device_state(a.device).status, max_ctas, kind[1], kind[2])
+        return out
+    if not a.is_cuda:
+        y = ref.grouped_gemm(a, w, expert_offsets, swiglu, act, unary)
+    elif a.dtype == torch.float32:
+        _count(1)
+        y = _core().gemm_simt(a, w, expert_offsets, *kind, None)
+    else:
+        if bn <= 0:
+            bn = grouped_tile(a.shape[0], *w.shape)
+        _count(1)
+        y = _core().grouped_gemm(a, w, expert_offsets, kind[0], bn, device_state(a.device).status, max_ctas, kind[1],
+                                 kind[2])
+    return y if out is None else out.copy_(y)
 
 
 # ------------------------------------------------------------- norm/activation
