@@ -211,6 +211,13 @@ class MLAAttention(nn.Module):
             lat = lat.reshape(total_blocks, gbs, lat.shape[-1])
         l = self.kv_lora_rank
         kv = self.kv_b_proj(lat[..., :l].reshape(total_blocks * gbs, l).contiguous())
+        if (q.is_cuda and q.dtype == kv.dtype == torch.bfloat16 and (self.nope, self.rope_dim, self.v_dim) == (128, 64, 128)
+                and ops.PREFILL_TCGEN05):
+            # the kernel reads keys, values and rotated parts where they are
+            first = torch.tensor(starts, dtype=torch.int32).mul_(gbs).to(dev, non_blocking=True)
+            qf = torch.cat([q[:, :, : self.nope], q_pe], dim=-1)
+            return ops.mla_prefill(qf, kv.view(total_blocks * gbs, n, 256), lat[..., l:].view(total_blocks * gbs, -1), first,
+                                   md.cu_q, md.seq_lens, md.num_seqs, md.max_q_len, self.scale)
         kv = kv.view(total_blocks, gbs, n, self.nope + self.v_dim)
         k_pe = lat[..., l:].unsqueeze(2).expand(total_blocks, gbs, n, self.rope_dim)
         k_paged = torch.cat([kv[..., : self.nope], k_pe], dim=-1).permute(0, 2, 1, 3).contiguous()

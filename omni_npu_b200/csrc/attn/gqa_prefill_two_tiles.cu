@@ -20,6 +20,11 @@
 // copies of the next item run under the end of this one.  Warps 0-3 and 4-7: softmax of tile 0 and 1; warp 8: TMA;
 // warp 9: MMA issue; warps 10 and 11 only complete the warpgroup that gives registers away.
 //
+// FLAT (latent attention, 128 + 64 rotated): keys and values are rows of the up-projection [rows, heads x (128 key, 128
+// value)] and the rotated part, shared by the heads, rows of the latents; a sequence's rows lie one after another, so that
+// a tile is one copy per 64 columns, and nothing is repacked into per-head pages (4 x 2048 tokens of 16 heads: the copies
+// that did took 250 us a layer, the attention 151, and 119 in this form).
+//
 // Every wait is bounded; on expiry the CTA records a status code, stops issuing, waits for what is in flight, frees its
 // TMEM and returns (its output rows are then not valid).
 //
@@ -111,11 +116,13 @@ __device__ __forceinline__ TwoTileItem two_tile_item(int idx, const TwoTileGrid&
   return it;
 }
 
-template <int DQK>
+// FLAT: tm_k covers the up-projected rows, tm_v the rotated parts; block_tables[b] is sequence b's first row.
+template <int DQK, bool FLAT>
 __global__ void __launch_bounds__(two::THREADS, 1)
 gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                              const __grid_constant__ CUtensorMap tm_v, const AttnParams p, const int box_rows,
                              const TwoTileGrid g) {
+  static_assert(!FLAT || DQK == 192, "latent attention");
   using namespace two;
   using C = Cfg<DQK>;
   constexpr int KS = C::KS, VS = C::VS;
@@ -189,9 +196,10 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
       const TwoTileItem it = two_tile_item(idx, g, p);
       if (it.n_max == 0) continue;
       const int* bt = p.block_tables + static_cast<long long>(it.b) * p.max_blocks;
+      const int first = FLAT ? bt[0] : 0;
       for (int j = 0; j < it.n_max; ++j) {
         const int n0 = j * BN;
-        const int nboxes = (min(BN, it.kv_len - n0) + box_rows - 1) / box_rows;
+        const int nboxes = FLAT ? 1 : (min(BN, it.kv_len - n0) + box_rows - 1) / box_rows;
         // keys (before the first tile's: the queries)
         if (j == 0) {
           if (q_loads > 0) ok = !*abort_flag && mbar_wait(q_empty, (q_loads - 1) & 1);
@@ -214,6 +222,15 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
         if (lane == 0) mbar_arrive_expect_tx(&k_full[ks], static_cast<uint32_t>(nboxes * box_rows * 128) * C::QK_SLABS);
         __syncwarp();
         for (int l = lane; l < nboxes * C::QK_SLABS; l += 32) {
+          if constexpr (FLAT) {
+            // (rows past the sequence are masked, rows past the end read as zero)
+            uint8_t* dst = smem + C::OFF_K + ks * C::K_BYTES + l * SLAB;
+            if (l < 2)
+              tma_load_2d(dst, &tm_k, &k_full[ks], it.h[0] * 256 + l * 64, first + n0);
+            else
+              tma_load_2d(dst, &tm_v, &k_full[ks], 0, first + n0);
+            continue;
+          }
           const int i = l / C::QK_SLABS, sl = l % C::QK_SLABS, key = n0 + i * box_rows;
           const int row = (bt[key / p.block_size] * p.Hk + it.kvh) * p.block_size + key % p.block_size;
           tma_load_2d(smem + C::OFF_K + ks * C::K_BYTES + sl * SLAB + i * box_rows * 128, &tm_k, &k_full[ks], sl * 64,
@@ -240,6 +257,11 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
         if (lane == 0) mbar_arrive_expect_tx(&v_full[vs], static_cast<uint32_t>(nboxes * box_rows * 128) * 2);
         __syncwarp();
         for (int l = lane; l < nboxes * 2; l += 32) {
+          if constexpr (FLAT) {
+            tma_load_2d(smem + C::OFF_V + vs * V_BYTES + l * SLAB, &tm_k, &v_full[vs], it.h[0] * 256 + 128 + l * 64,
+                        first + n0);
+            continue;
+          }
           const int i = l >> 1, sl = l & 1, key = n0 + i * box_rows;
           const int row = (bt[key / p.block_size] * p.Hk + it.kvh) * p.block_size + key % p.block_size;
           tma_load_2d(smem + C::OFF_V + vs * V_BYTES + sl * SLAB + i * box_rows * 128, &tm_v, &v_full[vs], sl * 64, row);
@@ -455,10 +477,10 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
   }
 }
 
-template <int DQK>
+template <int DQK, bool FLAT>
 static int launch_two_tiles(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p,
                             int box_rows, const TwoTileGrid& g, cudaStream_t stream) {
-  auto kern = gqa_prefill_two_tiles_kernel<DQK>;
+  auto kern = gqa_prefill_two_tiles_kernel<DQK, FLAT>;
   static_assert(two::Cfg<DQK>::SMEM <= 227 * 1024, "shared memory of an SM");
   static DeviceOnce once;
   int dev = 0;
@@ -536,6 +558,51 @@ extern "C" int b200_gqa_prefill_tc(const void* q, const void* k_cache, const voi
   const long long items = static_cast<long long>(g.m_units) * g.head_units * B;
   if (items > 0x7fffffffll) return 1;
   g.items = static_cast<int>(items);
-  return Dqk == 128 ? launch_two_tiles<128>(tq, tk, tv, p, box_rows, g, stream)
-                    : launch_two_tiles<192>(tq, tk, tv, p, box_rows, g, stream);
+  return Dqk == 128 ? launch_two_tiles<128, false>(tq, tk, tv, p, box_rows, g, stream)
+                    : launch_two_tiles<192, false>(tq, tk, tv, p, box_rows, g, stream);
+}
+
+// Non-absorbed latent attention over up-projected keys and values in place: q [T, H, 192] (pitch q_stride), kv [rows,
+// H, 256] (pitch kv_stride; 128 of the key, 128 of the value), pe [rows, 64] (pitch pe_stride); sequence b has seq_lens[b]
+// keys from row kv_start[b] on.  out [T, H, 128], causal.
+extern "C" int b200_mla_prefill(const void* q, const void* kv, const void* pe, void* out, const int* kv_start,
+                                const int* cu_q, const int* seq_lens, int B, int max_q_len, int H, long long rows,
+                                long long total_q_rows, long long q_stride, long long kv_stride, long long pe_stride,
+                                long long out_stride, float scale, int* status, cudaStream_t stream) {
+  if (B <= 0 || max_q_len <= 0 || total_q_rows <= 0 || rows <= 0) return 0;
+  if (H <= 0 || !(scale > 0.f) || rows > 0x7fffffffll || (out_stride & 7) != 0 ||
+      (reinterpret_cast<uintptr_t>(out) & 15) != 0)
+    return -1;
+  AttnParams p{};
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.block_tables = kv_start;
+  p.cu_q = cu_q;
+  p.seq_lens = seq_lens;
+  p.max_blocks = 1;
+  p.Hq = p.Hk = H;
+  p.out_stride = out_stride;
+  p.scale_log2 = scale * kLog2e;
+  p.causal = 1;
+  p.status = status;
+  CUtensorMap tq, tk, tp;
+  int r = make_tensormap_2d(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, q, static_cast<uint64_t>(total_q_rows),
+                            static_cast<uint64_t>(H) * 192, static_cast<uint64_t>(q_stride), two::BM, 64,
+                            CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r) return r - 1000;
+  r = make_tensormap_2d(&tk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, kv, static_cast<uint64_t>(rows),
+                        static_cast<uint64_t>(H) * 256, static_cast<uint64_t>(kv_stride), two::BN, 64,
+                        CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r) return r - 2000;
+  r = make_tensormap_2d(&tp, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, pe, static_cast<uint64_t>(rows), 64,
+                        static_cast<uint64_t>(pe_stride), two::BN, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r) return r - 3000;
+  TwoTileGrid g;
+  g.by_head = 0;
+  g.m_units = (max_q_len + 2 * two::BM - 1) / (2 * two::BM);
+  g.head_units = H;
+  g.B = B;
+  const long long items = static_cast<long long>(g.m_units) * H * B;
+  if (items > 0x7fffffffll) return -2;
+  g.items = static_cast<int>(items);
+  return launch_two_tiles<192, true>(tq, tk, tp, p, two::BN, g, stream);
 }

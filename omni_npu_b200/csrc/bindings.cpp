@@ -83,6 +83,10 @@ int b200_gqa_prefill_tc(const void* q, const void* k_cache, const void* v_cache,
                         int max_blocks, int block_size, int Hq, int Hk, int Dqk, int Dv, long long q_stride,
                         long long out_stride, float scale, int causal, int window, long long total_q_rows,
                         int num_cache_blocks, int* status, cudaStream_t stream);
+int b200_mla_prefill(const void* q, const void* kv, const void* pe, void* out, const int* kv_start, const int* cu_q,
+                     const int* seq_lens, int B, int max_q_len, int H, long long rows, long long total_q_rows,
+                     long long q_stride, long long kv_stride, long long pe_stride, long long out_stride, float scale,
+                     int* status, cudaStream_t stream);
 int b200_gqa_decode_ex(const void* q, const void* k_cache, const void* v_cache, void* out, float* lse,
                        const int* block_tables, const int* seq_lens, int B, int q_len, int max_blocks,
                        int block_size, int Hq, int Hk, int D, long long q_stride, long long out_stride,
@@ -559,6 +563,33 @@ std::tuple<Tensor, Tensor> gqa_prefill(const Tensor& q, const Tensor& k_cache, c
   return {out, lse};
 }
 
+// Latent attention of a prompt step: q [T, H, 192], kv [rows, H, 256] (key | value), pe [rows, 64]; sequence b's keys are
+// the rows kv_start[b] .. kv_start[b] + seq_lens[b].
+Tensor mla_prefill(const Tensor& q, const Tensor& kv, const Tensor& pe, const Tensor& kv_start, const Tensor& cu_q,
+                   const Tensor& seq_lens, int64_t num_seqs, int64_t max_q_len, double scale, const Tensor& status) {
+  CHECK_CUDA_BF16(q);
+  CHECK_CUDA_BF16(kv);
+  CHECK_CUDA_BF16(pe);
+  CHECK_I32(kv_start);
+  CHECK_I32(cu_q);
+  CHECK_I32(seq_lens);
+  TORCH_CHECK(q.dim() == 3 && q.size(2) == 192 && q.stride(2) == 1 && q.stride(1) == 192, "mla_prefill: q [T, H, 192]");
+  const int64_t T = q.size(0), H = q.size(1), rows = kv.size(0);
+  TORCH_CHECK(kv.dim() == 3 && kv.size(1) == H && kv.size(2) == 256 && kv.stride(2) == 1 && kv.stride(1) == 256,
+              "mla_prefill: kv [rows, H, 256]");
+  TORCH_CHECK(pe.dim() == 2 && pe.size(0) == rows && pe.size(1) == 64 && pe.stride(1) == 1, "mla_prefill: pe [rows, 64]");
+  TORCH_CHECK(kv_start.numel() >= num_seqs && cu_q.numel() > num_seqs && seq_lens.numel() >= num_seqs,
+              "mla_prefill: sequences");
+  c10::cuda::CUDAGuard guard(q.device());
+  Tensor out = torch::empty({T, H * 128}, q.options());
+  check(b200_mla_prefill(q.data_ptr(), kv.data_ptr(), pe.data_ptr(), out.data_ptr(), kv_start.data_ptr<int>(),
+                         cu_q.data_ptr<int>(), seq_lens.data_ptr<int>(), (int)num_seqs, (int)max_q_len, (int)H, rows, T,
+                         q.stride(0), kv.stride(0), pe.stride(0), H * 128, (float)scale, status.data_ptr<int>(),
+                         cur_stream()),
+        "mla_prefill");
+  return out;
+}
+
 int64_t gqa_decode_scratch_bytes(int64_t B, int64_t Hk, int64_t D, int64_t splits) {
   return (int64_t)b200_gqa_decode_scratch_bytes((int)B, (int)Hk, (int)D, (int)splits);
 }
@@ -689,6 +720,7 @@ TORCH_LIBRARY_FRAGMENT(omni_b200, m) {
   m.def("quant_fp8_1x128", &quant_fp8_1x128);
   m.def("rope_qk", &rope_qk);
   m.def("rope_cache_gqa", &rope_cache_gqa);
+  m.def("mla_prefill", &mla_prefill);
   m.def("mla_kv_rmsnorm_rope_cache", &mla_kv_rmsnorm_rope_cache);
   m.def("paged_scatter_rows", &paged_scatter_rows);
   m.def("gqa_cache_write", &gqa_cache_write);

@@ -540,6 +540,31 @@ def test_lse_merge_and_gather_cache():
     assert torch.equal(ops.gather_cache(cache, bt, sl).cpu(), ref.gather_cache(cache.cpu(), bt.cpu(), sl))
 
 
+@pytest.mark.parametrize("new,cached", [([1], [0]), ([300, 1, 128, 17], [0, 700, 3, 129]), ([257, 5], [0, 0])])
+def test_mla_prefill(new, cached):
+    """Latent attention over up-projected rows where they lie, sequences at starts of their own."""
+    torch.manual_seed(len(new))
+    h, lens = 3, [a + b for a, b in zip(new, cached)]
+    starts = [0]
+    for n in lens:
+        starts.append(starts[-1] + -(-n // 16) * 16)
+    kv = torch.randn(starts[-1], h, 256, device=DEV, dtype=torch.bfloat16)
+    lat = torch.randn(starts[-1], 576, device=DEV, dtype=torch.bfloat16)
+    q = torch.randn(sum(new), h, 192, device=DEV, dtype=torch.bfloat16)
+    cu = torch.tensor([0] + new).cumsum(0)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    out = ops.mla_prefill(q, kv, lat[:, 512:], torch.tensor(starts[:-1], **i32), cu.to(**i32), torch.tensor(lens, **i32), len(new),
+                          max(new), 192 ** -0.5)
+    for i, n in enumerate(lens):
+        rows = slice(starts[i], starts[i] + n)
+        k = torch.cat([kv[rows, :, :128], lat[rows, None, 512:].expand(-1, h, -1)], -1).double()
+        s = torch.einsum("qhd,khd->hqk", q[cu[i]: cu[i + 1]].double(), k) * 192 ** -0.5
+        hidden = torch.arange(n, device=DEV)[None] > cached[i] + torch.arange(new[i], device=DEV)[:, None]
+        want = torch.einsum("hqk,khd->qhd", s.masked_fill(hidden, -math.inf).softmax(-1), kv[rows, :, 128:].double())
+        # P is rounded to bf16 (2 ** -9 of values up to 4 or so), and so is the result
+        _close(out[cu[i]: cu[i + 1]], want.flatten(1).float(), 2e-2, 2 ** -7)
+
+
 @pytest.mark.parametrize("bs", [8, 16, 64])
 @pytest.mark.parametrize("dqk", [128, 192])
 def test_prefill_keeps_other_sequences_nans_out(bs, dqk):
