@@ -152,16 +152,14 @@ class MLAAttention(nn.Module):
             ops.mla_kv_rmsnorm_rope_cache(kv_all[:, : self.kv_lora_rank], kv_all[:, self.kv_lora_rank:],
                                           self.kv_a_layernorm.weight, cache, pc["positions_all"], pc["slot_all"],
                                           self.rotary.cos_sin_cache, self.kv_a_layernorm.eps, False)
+            q_pe = q[:, :, self.nope:].reshape(t, n * self.rope_dim).contiguous()
+            ops.rope_qk_(q_pe, q_pe.new_empty(t, 0), md.positions, self.rotary.cos_sin_cache, self.rope_dim, self.rope_dim,
+                         False)
+            q_pe = q_pe.view(t, n, self.rope_dim)
         else:
-            # fused: RMSNorm(c_kv), RoPE(k_pe), write [c_kv | k_pe] into the paged cache
-            ops.mla_kv_rmsnorm_rope_cache(kv_a[:, : self.kv_lora_rank], kv_a[:, self.kv_lora_rank:],
-                                          self.kv_a_layernorm.weight, cache, md.positions, md.slot_mapping,
-                                          self.rotary.cos_sin_cache, self.kv_a_layernorm.eps, False)
-        # RoPE on the rope part of q (k_pe is handled by the cache kernel)
-        q_pe = q[:, :, self.nope:].reshape(t, n * self.rope_dim).contiguous()
-        dummy_k = q_pe.new_empty(t, 0)
-        ops.rope_qk_(q_pe, dummy_k, md.positions, self.rotary.cos_sin_cache, self.rope_dim, self.rope_dim, False)
-        q_pe = q_pe.view(t, n, self.rope_dim)
+            # fused: RMSNorm(c_kv), RoPE(k_pe), [c_kv | k_pe] into the paged cache, RoPE on the rope part of q
+            q_pe = ops.mla_norm_rope_cache_(q, self.nope, kv_a, self.kv_a_layernorm.weight, cache, md.positions,
+                                            md.slot_mapping, self.rotary.cos_sin_cache, self.kv_a_layernorm.eps)
         nd = md.extra.get("num_decode_seqs", 0) if md.is_prefill and topk_indices is None else 0
         if nd and "md_decode" in md.extra:
             # mixed batch: rows [0, nd) are the single new tokens of decoding sequences: they take the
@@ -215,8 +213,10 @@ class MLAAttention(nn.Module):
                 and ops.PREFILL_TCGEN05):
             # the kernel reads keys, values and rotated parts where they are
             first = torch.tensor(starts, dtype=torch.int32).mul_(gbs).to(dev, non_blocking=True)
-            qf = torch.cat([q[:, :, : self.nope], q_pe], dim=-1)
-            return ops.mla_prefill(qf, kv.view(total_blocks * gbs, n, 256), lat[..., l:].view(total_blocks * gbs, -1), first,
+            # q_pe rotated in place: q is whole as it is
+            if q_pe.data_ptr() != q[:, :, self.nope:].data_ptr():
+                q = torch.cat([q[:, :, : self.nope], q_pe], dim=-1)
+            return ops.mla_prefill(q, kv.view(total_blocks * gbs, n, 256), lat[..., l:].view(total_blocks * gbs, -1), first,
                                    md.cu_q, md.seq_lens, md.num_seqs, md.max_q_len, self.scale)
         kv = kv.view(total_blocks, gbs, n, self.nope + self.v_dim)
         k_pe = lat[..., l:].unsqueeze(2).expand(total_blocks, gbs, n, self.rope_dim)

@@ -60,6 +60,10 @@ int b200_mla_kv_rmsnorm_rope_cache(const void* kv_c, const void* k_pe, const voi
                                    int L, int R, int neox, long long kvc_stride,
                                    long long kpe_stride, long long cache_row_stride,
                                    cudaStream_t stream);
+int b200_mla_norm_rope_cache(const void* kv_c, const void* k_pe, const void* w, void* cache, void* q_pe,
+                             const int* positions, const int* slot_mapping, const float* cos_sin, float eps, int T, int L,
+                             int R, int heads, long long kvc_stride, long long kpe_stride, long long cache_row_stride,
+                             long long q_stride, long long q_head_stride, cudaStream_t stream);
 int b200_paged_scatter_rows(void* dst, const void* src, const int* slot_mapping, int T,
                             int row_elems, long long src_stride, long long dst_row_stride,
                             cudaStream_t stream);
@@ -496,6 +500,35 @@ void mla_kv_rmsnorm_rope_cache(const Tensor& kv_c, const Tensor& k_pe, const Ten
         "mla_kv_rmsnorm_rope_cache");
 }
 
+// The latent row of every token into the cache, and the rotated parts q_pe [T, H, R] (a view) in place.  False (nothing
+// done): shapes or alignments that the kernel does not take.
+bool mla_norm_rope_cache(const Tensor& kv_c, const Tensor& k_pe, const Tensor& w, Tensor cache, Tensor q_pe,
+                         const Tensor& positions, const Tensor& slot_mapping, const Tensor& cos_sin, double eps) {
+  CHECK_CUDA_BF16(kv_c);
+  CHECK_CUDA_BF16(k_pe);
+  CHECK_CUDA_BF16(w);
+  CHECK_CUDA_BF16(cache);
+  CHECK_CUDA_BF16(q_pe);
+  CHECK_I32(positions);
+  CHECK_I32(slot_mapping);
+  const int T = kv_c.size(0), L = kv_c.size(1), R = k_pe.size(1);
+  TORCH_CHECK(kv_c.dim() == 2 && k_pe.dim() == 2 && q_pe.dim() == 3 && q_pe.size(2) == R && q_pe.size(0) == T &&
+                  k_pe.size(0) == T && kv_c.stride(1) == 1 && k_pe.stride(1) == 1 && q_pe.stride(2) == 1,
+              "mla_norm_rope_cache: kv_c [T, L], k_pe [T, R], q_pe [T, H, R]");
+  TORCH_CHECK(cache.is_contiguous() && cache.size(-1) >= L + R, "mla cache row too small");
+  TORCH_CHECK(w.is_contiguous() && w.numel() == L && positions.numel() >= T && slot_mapping.numel() >= T,
+              "mla_norm_rope_cache: sizes");
+  c10::cuda::CUDAGuard guard(kv_c.device());
+  const int rc = b200_mla_norm_rope_cache(kv_c.data_ptr(), k_pe.data_ptr(), w.data_ptr(), cache.data_ptr(), q_pe.data_ptr(),
+                                          positions.data_ptr<int>(), slot_mapping.data_ptr<int>(),
+                                          cos_sin.data_ptr<float>(), (float)eps, T, L, R, (int)q_pe.size(1),
+                                          kv_c.stride(0), k_pe.stride(0), cache.size(-1), q_pe.stride(0), q_pe.stride(1),
+                                          cur_stream());
+  if (rc == 1) return false;
+  check(rc, "mla_norm_rope_cache");
+  return true;
+}
+
 void paged_scatter_rows(Tensor dst, const Tensor& src, const Tensor& slot_mapping) {
   CHECK_CUDA_BF16(dst);
   CHECK_CUDA_BF16(src);
@@ -720,6 +753,7 @@ TORCH_LIBRARY_FRAGMENT(omni_b200, m) {
   m.def("quant_fp8_1x128", &quant_fp8_1x128);
   m.def("rope_qk", &rope_qk);
   m.def("rope_cache_gqa", &rope_cache_gqa);
+  m.def("mla_norm_rope_cache", &mla_norm_rope_cache);
   m.def("mla_prefill", &mla_prefill);
   m.def("mla_kv_rmsnorm_rope_cache", &mla_kv_rmsnorm_rope_cache);
   m.def("paged_scatter_rows", &paged_scatter_rows);

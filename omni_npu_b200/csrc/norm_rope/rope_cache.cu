@@ -450,6 +450,98 @@ mla_kv_rmsnorm_rope_cache_kernel(const __nv_bfloat16* __restrict__ kv_c,
   }
 }
 
+// The same with 16-byte accesses, neighbouring pairs, and the rotated part of every query head in place: one CTA per token,
+// all its loads ahead of the sum of squares.  8192 tokens of 16 heads: the kernel above 14.2 us, a copy of the queries'
+// rotated parts 15, their rotation 14 and their way back among the others 110; this one 22 for all of it.
+struct RopePairs {
+  uint4 x;
+  float4 c, s;
+};
+__device__ __forceinline__ RopePairs load_pairs(const __nv_bfloat16* src, const float* cs, int half, int j) {
+  return {*reinterpret_cast<const uint4*>(src + 8 * j), *reinterpret_cast<const float4*>(cs + 4 * j),
+          *reinterpret_cast<const float4*>(cs + half + 4 * j)};
+}
+__device__ __forceinline__ uint4 rotated_pairs(const RopePairs& r) {
+  const float c[4] = {r.c.x, r.c.y, r.c.z, r.c.w}, s[4] = {r.s.x, r.s.y, r.s.z, r.s.w};
+  uint4 out;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 x = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&r.x)[e]);
+    reinterpret_cast<__nv_bfloat162*>(&out)[e] = __floats2bfloat162_rn(x.x * c[e] - x.y * s[e], x.y * c[e] + x.x * s[e]);
+  }
+  return out;
+}
+
+static constexpr int kLatentThreads = 128, kLatentVecs = 4;      // vectors of the latent per thread: up to 4096 elements
+
+__global__ void __launch_bounds__(kLatentThreads)
+mla_norm_rope_cache_kernel(const __nv_bfloat16* __restrict__ kv_c, const __nv_bfloat16* __restrict__ k_pe,
+                           const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ cache,
+                           __nv_bfloat16* __restrict__ q_pe, const int* __restrict__ positions,
+                           const int* __restrict__ slot_mapping, const float* __restrict__ cos_sin, float eps, int L, int R,
+                           int heads, long long kvc_stride, long long kpe_stride, long long cache_row_stride,
+                           long long q_stride, long long q_head_stride) {
+  __shared__ float red[kLatentThreads / 32];
+  b200::pdl_trigger();
+  b200::pdl_wait();
+  const int t = blockIdx.x, tid = threadIdx.x;
+  const int slot = slot_mapping[t];
+  const int half = R >> 1, per_head = R >> 3, nvec = L >> 3;
+  const float* cs = cos_sin + static_cast<long long>(positions[t]) * R;
+  const __nv_bfloat16* src = kv_c + t * kvc_stride;
+  uint4 x[kLatentVecs], g[kLatentVecs];
+#pragma unroll
+  for (int i = 0; i < kLatentVecs; ++i) {
+    const int v = tid + i * kLatentThreads;
+    if (v < nvec) {
+      x[i] = reinterpret_cast<const uint4*>(src)[v];
+      g[i] = reinterpret_cast<const uint4*>(w)[v];
+    }
+  }
+  __nv_bfloat16* crow = slot >= 0 ? cache + static_cast<long long>(slot) * cache_row_stride : nullptr;
+  // the key's rotated part, then the queries'
+  for (int i = tid; i < per_head * (heads + 1); i += kLatentThreads) {
+    const int h = i / per_head - 1, j = i % per_head;
+    if (h < 0) {
+      if (crow) *reinterpret_cast<uint4*>(crow + L + 8 * j) = rotated_pairs(load_pairs(k_pe + t * kpe_stride, cs, half, j));
+    } else {
+      __nv_bfloat16* q = q_pe + t * q_stride + h * q_head_stride;
+      *reinterpret_cast<uint4*>(q + 8 * j) = rotated_pairs(load_pairs(q, cs, half, j));
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < kLatentVecs; ++i)
+    if (tid + i * kLatentThreads < nvec)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&x[i])[e]);
+        ss += f.x * f.x + f.y * f.y;
+      }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((tid & 31) == 0) red[tid >> 5] = ss;
+  __syncthreads();
+  float total = 0.f;
+#pragma unroll
+  for (int i = 0; i < kLatentThreads / 32; ++i) total += red[i];
+  const float inv = rsqrtf(total / static_cast<float>(L) + eps);
+  if (!crow) return;
+#pragma unroll
+  for (int i = 0; i < kLatentVecs; ++i) {
+    const int v = tid + i * kLatentThreads;
+    if (v >= nvec) continue;
+    uint4 out;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&x[i])[e]);
+      const float2 gw = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&g[i])[e]);
+      reinterpret_cast<__nv_bfloat162*>(&out)[e] = __floats2bfloat162_rn(f.x * inv * gw.x, f.y * inv * gw.y);
+    }
+    reinterpret_cast<uint4*>(crow)[v] = out;
+  }
+}
+
 // dst[slot_mapping[t], :] = src[t, :]  (row_elems a multiple of 8).
 __global__ void __launch_bounds__(128)
 paged_scatter_rows_kernel(__nv_bfloat16* __restrict__ dst, const __nv_bfloat16* __restrict__ src,
@@ -551,6 +643,28 @@ extern "C" int b200_mla_kv_rmsnorm_rope_cache(const void* kv_c, const void* k_pe
       static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(cache),
       static_cast<__nv_bfloat16*>(kv_c_out), static_cast<__nv_bfloat16*>(k_pe_out), positions,
       slot_mapping, cos_sin, eps, L, R, neox, kvc_stride, kpe_stride, cache_row_stride);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+// Latent row into the cache, and the rotated part of `heads` query heads (q_pe: the first one's of the first token) in place.
+// Neighbouring pairs.  Returns 1 (nothing done) for shapes and alignments that it does not take.
+extern "C" int b200_mla_norm_rope_cache(const void* kv_c, const void* k_pe, const void* w, void* cache, void* q_pe,
+                                        const int* positions, const int* slot_mapping, const float* cos_sin, float eps,
+                                        int T, int L, int R, int heads, long long kvc_stride, long long kpe_stride,
+                                        long long cache_row_stride, long long q_stride, long long q_head_stride,
+                                        cudaStream_t stream) {
+  const uintptr_t bases = reinterpret_cast<uintptr_t>(kv_c) | reinterpret_cast<uintptr_t>(k_pe) |
+                          reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(cache) |
+                          reinterpret_cast<uintptr_t>(q_pe) | reinterpret_cast<uintptr_t>(cos_sin);
+  const long long strides = kvc_stride | kpe_stride | cache_row_stride | q_stride | q_head_stride;
+  if ((bases & 15) != 0 || (strides & 7) != 0 || (L & 7) != 0 || (R & 7) != 0 || L > 8 * kLatentThreads * kLatentVecs)
+    return 1;
+  if (T <= 0) return 0;
+  b200::launch_pdl(mla_norm_rope_cache_kernel, dim3(T), dim3(kLatentThreads), 0, stream, 1,
+                   static_cast<const __nv_bfloat16*>(kv_c), static_cast<const __nv_bfloat16*>(k_pe),
+                   static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(cache),
+                   static_cast<__nv_bfloat16*>(q_pe), positions, slot_mapping, cos_sin, eps, L, R, heads, kvc_stride,
+                   kpe_stride, cache_row_stride, q_stride, q_head_stride);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

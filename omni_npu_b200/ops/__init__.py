@@ -584,6 +584,24 @@ def mla_kv_rmsnorm_rope_cache(kv_c: torch.Tensor, k_pe: torch.Tensor, w: torch.T
     return (kv_out, pe_out) if want_outputs else None
 
 
+def mla_norm_rope_cache_(q: torch.Tensor, nope: int, kv_a: torch.Tensor, w: torch.Tensor, cache: torch.Tensor,
+                         positions: torch.Tensor, slot_mapping: torch.Tensor, cos_sin: torch.Tensor,
+                         eps: float) -> torch.Tensor:
+    """One latent-attention layer's rows of a step: kv_a [T, latent + rope] into the paged cache (latent normed, the rest
+    rotated, neighbouring pairs), and the part of every query head of q [T, H, nope + rope] behind ``nope`` rotated.
+    Returns those parts, [T, H, rope]: views of q, rotated in place, or rows of their own."""
+    lat = w.shape[0]
+    kv_c, k_pe, q_pe = kv_a[:, :lat], kv_a[:, lat:], q[:, :, nope:]
+    if q.is_cuda and _C().mla_norm_rope_cache(kv_c, k_pe, w, cache, q_pe, positions, slot_mapping, cos_sin, eps):
+        _count(1)
+        return q_pe
+    mla_kv_rmsnorm_rope_cache(kv_c, k_pe, w, cache, positions, slot_mapping, cos_sin, eps, False)
+    t, n, rope = q_pe.shape
+    q_pe = q_pe.reshape(t, n * rope).contiguous()
+    rope_qk_(q_pe, q_pe.new_empty(t, 0), positions, cos_sin, rope, rope, False)
+    return q_pe.view(t, n, rope)
+
+
 # ------------------------------------------------------------------- attention
 def _pack_window(window: int, sink: int) -> int:
     """The kernels take the sliding window in the low 20 bits of one integer and the

@@ -540,6 +540,40 @@ def test_lse_merge_and_gather_cache():
     assert torch.equal(ops.gather_cache(cache, bt, sl).cpu(), ref.gather_cache(cache.cpu(), bt.cpu(), sl))
 
 
+@pytest.mark.parametrize("t,h,lat,rope,nope", [(1, 16, 512, 64, 128), (40, 3, 512, 64, 128), (7, 1, 8, 8, 16), (5, 2, 4096, 32, 64),
+                                               (9, 2, 260, 64, 128), (6, 2, 512, 64, 100)])
+def test_mla_norm_rope_cache(t, h, lat, rope, nope):
+    """Latent rows into the cache and the queries' rotated part in place (and shapes for which they are separate kernels)."""
+    torch.manual_seed(t)
+    q = torch.randn(t, h, nope + rope, device=DEV, dtype=torch.bfloat16)
+    kv = torch.randn(t, lat + rope, device=DEV, dtype=torch.bfloat16)
+    w = (torch.rand(lat, device=DEV) + 0.5).bfloat16()
+    pos = torch.randint(0, 500, (t,), device=DEV, dtype=torch.int32)
+    slots = torch.randperm(64)[:t].int()
+    if t > 2:
+        slots[2] = -1
+    cs = ref.build_cos_sin_cache(rope, 512, 10000.0).to(DEV)
+    cache = torch.zeros(4, 16, lat + rope, device=DEV, dtype=torch.bfloat16)
+    c, s = cs.double()[pos.long()].chunk(2, -1)
+
+    def turned(x):
+        x = x.double()
+        cc, ss = (c, s) if x.dim() == 2 else (c[:, None], s[:, None])
+        a, b = x[..., 0::2], x[..., 1::2]
+        return torch.stack([a * cc - b * ss, b * cc + a * ss], -1).flatten(-2)
+
+    want_q, head = turned(q[..., nope:]), q[..., :nope].clone()
+    row = kv[:, :lat].double()
+    row = torch.cat([row * torch.rsqrt(row.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double(), turned(kv[:, lat:])], -1)
+    got = ops.mla_norm_rope_cache_(q, nope, kv, w, cache, pos, slots.to(DEV), cs, 1e-6)
+    # one rounding to bf16
+    _close(got, want_q.float(), 1e-3, 2 ** -8)
+    assert torch.equal(q[..., :nope], head)
+    flat, used = cache.view(64, -1), [i for i in range(t) if slots[i] >= 0]
+    _close(flat[slots[used].long()], row[used].float(), 1e-3, 2 ** -8)
+    assert int((flat != 0).any(-1).sum()) == len(used)
+
+
 @pytest.mark.parametrize("new,cached", [([1], [0]), ([300, 1, 128, 17], [0, 700, 3, 129]), ([257, 5], [0, 0])])
 def test_mla_prefill(new, cached):
     """Latent attention over up-projected rows where they lie, sequences at starts of their own."""
