@@ -229,23 +229,20 @@ class MLAAttention(nn.Module):
                                self.scale, True, 0)
 
     def _absorb_q(self, q, q_pe):
-        """q_lat[h] = q_nope[h] @ W_UK[h] (heads act as the groups of a grouped GEMM); returns the
-        [t, n * 576] query of the latent-space kernel and the group offsets."""
+        """q_lat[h] = q_nope[h] @ W_UK[h]; returns the [t, n * 576] query of the latent-space kernel."""
         t, n, l = q.shape[0], self.num_heads, self.kv_lora_rank
         if self.w_uk is None:
             self.process_weights_after_loading()
-        q_nope = q[:, :, : self.nope].transpose(0, 1).reshape(n * t, self.nope).contiguous()
-        offs = torch.arange(0, (n + 1) * t, t, dtype=torch.int32, device=q.device)
-        q_lat = ops.grouped_gemm(q_nope, self.w_uk, offs).view(n, t, l).transpose(0, 1)
-        qf = torch.cat([q_lat, q_pe], dim=-1).reshape(t, n * (l + self.rope_dim)).contiguous()
-        return qf, offs
+        qf = q.new_empty(t, n, l + self.rope_dim)
+        ops.batched_gemm(q[:, :, : self.nope], self.w_uk, qf[:, :, :l])
+        qf[:, :, l:] = q_pe
+        return qf.view(t, n * (l + self.rope_dim))
 
-    def _unabsorb_o(self, o_lat, offs):
+    def _unabsorb_o(self, o_lat):
         """v[h] = o_lat[h] @ W_UV[h]^T -> [t, n * v_dim]."""
         t, n, l = o_lat.shape[0], self.num_heads, self.kv_lora_rank
-        o_lat = o_lat.view(t, n, l).transpose(0, 1).reshape(n * t, l).contiguous()
-        o = ops.grouped_gemm(o_lat, self.w_uv, offs).view(n, t, self.v_dim).transpose(0, 1)
-        return o.reshape(t, n * self.v_dim).contiguous()
+        o = o_lat.new_empty(t, n, self.v_dim)
+        return ops.batched_gemm(o_lat.view(t, n, l), self.w_uv, o).view(t, n * self.v_dim)
 
     @staticmethod
     def _rows_per_token(md: AttentionMetadata, t: int, device):
@@ -261,7 +258,7 @@ class MLAAttention(nn.Module):
 
     def _decode(self, q, q_pe, cache, md: AttentionMetadata, topk_indices) -> torch.Tensor:
         t, n = q.shape[0], self.num_heads
-        qf, offs = self._absorb_q(q, q_pe)
+        qf = self._absorb_q(q, q_pe)
         if md.is_prefill:
             # sparse prefill: every query token is its own "sequence" row for the kernel
             seq_of_tok = self._rows_per_token(md, t, q.device)
@@ -279,7 +276,7 @@ class MLAAttention(nn.Module):
         else:
             o_lat = ops.mla_decode(qf, cache, md.block_tables, md.seq_lens, md.num_seqs, n, self.scale, md.q_len,
                                    topk_indices, max_seq_len=md.max_seq_len)
-        return self._unabsorb_o(o_lat, offs)
+        return self._unabsorb_o(o_lat)
 
 
 class StaticSinkMLAAttention(MLAAttention):
@@ -335,7 +332,7 @@ class StaticSinkMLAAttention(MLAAttention):
 
     def _sink_window(self, q, q_pe, cache, md: AttentionMetadata) -> torch.Tensor:
         t, n, l = q.shape[0], self.num_heads, self.kv_lora_rank
-        qf, offs = self._absorb_q(q, q_pe)
+        qf = self._absorb_q(q, q_pe)
         pos = md.positions.reshape(-1)[:t].to(torch.int32)
         seq_of_tok = self._rows_per_token(md, t, q.device)
         bt = md.block_tables[seq_of_tok].contiguous()
@@ -348,7 +345,7 @@ class StaticSinkMLAAttention(MLAAttention):
         o_win, lse_win = ops.mla_decode(qf, cache, bt, sl, t, n, self.scale, 1, idx,
                                         max_seq_len=md.max_seq_len, return_lse=True)
         if not self.sink_len:
-            return self._unabsorb_o(o_win, offs)
+            return self._unabsorb_o(o_win)
         if self.sink_latent is None:
             self.process_weights_after_loading()
         sink = self.sink_latent.to(qf.dtype)                                              # [S, 576]
@@ -357,4 +354,4 @@ class StaticSinkMLAAttention(MLAAttention):
         o_s = (torch.softmax(sc, dim=-1).to(qf.dtype) @ sink[:, :l]).view(t, n, l)
         o_lat, _ = ops.merge_attn_states(torch.stack([o_win.view(t, n, l), o_s]),
                                          torch.stack([lse_win.view(t, n).float(), lse_s]))
-        return self._unabsorb_o(o_lat.reshape(t, n * l).to(qf.dtype), offs)
+        return self._unabsorb_o(o_lat.reshape(t, n * l).to(qf.dtype))

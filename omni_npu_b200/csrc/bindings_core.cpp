@@ -21,6 +21,8 @@ int b200_gemm_stream(const void* A, const void* W, void* C, const void* bias, co
 int b200_grouped_gemm_stream(const void* A, const void* W, void* C, const int* expert_offsets, int num_experts,
                              int total_rows, int N, int K, int lda, int ldc, int act, int tn, int* status, int max_ctas,
                              float act_alpha, float act_limit, cudaStream_t stream);
+int b200_batched_gemm(const void* A, const void* W, void* C, int T, int G, int N, int K, long long a_row, long long a_group,
+                      long long c_row, long long c_group, int tn, int* status, cudaStream_t stream);
 int b200_grouped_gemm_pair(const void* A, const void* W, void* C, const int* expert_offsets, int num_experts,
                            int total_rows, int N, int K, int lda, int ldc, int act, int* status, int max_ctas,
                            float act_alpha, float act_limit, cudaStream_t stream);
@@ -249,6 +251,25 @@ Tensor gemm_stream(const Tensor& a, const Tensor& w, const c10::optional<Tensor>
                          (int)max_ctas, (float)act_alpha, (float)act_limit, cur_stream()),
         "gemm_stream");
   return c;
+}
+
+// c[t, g] = a[t, g] w[g]^T: a [T, G, K] and c [T, G, N] views with any row and group pitch, w [G, N, K].  False (nothing
+// done): pitches or alignments that the kernel does not take.
+bool batched_gemm(const Tensor& a, const Tensor& w, Tensor c, int64_t tn, const Tensor& status) {
+  CHECK_CUDA_BF16(a);
+  CHECK_CUDA_BF16(w);
+  CHECK_CUDA_BF16(c);
+  TORCH_CHECK(a.dim() == 3 && w.dim() == 3 && c.dim() == 3 && w.is_contiguous() && a.stride(2) == 1 && c.stride(2) == 1 &&
+                  a.size(1) == w.size(0) && a.size(2) == w.size(2) && c.size(0) == a.size(0) && c.size(1) == w.size(0) &&
+                  c.size(2) == w.size(1),
+              "batched_gemm: a [T, G, K], w [G, N, K], c [T, G, N]");
+  c10::cuda::CUDAGuard guard(a.device());
+  const int rc = b200_batched_gemm(a.data_ptr(), w.data_ptr(), c.data_ptr(), (int)a.size(0), (int)a.size(1), (int)w.size(1),
+                                   (int)w.size(2), a.stride(0), a.stride(1), c.stride(0), c.stride(1), (int)tn,
+                                   status.data_ptr<int>(), cur_stream());
+  if (rc == 1) return false;
+  check(rc, "batched_gemm");
+  return true;
 }
 
 // tn: rows per tile of the weight-streaming kernel (gemm/gemm_stream.cu), 0: the kernel on CTA pairs (gemm/gemm_pair.cu).
@@ -1136,6 +1157,7 @@ TORCH_LIBRARY(omni_b200, m) {
   m.def("gemm", &gemm);
   m.def("gemm_pair", &gemm_pair);
   m.def("gemm_stream", &gemm_stream);
+  m.def("batched_gemm", &batched_gemm);
   m.def("grouped_gemm_rows", &grouped_gemm_rows);
   m.def("grouped_gemm", &grouped_gemm);
   m.def("moe_topk", &moe_topk);

@@ -464,6 +464,23 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, expert_offsets: torch.Tensor,
     return y if out is None else out.copy_(y)
 
 
+def batched_gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+    """``out[t, g] = a[t, g] @ w[g].T`` for a [T, G, K] and out [T, G, N] with any pitch between rows and groups (views of
+    larger rows are written and read as they lie), w [G, N, K]."""
+    t, g, k = a.shape
+    n = w.shape[1]
+    if a.is_cuda and a.dtype == out.dtype == torch.bfloat16:
+        # rows of A per tile: narrow ones while they are needed to fill the SMs
+        tiles = g * -(-n // 128)
+        tn = 32 if tiles * -(-t // 64) < 148 else 64 if t <= 64 else 128
+        if _core().batched_gemm(a, w, out, tn, device_state(a.device).status):
+            _count(1)
+            return out
+    rows = a.transpose(0, 1).reshape(g * t, k).contiguous()
+    offs = torch.arange(0, (g + 1) * t, max(t, 1), dtype=torch.int32, device=a.device)[: g + 1]
+    return out.copy_(grouped_gemm(rows, w, offs).view(g, t, n).transpose(0, 1))
+
+
 # ------------------------------------------------------------- norm/activation
 def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
     if not x.is_cuda:

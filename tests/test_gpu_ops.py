@@ -574,6 +574,22 @@ def test_mla_norm_rope_cache(t, h, lat, rope, nope):
     assert int((flat != 0).any(-1).sum()) == len(used)
 
 
+@pytest.mark.parametrize("t,g,n,k", [(1, 16, 512, 128), (33, 16, 128, 512), (130, 3, 200, 72), (300, 16, 512, 128), (5, 1, 24, 8),
+                                     (65, 128, 512, 64)])
+@pytest.mark.parametrize("at", [16, 4])
+def test_batched_gemm(t, g, n, k, at):
+    """Groups read and written where they lie among wider rows (from the fourth element on: an address that the copies do
+    not take)."""
+    torch.manual_seed(t + n)
+    a = torch.randn(t, g, k + 24, device=DEV, dtype=torch.bfloat16)[..., at: at + k]
+    w = (torch.randn(g, n, k, device=DEV) * k ** -0.5).bfloat16()
+    rows = torch.zeros(t, g, n + 64, device=DEV, dtype=torch.bfloat16)
+    out = ops.batched_gemm(a, w, rows[..., :n])
+    # one rounding to bf16
+    _close(out, torch.einsum("tgk,gnk->tgn", a.double(), w.double()).float(), 1e-3, 2 ** -8)
+    assert int(rows[..., n:].abs().max()) == 0
+
+
 @pytest.mark.parametrize("new,cached", [([1], [0]), ([300, 1, 128, 17], [0, 700, 3, 129]), ([257, 5], [0, 0])])
 def test_mla_prefill(new, cached):
     """Latent attention over up-projected rows where they lie, sequences at starts of their own."""
