@@ -264,7 +264,8 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
     st = device_state(a.device)
     m, k = a.shape
     n = w.shape[0]
-    if pair is None:
+    by_rule = pair is None
+    if by_rule:
         pair = PAIR_MIN_M > 0 and m >= PAIR_MIN_M and splits == 0 and bn == 0
     if pair:
         _count(1)
@@ -282,7 +283,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
         plan = C.gemm_plan(m, n, k, a.dtype.itemsize, gated, bn, 1 if gated else max(0, splits) if fused else splits)
         st.plans[key] = plan
     pbn, psplits, ws_bytes, ncnt, cluster = plan
-    if pair is None and m > PAIR_UNSPLIT_M and 0 < PAIR_MIN_M and a.dtype == torch.bfloat16 and bn == 0 and splits == 0 \
+    if by_rule and m > PAIR_UNSPLIT_M and 0 < PAIR_MIN_M and a.dtype == torch.bfloat16 and bn == 0 and splits == 0 \
             and psplits == 1:
         _count(1)
         return C.gemm_pair(a, w, bias, residual, out_dtype == torch.float32, kind[0], 0, st.status, max_ctas,
