@@ -8,12 +8,17 @@
 // 640 with a rank up to 512 (b200_latent_decode; the row holds zeros behind its last element).
 //
 // One CTA handles 16 query rows (heads) of one sequence (and one query token for
-// multi-token decode) over one split of the keys.  K tiles of 64 tokens x one row
-// come in through TMA (64-column slabs, 128B swizzle) into a two-stage
-// ring, issued by a producer warp.  Four compute warps:
-//   QK^T : warp w scores keys 16w..16w+15 of the tile,
+// multi-token decode) over one split of the keys.  K tiles of 32 tokens x one row
+// come in through TMA (64-column slabs, 128B swizzle) into a ring of five stages (four for rows above 576),
+// issued by a producer warp.  Three groups of two compute warps take the tiles in turn, each with a running
+// maximum, sum and output of its own, joined at the end:
+//   QK^T : a warp scores 16 keys, two accumulators in turn (one would wait for itself 36 times),
 //   softmax: tile-wide row max / sum through shared memory, P stored as bf16,
-//   P.V  : warp w accumulates a quarter of the output columns over all 64 keys.
+//   P.V  : a warp accumulates half of the output columns over the 32 keys.
+// A tile is a chain of scores, maximum, P and product; three chains side by side hide it.  128 sequences of 2300 tokens, 16
+// heads: 98.8 us with one group of four warps on tiles of 64 and one thread starting all copies (122 with the three key
+// splits chosen for it), 107 with the groups, 90 with the copies started by all lanes of the producer; 53 at the copy rate.
+// Four groups took 98: one stage less is on its way.
 // Split-KV partials are merged by a second kernel.  All waits are bounded.
 //
 // Replaces the decode call of npu_fused_infer_attention_score over the latent
@@ -24,6 +29,7 @@
 #include "attn_common.cuh"
 #include "../common/tensormap.h"
 #include "../common/device_once.h"
+#include "../common/pdl.cuh"
 
 namespace b200 {
 
@@ -31,13 +37,18 @@ static constexpr float kMlaLog2e = 1.4426950408889634f;
 static constexpr int kLat = 512;
 static constexpr int kRope = 64;
 static constexpr int kRow = kLat + kRope;     // 576
-static constexpr int kMlaBN = 64;
-static constexpr int kMlaStages = 2;
-static constexpr int kSlabBytes = kMlaBN * 128;           // 8 KB
-static constexpr int kPBytes = 16 * kMlaBN * 2;           // 2 KB
+static constexpr int kMlaBN = 32;                         // tokens of a tile
+static constexpr int kMlaGroups = 3;
+static constexpr int kMlaCompute = 64 * kMlaGroups, kMlaThreads = kMlaCompute + 32;
+static constexpr int kSlabBytes = kMlaBN * 128;           // 4 KB
+static constexpr int kPPitch = 80;                        // bytes of a row of P: 32 keys and 16 bytes against bank conflicts
+static constexpr int kPBytes = 16 * kPPitch;
 
-// shared memory for rows of `slabs` 64-column slabs: two key tiles, the queries, P, scratch
-static constexpr int mla_smem(int slabs) { return 1024 + slabs * (kMlaStages * kSlabBytes + 16 * 128) + kPBytes + 4096; }
+__host__ __device__ constexpr int mla_stages(int slabs) { return slabs <= 9 ? 5 : 4; }
+// shared memory for rows of `slabs` 64-column slabs: the ring, the queries, P, scratch
+static constexpr int mla_smem(int slabs) {
+  return 1024 + slabs * (mla_stages(slabs) * kSlabBytes + 16 * 128) + kMlaGroups * kPBytes + 4096;
+}
 
 struct MlaParams {
   const __nv_bfloat16* q;        // [T, N, row]
@@ -54,7 +65,7 @@ struct MlaParams {
   float scale_log2;
   int splits;
   int row, rank;                 // used by the instantiations whose sizes are not built in
-  float* o_part;                 // [B*q_len, head_tiles, splits, 16, 64 * CT]
+  float* o_part;                 // [B*q_len, head_tiles, splits, 16, 32 * CT]
   float* ml_part;                // [.., 16, 2]
   int* status;
 };
@@ -65,32 +76,49 @@ __device__ __forceinline__ uint32_t mla_off(int row, int chunk, int rows_per_sla
                                (((chunk & 7) ^ (row & 7)) << 4));
 }
 
-// ROW: elements of a cache row, 0 = p.row.  CT: 16-column output tiles of a warp (4 * 16 * CT >= rank).
+// ROW: elements of a cache row, 0 = p.row.  CT: 16-column output tiles of a warp (2 * 16 * CT >= rank).
 template <int ROW, int CT>
-__global__ void __launch_bounds__(160)
+__global__ void __launch_bounds__(kMlaThreads)
 mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, const int box_rows) {
   const int row_elems = ROW ? ROW : p.row;
   const int rank = ROW ? kLat : p.rank;
   const int slabs = ROW ? ROW / 64 : (p.row + 63) >> 6;
-  const int tile_bytes = slabs * kSlabBytes, q_bytes = slabs * 16 * 128;
+  const int tile_bytes = slabs * kSlabBytes, q_bytes = slabs * 16 * 128, stages = mla_stages(slabs);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sKV = smem;
-  uint8_t* sQ = sKV + kMlaStages * tile_bytes;
-  uint8_t* sP = sQ + q_bytes;                                  // [16][64] bf16, swizzled rows of 128 B
-  float* s_red = reinterpret_cast<float*>(sP + kPBytes);       // [2][4][16] max / sum exchange
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(s_red + 128);
-  uint64_t* empty_bar = full_bar + kMlaStages;
-  int* s_abort = reinterpret_cast<int*>(empty_bar + kMlaStages);
+  uint8_t* sQ = sKV + stages * tile_bytes;
+  uint8_t* sP_all = sQ + q_bytes;                              // [group][16][32] bf16
+  float* s_red_all = reinterpret_cast<float*>(sP_all + kMlaGroups * kPBytes);     // [group][max, sum][2][16]
+  float* s_ml = s_red_all + kMlaGroups * 64;                   // [group][16][max, sum]
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(s_ml + kMlaGroups * 32);
+  uint64_t* empty_bar = full_bar + 5;
+  int* s_abort = reinterpret_cast<int*>(empty_bar + 5);
   int* s_bt = s_abort + 4;                                     // up to 512 block-table entries
 
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  pdl_trigger();
+  if (tid == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 2);
+    }
+    *s_abort = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tm_c);
+  }
+  {
+    // rows that no copy writes (the last tile's, holes of a selection) must be finite: their P is zero
+    uint4* z = reinterpret_cast<uint4*>(sKV);
+    for (int i = tid; i < stages * tile_bytes / 16; i += kMlaThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  pdl_wait();
   const int tok = blockIdx.x;                 // b * q_len + qi
   const int b = tok / p.q_len;
   const int qi = tok % p.q_len;
   const int head0 = blockIdx.y * 16;
   const int split = blockIdx.z;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int seq_len = p.seq_lens[b];
   const int kv_len = p.topk_indices ? p.topk : (seq_len - p.q_len + qi + 1);   // causal limit
   const int* bt = p.block_tables + static_cast<long long>(b) * p.max_blocks;
@@ -102,78 +130,67 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
   const int t_end = min(n_tiles_all, t_begin + per);
   const int n_tiles = max(0, t_end - t_begin);
 
-  if (tid == 0) {
-    for (int s = 0; s < kMlaStages; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 4);
-    }
-    *s_abort = 0;
-    fence_barrier_init();
-    tma_prefetch_desc(&tm_c);
-  }
-  {
-    uint4* z = reinterpret_cast<uint4*>(sKV);
-    for (int i = tid; i < kMlaStages * tile_bytes / 16; i += 160) z[i] = make_uint4(0u, 0u, 0u, 0u);
-  }
   const int bt_first = sel ? 0 : (t_begin * kMlaBN) / p.block_size;
   const int bt_last = sel ? 0 : min(p.max_blocks, (min(kv_len, t_end * kMlaBN) + p.block_size - 1) / p.block_size);
   const bool bt_cached = !sel && (bt_last - bt_first) <= 512;
   if (bt_cached)
-    for (int i = bt_first + tid; i < bt_last; i += 160) s_bt[i - bt_first] = bt[i];
+    for (int i = bt_first + tid; i < bt_last; i += kMlaThreads) s_bt[i - bt_first] = bt[i];
   fence_proxy_async();
   __syncthreads();
   volatile int* abort_flag = s_abort;
 
-  if (warp == 4) {
+  if (warp == 2 * kMlaGroups) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
-      int issued = 0;
-      for (int it = 0; it < n_tiles; ++it) {
-        const int stage = it % kMlaStages;
-        if (it >= kMlaStages) {
-          const uint32_t parity = static_cast<uint32_t>(((it / kMlaStages) - 1) & 1);
-          if (*abort_flag || !mbar_wait(&empty_bar[stage], parity)) {
+    // (the lanes share out a tile's copies: one thread takes some 100 clocks for each, and 16-token pages make 18 a tile)
+    int issued = 0;
+    for (int it = 0; it < n_tiles; ++it) {
+      const int stage = it % stages;
+      if (it >= stages) {
+        const uint32_t parity = static_cast<uint32_t>(((it / stages) - 1) & 1);
+        const bool ok = !*abort_flag && mbar_wait(&empty_bar[stage], parity);
+        if (!__all_sync(0xffffffffu, ok)) {
+          if (lane == 0) {
             if (!*abort_flag && p.status) atomicCAS(p.status, 0, kStatusTimeoutEmptyBarrier);
             *abort_flag = 1;
-            break;
           }
+          break;
         }
-        const int n0 = (t_begin + it) * kMlaBN;
-        const int nvalid = min(kMlaBN, kv_len - n0);
-        uint8_t* dst_tile = sKV + stage * tile_bytes;
-        if (!sel) {
-          const int nboxes = (nvalid + box_rows - 1) / box_rows;
+      }
+      const int n0 = (t_begin + it) * kMlaBN;
+      const int nvalid = min(kMlaBN, kv_len - n0);
+      uint8_t* dst_tile = sKV + stage * tile_bytes;
+      if (!sel) {
+        const int nboxes = (nvalid + box_rows - 1) / box_rows;
+        if (lane == 0)
           mbar_arrive_expect_tx(&full_bar[stage], static_cast<uint32_t>(nboxes * box_rows * 128 * slabs));
-          for (int j = 0; j < nboxes; ++j) {
-            const int key = n0 + j * box_rows;
-            const int bi = key / p.block_size;
-            const int blk = bt_cached ? s_bt[bi - bt_first] : bt[bi];
-            const int row = blk * p.block_size + key % p.block_size;
-#pragma unroll
-            for (int s = 0; s < slabs; ++s)
-              tma_load_2d(dst_tile + s * kSlabBytes + j * box_rows * 128, &tm_c, &full_bar[stage], s * 64, row);
-          }
-        } else {
-          // sparse: one row per selected token (negative index = hole, left zero-scored)
-          int nrows = 0;
-          for (int j = 0; j < nvalid; ++j) nrows += sel[n0 + j] >= 0 ? 1 : 0;
-          mbar_arrive_expect_tx(&full_bar[stage], static_cast<uint32_t>(nrows * 128 * slabs));
-          for (int j = 0; j < nvalid; ++j) {
-            const int pos = sel[n0 + j];
-            if (pos < 0) continue;
-            const int row = bt[pos / p.block_size] * p.block_size + pos % p.block_size;
-#pragma unroll
-            for (int s = 0; s < slabs; ++s)
-              tma_load_2d(dst_tile + s * kSlabBytes + j * 128, &tm_c, &full_bar[stage], s * 64, row);
-          }
+        __syncwarp();
+        for (int l = lane; l < nboxes * slabs; l += 32) {
+          const int j = l / slabs, s = l - j * slabs;
+          const int key = n0 + j * box_rows;
+          const int bi = key / p.block_size;
+          const int blk = bt_cached ? s_bt[bi - bt_first] : bt[bi];
+          const int row = blk * p.block_size + key % p.block_size;
+          tma_load_2d(dst_tile + s * kSlabBytes + j * box_rows * 128, &tm_c, &full_bar[stage], s * 64, row);
         }
-        ++issued;
+      } else {
+        // sparse: one row per selected token (negative index = hole, left zero-scored), a token per lane
+        static_assert(kMlaBN == 32, "a token per lane");
+        const int pos = lane < nvalid ? sel[n0 + lane] : -1;
+        const int nrows = __popc(__ballot_sync(0xffffffffu, pos >= 0));
+        if (lane == 0) mbar_arrive_expect_tx(&full_bar[stage], static_cast<uint32_t>(nrows * 128 * slabs));
+        __syncwarp();
+        if (pos >= 0) {
+          const int row = bt[pos / p.block_size] * p.block_size + pos % p.block_size;
+          for (int s = 0; s < slabs; ++s)
+            tma_load_2d(dst_tile + s * kSlabBytes + lane * 128, &tm_c, &full_bar[stage], s * 64, row);
+        }
       }
-      if (*abort_flag) {
-        const int first = issued > kMlaStages ? issued - kMlaStages : 0;
-        for (int i = first; i < issued; ++i)
-          mbar_wait(&full_bar[i % kMlaStages], static_cast<uint32_t>((i / kMlaStages) & 1));
-      }
+      ++issued;
+    }
+    if (*abort_flag && lane == 0) {
+      const int first = issued > stages ? issued - stages : 0;
+      for (int i = first; i < issued; ++i)
+        mbar_wait(&full_bar[i % stages], static_cast<uint32_t>((i / stages) & 1));
     }
     __syncthreads();
     return;
@@ -181,7 +198,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
 
   // -------------------------------------------------------------- consumers
   const int chunks = slabs * 8;
-  for (int idx = tid; idx < 16 * chunks; idx += 128) {
+  for (int idx = tid; idx < 16 * chunks; idx += kMlaCompute) {
     const int row = idx / chunks, c = idx % chunks;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (head0 + row < p.N && c * 8 < row_elems)
@@ -189,8 +206,12 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
                                           static_cast<long long>(head0 + row) * row_elems + c * 8);
     *reinterpret_cast<uint4*>(sQ + mla_off(row, c, 16)) = v;
   }
-  asm volatile("bar.sync 1, 128;" ::: "memory");
+  asm volatile("bar.sync 1, %0;" ::"n"(kMlaCompute) : "memory");
 
+  const int group = warp >> 1, wi = warp & 1;
+  const int group_bar = 2 + group;            // named barrier of the group's 64 threads
+  uint8_t* sP = sP_all + group * kPBytes;
+  float* s_red = s_red_all + group * 64;
   float o_acc[2 * CT][4];
 #pragma unroll
   for (int i = 0; i < 2 * CT; ++i)
@@ -200,9 +221,10 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
   float row_sum[2] = {0.f, 0.f};
   const int r_a = lane >> 2;
 
-  for (int it = 0; it < n_tiles; ++it) {
-    const int stage = it % kMlaStages;
-    bool ok = !*abort_flag && mbar_wait(&full_bar[stage], static_cast<uint32_t>((it / kMlaStages) & 1));
+  int stage = group;
+  uint32_t phase = 0;
+  for (int it = group; it < n_tiles; it += kMlaGroups) {
+    bool ok = !*abort_flag && mbar_wait(&full_bar[stage], phase);
     ok = __all_sync(0xffffffffu, ok);
     if (!ok) {
       if (lane == 0) {
@@ -210,18 +232,19 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
         *abort_flag = 1;
       }
     }
-    // the decision must be uniform across the four warps (they share barriers below)
+    // the decision must be uniform across the group (its warps share barriers below); also: both are done with the
+    // tile before, whose P and scratch are rewritten now
     {
       uint32_t all_ok;
       asm volatile(
           "{\n\t"
           ".reg .pred p, q;\n\t"
           "setp.ne.u32 q, %1, 0;\n\t"
-          "bar.red.and.pred p, 1, 128, q;\n\t"
+          "bar.red.and.pred p, %2, 64, q;\n\t"
           "selp.u32 %0, 1, 0, p;\n\t"
           "}"
           : "=r"(all_ok)
-          : "r"(ok ? 1u : 0u)
+          : "r"(ok ? 1u : 0u), "r"(group_bar)
           : "memory");
       if (!all_ok) break;
     }
@@ -229,40 +252,46 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
     const int n0 = (t_begin + it) * kMlaBN;
 
     // ---- S = Q K^T for this warp's 16 keys
-    float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll 4
-    for (int ks = 0; ks < (row_elems + 15) / 16; ++ks) {
+    float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, s_odd[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    const int k_steps = (row_elems + 15) / 16;
+    const int krow = wi * 16 + (lane & 7) + ((lane >> 4) << 3);
+#pragma unroll 2
+    for (int ks = 0; ks < k_steps; ks += 2) {
       uint32_t qf[4], kf[4];
       ldmatrix_x4(qf, smem_u32(sQ) + mla_off(lane & 15, ks * 2 + (lane >> 4), 16));
-      const int krow = warp * 16 + (lane & 7) + ((lane >> 4) << 3);
       ldmatrix_x4(kf, kt + mla_off(krow, ks * 2 + ((lane >> 3) & 1), kMlaBN));
       mma_bf16_16816(s[0], qf, kf[0], kf[1]);
       mma_bf16_16816(s[1], qf, kf[2], kf[3]);
+      if (ks + 1 < k_steps) {
+        ldmatrix_x4(qf, smem_u32(sQ) + mla_off(lane & 15, ks * 2 + 2 + (lane >> 4), 16));
+        ldmatrix_x4(kf, kt + mla_off(krow, ks * 2 + 2 + ((lane >> 3) & 1), kMlaBN));
+        mma_bf16_16816(s_odd[0], qf, kf[0], kf[1]);
+        mma_bf16_16816(s_odd[1], qf, kf[2], kf[3]);
+      }
     }
     float tmax[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const int key = n0 + warp * 16 + i * 8 + (lane & 3) * 2 + (j & 1);
+        const int key = n0 + wi * 16 + i * 8 + (lane & 3) * 2 + (j & 1);
         bool keep = key < kv_len;
         if (sel && keep) keep = sel[key] >= 0;
-        const float v = keep ? s[i][j] * p.scale_log2 : -INFINITY;
+        const float v = keep ? (s[i][j] + s_odd[i][j]) * p.scale_log2 : -INFINITY;
         s[i][j] = v;
         tmax[j >> 1] = fmaxf(tmax[j >> 1], v);
       }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       tmax[r] = quad_max(tmax[r]);
-      if ((lane & 3) == 0) s_red[warp * 16 + r_a + 8 * r] = tmax[r];
+      if ((lane & 3) == 0) s_red[wi * 16 + r_a + 8 * r] = tmax[r];
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    asm volatile("bar.sync %0, 64;" ::"r"(group_bar) : "memory");
     float corr[2], m_use[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const int row = r_a + 8 * r;
-      const float tm = fmaxf(fmaxf(s_red[row], s_red[16 + row]), fmaxf(s_red[32 + row], s_red[48 + row]));
-      const float nm = fmaxf(row_max[r], tm);
+      const float nm = fmaxf(row_max[r], fmaxf(s_red[row], s_red[16 + row]));
       corr[r] = (nm == -INFINITY) ? 1.f : exp2f(row_max[r] - nm);
       row_max[r] = nm;
       m_use[r] = nm == -INFINITY ? 0.f : nm;
@@ -276,49 +305,44 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
         s[i][j] = e;
         psum[j >> 1] += e;
       }
-    // P (bf16) -> shared: row r, keys warp*16 + i*8 + (lane&3)*2
+    // P (bf16) -> shared: row r, keys wi*16 + i*8 + (lane&3)*2
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const int row = r_a + 8 * r;
-        const int key = warp * 16 + i * 8 + (lane & 3) * 2;
-        const uint32_t v = pack_bf16x2(s[i][2 * r], s[i][2 * r + 1]);
-        *reinterpret_cast<uint32_t*>(sP + row * 128 + (((key >> 3) ^ (row & 7)) << 4) + (key & 7) * 2) = v;
-      }
+      for (int r = 0; r < 2; ++r)
+        *reinterpret_cast<uint32_t*>(sP + (r_a + 8 * r) * kPPitch + (wi * 16 + i * 8 + (lane & 3) * 2) * 2) =
+            pack_bf16x2(s[i][2 * r], s[i][2 * r + 1]);
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       psum[r] = quad_sum(psum[r]);
-      if ((lane & 3) == 0) s_red[64 + warp * 16 + r_a + 8 * r] = psum[r];
+      if ((lane & 3) == 0) s_red[32 + wi * 16 + r_a + 8 * r] = psum[r];
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    asm volatile("bar.sync %0, 64;" ::"r"(group_bar) : "memory");
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const int row = r_a + 8 * r;
-      row_sum[r] = row_sum[r] * corr[r] + s_red[64 + row] + s_red[80 + row] + s_red[96 + row] + s_red[112 + row];
+      row_sum[r] = row_sum[r] * corr[r] + s_red[32 + row] + s_red[48 + row];
     }
+    if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {
 #pragma unroll
-    for (int i = 0; i < 2 * CT; ++i) {
-      o_acc[i][0] *= corr[0];
-      o_acc[i][1] *= corr[0];
-      o_acc[i][2] *= corr[1];
-      o_acc[i][3] *= corr[1];
+      for (int i = 0; i < 2 * CT; ++i) {
+        o_acc[i][0] *= corr[0];
+        o_acc[i][1] *= corr[0];
+        o_acc[i][2] *= corr[1];
+        o_acc[i][3] *= corr[1];
+      }
     }
     // ---- O (this warp's columns) += P V
 #pragma unroll
     for (int ks = 0; ks < kMlaBN / 16; ++ks) {
       uint32_t pf[4];
-      {
-        const int prow = lane & 15;
-        const int pchunk = ks * 2 + (lane >> 4);
-        ldmatrix_x4(pf, smem_u32(sP) + prow * 128 + ((pchunk ^ (prow & 7)) << 4));
-      }
+      ldmatrix_x4(pf, smem_u32(sP) + (lane & 15) * kPPitch + (ks * 2 + (lane >> 4)) * 16);
 #pragma unroll
       for (int dt = 0; dt < CT; ++dt) {
-        if (!ROW && (warp * CT + dt) * 16 >= rank) continue;
+        if (!ROW && (wi * CT + dt) * 16 >= rank) continue;
         uint32_t vf[4];
         const int vrow = ks * 16 + (lane & 15);
-        const int vchunk = warp * 2 * CT + dt * 2 + (lane >> 4);
+        const int vchunk = wi * 2 * CT + dt * 2 + (lane >> 4);
         ldmatrix_x4_trans(vf, kt + mla_off(vrow, vchunk, kMlaBN));
         mma_bf16_16816(o_acc[2 * dt], pf, vf[0], vf[1]);
         mma_bf16_16816(o_acc[2 * dt + 1], pf, vf[2], vf[3]);
@@ -326,26 +350,75 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty_bar[stage]);
-    // P and the reduction scratch are rewritten next tile: everyone must be done reading
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    stage += kMlaGroups;
+    if (stage >= stages) {
+      stage -= stages;
+      phase ^= 1;
+    }
   }
-  __syncthreads();
+  if (wi == 0 && (lane & 3) == 0) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      s_ml[(group * 16 + r_a + 8 * r) * 2] = row_max[r];
+      s_ml[(group * 16 + r_a + 8 * r) * 2 + 1] = row_sum[r];
+    }
+  }
+  __syncthreads();                 // also: every tile has been read
   if (*abort_flag) return;
 
-  // ---- write: every thread owns rows r_a, r_a+8 and two columns in eight of its warp's slice
+  // ---- the groups' shares, scaled to the common maximum, meet in the first group's threads
+  float l_all[2], m_all[2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    m_all[r] = -INFINITY;
+    l_all[r] = 0.f;
+#pragma unroll
+    for (int k = 0; k < kMlaGroups; ++k) m_all[r] = fmaxf(m_all[r], s_ml[(k * 16 + r_a + 8 * r) * 2]);
+#pragma unroll
+    for (int k = 0; k < kMlaGroups; ++k) {
+      const float m = s_ml[(k * 16 + r_a + 8 * r) * 2];
+      if (m != -INFINITY) l_all[r] += s_ml[(k * 16 + r_a + 8 * r) * 2 + 1] * exp2f(m - m_all[r]);
+    }
+    const float f = row_max[r] == -INFINITY ? 0.f : exp2f(row_max[r] - m_all[r]);
+#pragma unroll
+    for (int i = 0; i < 2 * CT; ++i) {
+      o_acc[i][2 * r] *= f;
+      o_acc[i][2 * r + 1] *= f;
+    }
+  }
+  float4* s_o = reinterpret_cast<float4*>(sKV);                // [group - 1][2 * CT][64 threads]
+  if (group > 0) {
+#pragma unroll
+    for (int i = 0; i < 2 * CT; ++i)
+      s_o[((group - 1) * 2 * CT + i) * 64 + wi * 32 + lane] = make_float4(o_acc[i][0], o_acc[i][1], o_acc[i][2], o_acc[i][3]);
+  }
+  asm volatile("bar.sync 1, %0;" ::"n"(kMlaCompute) : "memory");
+  if (group > 0) return;
+#pragma unroll
+  for (int k = 0; k < kMlaGroups - 1; ++k)
+#pragma unroll
+    for (int i = 0; i < 2 * CT; ++i) {
+      const float4 v = s_o[(k * 2 * CT + i) * 64 + wi * 32 + lane];
+      o_acc[i][0] += v.x;
+      o_acc[i][1] += v.y;
+      o_acc[i][2] += v.z;
+      o_acc[i][3] += v.w;
+    }
+
+  // ---- write: every thread owns rows r_a, r_a+8 and two columns in eight of its warp's half
   const size_t part_row = ((static_cast<size_t>(tok) * gridDim.y + blockIdx.y) * p.splits + split) * 16;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const int row = r_a + 8 * r;
     if (head0 + row >= p.N) continue;
-    const float l = row_sum[r];
+    const float l = l_all[r];
     if (p.splits == 1) {
       const float inv = l > 0.f ? 1.f / l : 0.f;
       __nv_bfloat16* dst = p.out + static_cast<long long>(tok) * p.out_stride +
                            static_cast<long long>(head0 + row) * rank;
 #pragma unroll
       for (int i = 0; i < 2 * CT; ++i) {
-        const int col = warp * 16 * CT + i * 8 + (lane & 3) * 2;
+        const int col = wi * 16 * CT + i * 8 + (lane & 3) * 2;
         const float o0 = o_acc[i][2 * r] * inv, o1 = o_acc[i][2 * r + 1] * inv;
         if (ROW || (col + 1 < rank && (rank & 1) == 0)) {
           *reinterpret_cast<uint32_t*>(dst + col) = pack_bf16x2(o0, o1);
@@ -354,18 +427,18 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
           if (col + 1 < rank) dst[col + 1] = __float2bfloat16(o1);
         }
       }
-      if (p.lse && warp == 0 && (lane & 3) == 0)
+      if (p.lse && wi == 0 && (lane & 3) == 0)
         p.lse[static_cast<long long>(tok) * p.N + head0 + row] =
-            l > 0.f ? (row_max[r] + log2f(l)) / kMlaLog2e : -INFINITY;
+            l > 0.f ? (m_all[r] + log2f(l)) / kMlaLog2e : -INFINITY;
     } else {
-      float* dst = p.o_part + (part_row + row) * (64 * CT) + warp * 16 * CT;
+      float* dst = p.o_part + (part_row + row) * (32 * CT) + wi * 16 * CT;
 #pragma unroll
       for (int i = 0; i < 2 * CT; ++i) {
         const int col = i * 8 + (lane & 3) * 2;
         *reinterpret_cast<float2*>(dst + col) = make_float2(o_acc[i][2 * r], o_acc[i][2 * r + 1]);
       }
-      if (warp == 0 && (lane & 3) == 0) {
-        p.ml_part[(part_row + row) * 2] = row_max[r];
+      if (wi == 0 && (lane & 3) == 0) {
+        p.ml_part[(part_row + row) * 2] = m_all[r];
         p.ml_part[(part_row + row) * 2 + 1] = l;
       }
     }
@@ -376,6 +449,8 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
 template <int CT>
 __global__ void __launch_bounds__(128)
 mla_merge_kernel(const MlaParams p, int total_tokens, int head_tiles) {
+  pdl_trigger();
+  pdl_wait();
   const long long gw = static_cast<long long>(blockIdx.x) * 4 + (threadIdx.x >> 5);
   if (gw >= static_cast<long long>(total_tokens) * p.N) return;
   const int lane = threadIdx.x & 31;
@@ -385,9 +460,9 @@ mla_merge_kernel(const MlaParams p, int total_tokens, int head_tiles) {
   float m = -INFINITY;
   for (int s = 0; s < p.splits; ++s) m = fmaxf(m, p.ml_part[(base + static_cast<size_t>(s) * 16) * 2]);
   float l = 0.f;
-  float acc[2 * CT];
+  float acc[CT];
 #pragma unroll
-  for (int i = 0; i < 2 * CT; ++i) acc[i] = 0.f;
+  for (int i = 0; i < CT; ++i) acc[i] = 0.f;
   for (int s = 0; s < p.splits; ++s) {
     const size_t pr = base + static_cast<size_t>(s) * 16;
     const float ms = p.ml_part[pr * 2];
@@ -395,19 +470,19 @@ mla_merge_kernel(const MlaParams p, int total_tokens, int head_tiles) {
     l += p.ml_part[pr * 2 + 1] * f;
     if (f == 0.f) continue;                  // (a split without keys has left its columns unwritten or zero)
 #pragma unroll
-    for (int i = 0; i < 2 * CT; ++i) acc[i] += p.o_part[pr * (64 * CT) + i * 32 + lane] * f;
+    for (int i = 0; i < CT; ++i) acc[i] += p.o_part[pr * (32 * CT) + i * 32 + lane] * f;
   }
   const float inv = l > 0.f ? 1.f / l : 0.f;
   __nv_bfloat16* dst = p.out + static_cast<long long>(tok) * p.out_stride + static_cast<long long>(head) * p.rank;
 #pragma unroll
-  for (int i = 0; i < 2 * CT; ++i)
+  for (int i = 0; i < CT; ++i)
     if (i * 32 + lane < p.rank) dst[i * 32 + lane] = __float2bfloat16(acc[i] * inv);
   if (p.lse && lane == 0)
     p.lse[static_cast<long long>(tok) * p.N + head] = l > 0.f ? (m + log2f(l)) / kMlaLog2e : -INFINITY;
 }
 
 
-static int mla_tiles_per_warp(int rank) { return rank <= 128 ? 2 : rank <= 256 ? 4 : 8; }
+static int mla_tiles_per_warp(int rank) { return rank <= 128 ? 4 : rank <= 256 ? 8 : 16; }
 
 template <int ROW, int CT>
 static int launch_mla(const MlaParams& p, const void* cache, int num_cache_blocks, int T, cudaStream_t stream) {
@@ -416,24 +491,25 @@ static int launch_mla(const MlaParams& p, const void* cache, int num_cache_block
   static DeviceOnce once;
   int cur_dev = 0;
   if (once.needed(&cur_dev)) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, mla_smem(ROW ? ROW / 64 : 10)) !=
-        cudaSuccess)
+    // (nine slabs, with one stage more, need the most)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, mla_smem(9)) != cudaSuccess)
       return -20;
     once.mark(cur_dev);
   }
   const int tiles = (p.N + 15) / 16;
-  const int box_rows = p.topk_indices ? 1 : (p.block_size < 64 ? p.block_size : 64);
+  const int box_rows = p.topk_indices ? 1 : (p.block_size < kMlaBN ? p.block_size : kMlaBN);
   CUtensorMap tm;
   const uint64_t rows = num_cache_blocks > 0 ? static_cast<uint64_t>(num_cache_blocks) * p.block_size : (1ull << 31);
   int r = make_tensormap_2d(&tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, cache, rows, p.row, p.row, box_rows, 64,
                             CU_TENSOR_MAP_SWIZZLE_128B);
   if (r) return r - 2000;
-  kern<<<dim3(T, tiles, p.splits), 160, smem, stream>>>(tm, p, box_rows);
-  if (cudaGetLastError() != cudaSuccess) return -21;
+  if (launch_pdl(kern, dim3(T, tiles, p.splits), dim3(kMlaThreads), smem, stream, 1, tm, p, box_rows) != cudaSuccess)
+    return -21;
   if (p.splits > 1) {
     const long long warps = static_cast<long long>(T) * p.N;
-    mla_merge_kernel<CT><<<static_cast<unsigned>((warps + 3) / 4), 128, 0, stream>>>(p, T, tiles);
-    if (cudaGetLastError() != cudaSuccess) return -22;
+    if (launch_pdl(mla_merge_kernel<CT>, dim3(static_cast<unsigned>((warps + 3) / 4)), dim3(128), 0, stream, 1, p, T,
+                   tiles) != cudaSuccess)
+      return -22;
   }
   return 0;
 }
@@ -445,7 +521,7 @@ using namespace b200;
 extern "C" size_t b200_latent_decode_scratch_bytes(int total_tokens, int N, int rank, int splits) {
   if (splits <= 1) return 0;
   const size_t tiles = (N + 15) / 16;
-  return static_cast<size_t>(total_tokens) * tiles * splits * 16 * (64 * mla_tiles_per_warp(rank) + 2) * sizeof(float);
+  return static_cast<size_t>(total_tokens) * tiles * splits * 16 * (32 * mla_tiles_per_warp(rank) + 2) * sizeof(float);
 }
 
 extern "C" size_t b200_mla_decode_scratch_bytes(int total_tokens, int N, int splits) {
@@ -483,13 +559,13 @@ static int mla_decode_any(const void* q, const void* cache, void* out, float* ls
   const int T = B * q_len;
   if (splits > 1) {
     p.o_part = static_cast<float*>(scratch);
-    p.ml_part = p.o_part + static_cast<size_t>(T) * ((N + 15) / 16) * splits * 16 * 64 * mla_tiles_per_warp(rank);
+    p.ml_part = p.o_part + static_cast<size_t>(T) * ((N + 15) / 16) * splits * 16 * 32 * mla_tiles_per_warp(rank);
   }
-  if (row == kRow && rank == kLat) return launch_mla<kRow, 8>(p, cache, num_cache_blocks, T, stream);
+  if (row == kRow && rank == kLat) return launch_mla<kRow, 16>(p, cache, num_cache_blocks, T, stream);
   switch (mla_tiles_per_warp(rank)) {
-    case 2: return launch_mla<0, 2>(p, cache, num_cache_blocks, T, stream);
     case 4: return launch_mla<0, 4>(p, cache, num_cache_blocks, T, stream);
-    default: return launch_mla<0, 8>(p, cache, num_cache_blocks, T, stream);
+    case 8: return launch_mla<0, 8>(p, cache, num_cache_blocks, T, stream);
+    default: return launch_mla<0, 16>(p, cache, num_cache_blocks, T, stream);
   }
 }
 

@@ -1131,6 +1131,18 @@ def contiguous_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out:
                             head_dim, head_dim_v, scale, 0, False, 0.0, 1, 0, device_state(q.device).status, True)
 
 
+def latent_splits(items: int, keys: int, sms: int = 148) -> int:
+    """Key splits of the latent decode kernel (one CTA per SM) for ``items`` (token, 16 heads) pairs and up to ``keys``
+    keys: fewest rounds of CTAs times a CTA's time, some 0.9 us per 32 keys and 5 for its start and end, 4 more for the
+    merge; at least 256 keys per split."""
+    tiles = -(-keys // 32)
+
+    def cost(s: int) -> float:
+        return -(-items * s // sms) * (-(-tiles // s) * 0.9 + 5.0) + (4.0 if s > 1 else 0.0)
+
+    return min(range(1, max(1, min(16, keys // 256)) + 1), key=cost)
+
+
 def latent_decode(q: torch.Tensor, cache: torch.Tensor, block_tables: torch.Tensor, seq_lens: torch.Tensor,
                   num_seqs: int, heads: int, rank: int, scale: float, out: torch.Tensor, max_seq_len: int = 0,
                   splits: int = 0) -> None:
@@ -1149,7 +1161,7 @@ def latent_decode(q: torch.Tensor, cache: torch.Tensor, block_tables: torch.Tens
     tiles = (heads + 15) // 16
     if splits <= 0:
         bound = max_seq_len if max_seq_len > 0 else block_tables.shape[1] * cache.shape[1]
-        splits = max(1, min((2 * 148 + num_seqs * tiles - 1) // max(1, num_seqs * tiles), max(1, bound // 256), 16))
+        splits = latent_splits(num_seqs * tiles, bound)
     scratch = None
     if splits > 1:
         nbytes = _core().latent_decode_scratch_bytes(num_seqs, heads, rank, splits)
@@ -1216,7 +1228,7 @@ def mla_decode(q: torch.Tensor, cache: torch.Tensor, block_tables: torch.Tensor,
     if splits <= 0:
         bound = topk_indices.shape[1] if topk_indices is not None else (
             max_seq_len if max_seq_len > 0 else block_tables.shape[1] * cache.shape[1])
-        splits = max(1, min((2 * 148 + t * tiles - 1) // max(1, t * tiles), max(1, bound // 256), 16))
+        splits = latent_splits(t * tiles, bound)
     scratch = None
     if splits > 1:
         nbytes = C.mla_decode_scratch_bytes(t, num_heads, splits)
