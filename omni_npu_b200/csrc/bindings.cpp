@@ -34,6 +34,13 @@ int b200_grouped_gemm_fp8_block(const void* A, const float* a_scales, const void
                                 const int* expert_offsets, int num_experts, int total_rows, int N, int K, int lda,
                                 int ldc, int scale_rows, int swiglu, int up_scale_row0, int* status, int max_ctas,
                                 cudaStream_t stream);
+int b200_gemm_fp8_stream(const void* A, const float* a_scales, const void* W, const float* w_scales, void* C,
+                         const void* bias, const void* residual, int M, int N, int K, int lda, int ldw, int ldc,
+                         int out_fp32, int* status, int max_ctas, cudaStream_t stream);
+int b200_grouped_gemm_fp8_stream(const void* A, const float* a_scales, const void* W, const float* w_scales, void* C,
+                                 const int* expert_offsets, int num_experts, int total_rows, int N, int K, int lda, int ldc,
+                                 int scale_rows, int swiglu, int up_scale_row0, int tn, int* status, int max_ctas,
+                                 cudaStream_t stream);
 int b200_dsa_indexer(const void* q, const float* w, const void* cache, const int* block_tables, const int* cu_q,
                      const int* positions, float* scores, int* topk_out, int T, int B, int H, int q_len,
                      long long num_blocks, int block_size, int max_blocks, long long ld, int max_ctx, int max_q,
@@ -234,7 +241,7 @@ std::tuple<Tensor, Tensor> quant_int8_per_token(const Tensor& x) {
 // [ceil(N/128), K/128]; every 128-wide K block's product is scaled before it is accumulated.
 Tensor gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tensor& w, const Tensor& w_scale,
                       const c10::optional<Tensor>& bias, const c10::optional<Tensor>& residual, bool out_fp32,
-                      const Tensor& status, int64_t max_ctas) {
+                      bool few_rows, const Tensor& status, int64_t max_ctas) {
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 2, "gemm_fp8_block: 2-D CUDA tensors");
   TORCH_CHECK(a.scalar_type() == at::kFloat8_e4m3fn && w.scalar_type() == at::kFloat8_e4m3fn,
               "gemm_fp8_block: float8_e4m3fn operands");
@@ -261,7 +268,9 @@ Tensor gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tensor& w, c
                 "gemm_fp8_block: residual [M, N] contiguous");
     res_p = residual->data_ptr();
   }
-  check(b200_gemm_fp8_block(a.data_ptr(), a_scale.data_ptr<float>(), w.data_ptr(), w_scale.data_ptr<float>(),
+  // few_rows: the weight-streaming kernel (gemm/gemm_fp8_stream.cu)
+  const auto product = few_rows ? b200_gemm_fp8_stream : b200_gemm_fp8_block;
+  check(product(a.data_ptr(), a_scale.data_ptr<float>(), w.data_ptr(), w_scale.data_ptr<float>(),
                             c.data_ptr(), bias_p, res_p, (int)M, (int)N, (int)K, (int)a.stride(0), (int)w.stride(0),
                             (int)N, out_fp32 ? 1 : 0, status.data_ptr<int>(), (int)max_ctas, cur_stream()),
         "gemm_fp8_block");
@@ -273,7 +282,7 @@ Tensor gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tensor& w, c
 // interleaved in groups of 8, their scale rows are gate blocks then up blocks (from row up_scale_row0).
 // The result goes into c [rows, N, or N / 2 with swiglu] (rows may lie further apart).
 void grouped_gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tensor& w, const Tensor& w_scale,
-                            const Tensor& expert_offsets, Tensor c, bool swiglu, int64_t up_scale_row0,
+                            const Tensor& expert_offsets, Tensor c, bool swiglu, int64_t up_scale_row0, int64_t tn,
                             const Tensor& status, int64_t max_ctas) {
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 3, "grouped_gemm_fp8_block: shapes");
   TORCH_CHECK(a.scalar_type() == at::kFloat8_e4m3fn && w.scalar_type() == at::kFloat8_e4m3fn,
@@ -295,6 +304,14 @@ void grouped_gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tensor
   TORCH_CHECK(c.is_cuda() && c.scalar_type() == at::kBFloat16 && c.dim() == 2 && c.size(0) == rows && c.size(1) == n_out &&
                   c.stride(1) == 1 && c.stride(0) >= n_out && c.device() == a.device(),
               "grouped_gemm_fp8_block: result bf16 [rows, N]");
+  if (tn > 0) {        // rows per tile of the weight-streaming kernel
+    check(b200_grouped_gemm_fp8_stream(a.data_ptr(), a_scale.data_ptr<float>(), w.data_ptr(), w_scale.data_ptr<float>(),
+                                       c.data_ptr(), expert_offsets.data_ptr<int>(), (int)E, (int)rows, (int)N, (int)K,
+                                       (int)a.stride(0), (int)c.stride(0), (int)R, swiglu ? 1 : 0, (int)up_scale_row0,
+                                       (int)tn, status.data_ptr<int>(), (int)max_ctas, cur_stream()),
+          "grouped_gemm_fp8_stream");
+    return;
+  }
   check(b200_grouped_gemm_fp8_block(a.data_ptr(), a_scale.data_ptr<float>(), w.data_ptr(), w_scale.data_ptr<float>(),
                                     c.data_ptr(), expert_offsets.data_ptr<int>(), (int)E, (int)rows, (int)N, (int)K,
                                     (int)a.stride(0), (int)c.stride(0), (int)R, swiglu ? 1 : 0, (int)up_scale_row0,

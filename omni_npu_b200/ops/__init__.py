@@ -307,6 +307,14 @@ def quant_int8_per_token(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     return _C().quant_int8_per_token(x)
 
 
+# Block-scaled products with at most this many rows (per group on average) stream their weights through
+# gemm_fp8_stream_kernel.  Us, gemm_fp8_block_kernel / here: 4096 x 7168 31.8 / 10.5 with one row, 32.2 / 13.7 with 64 (the
+# most that it takes), 18432 x 7168 34.4 / 33.7; 32 groups 4096 x 7168 with silu 214 / 159 at 32 rows each, 194 / 169 at 48,
+# 195 / 205 at 64, 7168 x 2048 111 / 88, 113 / 95 and 117 / 130.
+FP8_STREAM_ROWS = 64
+FP8_STREAM_GROUP_ROWS = 48
+
+
 def gemm_fp8_block(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor,
                    bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
                    out_dtype: Optional[torch.dtype] = None, max_ctas: int = 0) -> torch.Tensor:
@@ -317,7 +325,7 @@ def gemm_fp8_block(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.Tensor, 
     st = device_state(a_q.device)
     _count(1)
     return _C().gemm_fp8_block(a_q, a_scale.contiguous(), w_q, w_scale.contiguous(), bias, residual,
-                               out_dtype == torch.float32, st.status, max_ctas)
+                               out_dtype == torch.float32, a_q.shape[0] <= FP8_STREAM_ROWS, st.status, max_ctas)
 
 
 def grouped_gemm_fp8_block(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor,
@@ -333,9 +341,10 @@ def grouped_gemm_fp8_block(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.
     st = device_state(a_q.device)
     if out is None:
         out = torch.empty(a_q.shape[0], w_q.shape[1] // (2 if swiglu else 1), dtype=torch.bfloat16, device=a_q.device)
+    few = a_q.shape[0] <= FP8_STREAM_GROUP_ROWS * w_q.shape[0]
     _count(1)
     _C().grouped_gemm_fp8_block(a_q, a_scale.contiguous(), w_q, w_scale.contiguous(), expert_offsets, out, swiglu,
-                                up_scale_row0, st.status, max_ctas)
+                                up_scale_row0, 64 if few else 0, st.status, max_ctas)
     return out
 
 

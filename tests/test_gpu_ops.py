@@ -540,6 +540,41 @@ def test_lse_merge_and_gather_cache():
     assert torch.equal(ops.gather_cache(cache, bt, sl).cpu(), ref.gather_cache(cache.cpu(), bt.cpu(), sl))
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 4096, 7168), (33, 130, 128), (64, 1000, 640), (17, 7168, 2048), (5, 40000, 256)])
+def test_gemm_fp8_few_rows(m, n, k, monkeypatch):
+    """The weight-streaming block-scaled kernel against the one that it stands in for: K splits of 1 to 8, ragged N, epilogues."""
+    torch.manual_seed(m + n)
+    w = torch.randn(n, k, device=DEV).to(torch.float8_e4m3fn)
+    ws = torch.rand(-(-n // 128), k // 128, device=DEV) + 0.5
+    q, s = ops.quant_fp8_1x128(torch.randn(m, k, device=DEV, dtype=torch.bfloat16))
+    bias, res = torch.randn(n, device=DEV).bfloat16(), torch.randn(m, n, device=DEV).bfloat16()
+    got = [ops.gemm_fp8_block(q, s, w, ws, **kw) for kw in (dict(out_dtype=torch.float32), dict(bias=bias, residual=res))]
+    monkeypatch.setattr(ops, "FP8_STREAM_ROWS", 0)
+    want = [ops.gemm_fp8_block(q, s, w, ws, **kw) for kw in (dict(out_dtype=torch.float32), dict(bias=bias, residual=res))]
+    # the same fp32 products, summed in another order where K is split; one rounding to bf16
+    _close(got[0], want[0], 1e-5 * k ** 0.5, 1e-5)
+    _close(got[1], want[1], 1e-2, 2 ** -7)
+    ops.check_status()
+
+
+@pytest.mark.parametrize("counts,n,k,swiglu", [([0, 5, 64, 65, 0, 16, 17, 1], 512, 256, True), ([3], 130, 128, False),
+                                               ([33] * 40, 256, 384, True), ([0, 0, 90], 1000, 640, False)])
+def test_grouped_gemm_fp8_few_rows(counts, n, k, swiglu, monkeypatch):
+    torch.manual_seed(n)
+    offs = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device=DEV)
+    rows, e = sum(counts), len(counts)
+    assert rows <= ops.FP8_STREAM_GROUP_ROWS * e
+    w = torch.randn(e, n, k, device=DEV).to(torch.float8_e4m3fn)
+    up = n // 256 if swiglu else 0
+    ws = torch.rand(e, 2 * up if swiglu else -(-n // 128), k // 128, device=DEV) * 0.1
+    q, s = ops.quant_fp8_1x128(torch.randn(rows + 3, k, device=DEV, dtype=torch.bfloat16))
+    got = ops.grouped_gemm_fp8_block(q, s, w, ws, offs, swiglu, up)[:rows]
+    monkeypatch.setattr(ops, "FP8_STREAM_GROUP_ROWS", 0)
+    want = ops.grouped_gemm_fp8_block(q, s, w, ws, offs, swiglu, up)[:rows]
+    _close(got, want, 1e-3, 2 ** -7)       # the same sums, rounded once
+    ops.check_status()
+
+
 @pytest.mark.parametrize("t,h,lat,rope,nope", [(1, 16, 512, 64, 128), (40, 3, 512, 64, 128), (7, 1, 8, 8, 16), (5, 2, 4096, 32, 64),
                                                (9, 2, 260, 64, 128), (6, 2, 512, 64, 100)])
 def test_mla_norm_rope_cache(t, h, lat, rope, nope):
