@@ -210,6 +210,9 @@ SMALL_M_LIBRARY_ROWS = (64, 256)
 # 6144 x 4096 20 / 24: the rows of A, read again for every 128 columns, then weigh as much as the weights.
 STREAM_ROWS = 64
 STREAM_WIDE_ROWS, STREAM_WIDE_N = 128, 148 * 128
+# ... and with fewer than 64 weight rows (a small router), for which the other kernel has no split of K: 128 rows,
+# 32 x 7168, 35.7 / 13.4.
+STREAM_NARROW_N = 64
 
 GELU_TANH = "gelu_tanh"    # gated activation gelu(gate) * up, gelu in its tanh form
 RELU = "relu"              # gated activation max(gate, 0) * up
@@ -272,7 +275,8 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
         return C.gemm_pair(a, w, bias, residual, out_dtype == torch.float32, kind[0], bn, st.status, max_ctas,
                            kind[1], kind[2])
     fused, gated = kind[0] != 0, kind[0] in (1, 2, 4, 7)
-    if ((m < STREAM_ROWS or m <= STREAM_WIDE_ROWS and n >= STREAM_WIDE_N) and a.dtype == torch.bfloat16 and bn == 0 and splits == 0
+    if ((m < STREAM_ROWS or m <= STREAM_WIDE_ROWS and (n >= STREAM_WIDE_N or n < STREAM_NARROW_N))
+            and a.dtype == torch.bfloat16 and bn == 0 and splits == 0
             and not (gated and (residual is not None or out_dtype == torch.float32))):
         _count(1)
         return C.gemm_stream(a, w, bias, residual, out_dtype == torch.float32, kind[0], 0, st.status, max_ctas, kind[1],
