@@ -121,8 +121,8 @@ class LatentAttention(nn.Module):
             rows = ops.latent_gather(cache, bt, lens, shared["start"], n, shared["total"], md.max_seq_len)
             if self.rows_shared:
                 shared[cache_idx] = rows
-        k = ops.gemm(rows, self.w_key).view(-1, self.num_heads, 1, self.k_pad)
-        v = ops.gemm(rows, self.w_value).view(-1, self.num_heads, 1, self.v_pad)
+        k = ops.gemm(rows, self.w_key, w_ready=True).view(-1, self.num_heads, 1, self.k_pad)
+        v = ops.gemm(rows, self.w_value, w_ready=True).view(-1, self.num_heads, 1, self.v_pad)
         cu_q = md.extra["cu_q_prefill"] if nd else md.cu_q
         ops.contiguous_attention(q, k, v, out, cu_q, shared["start"], lens, n,
                                  md.extra["max_q_len_prefill"] if nd else md.max_q_len, self.num_heads, self.qk_dim,

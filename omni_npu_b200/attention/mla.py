@@ -231,10 +231,11 @@ class MLAAttention(nn.Module):
     def _absorb_q(self, q, q_pe):
         """q_lat[h] = q_nope[h] @ W_UK[h]; returns the [t, n * 576] query of the latent-space kernel."""
         t, n, l = q.shape[0], self.num_heads, self.kv_lora_rank
-        if self.w_uk is None:
+        made = self.w_uk is None          # by the kernel right ahead of the product, which then has to wait for it
+        if made:
             self.process_weights_after_loading()
         qf = q.new_empty(t, n, l + self.rope_dim)
-        ops.batched_gemm(q[:, :, : self.nope], self.w_uk, qf[:, :, :l])
+        ops.batched_gemm(q[:, :, : self.nope], self.w_uk, qf[:, :, :l], w_ready=not made)
         qf[:, :, l:] = q_pe
         return qf.view(t, n * (l + self.rope_dim))
 
@@ -242,7 +243,7 @@ class MLAAttention(nn.Module):
         """v[h] = o_lat[h] @ W_UV[h]^T -> [t, n * v_dim]."""
         t, n, l = o_lat.shape[0], self.num_heads, self.kv_lora_rank
         o = o_lat.new_empty(t, n, self.v_dim)
-        return ops.batched_gemm(o_lat.view(t, n, l), self.w_uv, o).view(t, n * self.v_dim)
+        return ops.batched_gemm(o_lat.view(t, n, l), self.w_uv, o, w_ready=True).view(t, n * self.v_dim)
 
     @staticmethod
     def _rows_per_token(md: AttentionMetadata, t: int, device):

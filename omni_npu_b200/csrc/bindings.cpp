@@ -36,7 +36,7 @@ int b200_grouped_gemm_fp8_block(const void* A, const float* a_scales, const void
                                 cudaStream_t stream);
 int b200_gemm_fp8_stream(const void* A, const float* a_scales, const void* W, const float* w_scales, void* C,
                          const void* bias, const void* residual, int M, int N, int K, int lda, int ldw, int ldc,
-                         int out_fp32, int* status, int max_ctas, cudaStream_t stream);
+                         int out_fp32, int* status, int max_ctas, int w_ready, cudaStream_t stream);
 int b200_grouped_gemm_fp8_stream(const void* A, const float* a_scales, const void* W, const float* w_scales, void* C,
                                  const int* expert_offsets, int num_experts, int total_rows, int N, int K, int lda, int ldc,
                                  int scale_rows, int swiglu, int up_scale_row0, int tn, int* status, int max_ctas,
@@ -52,7 +52,7 @@ int b200_silu_mul_quant(void* q, void* scales, const void* x, long long rows, in
                         cudaStream_t stream);
 int b200_gemm_scaled(const void* A, const void* W, void* C, const float* a_scales, const float* w_scales,
                      const void* bias, const void* residual, int M, int N, int K, int lda, int ldw, int ldc,
-                     int kind, int out_fp32, int BN, int* status, int max_ctas, cudaStream_t stream);
+                     int kind, int out_fp32, int BN, int* status, int max_ctas, int w_ready, cudaStream_t stream);
 int b200_rope_qk(void* q, void* k, const int* positions, const float* cos_sin, int T, int Hq,
                  int Hk, int D, int rot_dim, int neox, long long q_stride, long long k_stride,
                  int sec_t, int sec_h, int interleaved_mrope, cudaStream_t stream);
@@ -241,7 +241,7 @@ std::tuple<Tensor, Tensor> quant_int8_per_token(const Tensor& x) {
 // [ceil(N/128), K/128]; every 128-wide K block's product is scaled before it is accumulated.
 Tensor gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tensor& w, const Tensor& w_scale,
                       const c10::optional<Tensor>& bias, const c10::optional<Tensor>& residual, bool out_fp32,
-                      bool few_rows, const Tensor& status, int64_t max_ctas) {
+                      bool few_rows, const Tensor& status, int64_t max_ctas, bool w_ready) {
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 2, "gemm_fp8_block: 2-D CUDA tensors");
   TORCH_CHECK(a.scalar_type() == at::kFloat8_e4m3fn && w.scalar_type() == at::kFloat8_e4m3fn,
               "gemm_fp8_block: float8_e4m3fn operands");
@@ -268,12 +268,17 @@ Tensor gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tensor& w, c
                 "gemm_fp8_block: residual [M, N] contiguous");
     res_p = residual->data_ptr();
   }
-  // few_rows: the weight-streaming kernel (gemm/gemm_fp8_stream.cu)
-  const auto product = few_rows ? b200_gemm_fp8_stream : b200_gemm_fp8_block;
-  check(product(a.data_ptr(), a_scale.data_ptr<float>(), w.data_ptr(), w_scale.data_ptr<float>(),
-                            c.data_ptr(), bias_p, res_p, (int)M, (int)N, (int)K, (int)a.stride(0), (int)w.stride(0),
-                            (int)N, out_fp32 ? 1 : 0, status.data_ptr<int>(), (int)max_ctas, cur_stream()),
-        "gemm_fp8_block");
+  if (few_rows)        // the weight-streaming kernel (gemm/gemm_fp8_stream.cu)
+    check(b200_gemm_fp8_stream(a.data_ptr(), a_scale.data_ptr<float>(), w.data_ptr(), w_scale.data_ptr<float>(),
+                               c.data_ptr(), bias_p, res_p, (int)M, (int)N, (int)K, (int)a.stride(0), (int)w.stride(0),
+                               (int)N, out_fp32 ? 1 : 0, status.data_ptr<int>(), (int)max_ctas, w_ready ? 1 : 0,
+                               cur_stream()),
+          "gemm_fp8_stream");
+  else
+    check(b200_gemm_fp8_block(a.data_ptr(), a_scale.data_ptr<float>(), w.data_ptr(), w_scale.data_ptr<float>(),
+                              c.data_ptr(), bias_p, res_p, (int)M, (int)N, (int)K, (int)a.stride(0), (int)w.stride(0),
+                              (int)N, out_fp32 ? 1 : 0, status.data_ptr<int>(), (int)max_ctas, cur_stream()),
+          "gemm_fp8_block");
   return c;
 }
 
@@ -404,7 +409,7 @@ std::tuple<Tensor, Tensor> silu_and_mul_quant(const Tensor& x, int64_t kind) {
 // int8 x int8 (s32 accumulate) or e4m3 x e4m3 (fp32 accumulate).
 Tensor gemm_scaled(const Tensor& a, const Tensor& w, const Tensor& a_scale, const Tensor& w_scale,
                    const c10::optional<Tensor>& bias, const c10::optional<Tensor>& residual, bool out_fp32,
-                   int64_t bn, const Tensor& status, int64_t max_ctas) {
+                   int64_t bn, const Tensor& status, int64_t max_ctas, bool w_ready) {
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 2, "gemm_scaled: 2-D CUDA tensors");
   TORCH_CHECK(a.scalar_type() == w.scalar_type(), "gemm_scaled: dtype mismatch");
   const bool i8 = a.scalar_type() == at::kChar;
@@ -434,7 +439,7 @@ Tensor gemm_scaled(const Tensor& a, const Tensor& w, const Tensor& a_scale, cons
   check(b200_gemm_scaled(a.data_ptr(), w.data_ptr(), c.data_ptr(), a_scale.data_ptr<float>(),
                          w_scale.data_ptr<float>(), bias_p, res_p, M, N, K, (int)a.stride(0), (int)w.stride(0),
                          N, i8 ? 2 : 1, out_fp32 ? 1 : 0, (int)bn, status.data_ptr<int>(), (int)max_ctas,
-                         cur_stream()),
+                         w_ready ? 1 : 0, cur_stream()),
         "gemm_scaled");
   return c;
 }

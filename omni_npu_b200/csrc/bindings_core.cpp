@@ -14,22 +14,22 @@ void b200_gemm_plan(int M, int N, int K, int elem_bytes, int swiglu, int force_b
 int b200_gemm(const void* A, const void* W, void* C, const void* bias, const void* residual, int M,
               int N, int K, int lda, int ldw, int ldc, int dtype_fp8, int out_fp32, int swiglu,
               int BN, int splits, int cluster_split, void* workspace, int* counters, int* status,
-              int max_ctas, float act_alpha, float act_limit, cudaStream_t stream);
+              int max_ctas, float act_alpha, float act_limit, int w_ready, cudaStream_t stream);
 int b200_gemm_stream(const void* A, const void* W, void* C, const void* bias, const void* residual, int M, int N, int K,
                      int lda, int ldw, int ldc, int out_fp32, int act, int splits, int* status, int max_ctas,
-                     float act_alpha, float act_limit, cudaStream_t stream);
+                     float act_alpha, float act_limit, int w_ready, cudaStream_t stream);
 int b200_grouped_gemm_stream(const void* A, const void* W, void* C, const int* expert_offsets, int num_experts,
                              int total_rows, int N, int K, int lda, int ldc, int act, int tn, int* status, int max_ctas,
                              float act_alpha, float act_limit, cudaStream_t stream);
 int b200_batched_gemm(const void* A, const void* W, void* C, int T, int G, int N, int K, long long a_row, long long a_group,
-                      long long c_row, long long c_group, int tn, int* status, cudaStream_t stream);
+                      long long c_row, long long c_group, int tn, int* status, int w_ready, cudaStream_t stream);
 int b200_grouped_gemm_pair(const void* A, const void* W, void* C, const int* expert_offsets, int num_experts,
                            int total_rows, int N, int K, int lda, int ldc, int act, int* status, int max_ctas,
                            float act_alpha, float act_limit, cudaStream_t stream);
 int b200_gemm_pair(const void* A, const void* W, void* C, const void* bias, const void* residual,
                    int M, int N, int K, int lda, int ldw, int ldc, int dtype_fp8, int out_fp32,
                    int swiglu, int BN, int* status, int max_ctas, float act_alpha, float act_limit,
-                   cudaStream_t stream);
+                   int w_ready, cudaStream_t stream);
 int b200_grouped_gemm(const void* A, const void* W, void* C, const int* expert_offsets,
                       int num_experts, int total_rows, int N, int K, int lda, int ldc,
                       int dtype_fp8, int swiglu, int BN, int* status, int max_ctas, float act_alpha,
@@ -147,7 +147,7 @@ Tensor gemm(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& bias,
             const c10::optional<Tensor>& residual, bool out_fp32, int64_t act, int64_t bn,
             int64_t splits, bool cluster_split, const c10::optional<Tensor>& workspace,
             const c10::optional<Tensor>& counters, const Tensor& status, int64_t max_ctas, double act_alpha,
-            double act_limit) {
+            double act_limit, bool w_ready) {
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 2, "gemm: 2-D CUDA tensors");
   TORCH_CHECK(a.scalar_type() == w.scalar_type(), "gemm: dtype mismatch");
   const bool fp8 = a.scalar_type() == at::kFloat8_e4m3fn;
@@ -181,7 +181,7 @@ Tensor gemm(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& bias,
   check(b200_gemm(a.data_ptr(), w.data_ptr(), c.data_ptr(), bias_p, res_p, M, N, K,
                   (int)a.stride(0), (int)w.stride(0), n_out, fp8 ? 1 : 0, out_fp32 ? 1 : 0,
                   (int)act, (int)bn, (int)splits, cluster_split ? 1 : 0, ws_p, cnt_p,
-                  status.data_ptr<int>(), (int)max_ctas, (float)act_alpha, (float)act_limit, cur_stream()),
+                  status.data_ptr<int>(), (int)max_ctas, (float)act_alpha, (float)act_limit, w_ready ? 1 : 0, cur_stream()),
         "gemm");
   return c;
 }
@@ -189,7 +189,7 @@ Tensor gemm(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& bias,
 // Same contract as gemm() without split-K, run by CTA pairs (gemm/gemm_pair.cu); bn: rows of a per tile, 0 by rule.
 Tensor gemm_pair(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& bias,
                  const c10::optional<Tensor>& residual, bool out_fp32, int64_t act, int64_t bn,
-                 const Tensor& status, int64_t max_ctas, double act_alpha, double act_limit) {
+                 const Tensor& status, int64_t max_ctas, double act_alpha, double act_limit, bool w_ready) {
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 2, "gemm_pair: 2-D CUDA tensors");
   TORCH_CHECK(a.scalar_type() == w.scalar_type(), "gemm_pair: dtype mismatch");
   const bool fp8 = a.scalar_type() == at::kFloat8_e4m3fn;
@@ -216,7 +216,7 @@ Tensor gemm_pair(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& 
   check(b200_gemm_pair(a.data_ptr(), w.data_ptr(), c.data_ptr(), bias_p, res_p, M, N, K,
                        (int)a.stride(0), (int)w.stride(0), n_out, fp8 ? 1 : 0, out_fp32 ? 1 : 0,
                        (int)act, (int)bn, status.data_ptr<int>(), (int)max_ctas,
-                       (float)act_alpha, (float)act_limit, cur_stream()),
+                       (float)act_alpha, (float)act_limit, w_ready ? 1 : 0, cur_stream()),
         "gemm_pair");
   return c;
 }
@@ -224,7 +224,7 @@ Tensor gemm_pair(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& 
 // Same contract as gemm() for at most 128 bf16 rows: the weights are the tensor cores' M operand (gemm/gemm_stream.cu).
 Tensor gemm_stream(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& bias,
                    const c10::optional<Tensor>& residual, bool out_fp32, int64_t act, int64_t splits,
-                   const Tensor& status, int64_t max_ctas, double act_alpha, double act_limit) {
+                   const Tensor& status, int64_t max_ctas, double act_alpha, double act_limit, bool w_ready) {
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 2, "gemm_stream: 2-D CUDA tensors");
   TORCH_CHECK(a.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16, "gemm_stream: bf16 inputs");
   TORCH_CHECK(a.stride(1) == 1 && w.stride(1) == 1, "gemm_stream: K must be contiguous");
@@ -248,14 +248,14 @@ Tensor gemm_stream(const Tensor& a, const Tensor& w, const c10::optional<Tensor>
   }
   check(b200_gemm_stream(a.data_ptr(), w.data_ptr(), c.data_ptr(), bias_p, res_p, M, N, K, (int)a.stride(0),
                          (int)w.stride(0), n_out, out_fp32 ? 1 : 0, (int)act, (int)splits, status.data_ptr<int>(),
-                         (int)max_ctas, (float)act_alpha, (float)act_limit, cur_stream()),
+                         (int)max_ctas, (float)act_alpha, (float)act_limit, w_ready ? 1 : 0, cur_stream()),
         "gemm_stream");
   return c;
 }
 
 // c[t, g] = a[t, g] w[g]^T: a [T, G, K] and c [T, G, N] views with any row and group pitch, w [G, N, K].  False (nothing
 // done): pitches or alignments that the kernel does not take.
-bool batched_gemm(const Tensor& a, const Tensor& w, Tensor c, int64_t tn, const Tensor& status) {
+bool batched_gemm(const Tensor& a, const Tensor& w, Tensor c, int64_t tn, const Tensor& status, bool w_ready) {
   CHECK_CUDA_BF16(a);
   CHECK_CUDA_BF16(w);
   CHECK_CUDA_BF16(c);
@@ -266,7 +266,7 @@ bool batched_gemm(const Tensor& a, const Tensor& w, Tensor c, int64_t tn, const 
   c10::cuda::CUDAGuard guard(a.device());
   const int rc = b200_batched_gemm(a.data_ptr(), w.data_ptr(), c.data_ptr(), (int)a.size(0), (int)a.size(1), (int)w.size(1),
                                    (int)w.size(2), a.stride(0), a.stride(1), c.stride(0), c.stride(1), (int)tn,
-                                   status.data_ptr<int>(), cur_stream());
+                                   status.data_ptr<int>(), w_ready ? 1 : 0, cur_stream());
   if (rc == 1) return false;
   check(rc, "batched_gemm");
   return true;

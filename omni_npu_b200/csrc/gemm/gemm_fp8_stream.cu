@@ -40,6 +40,7 @@ constexpr int MAX_EXPERTS = 512;
 struct Fp8StreamParams {
   int M, N, k_slabs;
   int tn, box, stages, splits, num_n_tiles, num_experts, scale_rows, up_scale_row0, ldc, out_fp32, swiglu;
+  int w_ready;                // dense: no kernel still running writes W, its first ring goes ahead of the wait
   const float* a_scales;      // [rows, k_slabs]
   const float* w_scales;      // [E][scale_rows, k_slabs]
   void* C;
@@ -154,8 +155,8 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
   const int k_begin = rank * per, k_end = min(p.k_slabs, k_begin + per);
 
   pdl_trigger();
-  // dense: the weights are written by no kernel ahead of this one, their first ring is under way before the wait
-  const bool early = !GROUPED && threadIdx.x == 0;
+  // weights that no kernel ahead of this one writes (the caller says so): their first ring is under way before the wait
+  const bool early = !GROUPED && p.w_ready && threadIdx.x == 0;
   if (!early) pdl_wait();
 
   if (warp == 0) {
@@ -165,7 +166,7 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
       uint32_t phase = 0;
       bool ok = true;
       Fp8StreamTile tile;
-      if constexpr (!GROUPED) {
+      if (early) {
         if (fp8_stream_tile<GROUPED>(p, prefix, first_row, t_first, cursor, tile)) {
           const uint32_t bytes = W_BYTES + (tile.rows + p.box - 1) / p.box * p.box * SLAB;
           for (; preloaded < p.stages && k_begin + preloaded < k_end; ++preloaded) {
@@ -421,10 +422,10 @@ static int fp8_stream_splits(int n_tiles, int k_slabs) {
 
 using namespace b200;
 
-// The operands of b200_gemm_fp8_block, at most 64 rows.
+// The operands of b200_gemm_fp8_block, at most 64 rows.  w_ready: see Fp8StreamParams.
 extern "C" int b200_gemm_fp8_stream(const void* A, const float* a_scales, const void* W, const float* w_scales, void* C,
                                     const void* bias, const void* residual, int M, int N, int K, int lda, int ldw, int ldc,
-                                    int out_fp32, int* status, int max_ctas, cudaStream_t stream) {
+                                    int out_fp32, int* status, int max_ctas, int w_ready, cudaStream_t stream) {
   using namespace fp8s;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (M > MAX_ROWS || (K % SLAB) != 0) return -10;
@@ -440,6 +441,7 @@ extern "C" int b200_gemm_fp8_stream(const void* A, const float* a_scales, const 
   p.scale_rows = p.num_n_tiles;
   p.ldc = ldc;
   p.out_fp32 = out_fp32;
+  p.w_ready = w_ready;
   p.a_scales = a_scales;
   p.w_scales = w_scales;
   p.C = C;

@@ -49,6 +49,7 @@ struct PairParams {
   int slab_elems;          // elements of K in 128 bytes
   int width;               // dense: rows of A per tile
   int x_rows, stages;      // rows of A that a stage has room for, in each CTA; stages of the ring
+  int w_ready;             // dense: no kernel still running writes W, its first ring goes ahead of the wait
   float act_alpha, act_limit;
   void* C;
   const __nv_bfloat16* bias;
@@ -176,8 +177,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   const uint32_t tmem_base = *tmem_slot;
   const int t_first = blockIdx.x >> 1, t_stride = gridDim.x >> 1;
   pdl_trigger();
-  // dense: the weights are written by no kernel ahead of this one, their first ring is under way before the wait
-  const bool early = !GROUPED && threadIdx.x == 0;
+  // weights that no kernel ahead of this one writes (the caller says so): their first ring is under way before the wait
+  const bool early = !GROUPED && p.w_ready && threadIdx.x == 0;
   if (!early) pdl_wait();
 
   if (warp == 0) {
@@ -203,7 +204,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             tma_load_2d_pair(dst, &tm_w, bar, (k * KSUB + j) * p.slab_elems, tile.n0 + rank * 128);
         }
       };
-      if constexpr (!GROUPED) {
+      if (early) {
         if (pair_tile<GROUPED>(p, prefix, first_row, t_first, cursor, tile))
           for (; preloaded < p.stages && preloaded < p.k_iters; ++preloaded) {
             expect(preloaded);
@@ -449,9 +450,10 @@ static int pair_ctas(int max_ctas) {
 using namespace b200;
 
 // Same contract as b200_gemm (no split-K).  width: rows of A per tile, a multiple of 32 up to 256; 0: by rule.
+// w_ready: see PairParams.
 extern "C" int b200_gemm_pair(const void* A, const void* W, void* C, const void* bias, const void* residual, int M, int N,
                               int K, int lda, int ldw, int ldc, int dtype_fp8, int out_fp32, int act, int width,
-                              int* status, int max_ctas, float act_alpha, float act_limit, cudaStream_t stream) {
+                              int* status, int max_ctas, float act_alpha, float act_limit, int w_ready, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (width != 0 && (width < 32 || width > 256 || (width % 32) != 0)) return -10;
   if (act_is_gated(act) && (N % 16) != 0) return -11;
@@ -464,6 +466,7 @@ extern "C" int b200_gemm_pair(const void* A, const void* W, void* C, const void*
   p.x_rows = (p.width / 2 + pair::BOX - 1) / pair::BOX * pair::BOX;
   p.ldc = ldc;
   p.out_fp32 = out_fp32;
+  p.w_ready = w_ready;
   p.act = act;
   p.act_alpha = act_alpha;
   p.act_limit = act_limit;

@@ -49,6 +49,7 @@ struct StreamParams {
   int num_experts;        // groups (grouped, batched)
   long long c_group;      // batched: elements of C between groups
   int ldc, out_fp32, act;
+  int w_ready;            // no kernel still running writes W: its first ring goes ahead of the wait
   float act_alpha, act_limit;
   void* C;
   const __nv_bfloat16* bias;
@@ -199,8 +200,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   const int k_begin = rank * per, k_end = min(p.k_slabs, k_begin + per);
 
   pdl_trigger();
-  // the weights are written by no kernel ahead of this one: their first ring is under way before the wait
-  const bool early = !GROUPED && threadIdx.x == 0;
+  // weights that no kernel ahead of this one writes (the caller says so): their first ring is under way before the wait
+  const bool early = !GROUPED && p.w_ready && threadIdx.x == 0;
   if (!early) pdl_wait();
 
   if (warp == 0) {
@@ -210,7 +211,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       uint32_t phase = 0;
       bool ok = true;
       StreamTile tile;
-      if constexpr (!GROUPED) {
+      if (early) {
         if (stream_tile<MODE>(p, prefix, first_row, t_first, cursor, tile)) {
           const uint32_t bytes = W_BYTES + (tile.rows + p.box - 1) / p.box * p.box * 128;
           for (; preloaded < p.stages && k_begin + preloaded < k_end; ++preloaded) {
@@ -454,9 +455,10 @@ static int launch_stream(const CUtensorMap& tw, const CUtensorMap& tx, const Str
 using namespace b200;
 
 // A [M <= 128, K] (pitch lda), W [N, K] (pitch ldw), C [M, N, or N / 2 with a gated activation].  splits 0: by rule.
+// w_ready: see StreamParams.
 extern "C" int b200_gemm_stream(const void* A, const void* W, void* C, const void* bias, const void* residual, int M,
                                 int N, int K, int lda, int ldw, int ldc, int out_fp32, int act, int splits, int* status,
-                                int max_ctas, float act_alpha, float act_limit, cudaStream_t cu_stream) {
+                                int max_ctas, float act_alpha, float act_limit, int w_ready, cudaStream_t cu_stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (M > 128) return -10;
   if (act_is_gated(act) && ((N % 16) != 0 || out_fp32 || residual)) return -11;
@@ -475,6 +477,7 @@ extern "C" int b200_gemm_stream(const void* A, const void* W, void* C, const voi
   p.ldc = ldc;
   p.out_fp32 = out_fp32;
   p.act = act;
+  p.w_ready = w_ready;
   p.act_alpha = act_alpha;
   p.act_limit = act_limit;
   p.C = C;
@@ -543,7 +546,7 @@ extern "C" int b200_grouped_gemm_stream(const void* A, const void* W, void* C, c
 // C[t, g, :] = A[t, g, :] W[g]^T for T rows of G groups: A and C with pitches of their own between rows and groups (in
 // elements), W [G, N, K].  Returns 1 (nothing done) for pitches and alignments that the copies do not take.
 extern "C" int b200_batched_gemm(const void* A, const void* W, void* C, int T, int G, int N, int K, long long a_row,
-                                 long long a_group, long long c_row, long long c_group, int tn, int* status,
+                                 long long a_group, long long c_row, long long c_group, int tn, int* status, int w_ready,
                                  cudaStream_t cu_stream) {
   if (T <= 0 || G <= 0 || N <= 0 || K <= 0) return 0;
   if (tn != 16 && tn != 32 && tn != 64 && tn != 128) return -10;
@@ -562,6 +565,7 @@ extern "C" int b200_batched_gemm(const void* A, const void* W, void* C, int T, i
   p.splits = 1;
   p.num_experts = G;
   p.c_group = c_group;
+  p.w_ready = w_ready;
   p.ldc = static_cast<int>(c_row);
   p.C = C;
   p.status = status;

@@ -80,6 +80,7 @@ struct GemmParams {
   float act_alpha;        // constants of the clamped form
   float act_limit;
   int num_experts;        // grouped: number of local experts (0 = dense)
+  int w_ready;            // dense: no kernel still running writes W, its first ring goes ahead of the wait
   int cluster_split;      // 1: the `splits` CTAs of a cluster share one tile and reduce over DSMEM
   void* C;
   const __nv_bfloat16* bias;       // [N] or null
@@ -288,12 +289,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   volatile int* abort_flag = s_flags;
   const int groups = p.stages / p.ksub;   // barrier pairs in use
-  // Dependent launch: the next kernel of the stream may start its own prologue now.  This
-  // kernel's weights are written by no earlier kernel, so the producer thread of a dense
+  // Dependent launch: the next kernel of the stream may start its own prologue now.  Where the
+  // caller says that no kernel ahead writes the weights, the producer thread of a dense
   // problem streams the first ring of weight slabs before it waits for the kernels ahead;
   // every other thread waits here, before it reads anything those kernels produced.
   pdl_trigger();
-  const bool w_preload = !GROUPED && threadIdx.x == 0;
+  const bool w_preload = !GROUPED && p.w_ready && threadIdx.x == 0;
   uint32_t ar_epoch = 0;
   long long ar_slot_off = 0;
   if (!w_preload) {
@@ -314,7 +315,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       long long preloaded = 0;     // leading barrier groups whose weight slabs are already in flight
       bool ok = true;
       TileCoord tc;
-      if constexpr (!GROUPED) {
+      if (w_preload) {
         int c0 = 0;
         if (decode_tile<GROUPED>(p, s_tile_prefix, total_mn_tiles, t_first, cta_rank, c0, tc)) {
           int g = 0;
@@ -1403,16 +1404,17 @@ static int gemm_impl(const void* A, const void* W, void* C, const void* bias, co
                      int splits, int cluster_split, void* workspace, int* counters, int* status,
                      int max_ctas, cudaStream_t stream, const float* a_scales, const float* w_scales,
                      const ArArgs* ar = nullptr, const struct AgArgs* ag = nullptr,
-                     const struct RsArgs* rs = nullptr, float act_alpha = 0.f, float act_limit = 0.f);
+                     const struct RsArgs* rs = nullptr, float act_alpha = 0.f, float act_limit = 0.f, int w_ready = 1);
 
+// w_ready: see GemmParams (the fused collectives below take parameters of a loaded model as W: always ready).
 extern "C" int b200_gemm(const void* A, const void* W, void* C, const void* bias,
                          const void* residual, int M, int N, int K, int lda, int ldw, int ldc,
                          int dtype_fp8, int out_fp32, int swiglu, int BN, int splits,
                          int cluster_split, void* workspace, int* counters, int* status,
-                         int max_ctas, float act_alpha, float act_limit, cudaStream_t stream) {
+                         int max_ctas, float act_alpha, float act_limit, int w_ready, cudaStream_t stream) {
   return gemm_impl(A, W, C, bias, residual, M, N, K, lda, ldw, ldc, dtype_fp8, out_fp32, swiglu, BN, splits,
                    cluster_split, workspace, counters, status, max_ctas, stream, nullptr, nullptr, nullptr, nullptr,
-                   nullptr, act_alpha, act_limit);
+                   nullptr, act_alpha, act_limit, w_ready);
 }
 
 // Quantised product with per-row (a_scales[M]) and per-column (w_scales[N]) scales applied to
@@ -1420,11 +1422,11 @@ extern "C" int b200_gemm(const void* A, const void* W, void* C, const void* bias
 extern "C" int b200_gemm_scaled(const void* A, const void* W, void* C, const float* a_scales,
                                 const float* w_scales, const void* bias, const void* residual, int M, int N,
                                 int K, int lda, int ldw, int ldc, int kind, int out_fp32, int BN, int* status,
-                                int max_ctas, cudaStream_t stream) {
+                                int max_ctas, int w_ready, cudaStream_t stream) {
   if (kind != 1 && kind != 2) return -15;
   if (a_scales == nullptr || w_scales == nullptr) return -16;
   return gemm_impl(A, W, C, bias, residual, M, N, K, lda, ldw, ldc, kind, out_fp32, 0, BN, 1, 0, nullptr,
-                   nullptr, status, max_ctas, stream, a_scales, w_scales);
+                   nullptr, status, max_ctas, stream, a_scales, w_scales, nullptr, nullptr, nullptr, 0.f, 0.f, w_ready);
 }
 
 struct RsArgs {
@@ -1459,7 +1461,7 @@ static int gemm_impl(const void* A, const void* W, void* C, const void* bias, co
                      int splits, int cluster_split, void* workspace, int* counters, int* status,
                      int max_ctas, cudaStream_t stream, const float* a_scales, const float* w_scales,
                      const ArArgs* ar, const struct AgArgs* ag, const struct RsArgs* rs, float act_alpha,
-                     float act_limit);
+                     float act_limit, int w_ready);
 
 // Row-parallel projection of a tensor-parallel layer in ONE kernel: C = RMSNorm(residual +=
 // sum over ranks of (A @ W^T)) * norm_w  (norm_w null: C = sum (+ residual), residual untouched).
@@ -1552,7 +1554,8 @@ static int gemm_impl(const void* A, const void* W, void* C, const void* bias, co
                      int N, int K, int lda, int ldw, int ldc, int dtype_fp8, int out_fp32, int swiglu, int BN,
                      int splits, int cluster_split, void* workspace, int* counters, int* status,
                      int max_ctas, cudaStream_t stream, const float* a_scales, const float* w_scales,
-                     const ArArgs* ar, const AgArgs* ag, const RsArgs* rs, float act_alpha, float act_limit) {
+                     const ArArgs* ar, const AgArgs* ag, const RsArgs* rs, float act_alpha, float act_limit,
+                     int w_ready) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const int eb = dtype_fp8 ? 1 : 2;
   if (BN < 16 || BN > 256 || (BN % 16) != 0) return -10;
@@ -1585,6 +1588,7 @@ static int gemm_impl(const void* A, const void* W, void* C, const void* bias, co
   p.act_alpha = act_alpha;
   p.act_limit = act_limit;
   p.num_experts = 0;
+  p.w_ready = w_ready;
   p.C = C;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.residual = static_cast<const __nv_bfloat16*>(residual);

@@ -55,7 +55,7 @@ class VocabParallelEmbedding(nn.Module):
 class ParallelLMHead(VocabParallelEmbedding):
     def compute_logits(self, hidden: torch.Tensor, embedding_bias: Optional[torch.Tensor] = None) -> torch.Tensor:
         """hidden [B,H] -> logits [B, vocab] in fp32."""
-        logits = ops.gemm(hidden, self.weight, out_dtype=torch.float32)
+        logits = ops.gemm(hidden, self.weight, out_dtype=torch.float32, w_ready=True)
         if self.group.world_size > 1:
             logits = self.group.all_gather(logits, dim=-1)
         logits = logits[:, : self.vocab_size]

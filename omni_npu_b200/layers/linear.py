@@ -88,7 +88,7 @@ class UnquantizedLinearMethod:
               residual: Optional[torch.Tensor] = None, swiglu: bool = False,
               out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
         return ops.gemm(x, layer.weight, bias, residual, out_dtype, swiglu,
-                        act=getattr(layer, "gated_act", ops.SILU))
+                        act=getattr(layer, "gated_act", ops.SILU), w_ready=True)
 
 
 class Fp8BlockLinearMethod:
@@ -112,7 +112,7 @@ class Fp8BlockLinearMethod:
     def apply(self, layer, x, bias, residual=None, swiglu=False, out_dtype=None):
         from .quant_fp8 import fp8_block_gemm
         return fp8_block_gemm(x, layer.weight, layer.weight_scale_inv, bias, residual, self.block,
-                              swiglu=swiglu, out_dtype=out_dtype)
+                              swiglu=swiglu, out_dtype=out_dtype, w_ready=True)
 
 
 # -------------------------------------------------------------------- layers

@@ -67,7 +67,7 @@ class UnaryMLP(nn.Module):
                                            prefix=f"{prefix}.down_proj", group=group, reduce_results=reduce_results)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return self.down_proj(ops.gemm(x, self.up_proj.weight, unary=self.act))
+        return self.down_proj(ops.gemm(x, self.up_proj.weight, unary=self.act, w_ready=True))
 
 
 class XieluMLP(nn.Module):
@@ -91,4 +91,4 @@ class XieluMLP(nn.Module):
         self.constants = (p, 0.5 + q)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return self.down_proj(ops.gemm(x, self.up_proj.weight, xielu=self.constants))
+        return self.down_proj(ops.gemm(x, self.up_proj.weight, xielu=self.constants, w_ready=True))

@@ -43,15 +43,17 @@ def quantize_weight_per_channel(w: torch.Tensor):
 
 
 def int8_linear(x: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor, bias: Optional[torch.Tensor] = None,
-                residual: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+                residual: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
+                w_ready: bool = False) -> torch.Tensor:
     if isinstance(x, tuple):
         # already quantised by the producing kernel (norm + quant, SwiGLU + quant): (q [T,K], scale [T])
         xq, xs = x
-        return ops.gemm_scaled(xq, w_q, xs, w_scale, bias, residual, out_dtype or torch.bfloat16)
+        return ops.gemm_scaled(xq, w_q, xs, w_scale, bias, residual, out_dtype or torch.bfloat16, w_ready=w_ready)
     shape = x.shape
     x2 = x.reshape(-1, shape[-1])
     xq, xs = ops.quant_int8_per_token(x2)
-    y = ops.gemm_scaled(xq, w_q, xs, w_scale, bias, residual, out_dtype or (x.dtype if x.dtype.itemsize > 1 else None))
+    y = ops.gemm_scaled(xq, w_q, xs, w_scale, bias, residual, out_dtype or (x.dtype if x.dtype.itemsize > 1 else None),
+                        w_ready=w_ready)
     return y.reshape(*shape[:-1], w_q.shape[0])
 
 
@@ -70,7 +72,7 @@ class W8A8Int8LinearMethod:
 
     def apply(self, layer, x, bias, residual=None, swiglu=False, out_dtype=None):
         y = int8_linear(x, layer.weight, layer.weight_scale.view(-1), bias, residual,
-                        torch.float32 if swiglu else out_dtype)
+                        torch.float32 if swiglu else out_dtype, w_ready=True)
         if swiglu:
             # gate/up rows are interleaved in groups of 8 (the fused bf16 epilogue's layout):
             # undo it on the product and apply the activation
@@ -91,7 +93,7 @@ class W8A8Int8MoEMethod:
         return q.view(w.shape), s.view(w.shape[0], w.shape[1])
 
     def apply_expert(self, x: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor) -> torch.Tensor:
-        return int8_linear(x, w_q, w_scale)
+        return int8_linear(x, w_q, w_scale, w_ready=True)
 
 
 # -------------------------------------------------------------------- config

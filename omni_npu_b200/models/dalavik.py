@@ -191,7 +191,8 @@ class TokenSide(nn.Module):
         self.gate, self.proj, self.norm = param(pad8(dim), width), param(width, pad8(dim)), param(width)
 
     def forward(self, h: torch.Tensor, ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
-        return ops.gemm(ops.gelu_rows(ops.gemm(h, self.gate), ids, table, self.offset, self.dim), self.proj)
+        gate = ops.gemm(h, self.gate, w_ready=True)
+        return ops.gemm(ops.gelu_rows(gate, ids, table, self.offset, self.dim), self.proj, w_ready=True)
 
 
 class DalavikLayer(nn.Module):

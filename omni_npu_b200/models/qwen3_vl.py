@@ -61,7 +61,7 @@ class VisionConfig:
 
 def _linear(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor]) -> torch.Tensor:
     if x.is_cuda and x.dtype == torch.bfloat16:
-        return ops.gemm(x, w, b)
+        return ops.gemm(x, w, b, w_ready=True)
     return F.linear(x, w, b)
 
 

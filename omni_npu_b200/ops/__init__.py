@@ -244,7 +244,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
          residual: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
          swiglu: bool = False, bn: int = 0, splits: int = 0, max_ctas: int = 0,
          pair: Optional[bool] = None, act=SILU, xielu: Optional[Tuple[float, float]] = None,
-         unary: Optional[str] = None) -> torch.Tensor:
+         unary: Optional[str] = None, w_ready: bool = False) -> torch.Tensor:
     """``a[M,K] @ w[N,K].T`` (+bias, +residual).  bf16 or float8_e4m3fn inputs,
     fp32 accumulation, bf16 (default) or fp32 output.  ``swiglu`` fuses
     silu(gate)*up for weights laid out by :func:`ref.interleave_gate_up`; ``act`` = (slope, limit)
@@ -255,7 +255,9 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
     ``splits`` > 1 forces split-K (as a thread-block cluster when it fits), a
     negative value forces the workspace variant with |splits| slices.
     ``pair`` selects the CTA-pair kernel (tiles over two SMs, ``bn`` rows of ``a`` each); by default it runs for
-    M >= PAIR_MIN_M, and for bf16 above PAIR_UNSPLIT_M where K is not split, when neither was asked for."""
+    M >= PAIR_MIN_M, and for bf16 above PAIR_UNSPLIT_M where K is not split, when neither was asked for.
+    ``w_ready``: no kernel that may still run writes ``w`` (a parameter of a loaded model), so that its first tiles may be
+    loaded while the kernels ahead finish; otherwise nothing is read before they have."""
     if not a.is_cuda:
         return ref.gemm(a, w, bias, residual, out_dtype, swiglu, act, xielu, unary)
     C = _core()
@@ -273,14 +275,14 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
     if pair:
         _count(1)
         return C.gemm_pair(a, w, bias, residual, out_dtype == torch.float32, kind[0], bn, st.status, max_ctas,
-                           kind[1], kind[2])
+                           kind[1], kind[2], w_ready)
     fused, gated = kind[0] != 0, kind[0] in (1, 2, 4, 7)
     if ((m < STREAM_ROWS or m <= STREAM_WIDE_ROWS and (n >= STREAM_WIDE_N or n < STREAM_NARROW_N))
             and a.dtype == torch.bfloat16 and bn == 0 and splits == 0
             and not (gated and (residual is not None or out_dtype == torch.float32))):
         _count(1)
         return C.gemm_stream(a, w, bias, residual, out_dtype == torch.float32, kind[0], 0, st.status, max_ctas, kind[1],
-                             kind[2])
+                             kind[2], w_ready)
     key = (m, n, k, a.dtype.itemsize, kind[0], bn, splits)
     plan = st.plans.get(key)
     if plan is None:
@@ -291,7 +293,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
             and psplits == 1:
         _count(1)
         return C.gemm_pair(a, w, bias, residual, out_dtype == torch.float32, kind[0], 0, st.status, max_ctas,
-                           kind[1], kind[2])
+                           kind[1], kind[2], w_ready)
     if library_small_m(m, bool(cluster), residual is None and not fused and bn == 0
                        and splits == 0 and a.dtype == torch.bfloat16 and out_dtype in (None, torch.bfloat16)):
         return torch.nn.functional.linear(a, w, bias)    # a library kernel: not counted as a launch of ours
@@ -300,7 +302,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
         ws, cnt = st.gemm_workspace(torch.cuda.current_stream(a.device).cuda_stream, ws_bytes, ncnt)
     _count(1)
     return C.gemm(a, w, bias, residual, out_dtype == torch.float32, kind[0], pbn, psplits,
-                  bool(cluster), ws, cnt, st.status, max_ctas, kind[1], kind[2])
+                  bool(cluster), ws, cnt, st.status, max_ctas, kind[1], kind[2], w_ready)
 
 
 def quant_int8_per_token(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -321,7 +323,7 @@ FP8_STREAM_GROUP_ROWS = 48
 
 def gemm_fp8_block(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor,
                    bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
-                   out_dtype: Optional[torch.dtype] = None, max_ctas: int = 0) -> torch.Tensor:
+                   out_dtype: Optional[torch.dtype] = None, max_ctas: int = 0, w_ready: bool = False) -> torch.Tensor:
     """Block-scaled e4m3 product: ``a_q`` [M,K] with one scale per (row, 128 columns), ``w_q`` [N,K]
     with one scale per 128 x 128 block; each 128-wide K block is scaled before accumulation."""
     if not a_q.is_cuda:
@@ -329,7 +331,8 @@ def gemm_fp8_block(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.Tensor, 
     st = device_state(a_q.device)
     _count(1)
     return _C().gemm_fp8_block(a_q, a_scale.contiguous(), w_q, w_scale.contiguous(), bias, residual,
-                               out_dtype == torch.float32, a_q.shape[0] <= FP8_STREAM_ROWS, st.status, max_ctas)
+                               out_dtype == torch.float32, a_q.shape[0] <= FP8_STREAM_ROWS, st.status, max_ctas,
+                               w_ready)
 
 
 def grouped_gemm_fp8_block(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor,
@@ -402,9 +405,11 @@ def silu_and_mul_quant(x: torch.Tensor, kind: str = "int8") -> Tuple[torch.Tenso
 
 def gemm_scaled(a_q: torch.Tensor, w_q: torch.Tensor, a_scale: torch.Tensor, w_scale: torch.Tensor,
                 bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
-                out_dtype: Optional[torch.dtype] = None, bn: int = 0, max_ctas: int = 0) -> torch.Tensor:
+                out_dtype: Optional[torch.dtype] = None, bn: int = 0, max_ctas: int = 0,
+                w_ready: bool = False) -> torch.Tensor:
     """``(a_q @ w_q.T) * a_scale[:, None] * w_scale[None, :]`` (+bias, +residual) for int8 or
-    e4m3 operands; integer products accumulate exactly in 32 bits on the tensor cores."""
+    e4m3 operands; integer products accumulate exactly in 32 bits on the tensor cores
+    (``w_ready`` as in :func:`gemm`)."""
     if not a_q.is_cuda:
         return ref.gemm_scaled(a_q, w_q, a_scale, w_scale, bias, residual, out_dtype)
     st = device_state(a_q.device)
@@ -413,7 +418,7 @@ def gemm_scaled(a_q: torch.Tensor, w_q: torch.Tensor, a_scale: torch.Tensor, w_s
         bn = 256 if n >= 2048 else (128 if n >= 128 else max(16, (n + 15) // 16 * 16))
     _count(1)
     return _C().gemm_scaled(a_q, w_q, a_scale.contiguous(), w_scale.reshape(-1).contiguous(), bias, residual,
-                            out_dtype == torch.float32, bn, st.status, max_ctas)
+                            out_dtype == torch.float32, bn, st.status, max_ctas, w_ready)
 
 
 @functools.lru_cache(maxsize=4096)
@@ -478,16 +483,16 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, expert_offsets: torch.Tensor,
     return y if out is None else out.copy_(y)
 
 
-def batched_gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+def batched_gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, w_ready: bool = False) -> torch.Tensor:
     """``out[t, g] = a[t, g] @ w[g].T`` for a [T, G, K] and out [T, G, N] with any pitch between rows and groups (views of
-    larger rows are written and read as they lie), w [G, N, K]."""
+    larger rows are written and read as they lie), w [G, N, K] (``w_ready`` as in :func:`gemm`)."""
     t, g, k = a.shape
     n = w.shape[1]
     if a.is_cuda and a.dtype == out.dtype == torch.bfloat16:
         # rows of A per tile: narrow ones while they are needed to fill the SMs
         tiles = g * -(-n // 128)
         tn = 32 if tiles * -(-t // 64) < 148 else 64 if t <= 64 else 128
-        if _core().batched_gemm(a, w, out, tn, device_state(a.device).status):
+        if _core().batched_gemm(a, w, out, tn, device_state(a.device).status, w_ready):
             _count(1)
             return out
     rows = a.transpose(0, 1).reshape(g * t, k).contiguous()

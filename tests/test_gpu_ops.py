@@ -236,6 +236,37 @@ def test_grouped_gemm_tiles(counts, n, k):
     ops.check_status()
 
 
+@pytest.mark.parametrize("m,n,k", [(5, 256, 4096), (128, 20480, 1024), (300, 20480, 1024), (100, 4096, 4096), (1100, 2048, 1024)])
+def test_products_wait_for_weights_written_right_ahead(m, n, k):
+    """An operand that the kernel ahead writes, in memory that held another one: read once that kernel is through."""
+    torch.manual_seed(m)
+    a = torch.randn(m, k, device=DEV, dtype=torch.bfloat16)
+    q, s = ops.quant_fp8_1x128(a)
+    res = torch.randn(m, n, device=DEV, dtype=torch.bfloat16)
+    ones, scale = torch.ones(k, device=DEV, dtype=torch.bfloat16), torch.rand(-(-n // 128), k // 128, device=DEV)
+    row, col = torch.rand(m, device=DEV), torch.rand(n, device=DEV)
+    sources = [torch.randn(n, k, device=DEV, dtype=torch.bfloat16) for _ in range(4)]
+    calls = [(lambda x: ops.rms_norm(x, ones, 1e-6), lambda w: ops.gemm(a, w)),
+             (lambda x: ops.rms_norm(x, ones, 1e-6), lambda w: ops.gemm(a, w, residual=res)),
+             (lambda x: ops.quant_fp8_1x128(x)[0], lambda w: ops.gemm_fp8_block(q, s, w, scale)),
+             (lambda x: ops.quant_fp8_1x128(x)[0], lambda w: ops.gemm_scaled(q, w, row, col))]
+    for write, product in calls:
+        for i in range(12):
+            w = write(sources[i % 4])
+            got = product(w)
+            torch.cuda.synchronize()
+            assert torch.equal(got, product(w))
+            del w, got
+    h = torch.randn(64, 8192, device=DEV, dtype=torch.bfloat16)
+    batched = torch.randn(3, 16, 128, device=DEV, dtype=torch.bfloat16)
+    for i in range(12):
+        w = ops.rms_norm(sources[i % 4].view(-1, 1024)[:1024], ones[:1024], 1e-6).view(16, 512, 128)
+        got = ops.batched_gemm(batched, w, h.new_empty(3, 16, 512))
+        torch.cuda.synchronize()
+        assert torch.equal(got, ops.batched_gemm(batched, w, h.new_empty(3, 16, 512)))
+        del w, got
+
+
 def test_gemm_fp8_plain():
     torch.manual_seed(4)
     m, n, k = 256, 512, 1024
