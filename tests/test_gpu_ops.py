@@ -267,6 +267,24 @@ def test_products_wait_for_weights_written_right_ahead(m, n, k):
         del w, got
 
 
+@pytest.mark.parametrize("rows,h", [(1, 1024), (40, 4096), (3, 16384)])
+def test_norm_waits_for_weights_written_right_ahead(rows, h):
+    torch.manual_seed(h)
+    x, ones = torch.randn(rows, h, device=DEV, dtype=torch.bfloat16), torch.ones(h, device=DEV, dtype=torch.bfloat16)
+    sources = [torch.randn(1, h, device=DEV, dtype=torch.bfloat16) for _ in range(4)]
+    for i in range(24):
+        w = ops.rms_norm(sources[i % 4], ones, 1e-6)[0]
+        got, res = ops.rms_norm(x, w, 1e-6), x.clone()
+        added = ops.fused_add_rms_norm(x, res, ops.rms_norm(sources[(i + 1) % 4], ones, 1e-6)[0], 1e-6)
+        torch.cuda.synchronize()
+        exact = x.double() * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-6)
+        # one rounding to bf16; of the doubled row nothing changes but the weight of eps
+        _close(got, (exact * w.double()).float(), 1e-3, 2 ** -8)
+        other = ops.rms_norm(sources[(i + 1) % 4], ones, 1e-6)[0]
+        _close(added, (exact * other.double()).float(), 1e-3, 2 ** -8)
+        del w, got, added, other
+
+
 def test_gemm_fp8_plain():
     torch.manual_seed(4)
     m, n, k = 256, 512, 1024
