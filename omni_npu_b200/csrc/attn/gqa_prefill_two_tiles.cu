@@ -223,7 +223,7 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
         __syncwarp();
         for (int l = lane; l < nboxes * C::QK_SLABS; l += 32) {
           if constexpr (FLAT) {
-            // (rows past the sequence are masked, rows past the end read as zero)
+            // (keys past the sequence are masked, its values' rows cleared below; rows past the end read as zero)
             uint8_t* dst = smem + C::OFF_K + ks * C::K_BYTES + l * SLAB;
             if (l < 2)
               tma_load_2d(dst, &tm_k, &k_full[ks], it.h[0] * 256 + l * 64, first + n0);
@@ -240,20 +240,6 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
         if (v_loads >= VS) ok = !*abort_flag && mbar_wait(&v_empty[vs], ((v_loads / VS) - 1) & 1);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        // the product reads whole groups of 16 keys, and rows past the sequence would count if they were infinite or NaN
-        // (P is zero there): what no copy fills, with pages of 8 keys, is cleared; rows of other sequences never take part
-        {
-          const int filled = nboxes * box_rows, missing = ((min(BN, it.kv_len - n0) + 15) & ~15) - filled;
-          if (missing > 0) {
-            for (int i = lane; i < missing * 16; i += 32) {
-              const int sl = i / (missing * 8), at = i % (missing * 8);
-              *reinterpret_cast<uint4*>(smem + C::OFF_V + vs * V_BYTES + sl * SLAB + filled * 128 + at * 16) =
-                  make_uint4(0u, 0u, 0u, 0u);
-            }
-            fence_proxy_async();
-            __syncwarp();
-          }
-        }
         if (lane == 0) mbar_arrive_expect_tx(&v_full[vs], static_cast<uint32_t>(nboxes * box_rows * 128) * 2);
         __syncwarp();
         for (int l = lane; l < nboxes * 2; l += 32) {
@@ -347,11 +333,13 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
     const uint32_t lanes = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t s_col = tmem_base + lanes + COL_S + t * 128, o_col = tmem_base + lanes + COL_O + t * 128;
     const float scale = p.scale_log2;
-    uint32_t sc = 0, oc = 0;
+    uint32_t sc = 0, oc = 0, v_first = 0;                  // v_first: value tiles of the items before
     bool ok = true;
     for (int idx = blockIdx.x; ok && idx < g.items; idx += gridDim.x) {
       const TwoTileItem it = two_tile_item(idx, g, p);
       const int n = t ? it.n[1] : it.n[0], m0 = t ? it.m0[1] : it.m0[0], h = t ? it.h[1] : it.h[0];
+      const uint32_t v_item = v_first;
+      v_first += it.n_max;
       if (n == 0) continue;
       const int row_lo = it.ctx + m0 + quarter * 32;      // smallest position in this warp
       const int limit = p.causal ? min(it.kv_len - 1, it.ctx + m0 + r) : it.kv_len - 1;    // last key this row sees
@@ -367,6 +355,20 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
         for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(s_col + c * 32, sv[c]);
         tmem_ld_wait();
         const int n0 = j * BN;
+        // The second product reads whole groups of 16 keys.  Value rows past the sequence in the last one (the rest of a
+        // page, another sequence's rows, what an earlier tile left) would count if they were infinite or NaN, although P
+        // is zero there: the tile that the product comes first for clears them once they have landed.
+        const int left = it.kv_len - n0;
+        if (left < BN && (left & 15) != 0 && (t == 0 || j >= it.n[0])) {
+          const uint32_t v = v_item + j;
+          ok = __all_sync(0xffffffffu, mbar_wait(&v_full[v % VS], (v / VS) & 1));
+          if (!ok) break;
+          const int missing = 16 - (left & 15);
+          for (int i = r; i < missing * 16; i += BM)
+            *reinterpret_cast<uint4*>(smem + C::OFF_V + (v % VS) * V_BYTES + (i & 8 ? SLAB : 0) + (left + (i >> 4)) * 128 +
+                                      (i & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+          fence_proxy_async();
+        }
         // tiles that lie entirely below the diagonal and inside the sequence need no mask
         if (!(n0 + BN <= it.kv_len && (!p.causal || n0 + BN - 1 <= row_lo))) {
           const int last = limit - n0;

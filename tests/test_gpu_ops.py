@@ -728,6 +728,56 @@ def test_prefill_keeps_other_sequences_nans_out(bs, dqk):
     _close(out[tail], want, 2e-2, 2e-2)
 
 
+@pytest.mark.parametrize("bs", [8, 16, 64, 128])
+@pytest.mark.parametrize("dqk,hq,hk", [(128, 8, 2), (128, 3, 1), (192, 4, 4)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_prefill_keeps_the_rest_of_the_last_page_out(bs, dqk, hq, hk, causal):
+    """What an earlier owner left behind a sequence's last key takes no part, be it infinite or NaN."""
+    lens, new = [3, 17, 133, 250, 129, 8, 260, 120], [3, 16, 133, 1, 129, 8, 200, 2]
+    q, kc, vc, bt, cu, sl = _paged_setup(lens, new, hq, hk, dqk, bs, dv=128, seed=bs)
+    want = ref.paged_attention(q, kc, vc, bt, cu, sl, hq, dqk ** -0.5, causal, 0)
+    for i, n in enumerate(lens):
+        if n % bs:
+            last = int(bt[i, n // bs])
+            kc[last, :, n % bs:], vc[last, :, n % bs:] = float("nan"), float("nan") if i % 2 else float("-inf")
+    got = ops.gqa_prefill(q.to(DEV), kc.to(DEV), vc.to(DEV), bt.to(DEV), cu.to(DEV), sl.to(DEV), len(lens), max(new), hq,
+                          dqk ** -0.5, causal)
+    # P and the result are rounded to bf16 (2 ** -9 each) of values up to about 4
+    _close(got, want, 2e-2, 2e-2)
+
+
+@pytest.mark.parametrize("page", [8, 24])
+def test_mla_prefill_keeps_other_sequences_out(page):
+    """Sequences that start at any page, each followed by one with NaN and infinite values."""
+    torch.manual_seed(page)
+    h, lens, new = 2, [8, 3, 133, 40, 250, 5, 129], [8, 3, 133, 40, 20, 5, 129]
+    starts = [0]
+    for n in lens:
+        starts.append(starts[-1] + -(-n // page) * page)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    kv = torch.randn(starts[-1], h, 256, device=DEV, dtype=torch.bfloat16)
+    lat = torch.randn(starts[-1], 576, device=DEV, dtype=torch.bfloat16)
+    q = torch.randn(sum(new), h, 192, device=DEV, dtype=torch.bfloat16)
+    cu = torch.tensor([0] + new).cumsum(0)
+    args = (cu.to(**i32), torch.tensor(lens, **i32), len(new), max(new), 192 ** -0.5)
+    for sound in range(2):                       # of every two neighbours one is sound
+        bad = kv.clone()
+        for i, n in enumerate(lens):
+            bad[starts[i] + n: starts[i + 1]] = float("nan")
+            if i % 2 != sound:
+                bad[starts[i]: starts[i + 1]] = float("nan") if i % 4 < 2 else float("inf")
+        out = ops.mla_prefill(q, bad, lat[:, 512:], torch.tensor(starts[:-1], **i32), *args)
+        for i, n in enumerate(lens):
+            if i % 2 != sound:
+                continue
+            rows = slice(starts[i], starts[i] + n)
+            k = torch.cat([kv[rows, :, :128], lat[rows, None, 512:].expand(-1, h, -1)], -1).double()
+            s = torch.einsum("qhd,khd->hqk", q[cu[i]: cu[i + 1]].double(), k) * 192 ** -0.5
+            hidden = torch.arange(n, device=DEV)[None] > n - new[i] + torch.arange(new[i], device=DEV)[:, None]
+            want = torch.einsum("hqk,khd->qhd", s.masked_fill(hidden, -math.inf).softmax(-1), kv[rows, :, 128:].double())
+            _close(out[cu[i]: cu[i + 1]], want.flatten(1).float(), 2e-2, 2 ** -7)
+
+
 @pytest.mark.parametrize("t,hq,hk,d,rot,neox", [(1, 32, 4, 128, 128, True), (37, 3, 1, 16, 16, True), (300, 5, 2, 64, 64, True),
                                                 (9, 2, 2, 256, 256, True), (3, 1, 1, 512, 512, True),
                                                 (17, 4, 2, 128, 64, True), (5, 4, 2, 96, 96, True), (6, 4, 2, 128, 128, False)])
