@@ -109,7 +109,7 @@ __device__ __forceinline__ TwoTileItem two_tile_item(int idx, const TwoTileGrid&
     it.h[i] = g.by_head ? 2 * hu + i : hu;
     it.m0[i] = g.by_head ? mu * two::BM : (2 * mu + i) * two::BM;
     const int hi = p.causal ? min(it.kv_len, it.ctx + it.m0[i] + two::BM) : it.kv_len;
-    it.n[i] = it.m0[i] < it.q_len ? (hi + two::BN - 1) / two::BN : 0;
+    it.n[i] = it.m0[i] < it.q_len ? (max(hi, 0) + two::BN - 1) / two::BN : 0;
   }
   it.n_max = max(it.n[0], it.n[1]);
   it.kvh = it.h[0] / (p.Hq / p.Hk);
@@ -340,7 +340,17 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
       const int n = t ? it.n[1] : it.n[0], m0 = t ? it.m0[1] : it.m0[0], h = t ? it.h[1] : it.h[0];
       const uint32_t v_item = v_first;
       v_first += it.n_max;
-      if (n == 0) continue;
+      if (n == 0) {
+        // rows that see no key: zero, of weight zero
+        if (m0 + r < it.q_len) {
+          const long long row = it.q_begin + m0 + r;
+          uint4* dst = reinterpret_cast<uint4*>(p.out + row * p.out_stride + static_cast<long long>(h) * DV);
+#pragma unroll
+          for (int i = 0; i < DV / 8; ++i) dst[i] = make_uint4(0u, 0u, 0u, 0u);
+          if (p.lse) p.lse[row * p.Hq + h] = -INFINITY;
+        }
+        continue;
+      }
       const int row_lo = it.ctx + m0 + quarter * 32;      // smallest position in this warp
       const int limit = p.causal ? min(it.kv_len - 1, it.ctx + m0 + r) : it.kv_len - 1;    // last key this row sees
       float row_max = -INFINITY, row_sum = 0.f;

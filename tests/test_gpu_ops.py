@@ -746,6 +746,30 @@ def test_prefill_keeps_the_rest_of_the_last_page_out(bs, dqk, hq, hk, causal):
     _close(got, want, 2e-2, 2e-2)
 
 
+@pytest.mark.parametrize("hq,hk", [(8, 2), (3, 1)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_prefill_rows_without_keys_are_zero(hq, hk, causal):
+    """Sequences without keys (another rank's, or a padded one), and rows that lie ahead of the first key."""
+    lens, new = [0, 40, 0, 3, 0, 150], [5, 40, 200, 300, 1, 260]
+    q, kc, vc, bt, cu, sl = _paged_setup(lens, new, hq, hk, 128, 16, seed=hq)
+    junk = [torch.full((sum(new), hq * 128), 7.0, device=DEV, dtype=torch.bfloat16) for _ in range(4)]
+    del junk                                   # what the result's memory holds before
+    got, lse = ops.gqa_prefill(q.to(DEV), kc.to(DEV), vc.to(DEV), bt.to(DEV), cu.to(DEV), sl.to(DEV), len(lens), max(new), hq,
+                               128 ** -0.5, causal, 0, True)
+    got, lse = got.cpu().view(-1, hq, 128), lse.cpu()
+    for i, n in enumerate(lens):
+        for r in range(new[i]):
+            row, seen = int(cu[i]) + r, max(0, n - new[i] + r + 1) if causal else n
+            if seen == 0:
+                assert not got[row].any() and (lse[row] == -math.inf).all()
+            elif r % 37 == 0 or r == new[i] - 1:
+                k, v = (c[bt[i].long()].transpose(1, 2).flatten(0, 1)[:seen].double() for c in (kc, vc))
+                k, v = (x.repeat_interleave(hq // hk, 1) for x in (k, v))
+                s = torch.einsum("hd,khd->hk", q[row].view(hq, 128).double(), k) * 128 ** -0.5
+                _close(got[row], torch.einsum("hk,khd->hd", s.softmax(-1), v), 2e-2, 2e-2)
+                _close(lse[row], s.logsumexp(-1), 2e-2, 1e-2)
+
+
 @pytest.mark.parametrize("page", [8, 24])
 def test_mla_prefill_keeps_other_sequences_out(page):
     """Sequences that start at any page, each followed by one with NaN and infinite values."""
