@@ -216,8 +216,10 @@ class MLAAttention(nn.Module):
             # q_pe rotated in place: q is whole as it is
             if q_pe.data_ptr() != q[:, :, self.nope:].data_ptr():
                 q = torch.cat([q[:, :, : self.nope], q_pe], dim=-1)
-            return ops.mla_prefill(q, kv.view(total_blocks * gbs, n, 256), lat[..., l:].view(total_blocks * gbs, -1), first,
-                                   md.cu_q, md.seq_lens, md.num_seqs, md.max_q_len, self.scale)
+            out = ops.mla_prefill(q, kv.view(total_blocks * gbs, n, 256), lat[..., l:].view(total_blocks * gbs, -1), first,
+                                  md.cu_q, md.seq_lens, md.num_seqs, md.max_q_len, self.scale)
+            if out is not None:
+                return out
         kv = kv.view(total_blocks, gbs, n, self.nope + self.v_dim)
         k_pe = lat[..., l:].unsqueeze(2).expand(total_blocks, gbs, n, self.rope_dim)
         k_paged = torch.cat([kv[..., : self.nope], k_pe], dim=-1).permute(0, 2, 1, 3).contiguous()

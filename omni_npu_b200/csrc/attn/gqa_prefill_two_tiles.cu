@@ -46,7 +46,8 @@ constexpr int BN = 128;                 // keys per tile
 constexpr int DV = 128;
 constexpr int THREADS = 384;
 // registers: a thread of the softmax holds its row of S; the two warps that issue need few.  The shares must fit what
-// the launch takes (THREADS x MIN_REGS), or setmaxnreg would wait for good: checked before the first launch.
+// the launch takes (THREADS x MIN_REGS), or setmaxnreg would wait for good: checked before the first launch (a compiler
+// that gives the kernel fewer makes the callers take their other kernels).
 constexpr int SOFTMAX_REGS = 208, ISSUE_REGS = 56, MIN_REGS = 160;
 static_assert(256 * SOFTMAX_REGS + 128 * ISSUE_REGS <= THREADS * MIN_REGS, "register split");
 constexpr int SLAB = 128 * 128;         // 128 rows x 128 bytes
@@ -498,7 +499,8 @@ static int launch_two_tiles(const CUtensorMap& tq, const CUtensorMap& tk, const 
   int dev = 0;
   if (once.needed(&dev)) {
     cudaFuncAttributes fa{};
-    if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.numRegs < two::MIN_REGS) return -22;
+    if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return -22;
+    if (fa.numRegs < two::MIN_REGS) return 1;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, two::Cfg<DQK>::SMEM) != cudaSuccess)
       return -20;
     once.mark(dev);
@@ -576,15 +578,18 @@ extern "C" int b200_gqa_prefill_tc(const void* q, const void* k_cache, const voi
 
 // Non-absorbed latent attention over up-projected keys and values in place: q [T, H, 192] (pitch q_stride), kv [rows,
 // H, 256] (pitch kv_stride; 128 of the key, 128 of the value), pe [rows, 64] (pitch pe_stride); sequence b has seq_lens[b]
-// keys from row kv_start[b] on.  out [T, H, 128], causal.
+// keys from row kv_start[b] on.  out [T, H, 128], causal.  Returns 1 (nothing done) for scales, pitches and alignments that
+// the kernel does not take.
 extern "C" int b200_mla_prefill(const void* q, const void* kv, const void* pe, void* out, const int* kv_start,
                                 const int* cu_q, const int* seq_lens, int B, int max_q_len, int H, long long rows,
                                 long long total_q_rows, long long q_stride, long long kv_stride, long long pe_stride,
                                 long long out_stride, float scale, int* status, cudaStream_t stream) {
   if (B <= 0 || max_q_len <= 0 || total_q_rows <= 0 || rows <= 0) return 0;
-  if (H <= 0 || !(scale > 0.f) || rows > 0x7fffffffll || (out_stride & 7) != 0 ||
-      (reinterpret_cast<uintptr_t>(out) & 15) != 0)
-    return -1;
+  const uintptr_t bases = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kv) |
+                          reinterpret_cast<uintptr_t>(pe) | reinterpret_cast<uintptr_t>(out);
+  if (H <= 0 || !(scale > 0.f) || rows > 0x7fffffffll || (bases & 15) != 0 ||
+      ((q_stride | kv_stride | pe_stride | out_stride) & 7) != 0)
+    return 1;
   AttnParams p{};
   p.out = static_cast<__nv_bfloat16*>(out);
   p.block_tables = kv_start;
@@ -614,7 +619,7 @@ extern "C" int b200_mla_prefill(const void* q, const void* kv, const void* pe, v
   g.head_units = H;
   g.B = B;
   const long long items = static_cast<long long>(g.m_units) * H * B;
-  if (items > 0x7fffffffll) return -2;
+  if (items > 0x7fffffffll) return 1;
   g.items = static_cast<int>(items);
   return launch_two_tiles<192, true>(tq, tk, tp, p, two::BN, g, stream);
 }

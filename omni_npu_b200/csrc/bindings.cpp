@@ -619,8 +619,8 @@ std::tuple<Tensor, Tensor> gqa_prefill(const Tensor& q, const Tensor& k_cache, c
 }
 
 // Latent attention of a prompt step: q [T, H, 192], kv [rows, H, 256] (key | value), pe [rows, 64]; sequence b's keys are
-// the rows kv_start[b] .. kv_start[b] + seq_lens[b].
-Tensor mla_prefill(const Tensor& q, const Tensor& kv, const Tensor& pe, const Tensor& kv_start, const Tensor& cu_q,
+// the rows kv_start[b] .. kv_start[b] + seq_lens[b].  Nothing: scales or alignments that the kernel does not take.
+c10::optional<Tensor> mla_prefill(const Tensor& q, const Tensor& kv, const Tensor& pe, const Tensor& kv_start, const Tensor& cu_q,
                    const Tensor& seq_lens, int64_t num_seqs, int64_t max_q_len, double scale, const Tensor& status) {
   CHECK_CUDA_BF16(q);
   CHECK_CUDA_BF16(kv);
@@ -637,11 +637,12 @@ Tensor mla_prefill(const Tensor& q, const Tensor& kv, const Tensor& pe, const Te
               "mla_prefill: sequences");
   c10::cuda::CUDAGuard guard(q.device());
   Tensor out = torch::empty({T, H * 128}, q.options());
-  check(b200_mla_prefill(q.data_ptr(), kv.data_ptr(), pe.data_ptr(), out.data_ptr(), kv_start.data_ptr<int>(),
-                         cu_q.data_ptr<int>(), seq_lens.data_ptr<int>(), (int)num_seqs, (int)max_q_len, (int)H, rows, T,
-                         q.stride(0), kv.stride(0), pe.stride(0), H * 128, (float)scale, status.data_ptr<int>(),
-                         cur_stream()),
-        "mla_prefill");
+  const int rc = b200_mla_prefill(q.data_ptr(), kv.data_ptr(), pe.data_ptr(), out.data_ptr(), kv_start.data_ptr<int>(),
+                                  cu_q.data_ptr<int>(), seq_lens.data_ptr<int>(), (int)num_seqs, (int)max_q_len, (int)H, rows,
+                                  T, q.stride(0), kv.stride(0), pe.stride(0), H * 128, (float)scale, status.data_ptr<int>(),
+                                  cur_stream());
+  if (rc == 1) return c10::nullopt;
+  check(rc, "mla_prefill");
   return out;
 }
 

@@ -671,12 +671,15 @@ def gqa_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
 
 
 def mla_prefill(q: torch.Tensor, kv: torch.Tensor, pe: torch.Tensor, kv_start: torch.Tensor, cu_q: torch.Tensor,
-                seq_lens: torch.Tensor, num_seqs: int, max_q_len: int, scale: float) -> torch.Tensor:
+                seq_lens: torch.Tensor, num_seqs: int, max_q_len: int, scale: float) -> Optional[torch.Tensor]:
     """Causal latent attention of a prompt step over up-projected rows as they lie: q [T, H, 128 + 64], kv [rows, H,
     128 + 128] (key | value of every head), pe [rows, 64] (the keys' rotated part, of all heads); sequence b's keys are
-    the rows from kv_start[b] on, the last of them its last query's own.  bf16 on the GPU only."""
-    _count(1)
-    return _C().mla_prefill(q, kv, pe, kv_start, cu_q, seq_lens, num_seqs, max_q_len, scale, device_state(q.device).status)
+    the rows from kv_start[b] on, the last of them its last query's own.  bf16 on the GPU only.  None: a scale, a pitch or an
+    alignment that the kernel does not take."""
+    out = _C().mla_prefill(q, kv, pe, kv_start, cu_q, seq_lens, num_seqs, max_q_len, scale, device_state(q.device).status)
+    if out is not None:
+        _count(1)
+    return out
 
 
 def merge_attn_states(outs: torch.Tensor, lses: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:

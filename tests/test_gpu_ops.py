@@ -746,6 +746,16 @@ def test_prefill_keeps_the_rest_of_the_last_page_out(bs, dqk, hq, hk, causal):
     _close(got, want, 2e-2, 2e-2)
 
 
+@pytest.mark.parametrize("shift,scale", [(0, 192 ** -0.5), (4, 192 ** -0.5), (0, -0.07)])
+def test_mla_prefill_refuses_what_its_copies_do_not_take(shift, scale):
+    """Rotated parts off a 16-byte boundary and negative scales are the caller's to repack."""
+    q, kv = (torch.randn(8, 2, n, device=DEV, dtype=torch.bfloat16) for n in (192, 256))
+    pe = torch.randn(8, 64 + 8, device=DEV, dtype=torch.bfloat16)[:, shift: shift + 64]
+    i32 = dict(dtype=torch.int32, device=DEV)
+    out = ops.mla_prefill(q, kv, pe, torch.zeros(1, **i32), torch.tensor([0, 8], **i32), torch.tensor([8], **i32), 1, 8, scale)
+    assert (out is None) == (shift != 0 or scale < 0)
+
+
 @pytest.mark.parametrize("hq,hk", [(8, 2), (3, 1)])
 @pytest.mark.parametrize("causal", [True, False])
 def test_prefill_rows_without_keys_are_zero(hq, hk, causal):
