@@ -47,6 +47,21 @@ class RMSNorm(nn.Module):
         return (q, s), residual, y
 
 
+_RMS_FORWARD = RMSNorm.forward
+
+
+def fused_head_norms(q_norm: nn.Module, k_norm: nn.Module) -> Optional[Tuple[torch.Tensor, torch.Tensor, float]]:
+    """(q weight, k weight, eps) for a kernel that norms the heads of q and k itself, or None where the modules have to be
+    called: other classes, unequal eps, and modules whose calls somebody watches (hooks, a wrapped ``forward``)."""
+    for m in (q_norm, k_norm):
+        if type(m) is not RMSNorm or RMSNorm.forward is not _RMS_FORWARD or "forward" in m.__dict__ \
+                or m._forward_hooks or m._forward_pre_hooks:
+            return None
+    if q_norm.eps != k_norm.eps or nn.modules.module._has_any_global_hook():
+        return None
+    return q_norm.weight, k_norm.weight, q_norm.eps
+
+
 def reduce_add_rms_norm(norm: RMSNorm, x_partial: torch.Tensor, residual: torch.Tensor, group):
     """``residual += all_reduce(x_partial)``; returns (RMSNorm(residual), residual).
 

@@ -19,7 +19,7 @@ from ..layers.embedding import ParallelLMHead, VocabParallelEmbedding
 from ..layers.linear import row_parallel_add_rms_norm
 from ..layers.linear import QKVParallelLinear, RowParallelLinear
 from ..layers.mlp import FusedMLP
-from ..layers.norm import RMSNorm, reduce_add_rms_norm
+from ..layers.norm import RMSNorm, fused_head_norms, reduce_add_rms_norm
 from ..layers.rope import get_rope
 from ..attention.metadata import get_forward_context
 from ..parallel import state as pstate
@@ -46,10 +46,17 @@ class LlamaAttention(nn.Module):
                                  if self.rotary.mscale != 1.0 else cfg.head_dim ** -0.5,
                                  cfg.rotary_dim, cfg.rope_neox, cfg.sliding_window)
 
-    def forward(self, hidden: torch.Tensor, reduce: bool = True, fuse_norm=None):
+    def _attend(self, hidden: torch.Tensor) -> torch.Tensor:
         q, k, v = self.qkv_proj(hidden)
-        norm = (self.q_norm.weight, self.k_norm.weight, self.q_norm.eps) if self.qk_norm else None
-        o = self.attn(q, k, v, self.rotary.cos_sin_cache, norm=norm)
+        norm = None
+        if self.qk_norm:
+            norm = fused_head_norms(self.q_norm, self.k_norm)
+            if norm is None:
+                q, k = (m(x.reshape(-1, self.head_dim)).view(x.shape[0], -1) for m, x in ((self.q_norm, q), (self.k_norm, k)))
+        return self.attn(q, k, v, self.rotary.cos_sin_cache, norm=norm)
+
+    def forward(self, hidden: torch.Tensor, reduce: bool = True, fuse_norm=None):
+        o = self._attend(hidden)
         if fuse_norm is not None:
             # o_proj + tensor-parallel reduction + residual add + the following RMSNorm
             return row_parallel_add_rms_norm(self.o_proj, o, fuse_norm[0], fuse_norm[1])

@@ -64,9 +64,7 @@ class HeadToSequenceAttention(LlamaAttention):
     def forward(self, hidden, reduce: bool = True, fuse_norm=None, stream=None):
         if stream is None or not stream.enabled:
             return super().forward(hidden, reduce=reduce, fuse_norm=fuse_norm)
-        q, k, v = self.qkv_proj(hidden)
-        norm = (self.q_norm.weight, self.k_norm.weight, self.q_norm.eps) if self.qk_norm else None
-        o = self.attn(q, k, v, self.rotary.cos_sin_cache, norm=norm)
+        o = self._attend(hidden)
         if o.shape[0] != stream.padded:
             o = torch.cat([o, o.new_zeros(stream.padded - o.shape[0], o.shape[1])], dim=0)
         o = self.tp.comm.all_to_all(o, scatter_dim=0, gather_dim=-1)        # [T/tp, heads * d]

@@ -4,6 +4,7 @@ import torch
 
 from omni_npu_b200 import ops
 from omni_npu_b200.layers.linear import Fp8BlockLinearMethod, UnquantizedLinearMethod
+from omni_npu_b200.layers.norm import RMSNorm
 from omni_npu_b200.layers.quant_fp8 import fp8_block_gemm, quantize_weight_block
 
 
@@ -31,3 +32,72 @@ def test_only_parameters_are_read_ahead_of_the_kernels_before(monkeypatch):
     Fp8BlockLinearMethod().apply(layer, x, None)
     fp8_block_gemm(x, wq, ws, w_ready=True)
     assert len(calls) == 2 and not any(c.get("w_ready", False) for c in calls)
+
+
+def _qwen_attention():
+    """One attention layer of a small Qwen3 model, and what it returns for a prompt of five tokens."""
+    from omni_npu_b200.attention.metadata import AttentionMetadata, set_forward_context
+    from omni_npu_b200.config import ModelConfig
+    from omni_npu_b200.engine.llm import build_engine_config
+    from omni_npu_b200.models.llama import LlamaAttention
+    from omni_npu_b200.worker.worker import Worker
+    mc = ModelConfig(hidden_size=64, num_layers=1, num_heads=4, num_kv_heads=2, head_dim=16, intermediate_size=64,
+                     vocab_size=64, max_position_embeddings=64, qk_norm=True, dtype=torch.float32)
+    cfg = build_engine_config(mc, device="cpu", max_num_seqs=1, num_gpu_blocks=4, block_size=16)
+    Worker(cfg, local_rank=0, rank=0).init_device()
+    torch.manual_seed(0)
+    attn = LlamaAttention(mc, 0, "cpu", "attn")
+    for p in attn.parameters():
+        p.data.normal_(0.0, 0.2)
+    i32 = dict(dtype=torch.int32)
+    md = AttentionMetadata(is_prefill=True, num_seqs=1, num_tokens=5, max_q_len=5, max_seq_len=5, q_len=0,
+                           positions=torch.arange(5, **i32), slot_mapping=torch.arange(5, **i32),
+                           block_tables=torch.zeros(1, 1, **i32), seq_lens=torch.tensor([5], **i32),
+                           cu_q=torch.tensor([0, 5], **i32), num_actual_tokens=5, num_actual_seqs=1)
+    x = torch.randn(5, 64)
+
+    def run():
+        caches = [tuple(torch.zeros(4, 2, 16, 16) for _ in range(2))]
+        with set_forward_context(md, caches, cfg):
+            return attn(x)
+
+    return attn, run
+
+
+def test_head_norms_that_somebody_watches_are_called(monkeypatch):
+    """Hooks on the head norms, wrapped classes (the name-list tracer's) and modules of other classes see their calls."""
+    attn, run = _qwen_attention()
+    want, seen = run(), []
+    handle = attn.k_norm.register_forward_hook(lambda m, a, out: seen.append("hook"))
+    torch.testing.assert_close(run(), want)
+    handle.remove()
+    real = RMSNorm.forward
+    monkeypatch.setattr(RMSNorm, "forward", lambda self, *a, **k: (seen.append("class"), real(self, *a, **k))[1])
+    torch.testing.assert_close(run(), want)
+    monkeypatch.undo()
+    assert seen == ["hook", "class", "class"]
+
+    class Doubled(RMSNorm):
+        def forward(self, x):
+            return 2 * super().forward(x)
+
+    plain = attn.q_norm
+    attn.q_norm = Doubled(16, plain.eps, torch.float32)
+    attn.q_norm.weight.data.copy_(plain.weight)
+    doubled = run()
+    attn.q_norm = plain
+    plain.weight.data.mul_(2)
+    torch.testing.assert_close(doubled, run())
+
+
+def test_head_norms_keep_an_eps_of_their_own():
+    attn, run = _qwen_attention()
+    attn.q_norm.eps, attn.k_norm.eps = 1e-6, 10.0
+    got = run()
+    norms = [m.eps for m in (attn.q_norm, attn.k_norm)]
+    handle = attn.q_norm.register_forward_hook(lambda *a: None)         # the modules are called one by one
+    want = run()
+    handle.remove()
+    torch.testing.assert_close(got, want)
+    attn.k_norm.eps = 1e-6
+    assert norms == [1e-6, 10.0] and (run() - got).abs().max() > 1e-3
