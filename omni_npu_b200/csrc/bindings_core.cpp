@@ -18,6 +18,7 @@ int b200_gemm(const void* A, const void* W, void* C, const void* bias, const voi
 int b200_gemm_stream(const void* A, const void* W, void* C, const void* bias, const void* residual, int M, int N, int K,
                      int lda, int ldw, int ldc, int out_fp32, int act, int splits, int* status, int max_ctas,
                      float act_alpha, float act_limit, int w_ready, cudaStream_t stream);
+int b200_gemm_stream_splits(int N, int K, int max_ctas, int sms);
 int b200_grouped_gemm_stream(const void* A, const void* W, void* C, const int* expert_offsets, int num_experts,
                              int total_rows, int N, int K, int lda, int ldc, int act, int tn, int* status, int max_ctas,
                              float act_alpha, float act_limit, cudaStream_t stream);
@@ -251,6 +252,11 @@ Tensor gemm_stream(const Tensor& a, const Tensor& w, const c10::optional<Tensor>
                          (int)max_ctas, (float)act_alpha, (float)act_limit, w_ready ? 1 : 0, cur_stream()),
         "gemm_stream");
   return c;
+}
+
+// CTAs that share the K of a tile of gemm_stream.
+int64_t gemm_stream_splits(int64_t N, int64_t K, int64_t max_ctas, int64_t sms) {
+  return b200_gemm_stream_splits((int)N, (int)K, (int)max_ctas, (int)sms);
 }
 
 // c[t, g] = a[t, g] w[g]^T: a [T, G, K] and c [T, G, N] views with any row and group pitch, w [G, N, K].  False (nothing
@@ -1157,6 +1163,7 @@ TORCH_LIBRARY(omni_b200, m) {
   m.def("gemm", &gemm);
   m.def("gemm_pair", &gemm_pair);
   m.def("gemm_stream", &gemm_stream);
+  m.def("gemm_stream_splits", &gemm_stream_splits);
   m.def("batched_gemm", &batched_gemm);
   m.def("grouped_gemm_rows", &grouped_gemm_rows);
   m.def("grouped_gemm", &grouped_gemm);

@@ -23,6 +23,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tensormap.h"
 #include "column_store.cuh"
+#include "stream_split.cuh"
 
 namespace b200 {
 
@@ -408,16 +409,6 @@ static int launch_fp8_stream(const CUtensorMap& tw, const CUtensorMap& tx, const
              : -21;
 }
 
-// CTAs that share a tile's K: as many as keep all CTAs resident at two per SM, with at least four scale blocks each.
-static int fp8_stream_splits(int n_tiles, int k_slabs) {
-  int best = 1;
-  for (int s = 2; s <= 8; s *= 2) {
-    const int per = (k_slabs + s - 1) / s;
-    if (n_tiles * s <= 2 * sm_count() && per >= 4 && (s - 1) * per < k_slabs) best = s;
-  }
-  return best;
-}
-
 }  // namespace b200
 
 using namespace b200;
@@ -437,7 +428,7 @@ extern "C" int b200_gemm_fp8_stream(const void* A, const float* a_scales, const 
   p.box = p.tn;
   p.stages = RING / (W_BYTES + p.tn * SLAB);
   p.num_n_tiles = (N + BW - 1) / BW;
-  p.splits = fp8_stream_splits(p.num_n_tiles, p.k_slabs);
+  p.splits = stream_splits(p.num_n_tiles, p.k_slabs, max_ctas, sm_count());
   p.scale_rows = p.num_n_tiles;
   p.ldc = ldc;
   p.out_fp32 = out_fp32;

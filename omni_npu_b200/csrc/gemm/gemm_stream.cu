@@ -29,6 +29,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tensormap.h"
 #include "column_store.cuh"
+#include "stream_split.cuh"
 
 namespace b200 {
 
@@ -423,17 +424,6 @@ static size_t stream_smem(int tn, int stages, int num_experts) {
          (num_experts > 0 ? 2 * (num_experts + 1) * 4 : 0);
 }
 
-// CTAs that share a tile's K: as many (a power of two up to the portable cluster size) as keep all CTAs resident at two
-// per SM, with at least four slabs each.
-static int stream_splits(int n_tiles, int k_slabs) {
-  int best = 1;
-  for (int s = 2; s <= 8; s *= 2) {
-    const int per = (k_slabs + s - 1) / s;
-    if (n_tiles * s <= 2 * sm_count() && per >= 4 && (s - 1) * per < k_slabs) best = s;
-  }
-  return best;
-}
-
 template <int MODE, bool SPLIT>
 static int launch_stream(const CUtensorMap& tw, const CUtensorMap& tx, const StreamParams& p, int grid,
                          cudaStream_t stream) {
@@ -454,6 +444,11 @@ static int launch_stream(const CUtensorMap& tw, const CUtensorMap& tx, const Str
 
 using namespace b200;
 
+// CTAs of a cluster that b200_gemm_stream has share the K of one tile.
+extern "C" int b200_gemm_stream_splits(int N, int K, int max_ctas, int sms) {
+  return stream_splits((N + stream::BW - 1) / stream::BW, (K + stream::SLAB_K - 1) / stream::SLAB_K, max_ctas, sms);
+}
+
 // A [M <= 128, K] (pitch lda), W [N, K] (pitch ldw), C [M, N, or N / 2 with a gated activation].  splits 0: by rule.
 // w_ready: see StreamParams.
 extern "C" int b200_gemm_stream(const void* A, const void* W, void* C, const void* bias, const void* residual, int M,
@@ -471,7 +466,7 @@ extern "C" int b200_gemm_stream(const void* A, const void* W, void* C, const voi
   p.stages = stream_stages(p.tn);
   p.k_slabs = (K + stream::SLAB_K - 1) / stream::SLAB_K;
   p.num_n_tiles = (N + stream::BW - 1) / stream::BW;
-  p.splits = splits > 0 ? splits : stream_splits(p.num_n_tiles, p.k_slabs);
+  p.splits = splits > 0 ? splits : stream_splits(p.num_n_tiles, p.k_slabs, max_ctas, sm_count());
   if (p.splits != 1 && p.splits != 2 && p.splits != 4 && p.splits != 8) return -12;
   if ((p.splits - 1) * ((p.k_slabs + p.splits - 1) / p.splits) >= p.k_slabs) return -12;
   p.ldc = ldc;

@@ -1,0 +1,19 @@
+// How the weight-streaming kernels (gemm_stream.cu, gemm_fp8_stream.cu) share a tile's K among the CTAs of a cluster.
+#pragma once
+
+namespace b200 {
+
+// CTAs per tile of 128 weight rows: as many (a power of two up to the portable cluster size) as keep all CTAs resident at
+// two per SM, and within the caller's limit (0: none), with at least four slabs of K each.  Depends on the weights alone,
+// so that the result of a row does not depend on the number of rows.
+inline int stream_splits(int n_tiles, int k_slabs, int max_ctas, int sms) {
+  const int most = max_ctas > 0 && max_ctas < 2 * sms ? max_ctas : 2 * sms;
+  int best = 1;
+  for (int s = 2; s <= 8; s *= 2) {
+    const int per = (k_slabs + s - 1) / s;
+    if (static_cast<long long>(n_tiles) * s <= most && per >= 4 && (s - 1) * per < k_slabs) best = s;
+  }
+  return best;
+}
+
+}  // namespace b200

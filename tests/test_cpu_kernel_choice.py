@@ -101,3 +101,15 @@ def test_head_norms_keep_an_eps_of_their_own():
     torch.testing.assert_close(got, want)
     attn.k_norm.eps = 1e-6
     assert norms == [1e-6, 10.0] and (run() - got).abs().max() > 1e-3
+
+
+@pytest.mark.parametrize("n,k", [(128, 4096), (4096, 4096), (4096, 7168), (18944, 2048), (130, 256), (640, 64)])
+def test_split_products_keep_within_a_limit_of_ctas(n, k):
+    """A product that shares K among CTAs uses no more of them than its caller allows, and all of K's slabs."""
+    splits = ops._core().gemm_stream_splits
+    tiles, slabs = -(-n // 128), -(-k // 64)
+    for limit in (0, 1, 8, 32, 64, 100, 148, 296, 1000):
+        s = splits(n, k, limit, 148)
+        assert s in (1, 2, 4, 8) and (s == 1 or tiles * s <= min(limit or 296, 296))
+        assert s == 1 or ((s - 1) * -(-slabs // s) < slabs and -(-slabs // s) >= 4)
+        assert s <= splits(n, k, 0, 148)

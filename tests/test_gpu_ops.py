@@ -624,6 +624,22 @@ def test_grouped_gemm_fp8_few_rows(counts, n, k, swiglu, monkeypatch):
     ops.check_status()
 
 
+@pytest.mark.parametrize("limit", [1, 7, 40, 300])
+def test_few_rows_within_a_limit_of_ctas(limit):
+    torch.manual_seed(limit)
+    m, n, k = 20, 1000, 2048
+    a = torch.randn(m, k, device=DEV, dtype=torch.bfloat16)
+    w = (torch.randn(n, k, device=DEV) * k ** -0.5).bfloat16()
+    # fp32 sums of k products of size k ** -0.5
+    _close(ops.gemm(a, w, out_dtype=torch.float32, max_ctas=limit), (a.double() @ w.double().T).float(), k ** 0.5 * 2 ** -22, 0)
+    q, s = ops.quant_fp8_1x128(a)
+    w8, ws = torch.randn(n, k, device=DEV).to(torch.float8_e4m3fn), torch.rand(8, k // 128, device=DEV) + 0.5
+    full = w8.double() * ws.double().repeat_interleave(128, 0)[:n].repeat_interleave(128, 1)
+    want = (q.double() * s.double().repeat_interleave(128, 1)) @ full.T
+    # fp32 sums of products of size 1: k ** 0.5 of them in size, each off by some 2 ** -24 of the largest part
+    _close(ops.gemm_fp8_block(q, s, w8, ws, out_dtype=torch.float32, max_ctas=limit), want.float(), k ** 0.5 * 2 ** -16, 2 ** -16)
+
+
 @pytest.mark.parametrize("t,h,lat,rope,nope", [(1, 16, 512, 64, 128), (40, 3, 512, 64, 128), (7, 1, 8, 8, 16), (5, 2, 4096, 32, 64),
                                                (9, 2, 260, 64, 128), (6, 2, 512, 64, 100)])
 def test_mla_norm_rope_cache(t, h, lat, rope, nope):
