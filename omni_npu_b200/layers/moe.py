@@ -228,9 +228,11 @@ class FusedMoE(nn.Module):
         return moved
 
     # ----------------------------------------------------------------- forward
-    def _expert_rows(self, rows: torch.Tensor, offsets: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-        h = ops.grouped_gemm(rows, self.w13, offsets, swiglu=self.unary is None, act=self.act, unary=self.unary)
-        return ops.grouped_gemm(h, self.w2, offsets, out=out)
+    def _expert_rows(self, rows: torch.Tensor, offsets: torch.Tensor, out: Optional[torch.Tensor] = None,
+                     expected: Optional[int] = None) -> torch.Tensor:
+        h = ops.grouped_gemm(rows, self.w13, offsets, swiglu=self.unary is None, act=self.act, unary=self.unary,
+                             rows=expected)
+        return ops.grouped_gemm(h, self.w2, offsets, out=out, rows=expected)
 
     def forward(self, hidden: torch.Tensor) -> torch.Tensor:
         """hidden [T,H] (replicated across TP ranks) -> [T,H]."""
@@ -282,7 +284,7 @@ class FusedMoE(nn.Module):
             with torch.cuda.stream(self._side_stream):
                 shared_out = self.shared_experts(hidden)
         rows, offsets, handle = ep_dispatch(None, hidden, ids, w, self.num_physical, self.buffers)
-        y = self._expert_rows(rows, offsets)
+        y = self._expert_rows(rows, offsets, expected=handle.expected_rows)
         if shared_out is not None:
             cur.wait_stream(self._side_stream)
         return RoutedRows(y, handle.slots, w), shared_out
@@ -312,11 +314,12 @@ class FusedMoE(nn.Module):
                 # here), SwiGLU fused into the first product's epilogue, requantise, second product
                 rq, rs = rows if fp8_rows else ops.quant_fp8_1x128(rows)
                 h1 = ops.grouped_gemm_fp8_block(rq, rs, self.w13, self.w13_scale, offsets, swiglu=True,
-                                                up_scale_row0=(self.intermediate_size + 127) // 128)
+                                                up_scale_row0=(self.intermediate_size + 127) // 128,
+                                                rows=handle.expected_rows)
                 hq, hs = ops.quant_fp8_1x128(h1)
-                ops.grouped_gemm_fp8_block(hq, hs, self.w2, self.w2_scale, offsets, out=y)
+                ops.grouped_gemm_fp8_block(hq, hs, self.w2, self.w2_scale, offsets, out=y, rows=handle.expected_rows)
             else:
-                self._expert_rows(rows, offsets, out=y)
+                self._expert_rows(rows, offsets, out=y, expected=handle.expected_rows)
             if shared_out is not None:
                 torch.cuda.current_stream(x.device).wait_stream(self._side_stream)
             return ep_combine(comm, self.buffers.expert_y, handle, shared_out, self.buffers)

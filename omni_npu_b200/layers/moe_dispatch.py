@@ -60,6 +60,7 @@ class DispatchHandle:
     rows: int                       # rows of the local receive buffer in use (upper bound)
     expert_offsets: torch.Tensor    # [E_local+1] int32
     cpu_state: Optional[dict] = None
+    expected_rows: int = 0          # rows that hold tokens if these spread evenly over the experts: what kernels are chosen by
 
 
 class EpBuffers:
@@ -206,7 +207,9 @@ def ep_dispatch(comm, hidden: torch.Tensor, topk_ids: torch.Tensor, topk_weights
     ops._count(3 if buf.world == 1 else 6)  # count, layout, scatter (+ flag kernels)
     # static upper bound on the rows in use (device-side counts decide the real extent)
     rows = buf.cap_rows if buf.world > 1 else max(t * k, 1)
-    handle = DispatchHandle(topk_ids, topk_weights, buf.slots, t, rows, buf.expert_offsets)
+    # (each rank sends t * k rows, and gets as many where the experts are chosen evenly)
+    handle = DispatchHandle(topk_ids, topk_weights, buf.slots, t, rows, buf.expert_offsets,
+                            expected_rows=min(rows, max(t * k, 1)))
     if fp8:
         return (buf.recv_q[:rows], buf.recv_s[:rows]), buf.expert_offsets, handle
     return buf.recv_x[:rows], buf.expert_offsets, handle
@@ -266,7 +269,7 @@ def _cpu_dispatch(comm, hidden, topk_ids, topk_weights, num_experts):
     offsets[1:] = counts.cumsum(0)
     handle = DispatchHandle(topk_ids, topk_weights, None, t, rows.shape[0], offsets,
                             cpu_state=dict(pair_idx=pair_idx, lorder=lorder, send_counts=send_counts,
-                                           recv_counts=recv_counts, k=k))
+                                           recv_counts=recv_counts, k=k), expected_rows=rows.shape[0])
     return rows, offsets, handle
 
 

@@ -337,18 +337,20 @@ def gemm_fp8_block(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.Tensor, 
 
 def grouped_gemm_fp8_block(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor,
                            expert_offsets: torch.Tensor, swiglu: bool = False, up_scale_row0: int = 0,
-                           max_ctas: int = 0, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                           max_ctas: int = 0, out: Optional[torch.Tensor] = None,
+                           rows: Optional[int] = None) -> torch.Tensor:
     """Per-expert block-scaled e4m3 GEMM: rows ``expert_offsets[e]:expert_offsets[e+1]`` of ``a_q`` times
     ``w_q[e].T`` with ``w_scale[e]`` (one scale per 128 x 128 block).  ``swiglu``: gate / up rows of
     ``w_q`` are interleaved in groups of 8 and the result is ``silu(gate) * up``; the scale rows are the
-    gate blocks followed, from row ``up_scale_row0``, by the up blocks.  ``out``: where the result goes."""
+    gate blocks followed, from row ``up_scale_row0``, by the up blocks.  ``out``: where the result goes.
+    ``rows`` as in :func:`grouped_gemm`."""
     if not a_q.is_cuda:
         y = ref.grouped_gemm_fp8_block(a_q, a_scale, w_q, w_scale, expert_offsets, swiglu, up_scale_row0)
         return y if out is None else out.copy_(y)
     st = device_state(a_q.device)
     if out is None:
         out = torch.empty(a_q.shape[0], w_q.shape[1] // (2 if swiglu else 1), dtype=torch.bfloat16, device=a_q.device)
-    few = a_q.shape[0] <= FP8_STREAM_GROUP_ROWS * w_q.shape[0]
+    few = (a_q.shape[0] if rows is None else min(rows, a_q.shape[0])) <= FP8_STREAM_GROUP_ROWS * w_q.shape[0]
     _count(1)
     _C().grouped_gemm_fp8_block(a_q, a_scale.contiguous(), w_q, w_scale.contiguous(), expert_offsets, out, swiglu,
                                 up_scale_row0, 64 if few else 0, st.status, max_ctas)
@@ -442,7 +444,7 @@ def grouped_tile(rows: int, groups: int, n: int, k: int, sms: int = 148) -> int:
 
 @functools.lru_cache(maxsize=4096)
 def grouped_rows_tile(rows: int, groups: int, n: int, sms: int = 148) -> int:
-    """Kernel of a grouped bf16 product: rows of A per tile of gemm_stream_kernel, or 0 for grouped_pair_kernel.
+    """Kernel of a grouped bf16 product: rows of A per tile of gemm_stream_kernel, or 0 for gemm_pair_kernel.
 
     Streaming wins while the weights outweigh the rows (us, streaming / pair): 128 groups 1536 x 2048 with silu 132 / 136
     at 32 rows per group, 64 groups 2816 x 2048 117 / 125 at 48, but 128 groups 2048 x 768 110 / 79 at 64; with too few
@@ -457,14 +459,17 @@ def grouped_rows_tile(rows: int, groups: int, n: int, sms: int = 148) -> int:
 
 def grouped_gemm(a: torch.Tensor, w: torch.Tensor, expert_offsets: torch.Tensor,
                  swiglu: bool = False, bn: int = 0, max_ctas: int = 0,
-                 act=SILU, unary: Optional[str] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                 act=SILU, unary: Optional[str] = None, out: Optional[torch.Tensor] = None,
+                 rows: Optional[int] = None) -> torch.Tensor:
     """Per-expert GEMM: rows expert_offsets[e]:expert_offsets[e+1] of ``a`` times ``w[e].T``
-    (``swiglu`` / ``act`` / ``unary`` as in :func:`gemm`).  ``out``: where the result goes."""
+    (``swiglu`` / ``act`` / ``unary`` as in :func:`gemm`).  ``out``: where the result goes.  ``rows``: about how many rows the
+    groups hold, where the host knows it (the rest of a receive buffer is empty); the kernel is chosen by it."""
     kind = _act_kind(swiglu, act, None, unary)
     if a.is_cuda and a.dtype == torch.bfloat16 and bn <= 0:
-        rows, groups, n = a.shape[0], w.shape[0], w.shape[1]
+        groups, n = w.shape[0], w.shape[1]
+        rows = a.shape[0] if rows is None else min(rows, a.shape[0])
         if out is None:
-            out = a.new_empty(rows, n // 2 if kind[0] in (1, 2, 4, 7) else n)
+            out = a.new_empty(a.shape[0], n // 2 if kind[0] in (1, 2, 4, 7) else n)
         _count(1)
         _core().grouped_gemm_rows(a, w, expert_offsets, out, kind[0], grouped_rows_tile(rows, groups, n),
                                   device_state(a.device).status, max_ctas, kind[1], kind[2])

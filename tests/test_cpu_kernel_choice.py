@@ -113,3 +113,32 @@ def test_split_products_keep_within_a_limit_of_ctas(n, k):
         assert s in (1, 2, 4, 8) and (s == 1 or tiles * s <= min(limit or 296, 296))
         assert s == 1 or ((s - 1) * -(-slabs // s) < slabs and -(-slabs // s) >= 4)
         assert s <= splits(n, k, 0, 148)
+
+
+@pytest.mark.parametrize("quant", [None, "fp8"])
+def test_experts_choose_kernels_by_the_rows_of_the_step(monkeypatch, quant):
+    """Not by the size of the receive buffer, which on several ranks holds the largest step."""
+    from types import SimpleNamespace
+
+    from omni_npu_b200.layers import moe
+    from omni_npu_b200.layers.moe_dispatch import DispatchHandle
+    h, experts, cap = 128, 2, 4096
+    buffers = SimpleNamespace(fp8_dispatch=False, expert_y=torch.zeros(cap, h))
+    layer = SimpleNamespace(ep_size=1, buffers=buffers, shared_experts=None, quant=quant, num_physical=experts,
+                            intermediate_size=h, act=ops.SILU, unary=None, w13=torch.randn(experts, 2 * h, h),
+                            w2=torch.randn(experts, h, h), w13_scale=torch.ones(experts, 2, 1),
+                            w2_scale=torch.ones(experts, 1, 1))
+    layer._expert_rows = lambda *a, **k: moe.FusedMoE._expert_rows(layer, *a, **k)
+    handle = DispatchHandle(None, None, None, 5, cap, None, expected_rows=10)
+    monkeypatch.setattr(moe, "ep_dispatch", lambda *a, **k: (torch.zeros(cap, h), torch.tensor([0, 4, 10]), handle))
+    monkeypatch.setattr(moe, "ep_combine", lambda comm, y, *a: y)
+    seen = []
+    for name in ("grouped_gemm", "grouped_gemm_fp8_block"):
+        monkeypatch.setattr(ops, name, lambda a, *p, **k: (seen.append(k.get("rows")), torch.zeros(cap, h))[1])
+    moe.FusedMoE._routed(layer, SimpleNamespace(is_cuda=True, device=None), None, None)
+    assert seen == [10, 10]
+
+
+def test_rows_of_a_step_choose_the_grouped_kernel():
+    few, many = ops.grouped_rows_tile(16, 16, 1536), ops.grouped_rows_tile(131072, 16, 1536)
+    assert few > 0 and many == 0            # streamed weights; CTA pairs

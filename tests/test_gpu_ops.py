@@ -624,6 +624,24 @@ def test_grouped_gemm_fp8_few_rows(counts, n, k, swiglu, monkeypatch):
     ops.check_status()
 
 
+@pytest.mark.parametrize("used", [3, 200])
+def test_grouped_products_chosen_by_the_rows_in_use(used):
+    """Any estimate of the rows gives the same result."""
+    torch.manual_seed(used)
+    e, n, k, cap = 4, 512, 256, 3000
+    offs = (torch.arange(e + 1, device=DEV) * used // e).int()
+    a, w = torch.randn(cap, k, device=DEV).bfloat16(), (torch.randn(e, n, k, device=DEV) * k ** -0.5).bfloat16()
+    want = torch.cat([a[offs[i]: offs[i + 1]].double() @ w[i].double().T for i in range(e)]).float()
+    q, s = ops.quant_fp8_1x128(a)
+    w8, ws = torch.randn(e, n, k, device=DEV).to(torch.float8_e4m3fn), torch.rand(e, n // 128, k // 128, device=DEV)
+    want8 = ops.grouped_gemm_fp8_block(q[:used], s[:used], w8, ws, offs)
+    for rows in (None, used, 1, 10 * cap):
+        got = ops.grouped_gemm(a, w, offs, rows=rows)
+        assert got.shape == (cap, n)
+        _close(got[:used], want, 1e-3, 2 ** -8)      # one rounding to bf16
+        _close(ops.grouped_gemm_fp8_block(q, s, w8, ws, offs, rows=rows)[:used], want8, 1e-3, 2 ** -7)
+
+
 @pytest.mark.parametrize("limit", [1, 7, 40, 300])
 def test_few_rows_within_a_limit_of_ctas(limit):
     torch.manual_seed(limit)
