@@ -192,6 +192,26 @@ def test_gemm_few_rows(m, n, k):
     ops.check_status()
 
 
+@pytest.mark.parametrize("m,n,k", [(63, 2048, 512), (64, 130, 512), (33, 1000, 1024), (3, 48, 4096), (62, 258, 2048), (128, 56, 4096)])
+def test_gemm_few_rows_split(m, n, k):
+    """Sums over the CTAs of a cluster, four columns at a time: columns left over, results and residuals off 16 bytes."""
+    torch.manual_seed(m + n + k)
+    assert ops._core().gemm_stream_splits(n, k, 0, 148) > 1
+    a = torch.randn(m, k, device=DEV, dtype=torch.bfloat16)
+    w = (torch.randn(n, k, device=DEV) * k ** -0.5).bfloat16()
+    bias = torch.randn(n, device=DEV, dtype=torch.bfloat16)
+    exact = a.double() @ w.double().T
+    _close(ops.gemm(a, w, out_dtype=torch.float32), exact.float(), k ** 0.5 * 2 ** -22 + 1e-6, 0)
+    # one rounding to bf16
+    _close(ops.gemm(a, w, bias, unary="relu2"), (exact.clamp_min(0) ** 2 + bias.double()).float(), 1e-3, 2 ** -8)
+    for shift in (0, 1, 2):
+        res = torch.randn(m * n + 4, device=DEV, dtype=torch.bfloat16)[shift: shift + m * n].view(m, n)
+        _close(ops.gemm(a, w, bias, res), (exact + bias.double() + res.double()).float(), 1e-3, 2 ** -8)
+    if n % 16 == 0:
+        gate, up = (exact + bias.double()).view(m, -1, 2, 8).unbind(2)
+        _close(ops.gemm(a, w, bias, swiglu=True), (torch.nn.functional.silu(gate) * up).reshape(m, -1).float(), 1e-3, 2 ** -7)
+
+
 @pytest.mark.parametrize("m,n,k", [(65, 18944, 72), (129, 20000, 200), (257, 130, 64), (300, 1000, 136), (1023, 384, 1048),
                                    (1025, 257, 8), (2000, 48, 520), (33, 304, 128)])
 def test_gemm_pair_rows(m, n, k):
