@@ -68,6 +68,15 @@ __device__ __forceinline__ void store_gated_columns(const float (&v)[16], __nv_b
   }
 }
 
+// fp32 results without an activation: the 32 lanes' values of a row are 128 neighbouring bytes as they are.
+__device__ __forceinline__ void store_fp32_columns(const float (&v)[16], float* C, long long ldc, int n, int N, int rows) {
+  if (n >= N) return;
+  C += n;
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    if (i < rows) C[i * ldc] = v[i];
+}
+
 // Whether two neighbouring columns can be stored as one word.
 __device__ __forceinline__ bool columns_pair(const void* C, long long ldc, int N, bool gated) {
   return ((reinterpret_cast<uintptr_t>(C) & 3) == 0) && (ldc & 1) == 0 && (gated || (N & 1) == 0);

@@ -308,6 +308,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     // bf16 results without a residual, and without a bias behind a unary activation, are stored in pairs of columns
     const bool plain = act_is_gated(p.act) || (!p.out_fp32 && !p.residual && !(p.bias && act_is_unary(p.act)));
     const bool pairs = columns_pair(p.C, p.ldc, p.N, act_is_gated(p.act));
+    const bool plain32 = !GROUPED && p.out_fp32 && !p.residual && p.act == kActNone;
     int cursor = 0, acc = 0;
     uint32_t acc_phase = 0;
     PairTile tile;
@@ -345,6 +346,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           for (int i = 0; i < 16; ++i) x[i] += bias;
           store_act_columns(p.act, p.act_alpha, p.act_limit, x, static_cast<__nv_bfloat16*>(p.C) + at, p.ldc, n, p.N, rows,
                             pairs);
+        } else if (plain32) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) x[i] += bias;
+          store_fp32_columns(x, static_cast<float*>(p.C) + at, p.ldc, n, p.N, rows);
         } else if (n < p.N) {
           float add[16];
 #pragma unroll

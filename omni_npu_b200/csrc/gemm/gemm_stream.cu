@@ -369,6 +369,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     // bf16 results without a residual, and without a bias behind a unary activation: stored in pairs of columns
     const bool plain = !p.out_fp32 && !p.residual && !(p.bias && act_is_unary(p.act));
     const bool pairs = columns_pair(p.C, p.ldc | (BATCHED ? p.c_group : 0), p.N, act_is_gated(p.act));
+    const bool plain32 = MODE == kStreamDense && p.out_fp32 && !p.residual && p.act == kActNone;
     int cursor = 0, acc = 0;
     uint32_t acc_phase = 0;
     StreamTile tile;
@@ -383,7 +384,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       tc_fence_after_sync();
       const uint32_t col = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc * acc_stride);
       const int col_n = tile.n0 + r;
-      const float bias = plain && p.bias && col_n < p.N ? __bfloat162float(p.bias[col_n]) : 0.f;
+      const float bias = (plain || plain32) && p.bias && col_n < p.N ? __bfloat162float(p.bias[col_n]) : 0.f;
       float* part = reinterpret_cast<float*>(smem);      // split K: [row of A][128] (the ring has been read)
       for (int c = 0; c < tile.rows; c += 16) {
         uint32_t v[16];
@@ -408,6 +409,11 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                             static_cast<__nv_bfloat16*>(p.C) + (BATCHED ? tile.expert * p.c_group : 0) +
                                 static_cast<size_t>(tile.row0 + c) * p.ldc,
                             p.ldc, col_n, p.N, n, pairs);
+        } else if (plain32) {
+          float x[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(v[i]) + bias;
+          store_fp32_columns(x, static_cast<float*>(p.C) + static_cast<size_t>(tile.row0 + c) * p.ldc, p.ldc, col_n, p.N, n);
         } else {
 #pragma unroll
           for (int i = 0; i < 16; ++i)
