@@ -350,32 +350,53 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
   tc_fence_before_sync();
   __syncthreads();
   if constexpr (SPLIT) {
-    // one tile per CTA: the CTAs of the cluster share out its rows of A
+    // one tile per CTA: the CTAs of the cluster share out its rows of A, a row per warp and four columns per lane
+    // (gemm_stream.cu; 64 rows of 4096 x 1024 in two parts 12.4 us with all warps on one row, 8.2)
     cluster_sync_all();
     if (warp >= 2 && !*abort_flag) {
-      const int r = (warp & 3) * 32 + lane;
-      const int n = t_first * BW + r;
-      const float bias = p.bias && n < p.N ? __bfloat162float(p.bias[n]) : 0.f;
-      for (int row = rank; row < p.M; row += p.splits) {
-        const uint32_t at = smem_u32(smem) + static_cast<uint32_t>((row * BW + r) * 4);
-        float v[8];
+      const int n = t_first * BW + 4 * lane;
+      float bias[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) bias[i] = p.bias && n + i < p.N ? __bfloat162float(p.bias[n + i]) : 0.f;
+      const bool wide = n + 3 < p.N && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C) & (p.out_fp32 ? 15 : 7)) == 0;
+      for (int row = rank + p.splits * (warp - 2); row < p.M; row += 4 * p.splits) {
+        const uint32_t at = smem_u32(smem) + static_cast<uint32_t>((row * BW + 4 * lane) * 4);
+        float v[8][4];
 #pragma unroll
         for (int s = 0; s < 8; ++s) {
-          v[s] = 0.f;
-          if (s < p.splits)
-            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[s]) : "r"(mapa_shared(at, s)) : "memory");
-        }
-        float sum = v[0];
 #pragma unroll
-        for (int s = 1; s < 8; ++s) sum += v[s];
-        if (n >= p.N) continue;
+          for (int i = 0; i < 4; ++i) v[s][i] = 0.f;
+          if (s < p.splits)
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v[s][0]), "=f"(v[s][1]), "=f"(v[s][2]), "=f"(v[s][3])
+                         : "r"(mapa_shared(at, s))
+                         : "memory");
+        }
         const size_t o = static_cast<size_t>(row) * p.ldc + n;
-        sum += bias;
-        if (p.residual) sum += __bfloat162float(p.residual[o]);
-        if (p.out_fp32)
-          static_cast<float*>(p.C)[o] = sum;
-        else
-          static_cast<__nv_bfloat16*>(p.C)[o] = __float2bfloat16(sum);
+        float sum[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          sum[i] = v[0][i];
+#pragma unroll
+          for (int s = 1; s < 8; ++s) sum[i] += v[s][i];
+          sum[i] += bias[i];
+          if (p.residual && n + i < p.N) sum[i] += __bfloat162float(p.residual[o + i]);
+        }
+        if (wide && p.out_fp32) {
+          *reinterpret_cast<float4*>(static_cast<float*>(p.C) + o) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+        } else if (wide) {
+          *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.C) + o) =
+              make_uint2(columns_pack(sum[0], sum[1]), columns_pack(sum[2], sum[3]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (n + i >= p.N) break;
+            if (p.out_fp32)
+              static_cast<float*>(p.C)[o + i] = sum[i];
+            else
+              static_cast<__nv_bfloat16*>(p.C)[o + i] = __float2bfloat16(sum[i]);
+          }
+        }
       }
     }
     cluster_sync_all();

@@ -103,7 +103,8 @@ def test_head_norms_keep_an_eps_of_their_own():
     assert norms == [1e-6, 10.0] and (run() - got).abs().max() > 1e-3
 
 
-@pytest.mark.parametrize("n,k", [(128, 4096), (4096, 4096), (4096, 7168), (18944, 2048), (130, 256), (640, 64)])
+@pytest.mark.parametrize("n,k", [(128, 4096), (4096, 4096), (4096, 7168), (4700, 4096), (9216, 4096), (9000, 4096),
+                                 (18944, 2048), (130, 256), (640, 64)])
 def test_split_products_keep_within_a_limit_of_ctas(n, k):
     """A product that shares K among CTAs uses no more of them than its caller allows, and all of K's slabs."""
     splits = ops._core().gemm_stream_splits
@@ -113,6 +114,7 @@ def test_split_products_keep_within_a_limit_of_ctas(n, k):
         assert s in (1, 2, 4, 8) and (s == 1 or tiles * s <= min(limit or 296, 296))
         assert s == 1 or ((s - 1) * -(-slabs // s) < slabs and -(-slabs // s) >= 4)
         assert s <= splits(n, k, 0, 148)
+        assert tiles * s <= {1: tiles, 2: 296, 4: 284, 8: 264}[s]          # clusters that are resident at once
 
 
 @pytest.mark.parametrize("quant", [None, "fp8"])
