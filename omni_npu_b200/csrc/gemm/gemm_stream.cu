@@ -6,9 +6,10 @@
 // shared memory: two are resident, or one and the next kernel's, whose first ring of weights then flows while this
 // kernel finishes.
 //
-// Dense: N / 128 tiles; when these are fewer than the resident CTAs, the 2, 4 or 8 CTAs of a cluster share a tile's
+// Dense: N / 128 tiles; when these are fewer than half the SMs, the 2, 4 or 8 CTAs of a cluster share a tile's
 // K and sum their parts in rank order over distributed shared memory.  The split depends on N and K alone, so the
-// result of a row does not depend on the number of rows.
+// result of a row does not depend on the number of rows, up to the 128 that the kernel takes; products without a split
+// have the same bits on every kernel for bf16 operands (all add up K in steps of 16 in the tensor cores).
 // Grouped: tiles of all live experts, each read once; an expert with more rows than a tile takes several tiles side by
 // side, which share its weights in L2.
 // Batched: the same number of rows for every group, A and C with strides of their own for rows and groups (the heads of
@@ -508,9 +509,13 @@ static int launch_stream(const CUtensorMap& tw, const CUtensorMap& tx, const Str
 
 using namespace b200;
 
-// CTAs of a cluster that b200_gemm_stream has share the K of one tile.
+// CTAs of a cluster that b200_gemm_stream has share the K of one tile.  None where one CTA on half the SMs takes in what
+// the memory gives, nor for short rows, where the exchange costs what the split gains (us, no split / two parts, with 1 and
+// 64 rows: 12288 x 2048 with silu 13.4 / 13.9 and 15.9 / 19.9, 16384 x 2048 14.4 / 14.6 and 16.9 / 18.2, 18944 x 4096
+// 30.8 / 27.7 and 34.2 / 31.7, 2048 x 512 5.0 / 4.7 and 7.0 / 7.5).
 extern "C" int b200_gemm_stream_splits(int N, int K, int max_ctas, int sms) {
-  return stream_splits((N + stream::BW - 1) / stream::BW, (K + stream::SLAB_K - 1) / stream::SLAB_K, max_ctas, sms);
+  const int tiles = (N + stream::BW - 1) / stream::BW, slabs = (K + stream::SLAB_K - 1) / stream::SLAB_K;
+  return 2 * tiles > sms || slabs <= 8 ? 1 : stream_splits(tiles, slabs, max_ctas, sms);
 }
 
 // A [M <= 128, K] (pitch lda), W [N, K] (pitch ldw), C [M, N, or N / 2 with a gated activation].  splits 0: by rule.
@@ -530,7 +535,7 @@ extern "C" int b200_gemm_stream(const void* A, const void* W, void* C, const voi
   p.stages = stream_stages(p.tn);
   p.k_slabs = (K + stream::SLAB_K - 1) / stream::SLAB_K;
   p.num_n_tiles = (N + stream::BW - 1) / stream::BW;
-  p.splits = splits > 0 ? splits : stream_splits(p.num_n_tiles, p.k_slabs, max_ctas, sm_count());
+  p.splits = splits > 0 ? splits : b200_gemm_stream_splits(N, K, max_ctas, sm_count());
   if (p.splits != 1 && p.splits != 2 && p.splits != 4 && p.splits != 8) return -12;
   if ((p.splits - 1) * ((p.k_slabs + p.splits - 1) / p.splits) >= p.k_slabs) return -12;
   p.ldc = ldc;

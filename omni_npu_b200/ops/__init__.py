@@ -187,14 +187,14 @@ def check_status(device: Optional[torch.device] = None) -> None:
 SILU = (0.0, 0.0)          # gated activation silu(gate) * up: no slope, no limit
 # smallest M always routed to the CTA-pair GEMM (0 = never)
 PAIR_MIN_M = int(os.environ.get("OMNI_B200_GEMM_PAIR_MIN_M", "1024"))
-# ... and above this many bf16 rows products whose plan has no K split (gated, or wide enough to fill the SMs).  Us,
-# gemm_tcgen05_kernel / gemm_pair_kernel: 5632 x 2048 with silu 17.2 / 12.8 at 100 rows,
-# 24.6 / 16.7 at 512; 102400 x 2048 119 / 88.5 at 200, 317 / 223 at 700; 4096 x 4096 25.4 / 20.6 at 400.  With a split K
-# 128 x 2048 takes 7.9 / 10.6 at 200.
+# ... and above this many bf16 rows products whose plan has no K split (gated, or wide enough to fill the SMs), unless the
+# rules for up to 128 rows below say otherwise.  Us, gemm_tcgen05_kernel / gemm_pair_kernel: 5632 x 2048 with silu
+# 19.3 / 13.4 at 256 rows, 24.6 / 16.7 at 512; 102400 x 2048 119 / 88.5 at 200, 317 / 223 at 700; 4096 x 4096 25.4 / 20.6 at
+# 400.  With a split K 128 x 2048 takes 7.9 / 10.6 at 200.
 PAIR_UNSPLIT_M = 64
 # Plain bf16 products (no residual, SwiGLU, scales or fused collective) of a decode-sized batch
 # whose plan here is a cluster split-K: "library" hands them to cuBLAS, "own" keeps them on
-# gemm_tcgen05_kernel.  Measured at M = 128 inside a CUDA graph (us, own / cuBLAS): 4096 x 4096
+# gemm_stream_kernel (128 rows) and gemm_tcgen05_kernel.  Measured at M = 128 inside a CUDA graph (us, own / cuBLAS): 4096 x 4096
 # 19.0 / 10.6, 6144 x 4096 20.2 / 12.6, 4096 x 14336 37.4 / 26.3: every CTA of the own kernel re-reads
 # the 128-row activation slab of its K slice and the K slices meet in a 3-4 us exchange, which a
 # library kernel that may share one activation load between the CTAs of a cluster does not pay.
@@ -203,16 +203,20 @@ PAIR_UNSPLIT_M = 64
 SMALL_M_GEMM = os.environ.get("OMNI_B200_SMALL_M_GEMM", "library")
 SMALL_M_LIBRARY_ROWS = (64, 256)
 
-# Products with fewer bf16 rows than this stream their weights through gemm_stream_kernel; up to 128 rows with this many
-# weight rows at least (every SM then has a tile without splitting K).  Measured in a CUDA graph (us,
-# gemm_tcgen05_kernel / gemm_stream_kernel) with 1 and 63 rows: 4096 x 4096 17.5 / 9.2 and 17.6 / 12.5, 28672 x 4096 with
-# silu 71 / 40.6 and 60 / 43.3, 128256 x 4096 190 / 163 and 176 / 169; with 128 rows 61 / 47.4 and 184 / 181, but
-# 6144 x 4096 20 / 24: the rows of A, read again for every 128 columns, then weigh as much as the weights.
-STREAM_ROWS = 64
-STREAM_WIDE_ROWS, STREAM_WIDE_N = 128, 148 * 128
-# ... and with fewer than 64 weight rows (a small router), for which the other kernel has no split of K: 128 rows,
-# 32 x 7168, 35.7 / 13.4.
-STREAM_NARROW_N = 64
+# Products with at most this many bf16 rows whose weights gemm_stream_kernel shares out along K stream them through it, so
+# that the result of a row is the same for 1 to 128 rows (a decode step padded to a captured size gives the numbers of the
+# unpadded one); those that cuBLAS takes (above) change there.  Measured in a CUDA graph (us, gemm_tcgen05_kernel /
+# gemm_stream_kernel) with 1, 64 and 128 rows: 4096 x 4096 17.8 / 9.2, 17.6 / 11.8 and 19.0 / 14.9, 6144 x 4096 22 / 12.7,
+# 19.5 / 15.6 and 20.5 / 18.5, 64 x 2048 7.5 / 4.4, 7.5 / 6.0 and 7.9 / 7.6, 5632 x 2048 with silu 21.6 / 8.4, 17.3 / 12.4 and
+# 17.4 / 16.4 (12.8 on CTA pairs, which have no split).
+STREAM_ROWS = 128
+# Without a split all kernels give the same bits, and the row count may choose: up to 63 rows, up to 128 with this many weight
+# rows at least (every SM has a tile: 28672 x 4096 with silu 71 / 40.6 with one row, 61 / 47.4 with 128, 128256 x 4096
+# 190 / 163 and 184 / 181) or fewer than 64 (a small router: 32 x 7168 35.7 / 13.4 with 128), but only up to 16 between half
+# the SMs' tiles and all of them, where CTA pairs read the rows of A half as often (us, streaming / pairs: 12288 x 4096
+# 22.7 / 21.7 with one row, 23.3 / 20.9 with 16, 26.3 / 21.7 with 64; 12288 x 2048 with silu 13.4 / 13.7, 13.8 / 13.8, 15.9 / 14.1).
+STREAM_UNSPLIT_ROWS, STREAM_HALF_ROWS, STREAM_HALF_N = 63, 16, 74 * 128
+STREAM_WIDE_N, STREAM_NARROW_N = 148 * 128, 64
 
 GELU_TANH = "gelu_tanh"    # gated activation gelu(gate) * up, gelu in its tanh form
 RELU = "relu"              # gated activation max(gate, 0) * up
@@ -238,6 +242,19 @@ def library_small_m(m: int, cluster_split_plan: bool, plain_bf16: bool) -> bool:
     counts the comparison was measured on, and only while ``OMNI_B200_SMALL_M_GEMM`` says so."""
     return (SMALL_M_GEMM == "library" and plain_bf16 and cluster_split_plan
             and SMALL_M_LIBRARY_ROWS[0] <= m <= SMALL_M_LIBRARY_ROWS[1])
+
+
+@functools.lru_cache(maxsize=4096)
+def stream_parts(n: int, k: int, max_ctas: int = 0, sms: int = 148) -> int:
+    """CTAs that share the K of a tile of 128 weight rows in gemm_stream_kernel."""
+    return _core().gemm_stream_splits(n, k, max_ctas, sms)
+
+
+def stream_rows(n: int, k: int, max_ctas: int = 0, pair: bool = True) -> int:
+    """Most bf16 rows for which an [n, k] weight is streamed (``pair``: whether the CTA-pair kernel may take more)."""
+    if stream_parts(n, k, max_ctas) > 1 or n >= STREAM_WIDE_N or n < STREAM_NARROW_N or not pair:
+        return STREAM_ROWS
+    return STREAM_HALF_ROWS if n > STREAM_HALF_N else STREAM_UNSPLIT_ROWS
 
 
 def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
@@ -269,34 +286,38 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
     st = device_state(a.device)
     m, k = a.shape
     n = w.shape[0]
-    by_rule = pair is None
-    if by_rule:
-        pair = PAIR_MIN_M > 0 and m >= PAIR_MIN_M and splits == 0 and bn == 0
+    by_rule = pair is None and bn == 0 and splits == 0
+    pairs = by_rule and PAIR_MIN_M > 0
+    if pair is None:
+        pair = pairs and m >= PAIR_MIN_M
+
+    def run(kernel):
+        _count(1)
+        return kernel(a, w, bias, residual, out_dtype == torch.float32, kind[0], bn, st.status, max_ctas, kind[1], kind[2],
+                      w_ready)
+
     if pair:
-        _count(1)
-        return C.gemm_pair(a, w, bias, residual, out_dtype == torch.float32, kind[0], bn, st.status, max_ctas,
-                           kind[1], kind[2], w_ready)
+        return run(C.gemm_pair)
     fused, gated = kind[0] != 0, kind[0] in (1, 2, 4, 7)
-    if ((m < STREAM_ROWS or m <= STREAM_WIDE_ROWS and (n >= STREAM_WIDE_N or n < STREAM_NARROW_N))
-            and a.dtype == torch.bfloat16 and bn == 0 and splits == 0
-            and not (gated and (residual is not None or out_dtype == torch.float32))):
-        _count(1)
-        return C.gemm_stream(a, w, bias, residual, out_dtype == torch.float32, kind[0], 0, st.status, max_ctas, kind[1],
-                             kind[2], w_ready)
+    free = a.dtype == torch.bfloat16 and bn == 0 and splits == 0
+    plain = free and residual is None and not fused and out_dtype in (None, torch.bfloat16)
+    few = None           # the kernel of up to 128 rows
+    if free and m <= STREAM_ROWS and not (gated and (residual is not None or out_dtype == torch.float32)):
+        few = C.gemm_stream if m <= stream_rows(n, k, max_ctas, pairs) else C.gemm_pair
+        if not (plain and library_small_m(m, True, True)):      # (cuBLAS's products depend on gemm_tcgen05_kernel's plan)
+            return run(few)
     key = (m, n, k, a.dtype.itemsize, kind[0], bn, splits)
     plan = st.plans.get(key)
     if plan is None:
         plan = C.gemm_plan(m, n, k, a.dtype.itemsize, gated, bn, 1 if gated else max(0, splits) if fused else splits)
         st.plans[key] = plan
     pbn, psplits, ws_bytes, ncnt, cluster = plan
-    if by_rule and m > PAIR_UNSPLIT_M and 0 < PAIR_MIN_M and a.dtype == torch.bfloat16 and bn == 0 and splits == 0 \
-            and psplits == 1:
-        _count(1)
-        return C.gemm_pair(a, w, bias, residual, out_dtype == torch.float32, kind[0], 0, st.status, max_ctas,
-                           kind[1], kind[2], w_ready)
-    if library_small_m(m, bool(cluster), residual is None and not fused and bn == 0
-                       and splits == 0 and a.dtype == torch.bfloat16 and out_dtype in (None, torch.bfloat16)):
+    if plain and library_small_m(m, bool(cluster), True):
         return torch.nn.functional.linear(a, w, bias)    # a library kernel: not counted as a launch of ours
+    if few is not None:
+        return run(few)
+    if pairs and free and psplits == 1 and m > PAIR_UNSPLIT_M:
+        return run(C.gemm_pair)
     ws = cnt = None
     if psplits > 1 and not cluster:
         ws, cnt = st.gemm_workspace(torch.cuda.current_stream(a.device).cuda_stream, ws_bytes, ncnt)

@@ -144,3 +144,13 @@ def test_experts_choose_kernels_by_the_rows_of_the_step(monkeypatch, quant):
 def test_rows_of_a_step_choose_the_grouped_kernel():
     few, many = ops.grouped_rows_tile(16, 16, 1536), ops.grouped_rows_tile(131072, 16, 1536)
     assert few > 0 and many == 0            # streamed weights; CTA pairs
+
+
+def test_rows_that_stream_their_weights():
+    """Split products up to 128 rows whatever their width; others where the kernel is the fastest of equal ones."""
+    assert ops.stream_parts(4096, 4096) > 1 and ops.stream_rows(4096, 4096) == 128
+    assert ops.stream_parts(12288, 4096) == 1 and ops.stream_rows(12288, 4096) == 16
+    assert ops.stream_rows(12288, 4096, 0, False) == 128            # without the CTA-pair kernel
+    assert ops.stream_parts(2048, 512) == 1 and ops.stream_rows(2048, 512) == 63
+    assert ops.stream_rows(128256, 4096) == ops.stream_rows(32, 256) == 128
+    assert ops.stream_rows(4096, 4096, 8) == 63                     # a limit of CTAs leaves no split

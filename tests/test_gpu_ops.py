@@ -192,7 +192,7 @@ def test_gemm_few_rows(m, n, k):
     ops.check_status()
 
 
-@pytest.mark.parametrize("m,n,k", [(63, 2048, 512), (64, 130, 512), (33, 1000, 1024), (3, 48, 4096), (62, 258, 2048), (128, 56, 4096)])
+@pytest.mark.parametrize("m,n,k", [(63, 2048, 576), (64, 130, 576), (33, 1000, 1024), (3, 48, 4096), (62, 258, 2048), (128, 56, 4096)])
 def test_gemm_few_rows_split(m, n, k):
     """Sums over the CTAs of a cluster, four columns at a time: columns left over, results and residuals off 16 bytes."""
     torch.manual_seed(m + n + k)
@@ -210,6 +210,39 @@ def test_gemm_few_rows_split(m, n, k):
     if n % 16 == 0:
         gate, up = (exact + bias.double()).view(m, -1, 2, 8).unbind(2)
         _close(ops.gemm(a, w, bias, swiglu=True), (torch.nn.functional.silu(gate) * up).reshape(m, -1).float(), 1e-3, 2 ** -7)
+
+
+@pytest.mark.parametrize("n,k", [(64, 2048), (256, 7168), (4096, 4096), (6144, 4096), (9216, 2048), (12288, 2048), (18944, 1024),
+                                 (20000, 512), (2048, 512), (5632, 2048), (1000, 1408), (48, 256), (130, 4096)])
+def test_a_row_does_not_depend_on_the_rows_beside_it(n, k, monkeypatch):
+    """1 to 128 rows, on whichever kernels: a decode step padded to a captured size gives the unpadded one's numbers.
+    (Plain products of 64 rows and more may be cuBLAS's.)"""
+    torch.manual_seed(n + k)
+    a = torch.randn(128, k, device=DEV, dtype=torch.bfloat16)
+    w = (torch.randn(n, k, device=DEV) * k ** -0.5).bfloat16()
+    res = torch.randn(128, n, device=DEV, dtype=torch.bfloat16)
+    forms = [lambda m: ops.gemm(a[:m], w, out_dtype=torch.float32), lambda m: ops.gemm(a[:m], w, residual=res[:m]),
+             lambda m: ops.gemm(a[:m], w, unary="relu2")] + ([lambda m: ops.gemm(a[:m], w, swiglu=True)] if n % 16 == 0 else [])
+    monkeypatch.setattr(ops, "SMALL_M_GEMM", "own")
+    forms.append(lambda m: ops.gemm(a[:m], w))
+    for form in forms:
+        want = form(128)
+        for m in (1, 15, 16, 17, 33, 63, 64, 65, 96, 127):
+            assert torch.equal(form(m), want[:m]), (m,)
+
+
+@pytest.mark.parametrize("n,k", [(4096, 2048), (640, 1024), (18432, 512), (130, 256)])
+def test_an_e4m3_row_does_not_depend_on_the_rows_beside_it(n, k):
+    """On either side of the 64 rows that the weight-streaming kernel takes."""
+    torch.manual_seed(n + k)
+    q, s = ops.quant_fp8_1x128(torch.randn(300, k, device=DEV, dtype=torch.bfloat16))
+    w, ws = torch.randn(n, k, device=DEV).to(torch.float8_e4m3fn), torch.rand(-(-n // 128), k // 128, device=DEV)
+    want = ops.gemm_fp8_block(q, s, w, ws, out_dtype=torch.float32)
+    few = ops.gemm_fp8_block(q[:64], s[:64], w, ws, out_dtype=torch.float32)
+    for m in (1, 31, 32, 33, 63):
+        assert torch.equal(ops.gemm_fp8_block(q[:m], s[:m], w, ws, out_dtype=torch.float32), few[:m]), (m,)
+    for m in (65, 128, 129, 257):
+        assert torch.equal(ops.gemm_fp8_block(q[:m], s[:m], w, ws, out_dtype=torch.float32), want[:m]), (m,)
 
 
 @pytest.mark.parametrize("m,n,k", [(65, 18944, 72), (129, 20000, 200), (257, 130, 64), (300, 1000, 136), (1023, 384, 1048),
