@@ -100,17 +100,21 @@ argmax_kernel(const T* __restrict__ logits, int* __restrict__ out, int V, long l
 }
 
 // ---------------------------------------------------------------------------------------------- sampling
-// A thread-block cluster of eight CTAs per row.  Each CTA keeps its eighth of the row in shared memory, so
+// A thread-block cluster of CTAS = 8, 4 or 1 CTAs per row.  Each CTA keeps its part of the row in shared memory, so
 // that a row of 128 k fp32 logits is read from device memory once and the later passes (threshold of top-k,
 // threshold of top-p, draw) run from shared memory on eight SMs.  One CTA of 1024 threads per row, reading
 // the row from memory in every pass, took 615 us for 128 rows x 128256 (its histogram over the leading key bits
 // put most of the vocabulary into some thirty counters, and one thread walked the 2048 counters); this form is
 // bound by the passes over shared memory.
-static constexpr int kRowCtas = 8;
+// A row of temperature alone needs no threshold and is drawn from as it is read, without shared memory.
+// Fewer CTAs for short rows, whose time is the exchanges': see launch_sample.
+static constexpr int kMaxRowCtas = 8;
 static constexpr int kRowThreads = 512;
 static constexpr int kBins = 2048;
 static constexpr int kMaxKeys = kBins / 2;
 static constexpr int kMaxSlice = 50 * 1024;     // logits of a slice that fit shared memory
+// Rows of at most this many logits take one CTA, four CTAs.
+static constexpr int kOneCtaRow = 8 * 1024, kFourCtaRow = 48 * 1024;
 
 struct RowShared {
   union {
@@ -125,9 +129,9 @@ struct RowShared {
   MaxIdx red[32];
   float warp_sum[kRowThreads / 32];
   // one entry per CTA, which writes it into every CTA's copy: weight of its bins, its first bin at the target, weight before it
-  float share[kRowCtas];
-  int first[kRowCtas];
-  float before[kRowCtas];
+  float share[kMaxRowCtas];
+  int first[kMaxRowCtas];
+  float before[kMaxRowCtas];
   int own_first;
   float own_before;
   // CTA 0's, read by all
@@ -151,33 +155,40 @@ __device__ __forceinline__ void remote_store(const void* p, int rank, uint32_t v
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote_smem(p, rank)), "r"(v) : "memory");
 }
 __device__ __forceinline__ float remote_f32(const void* p, int rank) { return __uint_as_float(remote_u32(p, rank)); }
+template <int CTAS>
 __device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if constexpr (CTAS == 1)
+    __syncthreads();
+  else
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Best of the eight slices' entries (every thread of every CTA gets it); ends with all CTAs past the exchange.
+// Best of the slices' entries (every thread of every CTA gets it); ends with all CTAs past the exchange.
+template <int CTAS>
 __device__ __forceinline__ MaxIdx row_best(MaxIdx m, RowShared* sh) {
   m = block_argmax(m, sh->red);
-  if (threadIdx.x == 0) sh->top = m;
-  cluster_barrier();
+  if constexpr (CTAS > 1) {
+    if (threadIdx.x == 0) sh->top = m;
+    cluster_barrier<CTAS>();
 #pragma unroll
-  for (int r = 0; r < kRowCtas; ++r)
-    m = better(m, MaxIdx{remote_f32(&sh->top.v, r), static_cast<int>(remote_u32(&sh->top.i, r))});
-  cluster_barrier();
+    for (int r = 0; r < CTAS; ++r)
+      m = better(m, MaxIdx{remote_f32(&sh->top.v, r), static_cast<int>(remote_u32(&sh->top.i, r))});
+    cluster_barrier<CTAS>();
+  }
   return m;
 }
 
 // One pass of counters over the slices: ``bin_of(x)`` in [0, kBins) grows as logits fall, or is negative for
 // logits that take no part.  Finds the first bin at which the weight of the bins up to it reaches the target
-// (``target`` times the whole weight if SHARE); bin = -1 if rounding keeps the sum below the target.  Every CTA adds up an
-// eighth of the bins over the row's CTAs, one per thread.  (One CTA adding up all of them, 32 words of the other CTAs'
+// (``target`` times the whole weight if SHARE); bin = -1 if rounding keeps the sum below the target.  Every CTA adds up its
+// part of the bins over the row's CTAs.  (One CTA adding up all of them, 32 words of the other CTAs'
 // shared memory per thread, held the seven others up: 112.6 us for the mixture of 128 rows x 128256, 97.2 in this form.)
 struct PassResult {
   int bin;
   float above, target;
 };
 
-template <bool MASS, bool SHARE, typename Load, typename Bin>
+template <int CTAS, bool MASS, bool SHARE, typename Load, typename Bin>
 __device__ PassResult count_pass(Load load, int n, int rank, Bin bin_of, float target, float scale_log2, float max_scaled,
                                  RowShared* sh) {
   for (int i = threadIdx.x; i < kBins; i += kRowThreads) sh->count[i] = 0u;    // also 0.f
@@ -204,19 +215,24 @@ __device__ PassResult count_pass(Load load, int n, int rank, Bin bin_of, float t
     else
       atomicAdd(&sh->count[kBins - 1], static_cast<uint32_t>(far));
   }
-  cluster_barrier();
-  constexpr int OWN = kBins / kRowCtas;
-  static_assert(OWN <= kRowThreads, "a bin per thread");
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float w = 0.f;
-  if (threadIdx.x < OWN) {
-    uint32_t v[kRowCtas];
+  cluster_barrier<CTAS>();
+  constexpr int OWN = kBins / CTAS, PER = OWN > kRowThreads ? OWN / kRowThreads : 1;      // bins of a CTA, of a thread
+  static_assert(OWN % PER == 0 && OWN / PER <= kRowThreads, "bins of the threads");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, bin0 = rank * OWN + threadIdx.x * PER;
+  float w[PER], sum = 0.f;
 #pragma unroll
-    for (int r = 0; r < kRowCtas; ++r) v[r] = remote_u32(&sh->count[rank * OWN + threadIdx.x], r);
+  for (int i = 0; i < PER; ++i) {
+    w[i] = 0.f;
+    if (threadIdx.x < OWN / PER) {
+      uint32_t v[CTAS];
 #pragma unroll
-    for (int r = 0; r < kRowCtas; ++r) w += MASS ? __uint_as_float(v[r]) : static_cast<float>(v[r]);
+      for (int r = 0; r < CTAS; ++r) v[r] = CTAS == 1 ? sh->count[bin0 + i] : remote_u32(&sh->count[bin0 + i], r);
+#pragma unroll
+      for (int r = 0; r < CTAS; ++r) w[i] += MASS ? __uint_as_float(v[r]) : static_cast<float>(v[r]);
+    }
+    sum += w[i];
   }
-  float incl = w;
+  float incl = sum;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const float up = __shfl_up_sync(0xffffffffu, incl, o);
@@ -231,35 +247,44 @@ __device__ PassResult count_pass(Load load, int n, int rank, Bin bin_of, float t
     }
   }
   __syncthreads();
-  float run = incl - w, own = 0.f;
+  float run = incl - sum, own = 0.f;
 #pragma unroll
-  for (int i = 0; i < OWN / 32; ++i) {
+  for (int i = 0; i < OWN / PER / 32; ++i) {
     if (i < warp) run += sh->warp_sum[i];
     own += sh->warp_sum[i];
   }
-  if (threadIdx.x < kRowCtas) remote_store(&sh->share[rank], threadIdx.x, __float_as_uint(own));
-  cluster_barrier();
+  if (threadIdx.x < CTAS) remote_store(&sh->share[rank], threadIdx.x, __float_as_uint(own));
+  cluster_barrier<CTAS>();
   float total = 0.f;
 #pragma unroll
-  for (int r = 0; r < kRowCtas; ++r) {
+  for (int r = 0; r < CTAS; ++r) {
     if (r < rank) run += sh->share[r];
     total += sh->share[r];
   }
   if (SHARE) target *= total;
   // an empty bin is never chosen; the smallest bin that qualifies is
-  const bool mine = threadIdx.x < OWN && w > 0.f && run + w >= target;
-  if (mine) atomicMin(&sh->own_first, rank * OWN + static_cast<int>(threadIdx.x));
+  int mine = -1;
+  float mine_before = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    if (mine < 0 && w[i] > 0.f && run + w[i] >= target) {
+      mine = bin0 + i;
+      mine_before = run;
+    }
+    run += w[i];
+  }
+  if (mine >= 0) atomicMin(&sh->own_first, mine);
   __syncthreads();
-  if (mine && sh->own_first == rank * OWN + static_cast<int>(threadIdx.x)) sh->own_before = run;
+  if (mine >= 0 && sh->own_first == mine) sh->own_before = mine_before;
   __syncthreads();
-  if (threadIdx.x < kRowCtas) {
+  if (threadIdx.x < CTAS) {
     remote_store(&sh->first[rank], threadIdx.x, static_cast<uint32_t>(sh->own_first));
     remote_store(&sh->before[rank], threadIdx.x, __float_as_uint(sh->own_before));
   }
-  cluster_barrier();
+  cluster_barrier<CTAS>();
   PassResult res{-1, 0.f, target};
 #pragma unroll
-  for (int r = kRowCtas - 1; r >= 0; --r)
+  for (int r = CTAS - 1; r >= 0; --r)
     if (sh->first[r] != 0x7fffffff) {
       res.bin = sh->first[r];
       res.above = sh->before[r];
@@ -272,7 +297,7 @@ __device__ PassResult count_pass(Load load, int n, int rank, Bin bin_of, float t
 // The first counters are linear in the logit (1/32 of a power of two of probability below the maximum), which
 // spreads a vocabulary over them; the keys of the chosen bin are then compared with one another, or, if there are
 // more than kMaxKeys of them (equal logits), go through counters of their key bits.
-template <bool MASS, typename Load>
+template <int CTAS, bool MASS, typename Load>
 __device__ uint32_t row_threshold(Load load, int n, int rank, float target, uint32_t floor_key, float scale_log2,
                                   float max_scaled, RowShared* sh) {
   const auto linear = [=](float x) {
@@ -280,7 +305,7 @@ __device__ uint32_t row_threshold(Load load, int n, int rank, float target, uint
     return float_key(x) < floor_key ? -1 : min(max(b, 0), kBins - 1);
   };
   if (!(target > 0.f)) return 0xffffffffu;      // top_p <= 0: nothing qualifies, the caller falls back to the maximum
-  const PassResult first = count_pass<MASS, MASS>(load, n, rank, linear, target, scale_log2, max_scaled, sh);
+  const PassResult first = count_pass<CTAS, MASS, MASS>(load, n, rank, linear, target, scale_log2, max_scaled, sh);
   const int bin = first.bin;
   if (bin < 0) return 0u;
   target = first.target;
@@ -295,7 +320,7 @@ __device__ uint32_t row_threshold(Load load, int n, int rank, float target, uint
       asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote_smem(&sh->list.key[at], 0)), "r"(float_key(x))
                    : "memory");
   }
-  cluster_barrier();
+  cluster_barrier<CTAS>();
   const int found = static_cast<int>(remote_u32(&sh->num_keys, 0));
   if (found <= kMaxKeys) {
     if (rank == 0) {
@@ -319,7 +344,7 @@ __device__ uint32_t row_threshold(Load load, int n, int rank, float target, uint
         if (sum >= target || key == least) atomicMax(&sh->threshold, key);
       }
     }
-    cluster_barrier();
+    cluster_barrier<CTAS>();
     return remote_u32(&sh->threshold, 0);      // reset behind the first barrier of the next count_pass
   }
   uint32_t prefix = 0u, mask = 0u;
@@ -329,7 +354,7 @@ __device__ uint32_t row_threshold(Load load, int n, int rank, float target, uint
       const uint32_t key = float_key(x);
       return linear(x) != bin || (key & mask) != prefix ? -1 : 1023 - static_cast<int>((key >> shift) & 1023u);
     };
-    const PassResult res = count_pass<MASS, false>(load, n, rank, digit, target - above, scale_log2, max_scaled, sh);
+    const PassResult res = count_pass<CTAS, MASS, false>(load, n, rank, digit, target - above, scale_log2, max_scaled, sh);
     const int b = res.bin;
     if (b >= 0) above += res.above;
     const uint32_t d = b < 0 ? 0u : static_cast<uint32_t>(1023 - b);
@@ -340,24 +365,60 @@ __device__ uint32_t row_threshold(Load load, int n, int rank, float target, uint
     const uint32_t key = float_key(x);
     return linear(x) != bin || (key & mask) != prefix ? -1 : 3 - static_cast<int>(key & 3u);
   };
-  const int b = count_pass<MASS, false>(load, n, rank, tail, target - above, scale_log2, max_scaled, sh).bin;
+  const int b = count_pass<CTAS, MASS, false>(load, n, rank, tail, target - above, scale_log2, max_scaled, sh).bin;
   return prefix | (b < 0 ? 0u : static_cast<uint32_t>(3 - b));
 }
 
-template <typename T, bool CACHED>
-__global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
+struct DrawKey {
+  uint2 key;
+  uint32_t off_lo, off_hi;
+};
+__device__ __forceinline__ DrawKey draw_key(const long long* seeds, const long long* step_offset, int row) {
+  const uint64_t seed = seeds ? static_cast<uint64_t>(seeds[row]) : 0x9E3779B97F4A7C15ull;
+  const uint64_t off = step_offset ? static_cast<uint64_t>(step_offset[0]) : 0ull;
+  return {make_uint2(static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32)), static_cast<uint32_t>(off),
+          static_cast<uint32_t>(off >> 32)};
+}
+
+template <typename T, bool CACHED, int CTAS>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kRowThreads, 3)
 sample_kernel(const T* __restrict__ logits, int* __restrict__ out, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
               const long long* __restrict__ seeds, const long long* __restrict__ step_offset, int V,
               long long stride, int slice) {
   extern __shared__ __align__(16) float cached[];
   __shared__ RowShared sh;
-  const int rowi = blockIdx.x / kRowCtas;
-  const int rank = blockIdx.x % kRowCtas;
+  const int rowi = blockIdx.x / CTAS;
+  const int rank = blockIdx.x % CTAS;
   const int lo = min(V, rank * slice), n = min(V, lo + slice) - lo;
   const T* row = logits + static_cast<long long>(rowi) * stride + lo;
   const float temp = temperature ? temperature[rowi] : 1.f;
   const bool greedy = temp < 1e-5f;
+
+  const int k = top_k ? top_k[rowi] : 0;
+  const float p = top_p ? top_p[rowi] : 1.f;
+  const bool by_count = k > 0 && k < V, by_mass = p < 1.f;
+
+  // Gumbel-max over the kept set: four neighbours share a counter value
+  MaxIdx best{-INFINITY, 0x7fffffff};
+  const auto draw4 = [&](const DrawKey& d, const float (&x)[4], int i4, uint32_t floor_key) {
+    const uint4 r = philox4x32(make_uint4(static_cast<uint32_t>(lo / 4 + i4), d.off_lo, d.off_hi, static_cast<uint32_t>(rowi)),
+                               d.key);
+    const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int i = lo + i4 * 4 + j;
+      if (i4 * 4 + j >= n || float_key(x[j]) < floor_key) continue;
+      // u in (0,1]; e = -log(u) ~ Exp(1); score = x/T - log(e)
+      const float u = (static_cast<float>(rr[j] >> 8) + 1.0f) * (1.0f / 16777216.0f);
+      const float e = -__logf(u);
+      const float score = x[j] / temp - __logf(fmaxf(e, 1e-30f));
+      if (score > best.v || (score == best.v && i < best.i)) {
+        best.v = score;
+        best.i = i;
+      }
+    }
+  };
 
   // the maximum (the greedy answer), and the slice into shared memory
   MaxIdx m{-INFINITY, 0x7fffffff};
@@ -368,7 +429,27 @@ sample_kernel(const T* __restrict__ logits, int* __restrict__ out, const float* 
     }
   };
   int i0 = 0;
-  if (sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+  const bool by_four = sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(row) & 15) == 0;
+  if (!greedy && !by_count && !by_mass) {
+    // every token stays: drawn from as it is read
+    const DrawKey d = draw_key(seeds, step_offset, rowi);
+#pragma unroll 2
+    for (int i4 = threadIdx.x; i4 * 4 < n; i4 += kRowThreads) {
+      float x[4];
+      if (by_four && i4 * 4 + 3 < n) {
+        const float4 v = reinterpret_cast<const float4*>(row)[i4];
+        x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x[j] = i4 * 4 + j < n ? load_logit<T>(row, i4 * 4 + j) : -INFINITY;
+      }
+      draw4(d, x, i4, 0u);
+    }
+    best = row_best<CTAS>(best, &sh);
+    if (rank == 0 && threadIdx.x == 0) out[rowi] = best.i == 0x7fffffff ? 0 : best.i;
+    return;
+  }
+  if (by_four) {
     const float4* row4 = reinterpret_cast<const float4*>(row);
     const int n4 = n / 4;
 #pragma unroll 4
@@ -388,7 +469,7 @@ sample_kernel(const T* __restrict__ logits, int* __restrict__ out, const float* 
     if (CACHED && !greedy) cached[i] = v;
     see(v, lo + i);
   }
-  m = row_best(m, &sh);
+  m = row_best<CTAS>(m, &sh);
   if (greedy) {
     if (rank == 0 && threadIdx.x == 0) out[rowi] = m.i == 0x7fffffff ? 0 : m.i;
     return;
@@ -398,17 +479,12 @@ sample_kernel(const T* __restrict__ logits, int* __restrict__ out, const float* 
   const float max_scaled = m.v * scale_log2;
 
   uint32_t floor_key = 0;  // keep keys >= floor_key
-  const int k = top_k ? top_k[rowi] : 0;
-  if (k > 0 && k < V)
-    floor_key = row_threshold<false>(load, n, rank, static_cast<float>(k), 0u, scale_log2, max_scaled, &sh);
-  const float p = top_p ? top_p[rowi] : 1.f;
-  if (p < 1.f) floor_key = max(floor_key, row_threshold<true>(load, n, rank, p, floor_key, scale_log2, max_scaled, &sh));
+  if (by_count)
+    floor_key = row_threshold<CTAS, false>(load, n, rank, static_cast<float>(k), 0u, scale_log2, max_scaled, &sh);
+  if (by_mass)
+    floor_key = max(floor_key, row_threshold<CTAS, true>(load, n, rank, p, floor_key, scale_log2, max_scaled, &sh));
 
-  // Gumbel-max over the kept set; four neighbours share a counter value
-  const uint64_t seed = seeds ? static_cast<uint64_t>(seeds[rowi]) : 0x9E3779B97F4A7C15ull;
-  const uint64_t off = step_offset ? static_cast<uint64_t>(step_offset[0]) : 0ull;
-  const uint2 key = make_uint2(static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
-  MaxIdx best{-INFINITY, 0x7fffffff};
+  const DrawKey d = draw_key(seeds, step_offset, rowi);
   for (int i4 = threadIdx.x; i4 * 4 < n; i4 += kRowThreads) {
     float x[4];
     bool any = false;
@@ -417,49 +493,40 @@ sample_kernel(const T* __restrict__ logits, int* __restrict__ out, const float* 
       x[j] = i4 * 4 + j < n ? load(i4 * 4 + j) : 0.f;
       any |= i4 * 4 + j < n && float_key(x[j]) >= floor_key;
     }
-    if (!any) continue;
-    const uint4 r = philox4x32(make_uint4(static_cast<uint32_t>(lo / 4 + i4), static_cast<uint32_t>(off),
-                                          static_cast<uint32_t>(off >> 32), static_cast<uint32_t>(rowi)),
-                               key);
-    const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int i = lo + i4 * 4 + j;
-      if (i4 * 4 + j >= n || float_key(x[j]) < floor_key) continue;
-      // u in (0,1]; e = -log(u) ~ Exp(1); score = x/T - log(e)
-      const float u = (static_cast<float>(rr[j] >> 8) + 1.0f) * (1.0f / 16777216.0f);
-      const float e = -__logf(u);
-      const float score = x[j] / temp - __logf(fmaxf(e, 1e-30f));
-      if (score > best.v || (score == best.v && i < best.i)) {
-        best.v = score;
-        best.i = i;
-      }
-    }
+    if (any) draw4(d, x, i4, floor_key);
   }
-  best = row_best(best, &sh);
+  best = row_best<CTAS>(best, &sh);
   if (rank == 0 && threadIdx.x == 0) out[rowi] = best.i == 0x7fffffff ? (m.i == 0x7fffffff ? 0 : m.i) : best.i;
+}
+
+template <typename T, bool CACHED, int CTAS>
+int launch_sample_as(const void* logits, int* out, const float* temperature, const int* top_k, const float* top_p,
+                     const long long* seeds, const long long* step_offset, int B, int V, long long stride, int slice,
+                     cudaStream_t stream) {
+  const auto kern = sample_kernel<T, CACHED, CTAS>;
+  static DeviceOnce once;
+  int dev = 0;
+  if (CACHED && once.needed(&dev)) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSlice * 4) != cudaSuccess) return -4;
+    once.mark(dev);
+  }
+  kern<<<B * CTAS, kRowThreads, CACHED ? slice * 4 : 0, stream>>>(static_cast<const T*>(logits), out, temperature, top_k,
+                                                                 top_p, seeds, step_offset, V, stride, slice);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
 template <typename T>
 int launch_sample(const void* logits, int* out, const float* temperature, const int* top_k, const float* top_p,
                   const long long* seeds, const long long* step_offset, int B, int V, long long stride,
                   cudaStream_t stream) {
+  const int ctas = V <= kOneCtaRow ? 1 : V <= kFourCtaRow ? 4 : 8;
   // slices begin at a multiple of the four logits that share a draw
-  const int slice = ((V + kRowCtas - 1) / kRowCtas + 3) / 4 * 4;
-  const bool fits = slice <= kMaxSlice;
-  const auto kern = fits ? sample_kernel<T, true> : sample_kernel<T, false>;
-  const int smem = fits ? slice * 4 : 0;
-  static DeviceOnce once;
-  int dev = 0;
-  if (once.needed(&dev)) {
-    if (cudaFuncSetAttribute(sample_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSlice * 4) !=
-        cudaSuccess)
-      return -4;
-    once.mark(dev);
-  }
-  kern<<<B * kRowCtas, kRowThreads, smem, stream>>>(static_cast<const T*>(logits), out, temperature, top_k, top_p,
-                                                    seeds, step_offset, V, stride, slice);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  const int slice = ((V + ctas - 1) / ctas + 3) / 4 * 4;
+  const auto launch = ctas == 1            ? launch_sample_as<T, true, 1>
+                      : ctas == 4          ? launch_sample_as<T, true, 4>
+                      : slice <= kMaxSlice ? launch_sample_as<T, true, 8>
+                                           : launch_sample_as<T, false, 8>;
+  return launch(logits, out, temperature, top_k, top_p, seeds, step_offset, B, V, stride, slice, stream);
 }
 
 }  // namespace b200

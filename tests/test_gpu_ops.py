@@ -1076,6 +1076,28 @@ def test_sample_draws_the_best_race_among_the_kept_logits(v, dtype, pad):
         assert float(score[got[i]]) >= best - 1e-4 - 2e-6 / max(e, 1e-7)
 
 
+@pytest.mark.parametrize("v,dtype,pad", [(8192, torch.float32, 0), (8193, torch.float32, 3), (8190, torch.bfloat16, 2),
+                                         (49152, torch.float32, 0), (49154, torch.float32, 2), (32000, torch.bfloat16, 0)])
+def test_sample_on_one_four_and_eight_ctas(v, dtype, pad):
+    """The same draw on either side of the lengths at which a row takes more CTAs."""
+    test_sample_draws_the_best_race_among_the_kept_logits(v, dtype, pad)
+
+
+@pytest.mark.parametrize("v", [5, 1000, 20000, 128256])
+def test_sample_rows_without_numbers(v):
+    """NaN and infinite logits give a token of the vocabulary, with and without thresholds."""
+    rows = [float("nan"), float("-inf"), float("inf")]
+    logits = torch.tensor(rows, device=DEV).repeat_interleave(4).view(-1, 1).repeat(1, v)
+    logits = torch.cat([logits, torch.full((4, v), float("-inf"), device=DEV)])
+    logits[12:, v // 2] = 0.0                                   # one token possible
+    n = logits.shape[0]
+    top_k = torch.tensor([0, 3, 0, 3] * (n // 4), dtype=torch.int32, device=DEV)
+    top_p = torch.tensor([1.0, 1.0, 0.9, 0.9] * (n // 4), device=DEV)
+    got = ops.sample(logits, torch.full((n,), 0.7, device=DEV), top_k, top_p, torch.arange(n, device=DEV), None)
+    assert got.min() >= 0 and got.max() < v
+    assert (got[:4] == 0).all() and (got[12:] == v // 2).all()
+
+
 # --------------------------------------------------------------------- MoE
 @pytest.mark.parametrize("e,k,sigmoid,groups,bias", [(64, 6, False, (1, 1), False), (128, 8, False, (1, 1), False),
                                                       (256, 8, True, (8, 4), True), (8, 2, True, (4, 2), False)])
