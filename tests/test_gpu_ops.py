@@ -320,6 +320,15 @@ def test_products_wait_for_weights_written_right_ahead(m, n, k):
         del w, got
 
 
+@pytest.mark.parametrize("rows,h", [(5999, 1024), (6000, 1024), (6001, 1280), (6000, 1288), (7000, 1016)])
+def test_norm_of_many_short_rows(rows, h):
+    """On either side of the sizes at which a row takes a warp and a CTA."""
+    torch.manual_seed(rows)
+    x, w = torch.randn(rows, h, device=DEV).bfloat16(), (torch.rand(h, device=DEV) + 0.5).bfloat16()
+    want = x.double() * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    _close(ops.rms_norm(x, w, 1e-6), want.float(), 1e-3, 2 ** -8)      # one rounding to bf16
+
+
 @pytest.mark.parametrize("rows,h", [(1, 1024), (40, 4096), (3, 16384)])
 def test_norm_waits_for_weights_written_right_ahead(rows, h):
     torch.manual_seed(h)
