@@ -951,6 +951,13 @@ def test_rope_cache_gqa_norm(t, hq, hk, d, rot, neox, normed):
     assert int((vc != 0).any(-1).any(1).sum()) == written
 
 
+@pytest.mark.parametrize("t,hq,hk,d", [(5, 64, 8, 128), (3, 65, 1, 128), (2, 130, 2, 64), (1, 40, 30, 256)])
+@pytest.mark.parametrize("normed", [True, False])
+def test_rope_cache_gqa_many_heads(t, hq, hk, d, normed):
+    """More heads than a CTA takes at once."""
+    test_rope_cache_gqa_norm(t, hq, hk, d, d, True, normed)
+
+
 def test_rope_cache_gqa_and_cache_write():
     t, hq, hk, d, bs = 29, 8, 2, 128, 16
     qkv = torch.randn(t, (hq + 2 * hk) * d, device=DEV, dtype=torch.bfloat16)
