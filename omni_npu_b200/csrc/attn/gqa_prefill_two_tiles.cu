@@ -362,10 +362,15 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
         ++sc;
         tc_fence_after_sync();
         uint32_t sv[4][32];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(s_col + c * 32, sv[c]);
-        tmem_ld_wait();
         const int n0 = j * BN;
+        const bool whole = it.kv_len - n0 > BN / 2;           // else the second half of the tile's keys does not exist
+#pragma unroll
+        for (int c = 0; c < 2; ++c) tmem_ld_32x32b_x32(s_col + c * 32, sv[c]);
+        if (whole) {
+          tmem_ld_32x32b_x32(s_col + 64, sv[2]);
+          tmem_ld_32x32b_x32(s_col + 96, sv[3]);
+        }
+        tmem_ld_wait();
         // The second product reads whole groups of 16 keys.  Value rows past the sequence in the last one (the rest of a
         // page, another sequence's rows, what an earlier tile left) would count if they were infinite or NaN, although P
         // is zero there: the tile that the product comes first for clears them once they have landed.
@@ -416,6 +421,7 @@ gqa_prefill_two_tiles_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
         float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
+          if (half == 1 && !whole) break;
           uint32_t pk[32];
 #pragma unroll
           for (int c = 0; c < 32; ++c) {
@@ -564,7 +570,9 @@ extern "C" int b200_gqa_prefill_tc(const void* q, const void* k_cache, const voi
                         CU_TENSOR_MAP_SWIZZLE_128B);
   if (r) return r - 3000;
   TwoTileGrid g;
-  g.by_head = (Hq / Hk) % 2 == 0;
+  // (a single row tile per sequence and SMs to spare: one query tile per CTA, its keys read twice.  A prompt of 128 tokens,
+  // 32 + 8 heads, 10.5 us with two heads per CTA, 8.5 in this form.)
+  g.by_head = (Hq / Hk) % 2 == 0 && !(max_q_len <= two::BM && static_cast<long long>(Hq) * B <= sm_count());
   const int unit = g.by_head ? two::BM : 2 * two::BM;
   g.m_units = (max_q_len + unit - 1) / unit;
   g.head_units = g.by_head ? Hq / 2 : Hq;

@@ -480,6 +480,15 @@ def test_gqa_prefill_two_tiles(d, hq, hk, bs, seq_lens, q_lens, causal):
         _close(lse, lse_want, 2e-2, 1e-2)
 
 
+@pytest.mark.parametrize("d,hq,hk", [(128, 8, 2), (128, 64, 8), (192, 4, 2)])
+@pytest.mark.parametrize("seq_lens,q_lens", [([17], [17]), ([128, 1], [128, 1]), ([64, 65], [64, 65]), ([192, 193, 63], [128, 100, 1]),
+                                             ([129, 5], [129, 5])])
+@pytest.mark.parametrize("causal", [True, False])
+def test_gqa_prefill_small(d, hq, hk, seq_lens, q_lens, causal):
+    """Few short prompts, a query tile per CTA, and key tiles of which only the first half exists."""
+    test_gqa_prefill_two_tiles(d, hq, hk, 16, seq_lens, q_lens, causal)
+
+
 @pytest.mark.parametrize("d,bs", [(128, 16), (64, 16), (128, 128)])
 def test_gqa_prefill(d, bs):
     seq_lens, q_lens = [130, 64, 517, 9], [130, 33, 200, 9]
