@@ -108,8 +108,8 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
     fence_barrier_init();
     tma_prefetch_desc(&tm_c);
   }
-  {
-    // rows that no copy writes (the last tile's, holes of a selection) must be finite: their P is zero
+  if (p.topk_indices) {
+    // rows that no copy writes (holes of a selection) must be finite: their P is zero
     uint4* z = reinterpret_cast<uint4*>(sKV);
     for (int i = tid; i < stages * tile_bytes / 16; i += kMlaThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
   }
@@ -135,6 +135,15 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
   const bool bt_cached = !sel && (bt_last - bt_first) <= 512;
   if (bt_cached)
     for (int i = bt_first + tid; i < bt_last; i += kMlaThreads) s_bt[i - bt_first] = bt[i];
+  if (!sel && n_tiles > 0 && n_tiles <= stages) {
+    // and so must the rows that the last tile's pages leave, where no tile before it filled them
+    const int valid = kv_len - (t_end - 1) * kMlaBN;
+    const int filled = valid < kMlaBN ? min(kMlaBN, (valid + box_rows - 1) / box_rows * box_rows) : kMlaBN;
+    const int chunks = (kMlaBN - filled) * 8;                  // 16 bytes each, of a slab
+    uint8_t* tile = sKV + (n_tiles - 1) * tile_bytes + filled * 128;
+    for (int i = tid; i < chunks * slabs; i += kMlaThreads)
+      *reinterpret_cast<uint4*>(tile + i / chunks * kSlabBytes + i % chunks * 16) = make_uint4(0u, 0u, 0u, 0u);
+  }
   fence_proxy_async();
   __syncthreads();
   volatile int* abort_flag = s_abort;
@@ -387,7 +396,8 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
     }
   }
   float4* s_o = reinterpret_cast<float4*>(sKV);                // [group - 1][2 * CT][64 threads]
-  if (group > 0) {
+  const int live = min(kMlaGroups, n_tiles);                   // groups that had a tile
+  if (group > 0 && group < live) {
 #pragma unroll
     for (int i = 0; i < 2 * CT; ++i)
       s_o[((group - 1) * 2 * CT + i) * 64 + wi * 32 + lane] = make_float4(o_acc[i][0], o_acc[i][1], o_acc[i][2], o_acc[i][3]);
@@ -395,7 +405,8 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
   asm volatile("bar.sync 1, %0;" ::"n"(kMlaCompute) : "memory");
   if (group > 0) return;
 #pragma unroll
-  for (int k = 0; k < kMlaGroups - 1; ++k)
+  for (int k = 0; k < kMlaGroups - 1; ++k) {
+    if (k + 1 >= live) break;
 #pragma unroll
     for (int i = 0; i < 2 * CT; ++i) {
       const float4 v = s_o[(k * 2 * CT + i) * 64 + wi * 32 + lane];
@@ -404,6 +415,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tm_c, const MlaParams p, c
       o_acc[i][2] += v.z;
       o_acc[i][3] += v.w;
     }
+  }
 
   // ---- write: every thread owns rows r_a, r_a+8 and two columns in eight of its warp's half
   const size_t part_row = ((static_cast<size_t>(tok) * gridDim.y + blockIdx.y) * p.splits + split) * 16;

@@ -154,3 +154,14 @@ def test_rows_that_stream_their_weights():
     assert ops.stream_parts(2048, 512) == 1 and ops.stream_rows(2048, 512) == 63
     assert ops.stream_rows(128256, 4096) == ops.stream_rows(32, 256) == 128
     assert ops.stream_rows(4096, 4096, 8) == 63                     # a limit of CTAs leaves no split
+
+
+@pytest.mark.parametrize("items", [1, 8, 100, 148, 149, 2048])
+@pytest.mark.parametrize("keys", [1, 255, 256, 511, 512, 2300, 8192, 163840])
+def test_latent_splits_leave_keys_for_each(items, keys):
+    s = ops.latent_splits(items, keys)
+    assert 1 <= s <= 16 and (s == 1 or keys // s >= 256)
+    if items >= 148 * 16 or keys < 512:
+        assert s == 1
+    if items == 1 and keys >= 16 * 256:
+        assert s > 1

@@ -1201,6 +1201,31 @@ def test_mla_decode_sparse_selection():
     _close(got, want, 2e-2, 2e-2)
 
 
+@pytest.mark.parametrize("bs", [8, 16, 32, 64, 128])
+@pytest.mark.parametrize("seq_lens,n_heads,q_len", [([1, 31, 32, 33, 7], 16, 1), ([64, 95, 96, 97, 128, 130], 16, 1),
+                                                    ([159, 160, 161, 2000, 5], 20, 1), ([2, 40, 162], 16, 2)])
+def test_mla_decode_tiles(bs, seq_lens, n_heads, q_len):
+    """Pages smaller and larger than a tile of 32 keys, lengths around a tile, a tile per group and a ring, splits by rule;
+    what other kernels left in shared memory and in the rest of a page that no copy brings takes no part."""
+    torch.manual_seed(bs)
+    b = len(seq_lens)
+    max_blocks = max(-(-n // bs) for n in seq_lens) + 1
+    nblocks = b * max_blocks + 2
+    bt = torch.randperm(nblocks)[: b * max_blocks].view(b, max_blocks).to(torch.int32)
+    cache = torch.randn(nblocks, bs, 576).bfloat16()
+    q = (torch.randn(b * q_len, n_heads * 576) * 0.3).bfloat16()
+    sl = torch.tensor(seq_lens, dtype=torch.int32)
+    want, want_lse = ref.mla_decode(q, cache, bt, sl, b, q_len, n_heads, 0.07, None, True)
+    # NaN in the shared memory of every SM first
+    junk = torch.full((100, 16, 576), float("nan"), device=DEV, dtype=torch.bfloat16)
+    ops.mla_decode(torch.zeros(300, 16 * 576, device=DEV, dtype=torch.bfloat16), junk,
+                   torch.arange(10, device=DEV, dtype=torch.int32).repeat(300, 1),
+                   torch.full((300,), 160, device=DEV, dtype=torch.int32), 300, 16, 0.07, splits=1)
+    got, lse = ops.mla_decode(q.to(DEV), cache.to(DEV), bt.to(DEV), sl.to(DEV), b, n_heads, 0.07, q_len, return_lse=True)
+    _close(got, want, 2e-2, 2e-2)
+    _close(lse, want_lse, 2e-2, 2e-2)
+
+
 @pytest.mark.parametrize("kind", ["int8", "fp8"])
 @pytest.mark.parametrize("add", [False, True])
 def test_rms_norm_quant_fused(kind, add):
