@@ -446,7 +446,7 @@ def gemm_scaled(a_q: torch.Tensor, w_q: torch.Tensor, a_scale: torch.Tensor, w_s
 
 @functools.lru_cache(maxsize=4096)
 def grouped_tile(rows: int, groups: int, n: int, k: int, sms: int = 148) -> int:
-    """Tile width of a grouped e4m3 product whose ``rows`` rows spread evenly over the groups: 256, or the largest
+    """Tile width of a grouped product of gemm_tcgen05_kernel whose ``rows`` rows spread evenly over the groups: 256, or the largest
     power of two from 32 that divides n, unless another width is clearly better under the cost model of the
     dense plan (csrc/gemm/gemm_tcgen05.cu): fewer idle SMs in a decode step, less padding of n in a prompt."""
     live = max(1, min(groups, rows))
@@ -464,16 +464,25 @@ def grouped_tile(rows: int, groups: int, n: int, k: int, sms: int = 148) -> int:
 
 
 @functools.lru_cache(maxsize=4096)
-def grouped_rows_tile(rows: int, groups: int, n: int, sms: int = 148) -> int:
-    """Kernel of a grouped bf16 product: rows of A per tile of gemm_stream_kernel, or 0 for gemm_pair_kernel.
+def grouped_rows_tile(rows: int, groups: int, n: int, k: int = 0, sms: int = 148) -> int:
+    """Kernel of a grouped bf16 product: rows of A per tile of gemm_stream_kernel, 0 for gemm_pair_kernel, or -1 for
+    gemm_tcgen05_kernel.
 
     Streaming wins while the weights outweigh the rows (us, streaming / pair): 128 groups 1536 x 2048 with silu 132 / 136
     at 32 rows per group, 64 groups 2816 x 2048 117 / 125 at 48, but 128 groups 2048 x 768 110 / 79 at 64; with too few
-    tiles for the SMs, 4 groups 2048 x 2048 at 48 rows, 16.3 / 14.1.  A pair's tile is 256 weight rows: 16 groups
-    128 x 512 at 4096 rows 20.1 / 26.8.  Narrow tiles fill the SMs: there at 128 rows 7.9 with 32 and 9.2 with 64."""
+    tiles for the SMs, 4 groups 2048 x 2048 at 48 rows, 16.3 / 14.1.
+    Up to 128 weight rows, a single tile per group, are streamed through the narrowest tiles of A that are all resident (us,
+    32 / 64 / 128 rows, pair, gemm_tcgen05_kernel: 16 groups 128 x 512 at 512 rows 8.5 / 9.9 / 13.0, 12.6, 9.8, at 768
+    11.9 / 10.0 / 13.3, 12.7, 11.2, at 2048 19.6 / 14.6 / 14.0, 19.3, 16.3), but not along a K beyond some 768, which a CTA
+    walks through at half the rate of that kernel (8 groups 128 x 2048 at 64 rows 16.3 / 19.1 / 19.1, 13.1, 14.4, at 2048
+    29.9 / 20.5 / 27.4, 20.6, 17.8; 4 groups 128 x 1024 at 16 rows 9.5, 9.5, 10.5)."""
     per = -(-rows // groups)
     tiles = min(rows, groups) * -(-n // 128)
-    if n > 128 and per > (48 if tiles >= sms else 16):
+    if n <= 128:
+        if k > 768 and per > 16:
+            return -1
+        return next((t for t in (32, 64) if tiles * -(-per // t) <= 2 * sms), 128)
+    if per > (48 if tiles >= sms else 16):
         return 0
     return 32 if tiles * -(-per // 64) < sms else 64 if per <= 48 else 128
 
@@ -489,12 +498,14 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, expert_offsets: torch.Tensor,
     if a.is_cuda and a.dtype == torch.bfloat16 and bn <= 0:
         groups, n = w.shape[0], w.shape[1]
         rows = a.shape[0] if rows is None else min(rows, a.shape[0])
-        if out is None:
-            out = a.new_empty(a.shape[0], n // 2 if kind[0] in (1, 2, 4, 7) else n)
-        _count(1)
-        _core().grouped_gemm_rows(a, w, expert_offsets, out, kind[0], grouped_rows_tile(rows, groups, n),
-                                  device_state(a.device).status, max_ctas, kind[1], kind[2])
-        return out
+        tile = grouped_rows_tile(rows, groups, n, w.shape[2])
+        if tile >= 0:
+            if out is None:
+                out = a.new_empty(a.shape[0], n // 2 if kind[0] in (1, 2, 4, 7) else n)
+            _count(1)
+            _core().grouped_gemm_rows(a, w, expert_offsets, out, kind[0], tile, device_state(a.device).status, max_ctas,
+                                      kind[1], kind[2])
+            return out
     if not a.is_cuda:
         y = ref.grouped_gemm(a, w, expert_offsets, swiglu, act, unary)
     elif a.dtype == torch.float32:

@@ -144,6 +144,9 @@ def test_experts_choose_kernels_by_the_rows_of_the_step(monkeypatch, quant):
 def test_rows_of_a_step_choose_the_grouped_kernel():
     few, many = ops.grouped_rows_tile(16, 16, 1536), ops.grouped_rows_tile(131072, 16, 1536)
     assert few > 0 and many == 0            # streamed weights; CTA pairs
+    # a single tile of weight rows per group: never pairs; a long K with some rows: the kernel with rows of A as M
+    assert [ops.grouped_rows_tile(16 * r, 16, 128, 512) for r in (16, 512, 768, 1024, 2048)] == [32, 32, 64, 64, 128]
+    assert [ops.grouped_rows_tile(8 * r, 8, 128, 2048) for r in (16, 17, 4096)] == [32, -1, -1]
 
 
 def test_rows_that_stream_their_weights():

@@ -347,6 +347,26 @@ def test_norm_waits_for_weights_written_right_ahead(rows, h):
         del w, got, added, other
 
 
+@pytest.mark.parametrize("counts,n,k", [([17] * 8, 128, 1024), ([0, 70, 3, 128], 48, 2048), ([300] * 3, 128, 776), ([33, 0, 20], 16, 4096)])
+def test_grouped_gemm_narrow(counts, n, k):
+    """A single tile of weight rows per group and a long K, into rows of a wider tensor too."""
+    torch.manual_seed(n + k)
+    offs = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32)
+    rows, e = int(offs[-1]), len(counts)
+    assert ops.grouped_rows_tile(rows, e, n, k) == -1
+    a = torch.randn(rows, k, device=DEV, dtype=torch.bfloat16)
+    w = (torch.randn(e, n, k, device=DEV) * k ** -0.5).bfloat16()
+    exact = torch.cat([a[offs[i]: offs[i + 1]].double() @ w[i].double().T for i in range(e)])
+    out = torch.zeros(rows, 256, device=DEV, dtype=torch.bfloat16)
+    # one rounding to bf16
+    _close(ops.grouped_gemm(a, w, offs.to(DEV), out=out[:, :n]), exact.float(), 1e-3, 2 ** -8)
+    assert not out[:, n:].any()
+    gate, up = exact.view(rows, -1, 2, 8).unbind(2)
+    _close(ops.grouped_gemm(a, w, offs.to(DEV), swiglu=True), (torch.nn.functional.silu(gate) * up).reshape(rows, -1).float(),
+           1e-3, 2 ** -7)
+    ops.check_status()
+
+
 def test_gemm_fp8_plain():
     torch.manual_seed(4)
     m, n, k = 256, 512, 1024
