@@ -19,7 +19,7 @@ int b200_gather_cache(void* dst, const void* cache, const int* block_tables, con
 int b200_spec_verify(const int* draft, const int* target, const int* bonus, const int* cu, int* out,
                      int* num_out, int B, int max_spec, cudaStream_t stream);
 int b200_rmsnorm(void* out, const void* x, void* residual, const void* w, float eps, long long rows,
-                 int H, long long x_stride, long long out_stride, long long res_stride,
+                 int H, long long x_stride, long long out_stride, long long res_stride, int w_ready,
                  cudaStream_t stream);
 int b200_silu_mul(void* out, const void* x, long long rows, int I, long long x_stride,
                   long long out_stride, cudaStream_t stream);
@@ -171,7 +171,8 @@ std::tuple<Tensor, Tensor> spec_verify(const Tensor& draft, const Tensor& target
   return {out, num};
 }
 
-Tensor rms_norm(const Tensor& x, const Tensor& w, double eps) {
+// w_ready (here and below): no kernel still running writes w, which is then read early.
+Tensor rms_norm(const Tensor& x, const Tensor& w, double eps, bool w_ready) {
   CHECK_CUDA_BF16(x);
   CHECK_CUDA_BF16(w);
   TORCH_CHECK(x.stride(-1) == 1, "rms_norm: last dim contiguous");
@@ -180,13 +181,13 @@ Tensor rms_norm(const Tensor& x, const Tensor& w, double eps) {
   c10::cuda::CUDAGuard guard(x.device());
   Tensor out = torch::empty({x2.size(0), H}, x.options());
   check(b200_rmsnorm(out.data_ptr(), x2.data_ptr(), nullptr, w.data_ptr(), (float)eps, x2.size(0),
-                     H, x2.stride(0), H, 0, cur_stream()),
+                     H, x2.stride(0), H, 0, w_ready ? 1 : 0, cur_stream()),
         "rms_norm");
   return out.view(x.sizes());
 }
 
 // residual <- x + residual ; returns norm(residual) * w
-Tensor fused_add_rms_norm(const Tensor& x, Tensor residual, const Tensor& w, double eps) {
+Tensor fused_add_rms_norm(const Tensor& x, Tensor residual, const Tensor& w, double eps, bool w_ready) {
   CHECK_CUDA_BF16(x);
   CHECK_CUDA_BF16(residual);
   CHECK_CUDA_BF16(w);
@@ -196,7 +197,7 @@ Tensor fused_add_rms_norm(const Tensor& x, Tensor residual, const Tensor& w, dou
   c10::cuda::CUDAGuard guard(x.device());
   Tensor out = torch::empty({x.size(0), H}, x.options());
   check(b200_rmsnorm(out.data_ptr(), x.data_ptr(), residual.data_ptr(), w.data_ptr(), (float)eps,
-                     x.size(0), H, x.stride(0), H, residual.stride(0), cur_stream()),
+                     x.size(0), H, x.stride(0), H, residual.stride(0), w_ready ? 1 : 0, cur_stream()),
         "fused_add_rms_norm");
   return out;
 }

@@ -44,18 +44,23 @@ union Vec8 {
 
 // One CTA per row, VPT vectors of eight columns per thread.  ADD: x <- x + residual is written back to residual first.
 // What bounds it: memory in a prompt (a row of both inputs read, of both outputs written), the chain load - sum - store in
-// a decode step: all loads of a row are issued together, the weights' too.
+// a decode step: all loads of a row are issued together, the weights' ahead of the wait where no kernel still running writes
+// them (w_ready, by the caller's word: in a step they come from memory, the row from L2, 0.8 us later otherwise).
 // 8192 rows x 4096 with ADD: 58.5 us with loads, sums and stores vector by vector and room for eight vectors in every
 // thread, 41.4 in this form (41.7 at the copy rate); one row of 4096 2.8 and 2.2.
 template <bool ADD, int VPT>
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ x,
                __nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ w, float eps,
-               int H, long long x_stride, long long out_stride, long long res_stride) {
+               int H, long long x_stride, long long out_stride, long long res_stride, bool w_ready) {
   __shared__ float red[kNormThreads / 32];
   pdl_trigger();
   const int nvec = H >> 3, tid = threadIdx.x, step = blockDim.x;
   Vec8 g[VPT], a[VPT], b[VPT];
+  if (w_ready)
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+      if (tid + i * step < nvec) g[i].u = reinterpret_cast<const uint4*>(w)[tid + i * step];
   pdl_wait();
   const long long row = blockIdx.x;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * x_stride);
@@ -66,7 +71,7 @@ rmsnorm_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict_
     const bool live = tid + i * step < nvec;
     a[i].u = live ? xr[tid + i * step] : make_uint4(0u, 0u, 0u, 0u);
     if (ADD) b[i].u = live ? rr[tid + i * step] : make_uint4(0u, 0u, 0u, 0u);
-    if (live) g[i].u = reinterpret_cast<const uint4*>(w)[tid + i * step];
+    if (live && !w_ready) g[i].u = reinterpret_cast<const uint4*>(w)[tid + i * step];
   }
   float ss = 0.f;
 #pragma unroll
@@ -98,7 +103,7 @@ rmsnorm_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict_
 
 template <bool ADD>
 static void launch_rmsnorm(void* out, const void* x, void* residual, const void* w, float eps, long long rows, int H,
-                           long long x_stride, long long out_stride, long long res_stride, cudaStream_t stream) {
+                           long long x_stride, long long out_stride, long long res_stride, int w_ready, cudaStream_t stream) {
   const int nvec = H >> 3;
   int vpt = 1;
   while (vpt < kMaxVecPerThread && nvec > vpt * kNormThreads) vpt *= 2;
@@ -109,7 +114,7 @@ static void launch_rmsnorm(void* out, const void* x, void* residual, const void*
                                : rmsnorm_kernel<ADD, 8>;
   launch_pdl(kern, dim3(static_cast<unsigned>(rows)), dim3(threads), 0, stream, 1, static_cast<__nv_bfloat16*>(out),
              static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(residual),
-             static_cast<const __nv_bfloat16*>(w), eps, H, x_stride, out_stride, res_stride);
+             static_cast<const __nv_bfloat16*>(w), eps, H, x_stride, out_stride, res_stride, w_ready != 0);
 }
 
 // One warp per row, for short rows (per-head q/k norms, H <= 256*... up to 2048).
@@ -361,7 +366,7 @@ using namespace b200;
 
 extern "C" int b200_rmsnorm(void* out, const void* x, void* residual, const void* w, float eps,
                             long long rows, int H, long long x_stride, long long out_stride,
-                            long long res_stride, cudaStream_t stream) {
+                            long long res_stride, int w_ready, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if ((H & 7) != 0) return -1;
   // Rows of 1024 columns and more have a CTA's worth of vectors, but thousands of small CTAs take longer to start than a
@@ -376,9 +381,9 @@ extern "C" int b200_rmsnorm(void* out, const void* x, void* residual, const void
   }
   if (H > kNormThreads * kMaxVecPerThread * 8) return -2;
   if (residual)
-    launch_rmsnorm<true>(out, x, residual, w, eps, rows, H, x_stride, out_stride, res_stride, stream);
+    launch_rmsnorm<true>(out, x, residual, w, eps, rows, H, x_stride, out_stride, res_stride, w_ready, stream);
   else
-    launch_rmsnorm<false>(out, x, nullptr, w, eps, rows, H, x_stride, out_stride, 0LL, stream);
+    launch_rmsnorm<false>(out, x, nullptr, w, eps, rows, H, x_stride, out_stride, 0LL, w_ready, stream);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

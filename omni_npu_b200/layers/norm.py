@@ -28,11 +28,11 @@ class RMSNorm(nn.Module):
                 y_transform: Optional[str] = None
                 ) -> Union[torch.Tensor, Tuple[torch.Tensor, torch.Tensor]]:
         if residual is None:
-            y = ops.rms_norm(x, self.weight, self.eps)
+            y = ops.rms_norm(x, self.weight, self.eps, w_ready=True)
             if y_transform == "AG":
                 y = pstate.get_tp_group().all_gather(y, dim=0)
             return y
-        y = ops.fused_add_rms_norm(x, residual, self.weight, self.eps)
+        y = ops.fused_add_rms_norm(x, residual, self.weight, self.eps, w_ready=True)
         if y_transform == "AG":
             y = pstate.get_tp_group().all_gather(y, dim=0)
         return y, residual

@@ -43,9 +43,9 @@ if compat.vllm_available():
             shape = x.shape
             x2 = x.reshape(-1, shape[-1])
             if residual is None:
-                return ops.rms_norm(x2, self.weight.data, self.variance_epsilon).view(shape)
+                return ops.rms_norm(x2, self.weight.data, self.variance_epsilon, w_ready=True).view(shape)
             r2 = residual.reshape(-1, shape[-1])
-            y = ops.fused_add_rms_norm(x2, r2, self.weight.data, self.variance_epsilon)   # r2 updated in place
+            y = ops.fused_add_rms_norm(x2, r2, self.weight.data, self.variance_epsilon, w_ready=True)   # r2 updated in place
             return y.view(shape), r2.view(shape)
 
     REGISTERED += ["SiluAndMul", "RMSNorm"]

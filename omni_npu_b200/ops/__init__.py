@@ -538,20 +538,21 @@ def batched_gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, w_ready: b
 
 
 # ------------------------------------------------------------- norm/activation
-def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
+def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float, w_ready: bool = False) -> torch.Tensor:
+    """RMSNorm of the last dimension times ``w`` (``w_ready`` as in :func:`gemm`)."""
     if not x.is_cuda:
         return ref.rms_norm(x, w, eps)
     _count(1)
-    return _C().rms_norm(x, w, eps)
+    return _C().rms_norm(x, w, eps, w_ready)
 
 
 def fused_add_rms_norm(x: torch.Tensor, residual: torch.Tensor, w: torch.Tensor,
-                       eps: float) -> torch.Tensor:
-    """residual <- x + residual (in place); returns RMSNorm(residual) * w."""
+                       eps: float, w_ready: bool = False) -> torch.Tensor:
+    """residual <- x + residual (in place); returns RMSNorm(residual) * w (``w_ready`` as in :func:`gemm`)."""
     if not x.is_cuda:
         return ref.fused_add_rms_norm(x, residual, w, eps)
     _count(1)
-    return _C().fused_add_rms_norm(x, residual, w, eps)
+    return _C().fused_add_rms_norm(x, residual, w, eps, w_ready)
 
 
 def silu_and_mul(x: torch.Tensor) -> torch.Tensor:

@@ -34,6 +34,15 @@ def test_only_parameters_are_read_ahead_of_the_kernels_before(monkeypatch):
     assert len(calls) == 2 and not any(c.get("w_ready", False) for c in calls)
 
 
+def test_norm_layers_read_their_parameters_early(monkeypatch):
+    norm, x = RMSNorm(16, dtype=torch.float32), torch.randn(2, 16)
+    alone, added = _record(monkeypatch, "rms_norm"), _record(monkeypatch, "fused_add_rms_norm")
+    norm(x), norm(x, x.clone())
+    assert alone.pop()["w_ready"] is True and added.pop()["w_ready"] is True
+    ops.rms_norm(x, norm.weight.data, 1e-6)
+    assert not alone.pop().get("w_ready", False)
+
+
 def _qwen_attention():
     """One attention layer of a small Qwen3 model, and what it returns for a prompt of five tokens."""
     from omni_npu_b200.attention.metadata import AttentionMetadata, set_forward_context
