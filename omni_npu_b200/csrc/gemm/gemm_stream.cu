@@ -98,19 +98,19 @@ __device__ __forceinline__ bool stream_tile(const StreamParams& p, const int* pr
 }
 
 // One value of C per thread (column n; the 32 lanes of a warp hold neighbouring columns): epilogue and store.
-__device__ __forceinline__ void stream_store(const StreamParams& p, float v, int row, int n) {
+__device__ __forceinline__ void stream_store(const StreamParams& p, int act, float v, int row, int n) {
   const bool ok = n < p.N;
   const float bias = p.bias && ok ? __bfloat162float(p.bias[n]) : 0.f;
-  if (act_is_gated(p.act)) {
+  if (act_is_gated(act)) {
     v += bias;
     // columns alternate in groups of eight: gate, up (N is a multiple of 16)
     const float up = __shfl_xor_sync(0xffffffffu, v, 8);
     if (ok && !(n & 8))
       static_cast<__nv_bfloat16*>(p.C)[static_cast<size_t>(row) * p.ldc + (n >> 4) * 8 + (n & 7)] =
-          __float2bfloat16(gated_act(p.act, v, up, p.act_alpha, p.act_limit));
+          __float2bfloat16(gated_act(act, v, up, p.act_alpha, p.act_limit));
     return;
   }
-  if (act_is_unary(p.act)) v = unary_act(p.act, v, p.act_alpha, p.act_limit);
+  if (act_is_unary(act)) v = unary_act(act, v, p.act_alpha, p.act_limit);
   if (!ok) return;
   v += bias;
   const size_t at = static_cast<size_t>(row) * p.ldc + n;
@@ -123,11 +123,11 @@ __device__ __forceinline__ void stream_store(const StreamParams& p, float v, int
 
 // Four neighbouring values of a row per lane (column n, a multiple of four).  wide: C, the residual and their pitch let
 // four values be one access.
-__device__ __forceinline__ void stream_store4(const StreamParams& p, float (&v)[4], int row, int n, bool wide) {
-  const bool gated = act_is_gated(p.act), whole = n + 3 < p.N;
-  if (act_is_unary(p.act))
+__device__ __forceinline__ void stream_store4(const StreamParams& p, int act, float (&v)[4], int row, int n, bool wide) {
+  const bool gated = act_is_gated(act), whole = n + 3 < p.N;
+  if (act_is_unary(act))
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = unary_act(p.act, v[i], p.act_alpha, p.act_limit);
+    for (int i = 0; i < 4; ++i) v[i] = unary_act(act, v[i], p.act_alpha, p.act_limit);
   if (p.bias)
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -140,7 +140,7 @@ __device__ __forceinline__ void stream_store4(const StreamParams& p, float (&v)[
     for (int i = 0; i < 4; ++i) up[i] = __shfl_xor_sync(0xffffffffu, v[i], 2);
     if (!whole || (n & 8)) return;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = gated_act(p.act, v[i], up[i], p.act_alpha, p.act_limit);
+    for (int i = 0; i < 4; ++i) v[i] = gated_act(act, v[i], up[i], p.act_alpha, p.act_limit);
     at = static_cast<size_t>(row) * p.ldc + (n >> 4) * 8 + (n & 7);
   }
   if (wide && whole) {
@@ -168,13 +168,16 @@ __device__ __forceinline__ void stream_store4(const StreamParams& p, float (&v)[
   }
 }
 
-// SPLIT: the CTAs of a cluster share a tile's K.
-template <int MODE, bool SPLIT>
+// SPLIT: the CTAs of a cluster share a tile's K.  ACT: p.act is looked at.  (With every activation's code the kernel takes
+// 168 registers instead of 64, which leaves the kernel behind it no room beside two of its CTAs: latent decode step of 128
+// rows, 4 layers, 1334 us with one kernel for all, 1312.)
+template <int MODE, bool SPLIT, bool ACT>
 __global__ void __launch_bounds__(stream::THREADS, 2)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                    const StreamParams p) {
   using namespace stream;
   constexpr bool GROUPED = MODE == kStreamGrouped, BATCHED = MODE == kStreamBatched;
+  const int act = ACT ? p.act : static_cast<int>(kActNone);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -368,9 +371,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;      // row of the W tile
     // bf16 results without a residual, and without a bias behind a unary activation: stored in pairs of columns
-    const bool plain = !p.out_fp32 && !p.residual && !(p.bias && act_is_unary(p.act));
-    const bool pairs = columns_pair(p.C, p.ldc | (BATCHED ? p.c_group : 0), p.N, act_is_gated(p.act));
-    const bool plain32 = MODE == kStreamDense && p.out_fp32 && !p.residual && p.act == kActNone;
+    const bool plain = !p.out_fp32 && !p.residual && !(p.bias && act_is_unary(act));
+    const bool pairs = columns_pair(p.C, p.ldc | (BATCHED ? p.c_group : 0), p.N, act_is_gated(act));
+    const bool plain32 = MODE == kStreamDense && p.out_fp32 && !p.residual && act == kActNone;
     int cursor = 0, acc = 0;
     uint32_t acc_phase = 0;
     StreamTile tile;
@@ -406,7 +409,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
           float x[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(v[i]) + bias;
-          store_act_columns(p.act, p.act_alpha, p.act_limit, x,
+          store_act_columns(act, p.act_alpha, p.act_limit, x,
                             static_cast<__nv_bfloat16*>(p.C) + (BATCHED ? tile.expert * p.c_group : 0) +
                                 static_cast<size_t>(tile.row0 + c) * p.ldc,
                             p.ldc, col_n, p.N, n, pairs);
@@ -418,7 +421,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         } else {
 #pragma unroll
           for (int i = 0; i < 16; ++i)
-            if (i < n) stream_store(p, __uint_as_float(v[i]), tile.row0 + c + i, col_n);
+            if (i < n) stream_store(p, act, __uint_as_float(v[i]), tile.row0 + c + i, col_n);
         }
       }
       tc_fence_before_sync();
@@ -462,7 +465,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 #pragma unroll
           for (int s = 1; s < 8; ++s) sum[i] += v[s][i];
         }
-        stream_store4(p, sum, row, n, wide);
+        stream_store4(p, act, sum, row, n, wide);
       }
     }
     cluster_sync_all();
@@ -489,10 +492,10 @@ static size_t stream_smem(int tn, int stages, int num_experts) {
          (num_experts > 0 ? 2 * (num_experts + 1) * 4 : 0);
 }
 
-template <int MODE, bool SPLIT>
+template <int MODE, bool SPLIT, bool ACT>
 static int launch_stream(const CUtensorMap& tw, const CUtensorMap& tx, const StreamParams& p, int grid,
                          cudaStream_t stream) {
-  auto kern = gemm_stream_kernel<MODE, SPLIT>;
+  auto kern = gemm_stream_kernel<MODE, SPLIT, ACT>;
   static DeviceOnce once;
   int dev = 0;
   if (once.needed(&dev)) {
@@ -560,8 +563,11 @@ extern "C" int b200_gemm_stream(const void* A, const void* W, void* C, const voi
     const int most = max_ctas > 0 ? max_ctas : 2 * sm_count();
     if (grid > most) grid = most;
   }
-  return p.splits > 1 ? launch_stream<kStreamDense, true>(tw, tx, p, grid, cu_stream)
-                      : launch_stream<kStreamDense, false>(tw, tx, p, grid, cu_stream);
+  if (act == kActNone)
+    return p.splits > 1 ? launch_stream<kStreamDense, true, false>(tw, tx, p, grid, cu_stream)
+                        : launch_stream<kStreamDense, false, false>(tw, tx, p, grid, cu_stream);
+  return p.splits > 1 ? launch_stream<kStreamDense, true, true>(tw, tx, p, grid, cu_stream)
+                      : launch_stream<kStreamDense, false, true>(tw, tx, p, grid, cu_stream);
 }
 
 // A [total_rows, K], W [E, N, K]; rows expert_offsets[e] .. expert_offsets[e + 1] (device) belong to expert e.
@@ -604,7 +610,8 @@ extern "C" int b200_grouped_gemm_stream(const void* A, const void* W, void* C, c
   if (r) return r - 1000;
   int grid = max_ctas > 0 ? max_ctas : 2 * sm_count();
   if (row_tiles * p.num_n_tiles < grid) grid = static_cast<int>(row_tiles * p.num_n_tiles);
-  return launch_stream<kStreamGrouped, false>(tw, tx, p, grid, cu_stream);
+  return act == kActNone ? launch_stream<kStreamGrouped, false, false>(tw, tx, p, grid, cu_stream)
+                         : launch_stream<kStreamGrouped, false, true>(tw, tx, p, grid, cu_stream);
 }
 
 // C[t, g, :] = A[t, g, :] W[g]^T for T rows of G groups: A and C with pitches of their own between rows and groups (in
@@ -643,5 +650,5 @@ extern "C" int b200_batched_gemm(const void* A, const void* W, void* C, int T, i
                         static_cast<uint64_t>(a_row), p.box, stream::SLAB_K, CU_TENSOR_MAP_SWIZZLE_128B);
   if (r) return r - 1000;
   const int grid = tiles < 2 * sm_count() ? static_cast<int>(tiles) : 2 * sm_count();
-  return launch_stream<kStreamBatched, false>(tw, tx, p, grid, cu_stream);
+  return launch_stream<kStreamBatched, false, false>(tw, tx, p, grid, cu_stream);
 }
