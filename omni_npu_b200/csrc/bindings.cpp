@@ -39,7 +39,7 @@ int b200_gemm_fp8_stream(const void* A, const float* a_scales, const void* W, co
                          int out_fp32, int* status, int max_ctas, int w_ready, cudaStream_t stream);
 int b200_grouped_gemm_fp8_stream(const void* A, const float* a_scales, const void* W, const float* w_scales, void* C,
                                  const int* expert_offsets, int num_experts, int total_rows, int N, int K, int lda, int ldc,
-                                 int scale_rows, int swiglu, int up_scale_row0, int tn, int* status, int max_ctas,
+                                 int scale_rows, int swiglu, int up_scale_row0, int* status, int max_ctas,
                                  cudaStream_t stream);
 int b200_dsa_indexer(const void* q, const float* w, const void* cache, const int* block_tables, const int* cu_q,
                      const int* positions, float* scores, int* topk_out, int T, int B, int H, int q_len,
@@ -288,7 +288,7 @@ Tensor gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tensor& w, c
 // interleaved in groups of 8, their scale rows are gate blocks then up blocks (from row up_scale_row0).
 // The result goes into c [rows, N, or N / 2 with swiglu] (rows may lie further apart).
 void grouped_gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tensor& w, const Tensor& w_scale,
-                            const Tensor& expert_offsets, Tensor c, bool swiglu, int64_t up_scale_row0, int64_t tn,
+                            const Tensor& expert_offsets, Tensor c, bool swiglu, int64_t up_scale_row0, bool few_rows,
                             const Tensor& status, int64_t max_ctas) {
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 3, "grouped_gemm_fp8_block: shapes");
   TORCH_CHECK(a.scalar_type() == at::kFloat8_e4m3fn && w.scalar_type() == at::kFloat8_e4m3fn,
@@ -310,11 +310,11 @@ void grouped_gemm_fp8_block(const Tensor& a, const Tensor& a_scale, const Tensor
   TORCH_CHECK(c.is_cuda() && c.scalar_type() == at::kBFloat16 && c.dim() == 2 && c.size(0) == rows && c.size(1) == n_out &&
                   c.stride(1) == 1 && c.stride(0) >= n_out && c.device() == a.device(),
               "grouped_gemm_fp8_block: result bf16 [rows, N]");
-  if (tn > 0) {        // rows per tile of the weight-streaming kernel
+  if (few_rows) {      // the weight-streaming kernel
     check(b200_grouped_gemm_fp8_stream(a.data_ptr(), a_scale.data_ptr<float>(), w.data_ptr(), w_scale.data_ptr<float>(),
                                        c.data_ptr(), expert_offsets.data_ptr<int>(), (int)E, (int)rows, (int)N, (int)K,
                                        (int)a.stride(0), (int)c.stride(0), (int)R, swiglu ? 1 : 0, (int)up_scale_row0,
-                                       (int)tn, status.data_ptr<int>(), (int)max_ctas, cur_stream()),
+                                       status.data_ptr<int>(), (int)max_ctas, cur_stream()),
           "grouped_gemm_fp8_stream");
     return;
   }

@@ -16,7 +16,7 @@ int b200_gemm(const void* A, const void* W, void* C, const void* bias, const voi
               int BN, int splits, int cluster_split, void* workspace, int* counters, int* status,
               int max_ctas, float act_alpha, float act_limit, int w_ready, cudaStream_t stream);
 int b200_gemm_stream(const void* A, const void* W, void* C, const void* bias, const void* residual, int M, int N, int K,
-                     int lda, int ldw, int ldc, int out_fp32, int act, int splits, int* status, int max_ctas,
+                     int lda, int ldw, int ldc, int out_fp32, int act, int* status, int max_ctas,
                      float act_alpha, float act_limit, int w_ready, cudaStream_t stream);
 int b200_gemm_stream_splits(int N, int K, int max_ctas, int sms);
 int b200_grouped_gemm_stream(const void* A, const void* W, void* C, const int* expert_offsets, int num_experts,
@@ -224,8 +224,8 @@ Tensor gemm_pair(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& 
 
 // Same contract as gemm() for at most 128 bf16 rows: the weights are the tensor cores' M operand (gemm/gemm_stream.cu).
 Tensor gemm_stream(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& bias,
-                   const c10::optional<Tensor>& residual, bool out_fp32, int64_t act, int64_t splits,
-                   const Tensor& status, int64_t max_ctas, double act_alpha, double act_limit, bool w_ready) {
+                   const c10::optional<Tensor>& residual, bool out_fp32, int64_t act, const Tensor& status,
+                   int64_t max_ctas, double act_alpha, double act_limit, bool w_ready) {
   TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 2, "gemm_stream: 2-D CUDA tensors");
   TORCH_CHECK(a.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16, "gemm_stream: bf16 inputs");
   TORCH_CHECK(a.stride(1) == 1 && w.stride(1) == 1, "gemm_stream: K must be contiguous");
@@ -248,7 +248,7 @@ Tensor gemm_stream(const Tensor& a, const Tensor& w, const c10::optional<Tensor>
     res_p = residual->data_ptr();
   }
   check(b200_gemm_stream(a.data_ptr(), w.data_ptr(), c.data_ptr(), bias_p, res_p, M, N, K, (int)a.stride(0),
-                         (int)w.stride(0), n_out, out_fp32 ? 1 : 0, (int)act, (int)splits, status.data_ptr<int>(),
+                         (int)w.stride(0), n_out, out_fp32 ? 1 : 0, (int)act, status.data_ptr<int>(),
                          (int)max_ctas, (float)act_alpha, (float)act_limit, w_ready ? 1 : 0, cur_stream()),
         "gemm_stream");
   return c;

@@ -23,6 +23,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tensormap.h"
 #include "column_store.cuh"
+#include "group_tiles.cuh"
 #include "stream_split.cuh"
 
 namespace b200 {
@@ -121,30 +122,9 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
   }
   if constexpr (GROUPED) {
     pdl_wait();      // the offsets come from an earlier kernel
-    if (warp == 2) {
-      const int per = (p.num_experts + 31) / 32;
-      const int e0 = min(p.num_experts, lane * per), e1 = min(p.num_experts, e0 + per);
-      int tiles = 0;
-      for (int e = e0; e < e1; ++e)
-        tiles += (p.expert_offsets[e + 1] - p.expert_offsets[e] + p.tn - 1) / p.tn * p.num_n_tiles;
-      int incl = tiles;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int up = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += up;
-      }
-      int before = incl - tiles;
-      for (int e = e0; e < e1; ++e) {
-        const int a = p.expert_offsets[e], b = p.expert_offsets[e + 1];
-        prefix[e] = before;
-        first_row[e] = a;
-        before += (b - a + p.tn - 1) / p.tn * p.num_n_tiles;
-        if (e + 1 == p.num_experts) {
-          prefix[e + 1] = before;
-          first_row[e + 1] = b;
-        }
-      }
-    }
+    if (warp == 2)
+      group_tiles(p.expert_offsets, p.num_experts, prefix, first_row,
+                  [&](int rows) { return (rows + p.tn - 1) / p.tn * p.num_n_tiles; });
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -361,24 +341,11 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
       const bool wide = n + 3 < p.N && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C) & (p.out_fp32 ? 15 : 7)) == 0;
       for (int row = rank + p.splits * (warp - 2); row < p.M; row += 4 * p.splits) {
         const uint32_t at = smem_u32(smem) + static_cast<uint32_t>((row * BW + 4 * lane) * 4);
-        float v[8][4];
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) v[s][i] = 0.f;
-          if (s < p.splits)
-            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                         : "=f"(v[s][0]), "=f"(v[s][1]), "=f"(v[s][2]), "=f"(v[s][3])
-                         : "r"(mapa_shared(at, s))
-                         : "memory");
-        }
         const size_t o = static_cast<size_t>(row) * p.ldc + n;
         float sum[4];
+        split_sum(at, p.splits, sum);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          sum[i] = v[0][i];
-#pragma unroll
-          for (int s = 1; s < 8; ++s) sum[i] += v[s][i];
           sum[i] += bias[i];
           if (p.residual && n + i < p.N) sum[i] += __bfloat162float(p.residual[o + i]);
         }
@@ -476,23 +443,23 @@ extern "C" int b200_gemm_fp8_stream(const void* A, const float* a_scales, const 
                     : launch_fp8_stream<64, false, true>(tw, tx, p, grid, stream);
 }
 
-// The operands of b200_grouped_gemm_fp8_block; tn: rows of A per tile, 64.
+// The operands of b200_grouped_gemm_fp8_block.
 extern "C" int b200_grouped_gemm_fp8_stream(const void* A, const float* a_scales, const void* W, const float* w_scales,
                                             void* C, const int* expert_offsets, int num_experts, int total_rows, int N,
-                                            int K, int lda, int ldc, int scale_rows, int swiglu, int up_scale_row0, int tn,
+                                            int K, int lda, int ldc, int scale_rows, int swiglu, int up_scale_row0,
                                             int* status, int max_ctas, cudaStream_t stream) {
   using namespace fp8s;
   if (total_rows <= 0 || num_experts <= 0 || N <= 0 || K <= 0) return 0;
   if (num_experts > MAX_EXPERTS) return -13;
-  if ((K % SLAB) != 0 || tn != MAX_ROWS) return -10;
+  if ((K % SLAB) != 0) return -10;
   if (swiglu && (N % 16) != 0) return -11;
   Fp8StreamParams p{};
   p.M = total_rows;
   p.N = N;
   p.k_slabs = K / SLAB;
-  p.tn = tn;
+  p.tn = MAX_ROWS;
   p.box = 16;
-  p.stages = RING / (W_BYTES + tn * SLAB);
+  p.stages = RING / (W_BYTES + p.tn * SLAB);
   p.num_n_tiles = (N + BW - 1) / BW;
   p.splits = 1;
   p.num_experts = num_experts;
@@ -505,7 +472,7 @@ extern "C" int b200_grouped_gemm_fp8_stream(const void* A, const float* a_scales
   p.C = C;
   p.expert_offsets = expert_offsets;
   p.status = status;
-  const long long row_tiles = total_rows / tn + (num_experts < total_rows ? num_experts : total_rows);
+  const long long row_tiles = total_rows / p.tn + (num_experts < total_rows ? num_experts : total_rows);
   if (row_tiles * p.num_n_tiles > 0x3fffffffll) return -14;
   CUtensorMap tw, tx;
   int r = make_tensormap_3d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, W, num_experts, N, K, static_cast<uint64_t>(N) * K, K, BW,

@@ -30,6 +30,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tensormap.h"
 #include "column_store.cuh"
+#include "group_tiles.cuh"
 
 namespace b200 {
 
@@ -142,33 +143,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   }
   if constexpr (GROUPED) {
     pdl_wait();      // the offsets come from an earlier kernel
-    if (warp == 2) {
-      const int per = (p.num_experts + 31) / 32;
-      const int e0 = min(p.num_experts, lane * per), e1 = min(p.num_experts, e0 + per);
-      const auto tiles_of = [&](int rows) {
+    if (warp == 2)
+      group_tiles(p.expert_offsets, p.num_experts, prefix, first_row, [&](int rows) {
         const int w = pair_group_width(rows);
         return (rows + w - 1) / w * p.num_n_tiles;
-      };
-      int tiles = 0;
-      for (int e = e0; e < e1; ++e) tiles += tiles_of(p.expert_offsets[e + 1] - p.expert_offsets[e]);
-      int incl = tiles;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int up = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += up;
-      }
-      int before = incl - tiles;
-      for (int e = e0; e < e1; ++e) {
-        const int a = p.expert_offsets[e], b = p.expert_offsets[e + 1];
-        prefix[e] = before;
-        first_row[e] = a;
-        before += tiles_of(b - a);
-        if (e + 1 == p.num_experts) {
-          prefix[e + 1] = before;
-          first_row[e + 1] = b;
-        }
-      }
-    }
+      });
   }
   tc_fence_before_sync();
   __syncthreads();

@@ -30,6 +30,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tensormap.h"
 #include "column_store.cuh"
+#include "group_tiles.cuh"
 #include "stream_split.cuh"
 
 namespace b200 {
@@ -45,7 +46,7 @@ constexpr int MAX_EXPERTS = 512;
 
 struct StreamParams {
   int M, N, K;
-  int tn;                 // rows of A per tile: 16, 32, 64 or 128
+  int tn;                 // rows of A per tile: 32, 64 or 128; dense 16 too
   int box;                // rows of A per copy: dense tn (rows past the end cost nothing), grouped 16
   int stages, k_slabs, splits, num_n_tiles;
   int num_experts;        // groups (grouped, batched)
@@ -168,9 +169,9 @@ __device__ __forceinline__ void stream_store4(const StreamParams& p, int act, fl
   }
 }
 
-// SPLIT: the CTAs of a cluster share a tile's K.  ACT: p.act is looked at.  (With every activation's code the kernel takes
-// 168 registers instead of 64, which leaves the kernel behind it no room beside two of its CTAs: latent decode step of 128
-// rows, 4 layers, 1334 us with one kernel for all, 1312.)
+// SPLIT: the CTAs of a cluster share a tile's K.  ACT: p.act is looked at.  (With every activation's code the
+// unsplit kernels take 168 registers, which leave the kernel behind no room beside two of their CTAs, without it 113 to 137:
+// latent decode step of 128 rows, 4 layers, 1334 us with one kernel for all, 1312.)
 template <int MODE, bool SPLIT, bool ACT>
 __global__ void __launch_bounds__(stream::THREADS, 2)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
@@ -217,30 +218,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   }
   if constexpr (GROUPED) {
     pdl_wait();      // the offsets come from an earlier kernel
-    if (warp == 2) {
-      const int per = (p.num_experts + 31) / 32;
-      const int e0 = min(p.num_experts, lane * per), e1 = min(p.num_experts, e0 + per);
-      int tiles = 0;
-      for (int e = e0; e < e1; ++e)
-        tiles += (p.expert_offsets[e + 1] - p.expert_offsets[e] + p.tn - 1) / p.tn * p.num_n_tiles;
-      int incl = tiles;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int up = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += up;
-      }
-      int before = incl - tiles;
-      for (int e = e0; e < e1; ++e) {
-        const int a = p.expert_offsets[e], b = p.expert_offsets[e + 1];
-        prefix[e] = before;
-        first_row[e] = a;
-        before += (b - a + p.tn - 1) / p.tn * p.num_n_tiles;
-        if (e + 1 == p.num_experts) {
-          prefix[e + 1] = before;
-          first_row[e + 1] = b;
-        }
-      }
-    }
+    if (warp == 2)
+      group_tiles(p.expert_offsets, p.num_experts, prefix, first_row,
+                  [&](int rows) { return (rows + p.tn - 1) / p.tn * p.num_n_tiles; });
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -447,24 +427,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                         (reinterpret_cast<uintptr_t>(p.residual) & 7) == 0;
       for (int row = rank + p.splits * (warp - 2); row < p.M; row += 4 * p.splits) {
         const uint32_t at = smem_u32(smem) + static_cast<uint32_t>((row * BW + 4 * lane) * 4);
-        float v[8][4];
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) v[s][i] = 0.f;
-          if (s < p.splits)
-            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                         : "=f"(v[s][0]), "=f"(v[s][1]), "=f"(v[s][2]), "=f"(v[s][3])
-                         : "r"(mapa_shared(at, s))
-                         : "memory");
-        }
         float sum[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          sum[i] = v[0][i];
-#pragma unroll
-          for (int s = 1; s < 8; ++s) sum[i] += v[s][i];
-        }
+        split_sum(at, p.splits, sum);
         stream_store4(p, act, sum, row, n, wide);
       }
     }
@@ -521,10 +485,10 @@ extern "C" int b200_gemm_stream_splits(int N, int K, int max_ctas, int sms) {
   return 2 * tiles > sms || slabs <= 8 ? 1 : stream_splits(tiles, slabs, max_ctas, sms);
 }
 
-// A [M <= 128, K] (pitch lda), W [N, K] (pitch ldw), C [M, N, or N / 2 with a gated activation].  splits 0: by rule.
+// A [M <= 128, K] (pitch lda), W [N, K] (pitch ldw), C [M, N, or N / 2 with a gated activation].
 // w_ready: see StreamParams.
 extern "C" int b200_gemm_stream(const void* A, const void* W, void* C, const void* bias, const void* residual, int M,
-                                int N, int K, int lda, int ldw, int ldc, int out_fp32, int act, int splits, int* status,
+                                int N, int K, int lda, int ldw, int ldc, int out_fp32, int act, int* status,
                                 int max_ctas, float act_alpha, float act_limit, int w_ready, cudaStream_t cu_stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (M > 128) return -10;
@@ -538,9 +502,7 @@ extern "C" int b200_gemm_stream(const void* A, const void* W, void* C, const voi
   p.stages = stream_stages(p.tn);
   p.k_slabs = (K + stream::SLAB_K - 1) / stream::SLAB_K;
   p.num_n_tiles = (N + stream::BW - 1) / stream::BW;
-  p.splits = splits > 0 ? splits : b200_gemm_stream_splits(N, K, max_ctas, sm_count());
-  if (p.splits != 1 && p.splits != 2 && p.splits != 4 && p.splits != 8) return -12;
-  if ((p.splits - 1) * ((p.k_slabs + p.splits - 1) / p.splits) >= p.k_slabs) return -12;
+  p.splits = b200_gemm_stream_splits(N, K, max_ctas, sm_count());
   p.ldc = ldc;
   p.out_fp32 = out_fp32;
   p.act = act;
@@ -571,14 +533,14 @@ extern "C" int b200_gemm_stream(const void* A, const void* W, void* C, const voi
 }
 
 // A [total_rows, K], W [E, N, K]; rows expert_offsets[e] .. expert_offsets[e + 1] (device) belong to expert e.
-// tn: rows of A per tile, 16, 32, 64 or 128.
+// tn: rows of A per tile, 32, 64 or 128.
 extern "C" int b200_grouped_gemm_stream(const void* A, const void* W, void* C, const int* expert_offsets,
                                         int num_experts, int total_rows, int N, int K, int lda, int ldc, int act, int tn,
                                         int* status, int max_ctas, float act_alpha, float act_limit,
                                         cudaStream_t cu_stream) {
   if (total_rows <= 0 || num_experts <= 0 || N <= 0 || K <= 0) return 0;
   if (num_experts > stream::MAX_EXPERTS) return -13;
-  if (tn != 16 && tn != 32 && tn != 64 && tn != 128) return -10;
+  if (tn != 32 && tn != 64 && tn != 128) return -10;
   if (act_is_gated(act) && (N % 16) != 0) return -11;
   StreamParams p{};
   p.M = total_rows;
@@ -620,7 +582,7 @@ extern "C" int b200_batched_gemm(const void* A, const void* W, void* C, int T, i
                                  long long a_group, long long c_row, long long c_group, int tn, int* status, int w_ready,
                                  cudaStream_t cu_stream) {
   if (T <= 0 || G <= 0 || N <= 0 || K <= 0) return 0;
-  if (tn != 16 && tn != 32 && tn != 64 && tn != 128) return -10;
+  if (tn != 32 && tn != 64 && tn != 128) return -10;
   if (((a_row | a_group | K) & 7) != 0 || ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) != 0 ||
       a_row <= 0 || (G > 1 && a_group <= 0) || c_row > 0x7fffffffll)
     return 1;

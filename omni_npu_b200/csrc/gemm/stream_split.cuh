@@ -1,6 +1,8 @@
 // How the weight-streaming kernels (gemm_stream.cu, gemm_fp8_stream.cu) share a tile's K among the CTAs of a cluster.
 #pragma once
 
+#include "../common/ptx.cuh"
+
 namespace b200 {
 
 // CTAs per tile of 128 weight rows: as many (a power of two up to the portable cluster size) as keep all CTAs resident at
@@ -18,6 +20,27 @@ inline int stream_splits(int n_tiles, int k_slabs, int max_ctas, int sms) {
     if (static_cast<long long>(n_tiles) * s <= room && per >= 4 && (s - 1) * per < k_slabs) best = s;
   }
   return best;
+}
+
+// Four neighbouring values of the CTAs' parts, in rank order; at: their address in this CTA's shared memory.
+__device__ __forceinline__ void split_sum(uint32_t at, int splits, float (&sum)[4]) {
+  float v[8][4];
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[s][i] = 0.f;
+    if (s < splits)
+      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                   : "=f"(v[s][0]), "=f"(v[s][1]), "=f"(v[s][2]), "=f"(v[s][3])
+                   : "r"(mapa_shared(at, s))
+                   : "memory");
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    sum[i] = v[0][i];
+#pragma unroll
+    for (int s = 1; s < 8; ++s) sum[i] += v[s][i];
+  }
 }
 
 }  // namespace b200

@@ -293,7 +293,8 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
 
     def run(kernel):
         _count(1)
-        return kernel(a, w, bias, residual, out_dtype == torch.float32, kind[0], bn, st.status, max_ctas, kind[1], kind[2],
+        tile = (bn,) if kernel is C.gemm_pair else ()
+        return kernel(a, w, bias, residual, out_dtype == torch.float32, kind[0], *tile, st.status, max_ctas, kind[1], kind[2],
                       w_ready)
 
     if pair:
@@ -374,7 +375,7 @@ def grouped_gemm_fp8_block(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.
     few = (a_q.shape[0] if rows is None else min(rows, a_q.shape[0])) <= FP8_STREAM_GROUP_ROWS * w_q.shape[0]
     _count(1)
     _C().grouped_gemm_fp8_block(a_q, a_scale.contiguous(), w_q, w_scale.contiguous(), expert_offsets, out, swiglu,
-                                up_scale_row0, 64 if few else 0, st.status, max_ctas)
+                                up_scale_row0, few, st.status, max_ctas)
     return out
 
 
