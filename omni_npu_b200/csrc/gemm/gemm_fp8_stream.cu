@@ -9,10 +9,11 @@
 // loaded one per lane, a stage ahead, and passed around by shuffles.
 //
 // Dense: when the tiles are fewer than the resident CTAs, the 2, 4 or 8 CTAs of a cluster share a tile's K and sum their
-// parts in rank order; the split depends on N and K alone.  Grouped: tiles of all live experts.
+// parts in rank order; the split depends on N and K alone, so that up to 64 rows the result of a row does not depend on the
+// others (gemm_fp8_block.cu, beyond, has no split).  Grouped: tiles of all live experts.
 //
 // Measured in a CUDA graph (us, gemm_fp8_block_kernel / here / the weights at 6.4 TB/s): one row 4096 x 7168
-// 31.8 / 10.5 / 4.6, 18432 x 7168 41.4 / 25.2 / 20.5; 32 experts, 32 rows each, 4096 x 7168 with silu 214 / 159 / 146,
+// 31.8 / 10.2 / 4.6, 18432 x 7168 41.4 / 25.1 / 20.5; 32 experts, 32 rows each, 4096 x 7168 with silu 214 / 159 / 146,
 // 7168 x 2048 111 / 88 / 73.  Tiles of 32 rows take as long as those of 64 up to 16 rows per expert, and longer beyond.
 //
 // Per CTA (192 threads): warp 0 TMA, warp 1 MMA, warps 2-5 epilogue.  Every wait is bounded; on expiry the CTA records a

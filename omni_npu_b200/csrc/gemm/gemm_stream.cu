@@ -18,7 +18,7 @@
 //
 // Measured in a CUDA graph, one row (us, gemm_tcgen05_kernel / here / the weights at 6.4 TB/s): 4096 x 4096
 // 17.5 / 9.2 / 5.2, 6144 x 4096 22.7 / 12.5 / 7.8, 4096 x 14336 35.2 / 21.5 / 18.2, 28672 x 4096 with silu 71.5 / 41.4 /
-// 36.5, 128256 x 4096 193 / 162 / 163; 83 of 128 experts live, 1536 x 2048 with silu 121 / 83 / 81.
+// 36.5, 128256 x 4096 193 / 164 / 163; 83 of 128 experts live, 1536 x 2048 with silu 121 / 83 / 81.
 // Against 8 CTAs per cluster throughout: 6144 x 4096 takes 16.0 (only what stays resident at once pays).
 //
 // Per CTA (192 threads): warp 0 TMA, warp 1 MMA, warps 2-5 epilogue (a thread holds one column of C and the rows of A

@@ -336,9 +336,10 @@ def quant_int8_per_token(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
 
 
 # Block-scaled products with at most this many rows (per group on average) stream their weights through
-# gemm_fp8_stream_kernel.  Us, gemm_fp8_block_kernel / here: 4096 x 7168 31.8 / 10.5 with one row, 32.2 / 13.7 with 64 (the
-# most that it takes), 18432 x 7168 34.4 / 33.7; 32 groups 4096 x 7168 with silu 214 / 159 at 32 rows each, 194 / 169 at 48,
-# 195 / 205 at 64, 7168 x 2048 111 / 88, 113 / 95 and 117 / 130.
+# gemm_fp8_stream_kernel.  Us, gemm_fp8_block_kernel / here: 4096 x 7168 31.8 / 10.2 with one row, 31.5 / 12.5 with 64 (the
+# most that it takes), 18432 x 7168 34.5 / 28.9 with 64, 12288 x 4096 21.9 / 20.8, 4096 x 1024 8.3 / 8.2; 32 groups 4096 x 7168
+# with silu 214 / 159 at 32 rows each, 194 / 169 at 48, 195 / 205 at 64, 7168 x 2048 111 / 88, 113 / 95 and 117 / 130.
+# A row's bits are one thing up to 64 dense rows, where K may be split, and another beyond.
 FP8_STREAM_ROWS = 64
 FP8_STREAM_GROUP_ROWS = 48
 

@@ -733,6 +733,44 @@ def test_grouped_products_chosen_by_the_rows_in_use(used):
         _close(ops.grouped_gemm_fp8_block(q, s, w8, ws, offs, rows=rows)[:used], want8, 1e-3, 2 ** -7)
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 130, 128), (33, 1000, 640), (64, 4096, 1024), (65, 260, 384)])
+def test_gemm_fp8_block_against_64_bits(m, n, k):
+    """Scale rows of a ragged N, K splits, epilogues, on either side of the 64 rows of the weight-streaming kernel."""
+    torch.manual_seed(m + n + k)
+    q, s = ops.quant_fp8_1x128(torch.randn(m, k, device=DEV, dtype=torch.bfloat16))
+    w, ws = torch.randn(n, k, device=DEV).to(torch.float8_e4m3fn), torch.rand(-(-n // 128), k // 128, device=DEV) + 0.5
+    full = w.double() * ws.double().repeat_interleave(128, 0)[:n].repeat_interleave(128, 1)
+    exact = (q.double() * s.double().repeat_interleave(128, 1)) @ full.T
+    bias, res = torch.randn(n, device=DEV).bfloat16(), torch.randn(m, n, device=DEV).bfloat16()
+    # fp32 sums of k products of size 1
+    _close(ops.gemm_fp8_block(q, s, w, ws, out_dtype=torch.float32), exact.float(), k ** 0.5 * 2 ** -16, 2 ** -16)
+    # one rounding to bf16
+    _close(ops.gemm_fp8_block(q, s, w, ws, bias, res), (exact + bias.double() + res.double()).float(), 1e-2, 2 ** -8)
+
+
+@pytest.mark.parametrize("counts,n,k,swiglu", [([0, 5, 64, 65, 0, 16], 512, 256, True), ([3, 40], 130, 128, False),
+                                               ([70, 1], 768, 384, True), ([200, 180], 512, 256, True)])
+def test_grouped_gemm_fp8_block_against_64_bits(counts, n, k, swiglu):
+    """Scale rows of alternating gate and up rows, groups of any size, few rows per group and many."""
+    torch.manual_seed(n + k)
+    offs = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32)
+    rows, e = int(offs[-1]), len(counts)
+    w = torch.randn(e, n, k, device=DEV).to(torch.float8_e4m3fn)
+    r = torch.arange(n)
+    up = n // 256 if swiglu else 0
+    block = torch.where((r & 8) != 0, up, 0) + (r // 16 * 8 + r % 8) // 128 if swiglu else r // 128
+    ws = torch.rand(e, 2 * up if swiglu else -(-n // 128), k // 128, device=DEV) * 0.2 + 0.05
+    q, s = ops.quant_fp8_1x128(torch.randn(rows, k, device=DEV, dtype=torch.bfloat16))
+    x = q.double() * s.double().repeat_interleave(128, 1)
+    full = w.double() * ws.double()[:, block.to(DEV)].repeat_interleave(128, 2)
+    exact = torch.cat([x[offs[i]: offs[i + 1]] @ full[i].T for i in range(e)])
+    if swiglu:
+        gate, upper = exact.view(rows, -1, 2, 8).unbind(2)
+        exact = (torch.nn.functional.silu(gate) * upper).reshape(rows, -1)
+    # one rounding to bf16, of fp32 sums
+    _close(ops.grouped_gemm_fp8_block(q, s, w, ws, offs.to(DEV), swiglu, up), exact.float(), 1e-2, 2 ** -7)
+
+
 @pytest.mark.parametrize("limit", [1, 7, 40, 300])
 def test_few_rows_within_a_limit_of_ctas(limit):
     torch.manual_seed(limit)
